@@ -111,6 +111,12 @@ int qgemm_w8a8_grouped(const int8_t* A, const int8_t* B, const float* scale_b, c
                        int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
                        int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len, int out_dtype,
                        int b_layout, uint32_t* status, void* stream);
+/* The same, and rows of C that no block covers are set to zero (for callers that allocate C and would otherwise have to
+ * clear all of it first); acc_out is left untouched there. */
+int qgemm_w8a8_grouped_zeroed(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
+                              int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
+                              int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len, int out_dtype,
+                              int b_layout, uint32_t* status, void* stream);
 
 /* Bytes of scratch memory qgemm_w4a16 needs for this problem on the current device (split-K partial
  * sums and arrival counters, the prepared activations and, from 1792 tokens on, the weights as f16: 2*N*K).
@@ -190,6 +196,10 @@ int qgemm_w4a16_batched(const void* A, const uint8_t* B_packed, const void* scal
 #define QGEMM_ZERO_RESCALE 1
 #define QGEMM_ZERO_QUANTIZED 2
 int64_t qgemm_w4a16_ex_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int has_zeros_tensor);
+/* The scratch bytes of one particular qgemm_w4a16_ex call (never more than qgemm_w4a16_ex_workspace_bytes): knows
+ * which kernel the group size, the scales and the zero mode select. */
+int64_t qgemm_w4a16_call_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t group, int has_scales,
+                                         int has_zeros_tensor, int zero_mode);
 int qgemm_w4a16_ex(const void* A, const uint8_t* B_packed, const void* scales, const void* zeros, int zero,
                    int zero_mode, int weight_format, int64_t group, void* C, void* workspace, int64_t workspace_bytes,
                    int64_t batch, int64_t M, int64_t N, int64_t K, int a_dtype, int out_dtype, uint32_t* status,

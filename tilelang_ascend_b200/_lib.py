@@ -9,10 +9,12 @@ There is no fallback: if the library is missing or a call is rejected, an except
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 
 PKG = os.path.dirname(os.path.abspath(__file__))
+HOST_PATH = os.path.join(PKG, "_qhost.so")
 LIB_PATH = os.environ.get("QGEMM_LIB") or os.path.join(PKG, "libqgemm.so")  # QGEMM_LIB: another build of the library
 
 DT_F16, DT_BF16, DT_I32 = 0, 1, 2
@@ -36,6 +38,9 @@ SIGNATURES = {
     "qgemm_w8a8_grouped": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                       _c.c_void_p, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64,
                                       _c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
+    "qgemm_w8a8_grouped_zeroed": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p,
+                                             _c.c_void_p, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64,
+                                             _c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "qgemm_w4a16_workspace_bytes": (_c.c_int64, [_c.c_int64, _c.c_int64, _c.c_int64]),
     "qgemm_w4a16_counter_bytes": (_c.c_int64, []),
     "qgemm_w4a16": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int64, _c.c_void_p,
@@ -46,6 +51,8 @@ SIGNATURES = {
                                        _c.c_void_p, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64,
                                        _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "qgemm_w4a16_ex_workspace_bytes": (_c.c_int64, [_c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int]),
+    "qgemm_w4a16_call_workspace_bytes": (_c.c_int64, [_c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int,
+                                                      _c.c_int, _c.c_int]),
     "qgemm_w4a16_ex": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int,
                                   _c.c_int64, _c.c_void_p, _c.c_void_p, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int64,
                                   _c.c_int64, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
@@ -69,8 +76,13 @@ SIGNATURES = {
                                    _c.c_void_p]),
 }
 
-_lock = threading.Lock()
+_lock = threading.RLock()
 _lib = None
+_host = None
+
+# entry points the native call path (csrc/host.cpp) is handed, in the order its init() takes them
+_HOST_ENTRY_POINTS = ("qgemm_w8a8", "qgemm_w8a8_grouped", "qgemm_w4a16_call_workspace_bytes", "qgemm_w4a16_ex", "qgemm_w4a8",
+                      "qgemm_w4a8_act_quant", "qgemm_act_quant", "qgemm_w8a8_grouped_zeroed")
 
 
 class QGemmError(RuntimeError):
@@ -89,7 +101,7 @@ def load() -> ctypes.CDLL:
                 if _build.needs_build():
                     _build.build()
             except Exception:
-                if not os.path.isfile(LIB_PATH):
+                if not (os.path.isfile(LIB_PATH) and os.path.isfile(HOST_PATH)):
                     raise
         if not os.path.isfile(LIB_PATH):
             raise QGemmError(f"{LIB_PATH} not found: build it with `python -m tilelang_ascend_b200.build`")
@@ -100,6 +112,22 @@ def load() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = lib
         return lib
+
+
+def host():
+    """The native call path (extension module _qhost), bound to the loaded library's entry points."""
+    global _host
+    with _lock:
+        if _host is None:
+            lib = load()
+            if not os.path.isfile(HOST_PATH):
+                raise QGemmError(f"{HOST_PATH} not found: build it with `python -m tilelang_ascend_b200.build`")
+            spec = importlib.util.spec_from_file_location("_qhost", HOST_PATH)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            mod.init(*[_c.cast(getattr(lib, n), _c.c_void_p).value for n in _HOST_ENTRY_POINTS])
+            _host = mod
+        return _host
 
 
 def last_error() -> str:

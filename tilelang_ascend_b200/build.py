@@ -1,9 +1,10 @@
-"""Build libqgemm.so (the C-ABI shared library) in-tree with nvcc for sm_100a.
+"""Build libqgemm.so (the C-ABI shared library, nvcc for sm_100a) and _qhost.so (the operators' native call
+path, g++ against torch's headers) in-tree.
 
     python -m tilelang_ascend_b200.build [--force] [--verbose]
 
-The library lands next to this file as ``tilelang_ascend_b200/libqgemm.so``; it is rebuilt
-when a source under ``csrc/`` or ``include/qgemm.h`` is newer than it.
+Both land next to this file; each is rebuilt when one of its sources under ``csrc/`` or ``include/qgemm.h`` is newer
+than it.
 """
 from __future__ import annotations
 
@@ -16,6 +17,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libqgemm.so")
+HOST_LIB = os.path.join(PKG, "_qhost.so")
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 SOURCES = ["qgemm_api.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -31,11 +34,23 @@ def _deps():
     return deps
 
 
-def needs_build() -> bool:
-    if not os.path.isfile(LIB):
+def _stale(target, deps) -> bool:
+    if not os.path.isfile(target):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(d) > t for d in _deps())
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _lib_stale() -> bool:
+    return _stale(LIB, _deps())
+
+
+def _host_stale() -> bool:
+    return _stale(HOST_LIB, [os.path.join(ROOT, "include", "qgemm.h"), HOST_SOURCE])
+
+
+def needs_build() -> bool:
+    return _lib_stale() or _host_stale()
 
 
 def find_nvcc() -> str:
@@ -45,18 +60,37 @@ def find_nvcc() -> str:
     raise RuntimeError("nvcc not found; libqgemm.so cannot be built")
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
-    cmd = [find_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB]
+def _run(cmd, verbose):
     res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd))
+        raise RuntimeError("build failed:\n" + " ".join(cmd))
+
+
+def _host_command():
+    import sysconfig
+
+    import torch
+    base = os.path.join(os.path.dirname(torch.__file__))
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")]
+    lib = os.path.join(base, "lib")
+    return ([os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            + [f"-I{d}" for d in inc]
+            + [HOST_SOURCE, "-o", HOST_LIB, f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda",
+               "-lc10", "-lc10_cuda"])
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    if force or _lib_stale():
+        cmd = [find_nvcc(), *NVCC_FLAGS]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        _run(cmd + [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB], verbose)
+    if force or _host_stale():
+        _run(_host_command(), verbose)
     return LIB
 
 

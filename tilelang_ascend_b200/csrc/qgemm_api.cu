@@ -2,6 +2,7 @@
 // The exported functions are declared and documented in include/qgemm.h.
 #include "../../include/qgemm.h"
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -40,7 +41,7 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 
 constexpr int kMaxDevices = 64;
 struct DeviceState {
-  bool ready = false;
+  std::atomic<bool> ready{false};
   int sm_count = 0;
 };
 std::mutex g_mu;
@@ -114,9 +115,13 @@ int ensure_device(int* sm_count) {
   int dev = 0;
   CUDA_OK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) return fail("device index %d out of range", dev);
-  std::lock_guard<std::mutex> lock(g_mu);
   DeviceState& st = g_dev[dev];
-  if (!st.ready) {
+  if (st.ready.load(std::memory_order_acquire)) {  // every call but the first one per device
+    *sm_count = st.sm_count;
+    return 0;
+  }
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (!st.ready.load(std::memory_order_relaxed)) {
     cudaDeviceProp prop;
     CUDA_OK(cudaGetDeviceProperties(&prop, dev));
     if (prop.major != 10) return fail("libqgemm needs an sm_100a device (B200); device %d is sm_%d%d", dev, prop.major, prop.minor);
@@ -133,7 +138,7 @@ int ensure_device(int* sm_count) {
     if (set_smem_w4i8<16>() || set_smem_w4i8<32>() || set_smem_w4i8<64>() || set_smem_w4i8<128>()) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
-    st.ready = true;
+    st.ready.store(true, std::memory_order_release);
   }
   *sm_count = st.sm_count;
   return 0;
@@ -461,7 +466,7 @@ int qgemm_init(void) {
 static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
                      int32_t* acc_out, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t scale_b_len,
                      int64_t scale_a_len, int out_dtype, int b_layout, uint32_t* status, void* stream,
-                     const int* meta, int64_t num_blocks) {
+                     const int* meta, int64_t num_blocks, bool zero_uncovered = false) {
   const int64_t batchA = meta ? 1 : batch;  // batch extent of A, C and scale_a
   if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) return fail("qgemm_w8a8: batch, M, N, K must be positive (got %lld, %lld, %lld, %lld)", (long long)batch, (long long)M, (long long)N, (long long)K);
   if (M > (1ll << 30) || N > (1ll << 30) || K > (1ll << 30) || batch > 65535) return fail("qgemm_w8a8: dimension too large");
@@ -542,6 +547,8 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.acc_out = acc_out;
   p.batch = (int)batchA;
   p.meta = meta;
+  p.num_blocks = meta ? (int)num_blocks : 0;
+  p.zero_uncovered = zero_uncovered && C != nullptr ? 1 : 0;
   p.groups = (int)batch;
   p.M = (int)M;
   p.N = (int)N;
@@ -592,17 +599,38 @@ int qgemm_w8a8(const int8_t* A, const int8_t* B, const float* scale_b, const flo
                    status, stream, nullptr, 0);
 }
 
-int qgemm_w8a8_grouped(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
-                       int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
-                       int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len, int out_dtype,
-                       int b_layout, uint32_t* status, void* stream) {
+static int w8a8_grouped_impl(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
+                             int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
+                             int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len, int out_dtype,
+                             int b_layout, uint32_t* status, void* stream, bool zero_uncovered) {
   if (num_blocks < 0) return fail("qgemm_w8a8_grouped: num_blocks must not be negative (got %lld)", (long long)num_blocks);
-  if (num_blocks == 0 || total_M == 0) return 0;  // no rows: nothing to compute
+  if (total_M == 0) return 0;  // no rows: nothing to compute
+  if (num_blocks == 0) {       // no row is covered
+    if (zero_uncovered && C != nullptr && total_M > 0 && N > 0)
+      CUDA_OK(cudaMemsetAsync(C, 0, (size_t)total_M * (size_t)N * (out_dtype == QGEMM_DT_I32 ? 4 : 2), static_cast<cudaStream_t>(stream)));
+    return 0;
+  }
   if (block_metadata == nullptr) return fail("qgemm_w8a8_grouped: block_metadata must not be null");
   if ((reinterpret_cast<uintptr_t>(block_metadata) & 3u) != 0) return fail("qgemm_w8a8_grouped: block_metadata must be 4-byte aligned");
   if (num_blocks > (1ll << 24)) return fail("qgemm_w8a8_grouped: too many row blocks (%lld)", (long long)num_blocks);
   return w8a8_impl(A, B, scale_b, scale_a, C, acc_out, groups, total_M, N, K, scale_b_len, scale_a_len, out_dtype,
-                   b_layout, status, stream, block_metadata, num_blocks);
+                   b_layout, status, stream, block_metadata, num_blocks, zero_uncovered);
+}
+
+int qgemm_w8a8_grouped(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
+                       int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
+                       int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len, int out_dtype,
+                       int b_layout, uint32_t* status, void* stream) {
+  return w8a8_grouped_impl(A, B, scale_b, scale_a, C, acc_out, block_metadata, num_blocks, groups, total_M, N, K, scale_b_len,
+                           scale_a_len, out_dtype, b_layout, status, stream, false);
+}
+
+int qgemm_w8a8_grouped_zeroed(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
+                              int32_t* acc_out, const int32_t* block_metadata, int64_t num_blocks, int64_t groups,
+                              int64_t total_M, int64_t N, int64_t K, int64_t scale_b_len, int64_t scale_a_len,
+                              int out_dtype, int b_layout, uint32_t* status, void* stream) {
+  return w8a8_grouped_impl(A, B, scale_b, scale_a, C, acc_out, block_metadata, num_blocks, groups, total_M, N, K, scale_b_len,
+                           scale_a_len, out_dtype, b_layout, status, stream, true);
 }
 
 int64_t qgemm_w4a16_counter_bytes(void) { return kW4CounterBytes; }
@@ -642,6 +670,18 @@ int64_t qgemm_w4a16_batched_workspace_bytes(int64_t batch, int64_t M, int64_t N,
 
 int64_t qgemm_w4a16_ex_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int has_zeros_tensor) {
   return w4_workspace_bytes(batch, M, N, K, has_zeros_tensor != 0);
+}
+
+// Whether a zeros tensor is taken in flight by the group-sum kernel (see w4a16_impl).
+static bool w4_zeros_inflight(int64_t M, int64_t N, int64_t K, int64_t group, int zero_mode) {
+  static const int on = getenv("QGEMM_W4_ZEROS_INFLIGHT") ? atoi(getenv("QGEMM_W4_ZEROS_INFLIGHT")) : 1;
+  return on && zero_mode == QGEMM_ZERO_QUANTIZED && !w4_use_f16_gemm(M, N) && w4_gs_shape_ok(M, true, group, K);
+}
+
+int64_t qgemm_w4a16_call_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t group, int has_scales,
+                                         int has_zeros_tensor, int zero_mode) {
+  const bool zeros = has_scales && has_zeros_tensor;
+  return w4_workspace_bytes(batch, M, N, K, zeros && !w4_zeros_inflight(M, N, K, group, zero_mode));
 }
 
 int64_t qgemm_w4a16_workspace_bytes(int64_t M, int64_t N, int64_t K) {
@@ -791,9 +831,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   // A zeros tensor of mode "quantized" (integer zero points) is taken in flight by the group-sum kernel wherever that
   // kernel applies; the other zero modes, whose f16 roundings per weight the group-sum form cannot reproduce, and all
   // other shapes go through the whole-matrix dequantisation.  QGEMM_W4_ZEROS_INFLIGHT=0 sends every zeros tensor there.
-  static const int zeros_inflight_on = getenv("QGEMM_W4_ZEROS_INFLIGHT") ? atoi(getenv("QGEMM_W4_ZEROS_INFLIGHT")) : 1;
-  const bool zeros_inflight = zeros != nullptr && zeros_inflight_on && zero_mode == QGEMM_ZERO_QUANTIZED && gd == nullptr &&
-                              !w4_use_f16_gemm(M, N) && w4_gs_shape_ok(M, true, group, K);
+  const bool zeros_inflight = zeros != nullptr && gd == nullptr && w4_zeros_inflight(M, N, K, group, zero_mode);
   const bool dequant_once = (zeros != nullptr && !zeros_inflight) || w4_use_f16_gemm(M, N);
   // a zeros tensor that is taken in flight needs no room for dequantised weights
   const int64_t need = w4_workspace_bytes(batch, M, N, K, zeros != nullptr && !zeros_inflight);

@@ -31,6 +31,8 @@ struct W8A8Params {
   // of the table is (group, first row, valid rows <= 128).  Null for the plain and batched forms.
   const int* meta;
   int groups;
+  int num_blocks;       // rows of the table
+  int zero_uncovered;   // rows of C (16-bit outputs) that no block covers are set to zero
   // Tail split: work items from `split_from` on are half-width tiles (item split_from + 2i + h is the left or
   // right half of tile split_from + i), so that the last, partly filled round of the persistent grid keeps
   // twice as many SMs busy for about half as long.  num_items = num_tiles when nothing is split.
@@ -109,6 +111,39 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
     t.rows = min(t.rows, p.M - t.m0);
   }
   return t;
+}
+
+// Grouped form, rows of C that no table entry covers: set to zero by the four epilogue warps before their first tile
+// (they would otherwise wait for it), CTA c looking after every grid-th block of 128 rows.  A clear of the whole output in front
+// of the launch cost a pass over C (33 MB for 8192 x 2048: 10 us of 125) although normally every row is covered.
+__device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4, int lane) {
+  // a warp takes 32 rows at a time, one per lane, and walks the table once for them
+  for (long long base = (long long)blockIdx.x * 128 + warp4 * 32; base < p.M; base += (long long)gridDim.x * 128) {
+    const int row = (int)base + lane;
+    bool covered = row >= p.M;
+    for (int i = 0; i < p.num_blocks; i += 32) {
+      int first = 0, rows = 0;
+      if (i + lane < p.num_blocks) {
+        const int g = __ldg(p.meta + 3 * (i + lane));
+        first = __ldg(p.meta + 3 * (i + lane) + 1);
+        rows = min(__ldg(p.meta + 3 * (i + lane) + 2), W8_BM);
+        if (g < 0 || g >= p.groups || first < 0 || first >= p.M) rows = 0;  // as in w8_tile
+      }
+      const int n_here = min(32, p.num_blocks - i);
+      for (int j = 0; j < n_here; ++j) {
+        const int f = __shfl_sync(0xffffffffu, first, j), r = __shfl_sync(0xffffffffu, rows, j);
+        covered = covered || (row >= f && row - f < r);
+      }
+      if (__all_sync(0xffffffffu, covered)) break;
+    }
+    uint32_t open_rows = __ballot_sync(0xffffffffu, !covered);
+    while (open_rows) {
+      const int r = __ffs(open_rows) - 1;
+      open_rows &= open_rows - 1;
+      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + ((size_t)base + r) * (size_t)p.N);
+      for (int c = lane; c < p.N / 8; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);  // N is a multiple of 16
+    }
+  }
 }
 
 // F16 = true runs the same pipeline on f16 operands (kind::f16, fp32 accumulators, no scales): one MMA K step
@@ -286,6 +321,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     float* sb_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES) + q * BN;
     uint8_t* my_stage = out_stage + q * 4096;  // [32 rows][128 B], 16-byte piece j of row r at (j ^ (r & 7))
     int it = 0;
+    if (p.zero_uncovered) w8_zero_uncovered(p, q, lane);
     // split form: the other CTA's accumulators travel through CTA 0's pipeline stages, one 16-byte piece per
     // (row, four columns): piece (col / 4, row) at ((col / 4) * 128 + row) * 16, so that a warp's 32 rows are
     // 512 contiguous bytes for the sender's stores and the receiver's loads alike

@@ -30,6 +30,19 @@ _TORCH_DT = {"float16": torch.float16, "bfloat16": torch.bfloat16, "float32": to
 _ABI_DT = {torch.float16: _lib.DT_F16, torch.bfloat16: _lib.DT_BF16, torch.int32: _lib.DT_I32}
 
 
+_host = None
+
+
+def _native():
+    """The native call path (csrc/host.cpp): one function per operator that does the whole ordinary call - metadata
+    checks, output and scratch allocation, current stream, launch - and returns None, having done nothing, for any call
+    that is not ordinary; the Python code below then checks everything and raises or handles it."""
+    global _host
+    if _host is None:
+        _host = _lib.host()
+    return _host
+
+
 def _dt(x):
     if isinstance(x, torch.dtype):
         return x
@@ -84,6 +97,10 @@ def quant_matmul(A, B, scale, scale_a=None, out_dtype=torch.float16, b_layout="K
     (``"NK"``).  scale: fp32 [1], [N] or [Batch, N].  scale_a: optional fp32 [M] or [Batch, M].
     ``out_dtype`` float16 / bfloat16, or int32 for the raw accumulators.
     """
+    if stream is None and status is None and not return_accumulators and b_layout in ("KN", "NK"):
+        C = (_host or _native()).w8a8(A, B, scale, scale_a, out_dtype, b_layout == "NK", -1, 0, 0, 0)
+        if C is not None:
+            return C
     lib = _lib.load()
     _require_cuda(A, "A")
     dev = A.device
@@ -139,16 +156,25 @@ class _QuantMatmulKernel:
         self.batch, self.M, self.N, self.K = batch, M, N, K
         self.scale_size = scale_size
         self.out_dtype = out_dtype
+        n_scale = N if str(scale_size) == "N" else 1
+        self._scale_lengths = {n_scale} | ({batch * N} if (batch and n_scale != 1) else set())
+
+    def _scale_fits(self, scale):
+        return isinstance(scale, torch.Tensor) and scale.numel() in self._scale_lengths
 
     def __call__(self, A, B, scale, scale_a=None, stream=None, return_accumulators=False):
+        # (a per-token scale_a comes with any scale shape; without it the factory's scale_size decides)
+        if stream is None and not return_accumulators and (scale_a is not None or self._scale_fits(scale)):
+            C = (_host or _native()).w8a8(A, B, scale, scale_a, self.out_dtype, False, self.batch or 0, self.M, self.N, self.K)
+            if C is not None:
+                return C
         lead = () if self.batch is None else (self.batch,)
         _require_cuda(A, "A")
         _check_tensor(A, 0, "A", torch.int8, lead + (self.M, self.K), A.device)
         _check_tensor(B, 1, "B", torch.int8, lead + (self.K, self.N), A.device)
         if isinstance(scale, torch.Tensor) and scale_a is None:
             n_scale = self.N if str(self.scale_size) == "N" else 1
-            allowed = {n_scale} | ({self.batch * self.N} if (self.batch and n_scale != 1) else set())
-            if scale.numel() not in allowed:
+            if scale.numel() not in self._scale_lengths:
                 raise ValueError(f"Static shape mismatch for parameter scale: expected [{n_scale}], got {tuple(scale.shape)}")
         return quant_matmul(A, B, scale, scale_a=scale_a, out_dtype=self.out_dtype, stream=stream,
                             return_accumulators=return_accumulators)
@@ -206,7 +232,7 @@ def release_workspaces():
     allocates its workspaces, tilelang/jit/adapter/cython/cython_wrapper.pyx:102-141), so there is nothing to drop."""
 
 
-def _w4a16_workspace(lib, batch, M, N, K, device, stream_handle, zeros_tensor=False):
+def _w4a16_workspace(lib, batch, M, N, K, device, stream_handle, group, has_scales, zeros_tensor=False, zero_mode=0):
     """Scratch buffer of one call (split-K partial sums + arrival counters + prepared activations, and from 1024
     tokens on, or with a zeros tensor, the f16 copy of the weights).
 
@@ -214,9 +240,9 @@ def _w4a16_workspace(lib, batch, M, N, K, device, stream_handle, zeros_tensor=Fa
     call from torch's caching allocator, so no launch ever sees a buffer that another call may still be using or
     that a captured CUDA graph still points to; when the launch stream is not torch's current stream the buffer
     is tied to that stream so that the allocator does not hand it out again too early."""
-    need = lib.qgemm_w4a16_ex_workspace_bytes(batch, M, N, K, 1 if zeros_tensor else 0)
+    need = lib.qgemm_w4a16_call_workspace_bytes(batch, M, N, K, int(group), 1 if has_scales else 0, 1 if zeros_tensor else 0, zero_mode)
     if need < 0:
-        raise _lib.QGemmError("qgemm_w4a16_ex_workspace_bytes: " + _lib.last_error())
+        raise _lib.QGemmError("qgemm_w4a16_call_workspace_bytes: " + _lib.last_error())
     ws = torch.empty(need, dtype=torch.uint8, device=device)
     if stream_handle != torch.cuda.current_stream(device).cuda_stream:
         ws.record_stream(torch.cuda.ExternalStream(stream_handle, device=device))
@@ -240,6 +266,11 @@ def w4a16_gemm(A, B_packed, scales=None, zeros=8, group_size=128, out_dtype=None
     ``status``: optional int32 CUDA tensor of one element that receives a non-zero code if a bounded wait inside
     the kernel ran out (the result is then unspecified).  ``check_status=True`` allocates that word, waits for the
     launch to finish and raises ``QGemmError`` if it is non-zero - a synchronising debug aid, off by default."""
+    if stream is None and status is None and not check_status and zeros_mode in _ZERO_MODES and weight_layout in _WEIGHT_LAYOUTS:
+        C = (_host or _native()).w4a16(A, B_packed, scales, zeros, group_size, out_dtype, _ZERO_MODES[zeros_mode],
+                                       _WEIGHT_LAYOUTS[weight_layout], -1, 0, 0)
+        if C is not None:
+            return C
     lib = _lib.load()
     _require_cuda(A, "A")
     dev = A.device
@@ -288,12 +319,8 @@ def w4a16_gemm(A, B_packed, scales=None, zeros=8, group_size=128, out_dtype=None
     if check_status and status is None:
         status = torch.zeros(1, dtype=torch.int32, device=dev)
     with torch.cuda.device(dev):
-        # integer zero points at decode sizes are taken in flight: no room for dequantised weights is needed
-        inflight = (zeros_t is not None and zeros_mode == "quantized" and M <= 64
-                    and (group_size == 128 or group_size % 256 == 0 or group_size >= K)
-                    and os.environ.get("QGEMM_W4_ZEROS_INFLIGHT", "1") != "0" and os.environ.get("QGEMM_W4_GS", "1") != "0"
-                    and "QGEMM_W4_GS_MIN_M" not in os.environ)
-        ws, need = _w4a16_workspace(lib, batch, M, N, K, dev, sh, zeros_t is not None and not inflight)
+        ws, need = _w4a16_workspace(lib, batch, M, N, K, dev, sh, group_size, scales is not None, zeros_t is not None,
+                                    _ZERO_MODES[zeros_mode])
         rc = lib.qgemm_w4a16_ex(A.data_ptr(), B_packed.data_ptr(), _ptr(scales), _ptr(zeros_t), int(zeros),
                                 _ZERO_MODES[zeros_mode], _WEIGHT_LAYOUTS[weight_layout], int(group_size),
                                 C.data_ptr(), ws.data_ptr(), need, batch, M, N, K, _ABI_DT[A.dtype],
@@ -340,7 +367,7 @@ def w4a16_gemm_gather(A, B_packed, scales, zeros, group_size, dst_ptrs, ldc, col
     sh = _stream_handle(stream, dev)
     ptr_array = (ctypes.c_void_p * len(dst_ptrs))(*[int(x) for x in dst_ptrs])
     with torch.cuda.device(dev):
-        ws, need = _w4a16_workspace(lib, 1, M, N, K, dev, sh)
+        ws, need = _w4a16_workspace(lib, 1, M, N, K, dev, sh, group_size, scales is not None)
         rc = lib.qgemm_w4a16_gather(A.data_ptr(), B_packed.data_ptr(), _ptr(scales), int(zeros), int(group_size),
                                     ctypes.cast(ptr_array, ctypes.c_void_p), len(dst_ptrs), int(ldc), int(col0),
                                     ws.data_ptr(), need, M, N, K, _ABI_DT[A.dtype], _ABI_DT[out_dtype], _ptr(status), sh)
@@ -435,6 +462,10 @@ def dequant_gemm_fp16_wrapper(M: int, N: int, K: int, block_M: int, block_N: int
         raise ValueError("input_dtype / output_dtype must be float16 or bfloat16")
 
     def wrapper(A: torch.Tensor, B_packed: torch.Tensor, scales=None, zeros: int = 8, group_size: int = 128):
+        if A.dtype == in_dt and A.is_cuda:
+            C = (_host or _native()).w4a16(A, B_packed, scales, zeros, group_size, out_dt, 0, 0, M, N, K)
+            if C is not None:
+                return C
         if tuple(A.shape) != (M, K) or tuple(B_packed.shape) != (N, K // 2):
             raise ValueError(f"Static shape mismatch: expected A {(M, K)}, B_packed {(N, K // 2)}; "
                              f"got {tuple(A.shape)}, {tuple(B_packed.shape)}")
@@ -494,6 +525,8 @@ def w4a8_gemm_cv(M: int, N: int, K: int):
     (two's-complement) nibbles; like the reference, the caller provides ``workspace`` and ``C`` (:174-177)."""
 
     def kernel(A, qB, workspace, C, stream=None):
+        if stream is None and (_host or _native()).w4a8(A, qB, workspace, C, M, N, K):
+            return C
         _require_cuda(A, "A")
         dev = A.device
         _check_tensor(A, 0, "A", torch.int8, (M, K), dev)
@@ -514,7 +547,13 @@ def w4a8_gemm_act_quant(M: int, N: int, K: int, round_scale: bool = False):
     with ``C`` and ``scale_a`` bit-identical to ``act_quant`` followed by ``w4a8_gemm_cv``; the dequantised product is
     ``C * scale_a[:, None] * weight_scale``."""
 
+    round_scale = bool(round_scale)
+
     def kernel(X, qB, workspace, C, stream=None, status=None):
+        if stream is None and status is None:
+            s = (_host or _native()).w4a8_aq(X, qB, workspace, C, M, N, K, round_scale)
+            if s is not None:
+                return C, s
         lib = _lib.load()
         _require_cuda(X, "X")
         dev = X.device
@@ -574,6 +613,10 @@ def act_quant(x, round_scale: bool = False, stream=None):
     (examples/deepseek_v4/act_quant.py:112-142), computed on the GPU: per row ``scale = max(amax, 1e-4) / 127``
     (a power of two not below it when ``round_scale``), ``y = round(clamp(x / scale, -127, 127))``.  The
     outputs are what ``quant_matmul`` takes as ``A`` and ``scale_a``."""
+    if stream is None:
+        ys = (_host or _native()).act_quant(x, bool(round_scale), -1)
+        if ys is not None:
+            return ys
     lib = _lib.load()
     _require_cuda(x, "x")
     dev = x.device
@@ -606,7 +649,13 @@ def act_quant_kernel_int8_optimized(N: int, block_M: int = 32, block_N: int = 32
     if block_M <= 0 or block_N <= 0:
         raise ValueError("block_M and block_N must be positive")
 
+    round_scale = bool(round_scale)
+
     def kernel(X, stream=None):
+        if stream is None:
+            ys = (_host or _native()).act_quant(X, round_scale, N)
+            if ys is not None:
+                return ys
         if X.dim() != 2 or X.shape[1] != N:
             raise ValueError(f"X must have shape [M, {N}], got {tuple(X.shape)}")
         y, s = act_quant(X, round_scale=round_scale, stream=stream)
@@ -644,6 +693,10 @@ def grouped_quant_matmul(A, B, block_metadata, scale, scale_a=None, out_dtype=to
     A: [total_M, K] int8; B: [G, K, N] (``"KN"``) or [G, N, K] (``"NK"``) int8; block_metadata: CUDA int32
     [blocks, 3] with at most 128 rows per block; scale: fp32 [1], [N] or [G, N]; scale_a: optional fp32 [total_M].
     Rows of the result that no block covers keep the contents of ``out`` (zeros when ``out`` is not given)."""
+    if stream is None and status is None and not return_accumulators and b_layout in ("KN", "NK"):
+        C = (_host or _native()).grouped(A, B, block_metadata, scale, scale_a, out_dtype, b_layout == "NK", out, -1, 0, 0, 0)
+        if C is not None:
+            return C
     lib = _lib.load()
     _require_cuda(A, "A")
     dev = A.device
@@ -711,6 +764,11 @@ def grouped_quant_gemm(batch_sizes_list, K: int, N: int, block_M: int = 128, blo
     blocks = sum((x + block_M - 1) // block_M for x in sizes)
 
     def kernel(A, B, block_metadata, scale, scale_a=None, stream=None, return_accumulators=False):
+        if stream is None and not return_accumulators and b_layout in ("KN", "NK"):
+            C = (_host or _native()).grouped(A, B, block_metadata, scale, scale_a, out_dtype, b_layout == "NK", None,
+                                             total_M, K, G, blocks)
+            if C is not None:
+                return C
         if A.dim() != 2 or tuple(A.shape) != (total_M, K):
             raise ValueError(f"Static shape mismatch for parameter A: expected ({total_M}, {K}), got {tuple(A.shape)}")
         if B.dim() != 3 or B.shape[0] != G:
