@@ -97,12 +97,13 @@ int set_smem_w4() {
 template <int MT>
 int set_smem_w4g() {
   using C = qg::W4GCfg<MT>;
+  constexpr int zt_bytes = qg::W4GCfg<MT, true>::SMEM_BYTES;
   if (set_smem(qg::w4a16_gs_kernel<MT, false>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w4a16_gs_kernel<MT, true>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w4a16_gs_kernel<MT, false, true>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w4a16_gs_kernel<MT, true, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, false, false, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, true, false, true>, C::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, false, false, true>, zt_bytes)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, true, false, true>, zt_bytes)) return -1;
   if constexpr (MT == 16) {
     if (set_smem(qg::w4a16_gs_kernel<16, false, false, false, true>, C::SMEM_BYTES)) return -1;
     if (set_smem(qg::w4a16_gs_kernel<16, true, false, false, true>, C::SMEM_BYTES)) return -1;
@@ -235,32 +236,45 @@ int launch_w4(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUt
   if (bf) return launch_pdl(qg::w4a16_gemm_kernel<MT, true>, grid, qg::W4_THREADS, qg::W4Cfg<MT>::SMEM_BYTES, s, tmW, tmS, tmA, p);
   return launch_pdl(qg::w4a16_gemm_kernel<MT, false>, grid, qg::W4_THREADS, qg::W4Cfg<MT>::SMEM_BYTES, s, tmW, tmS, tmA, p);
 }
+constexpr int64_t kW4MaxGrid = 1024;
+constexpr int64_t kW4CounterBytes = kW4MaxGrid * 4;
+
 // Test hook (qgemm_debug_withhold_commit): see W4GDebug.
 int g_w4g_withhold_commit = 0;
 
 // `tmZ` non-null: the zeros-tensor instantiation (not combined with the gathered form).
 template <int MT>
-int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap* tmZ, const CUtensorMap& tmA,
-               const qg::W4A16Params& p, int grid, cudaStream_t s) {
+int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap* tmZ, const qg::W4A16Params& p,
+               int grid, cudaStream_t s) {
   qg::W4GDebug dbg;
   dbg.withhold_last_commit = g_w4g_withhold_commit;
-  constexpr int smem = qg::W4GCfg<MT>::SMEM_BYTES;
+  constexpr int smem = qg::W4GCfg<MT>::SMEM_BYTES, smem_zt = qg::W4GCfg<MT, true>::SMEM_BYTES;
   if (tmZ != nullptr) {
-    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, *tmZ, tmA, p, dbg);
-    return launch_pdl(qg::w4a16_gs_kernel<MT, false, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, *tmZ, tmA, p, dbg);
+    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, p, dbg);
+    return launch_pdl(qg::w4a16_gs_kernel<MT, false, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, p, dbg);
   }
   if (p.n_dst > 0) {
-    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
-    return launch_pdl(qg::w4a16_gs_kernel<MT, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
+    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+    return launch_pdl(qg::w4a16_gs_kernel<MT, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
   }
-  if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
-  return launch_pdl(qg::w4a16_gs_kernel<MT, false>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
+  if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+  return launch_pdl(qg::w4a16_gs_kernel<MT, false>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+}
+
+// The pre-pass of the group-sum kernel: activations -> stage images.
+template <int MT>
+int launch_w4g_prepare(const void* A, void* out, const qg::W4A16Params& p, bool is_bf16, cudaStream_t s) {
+  const long long threads = (long long)p.batch * p.m_tiles * (2 * p.KS) * MT * 4;
+  const long long blocks = (threads + 127) / 128;
+  if (blocks > 0x7fffffffll) return fail("qgemm_w4a16: activation tensor too large");
+  return launch_pdl(qg::w4g_prepare_activations<MT>, (int)blocks, 128, 0, s, static_cast<const uint4*>(A),
+                    static_cast<uint8_t*>(out), p.batch, p.M, p.K, p.m_tiles, 2 * p.KS, is_bf16 ? 1 : 0,
+                    p.ws_counters, (int)(kW4CounterBytes / 4));
 }
 
 // Single-launch form of the group-sum kernel (see its SMALL parameter): clusters of `cluster` CTAs, one tile per cluster,
 // no pre-pass in front.  Still a programmatic dependent of whatever is in front of it on the stream.
-int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap& tmA,
-                     const qg::W4A16Params& p, int grid, int cluster, cudaStream_t s) {
+int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const qg::W4A16Params& p, int grid, int cluster, cudaStream_t s) {
   static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   qg::W4GDebug dbg;
   dbg.withhold_last_commit = g_w4g_withhold_commit;
@@ -278,8 +292,8 @@ int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, co
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
-  if (bf) CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, true, false, false, true>, tmW, tmS, tmS, tmA, p, dbg));
-  else CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, false, false, false, true>, tmW, tmS, tmS, tmA, p, dbg));
+  if (bf) CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, true, false, false, true>, tmW, tmS, tmS, p, dbg));
+  else CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, false, false, false, true>, tmW, tmS, tmS, p, dbg));
   return 0;
 }
 
@@ -328,9 +342,6 @@ int w4_pick_mt(int64_t M, bool gs) {
   if (w4_use_decode(M)) return M <= 8 ? 8 : 16;
   return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
 }
-
-constexpr int64_t kW4MaxGrid = 1024;
-constexpr int64_t kW4CounterBytes = kW4MaxGrid * 4;
 
 __global__ void unpack_int4_kernel(const uint8_t* __restrict__ packed, int8_t* __restrict__ out, long long n_bytes,
                                    int signed_nibbles) {
@@ -657,10 +668,16 @@ static int64_t w4_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K
   const int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   // sized for whichever small-token kernel the scale groups will select (the group-sum kernel's tile is the taller)
   const int mt = M <= 64 ? w4_pick_mt(M, true) : w4_pick_mt(M, false);
+  // prepared activations: plain f16 [M, K], or the group-sum kernel's stage images (token tiles padded)
+  int64_t a_bytes = batch * M * K * 2;
+  if (M <= 64) {
+    const int64_t images = batch * ((K + 255) / 256) * 2 * (int64_t)qg::w4g_half_bytes(mt);
+    if (images > a_bytes) a_bytes = images;
+  }
   // the arrival counters first (fixed place whatever the tile height), then two partial slots of
   // [MT][128] fp32 per CTA, then the f16 copy of the activations in the kernel's K order
   // ... and, for the large-token path, the dequantised f16 weights
-  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + batch * M * K * 2 +
+  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + a_bytes +
          ((dequant_once || w4_use_f16_gemm(M, N)) ? batch * N * K * 2 : 0);
 }
 
@@ -867,7 +884,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   }
   const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   uint8_t* a_prepared = static_cast<uint8_t*>(workspace) + kW4CounterBytes + grid_max * 2 * (int64_t)mt * 128 * 4;
-  {
+  if (!use_gs) {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)M * (uint64_t)K * 2};
     const uint32_t box[3] = {64, (uint32_t)mt, 1};
@@ -905,7 +922,8 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
   p.A_raw = nullptr;
-  p.a_is_bf16 = p.a_permute = 0;
+  p.a_is_bf16 = 0;
+  p.w_interleaved = weight_format == QGEMM_W4_SEQUENTIAL ? 0 : 1;
   int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   if (p.total_items < grid) grid = p.total_items;
   // Small problems (a few slabs per CTA): prefer a slightly smaller grid that cuts every tile into equal K ranges,
@@ -920,18 +938,16 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
       }
     }
   }
-  // Group-sum kernel, 16-token tile: whole tiles per CTA where there are enough, and only the remainder (plus one
-  // round when the remainder alone would give every CTA a sliver of a tile) cut stream-K fashion, processed first, so
-  // that the launch ends with plain tile writes instead of the partial tiles' hand-overs (K=8192, N=28672: 38.2 ->
-  // 36.5 us at 16 tokens, 37.7 -> 36.1 at 8).  The taller tiles keep the even cut: their drain warps set the pace,
-  // and a hand-over in the middle of a CTA's work stalls them where one at the end only delays the exit (measured
-  // 4 % slower at 32 tokens, 3 % at 64).  QGEMM_W4_HYBRID=0 cuts all tiles stream-K fashion.
+  // Group-sum kernel: whole tiles per CTA where there are enough, and only the remainder (plus one round when the
+  // remainder alone would give every CTA a sliver of a tile) cut stream-K fashion, processed first, so that its hand-overs
+  // run beside the whole tiles' work and the launch ends with plain tile writes.  QGEMM_W4_HYBRID=0 cuts all tiles
+  // stream-K fashion.
   p.sk_tiles = p.num_tiles;
   p.dp_rounds = 0;
   {
     static const int hybrid = getenv("QGEMM_W4_HYBRID") ? atoi(getenv("QGEMM_W4_HYBRID")) : 1;
     const int64_t rounds = num_tiles / grid, r = num_tiles % grid;
-    if (hybrid && use_gs && mt == 16 && rounds >= 1) {
+    if (hybrid && use_gs && rounds >= 1) {
       const bool borrow = r != 0 && 2 * r < grid;
       p.dp_rounds = (int)(borrow ? rounds - 1 : rounds);
       p.sk_tiles = (int)(borrow ? r + grid : r);
@@ -953,10 +969,17 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
       if (cluster > 0 && num_tiles * cluster <= (int64_t)small_waves * sms) {
         p.A_raw = A;
         p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
-        p.a_permute = weight_format == QGEMM_W4_SEQUENTIAL ? 1 : 0;
-        return launch_w4g_small(bf, tmW, tmS, tmA, p, (int)(num_tiles * cluster), cluster, s);
+        return launch_w4g_small(bf, tmW, tmS, p, (int)(num_tiles * cluster), cluster, s);
       }
     }
+  }
+  if (use_gs) {
+    const CUtensorMap* tz = zeros_inflight ? &tmZ : nullptr;
+    const bool a_bf = a_dtype == QGEMM_DT_BF16;
+    p.A_raw = a_prepared;
+    if (mt == 16) return launch_w4g_prepare<16>(A, a_prepared, p, a_bf, s) || launch_w4g<16>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
+    if (mt == 32) return launch_w4g_prepare<32>(A, a_prepared, p, a_bf, s) || launch_w4g<32>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
+    return launch_w4g_prepare<64>(A, a_prepared, p, a_bf, s) || launch_w4g<64>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
   }
   {
     const long long n_chunks = (long long)batch * M * K / 8;
@@ -985,12 +1008,6 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
                                                              (int)N, (int)K, (int)geff, zero);
     CUDA_OK(cudaGetLastError());
     return w4_f16_gemm(a_prepared, w16, C, batch, M, N, K, bf, status, s, sms, gd);
-  }
-  if (use_gs) {
-    const CUtensorMap* tz = zeros_inflight ? &tmZ : nullptr;
-    if (mt == 16) return launch_w4g<16>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
-    if (mt == 32) return launch_w4g<32>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
-    return launch_w4g<64>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
   }
   if (gd == nullptr && w4_use_decode(M) && mt <= 16 && M <= w4_decode_max_m()) {
     if (scales == nullptr) return launch_w4d<0>(bf, mt, tmW, tmS, tmA, p, (int)grid, s);
@@ -1225,7 +1242,7 @@ constexpr int64_t kStaticMaxM = QGEMM_W4A16_NOALLOC_MAX_M;
 constexpr int64_t kStaticMaxK = QGEMM_W4A16_NOALLOC_MAX_K;
 constexpr int64_t kStaticMaxSms = 160;
 constexpr int64_t kStaticScratchBytes =
-    kW4CounterBytes + kStaticMaxSms * 2 * kStaticMaxM * 128 * 4 + kStaticMaxM * kStaticMaxK * 2;  // about 6.3 MB
+    kW4CounterBytes + kStaticMaxSms * 2 * kStaticMaxM * 128 * 4 + (kStaticMaxK / 128) * qg::w4g_half_bytes(kStaticMaxM);  // about 6.4 MB
 
 static __device__ __align__(256) unsigned char g_w4a16_static_scratch[kStaticScratchBytes];
 

@@ -44,10 +44,10 @@ struct W4A16Params {
   // Group-sum kernel only: tiles 0 .. sk_tiles - 1 are cut stream-K fashion over all CTAs, then CTA c takes dp_rounds
   // whole tiles sk_tiles + c + j * grid.  The other kernels deal all (tile, slab) items evenly (total_items).
   int sk_tiles, dp_rounds;
-  // Single-launch form of the group-sum kernel (no pre-pass): the caller's activations [batch, M, K], whether they
-  // are bf16, and whether every group of eight k is to be reordered (sequential weight layout).
+  // Group-sum kernel: the prepared activations (stage images) or, in its single-launch form (no pre-pass), the caller's
+  // activations [batch, M, K] and whether they are bf16; and whether the weight layout is the interleaved one.
   const void* A_raw;
-  int a_is_bf16, a_permute;
+  int a_is_bf16, w_interleaved;
   int scale_rows;       // scale rows fetched per slab (256 / group, at least 1)
   long long total_items;
   uint32_t* status;
@@ -124,6 +124,20 @@ __device__ __forceinline__ void w4_store_out(const W4A16Params& p, uint16_t* Cou
 #pragma unroll
     for (int d = 0; d < 8; ++d)
       if (d < p.n_dst) reinterpret_cast<uint16_t*>(p.c_dst[d])[off] = h;
+  }
+}
+
+// Four consecutive output features n .. n + 3 of token m (N, ldc and col0 are multiples of 8): one 8-byte store each.
+template <bool OUT_BF16, bool GATHER = true>
+__device__ __forceinline__ void w4_store_out4(const W4A16Params& p, uint16_t* Cout, int m, int n, const float4& v) {
+  const uint2 h = make_uint2(pack_out2<OUT_BF16>(v.x, v.y), pack_out2<OUT_BF16>(v.z, v.w));
+  if (!GATHER || p.n_dst == 0) {
+    *reinterpret_cast<uint2*>(Cout + (size_t)m * p.N + n) = h;
+  } else {
+    const size_t off = (size_t)m * p.ldc + p.col0 + n;
+#pragma unroll
+    for (int d = 0; d < 8; ++d)
+      if (d < p.n_dst) *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.c_dst[d]) + off) = h;
   }
 }
 

@@ -5,33 +5,31 @@
 // and is rounded once, to the output type); in general it differs from scaling each weight in f16 first
 // only by that product's own rounding (2^-11 relative per term), well inside the operator's tolerance.
 //
-// Why: these shapes are bound by instruction issue on the SM, not by memory (a warp gets an issue slot
-// only every ~10 cycles once 28 warps share four schedulers, and the ALU and FP16 pipes run at half
-// rate), so the kernel is written to execute as few instructions per weight as possible:
-//  - 9 instead of 13 instructions per eight weights in the dequant warps (no f16x2 scale multiplies; the
-//    scale work is one fp32 FMA per (token, 128 k) in four drain warps, on the otherwise idle FMA pipe);
-//  - ring stages and barrier parities are compile-time constants of unrolled loops, barrier addresses
-//    are one base register plus an immediate, a wait is a try_wait and a branch on its fast path;
-//  - a dequant warp converts a whole 128-k half of its 32 rows per hand-over (two sets of eight warps
-//    take alternate slabs), so the hand-over cost is paid once per 16 packed words;
-//  - the MMA-issuing warps run warp-convergent, one hardware-elected lane issues the eight MMAs of a half
-//    and their commits (see w4g_elect_one), and they know nothing about tiles: every 128-k half starts a
-//    fresh accumulator.
+// What bounds these shapes is not memory but the number of instructions and hand-overs an SM spends per 16 KB slab of
+// packed weights (a slab's HBM time is about 700 cycles per SM), so the kernel is built to spend few:
+//  - Conversion in five integer instructions per eight weights, no arithmetic at all.  A nibble q in bits 0..3 of an f16
+//    word IS the number q * 2^-24 (a subnormal), one in bits 4..7 is q * 2^-20, and the tensor core takes subnormals at
+//    full precision; so masking is converting: x & 0x000f000f, x & 0x00f000f0, and the same of x >> 8.  The MMAs of a
+//    128-k half first sum the "high" words (16 times too large), then the "low" ones, the first of which scales what has
+//    been accumulated by 2^-4 (tcgen05.mma's scale-input-d): exact, as is the factor 2^24 that the group scale carries.
+//  - The zero point enters as one more MMA per half: a constant weight column -zero against the activations' sum over the
+//    half, which the pre-pass provides as three f16 parts (about 33 bits, see w4g_sum_parts).
+//  - Activations are laid out by the pre-pass in the exact image of a shared-memory stage (swizzle, K order, sum
+//    columns), so that a stage is one untiled bulk copy.
+//  - All hand-overs are by whole slabs; one commit per slab signals one barrier that the weight stage, the activation
+//    stage and the accumulators share; the group scales arrive with the packed bytes and need no barrier of their own.
 //
-// Structure (persistent stream-K over (tile, 256-wide K slab) items, as in w4a16.cuh):
-//   warp 0        TMA: packed weights [128 rows x 128 B] per slab into the raw ring
-//   warp 1        TMA: prepared activations [MT x 256 k] per slab into their ring
-//   warp 2        tensor-memory allocation; TMA: the slab's scale rows [1 or 2 x 128] into the scale ring
-//   warps 4..7, 28..31  drain (two sets of four on alternate slabs: one warp's instruction stream per slab is a
-//                 serial chain of ~85 instructions, too long for one warp per 32 rows at the slab rate):
-//                 one tcgen05.ld of the slab's two accumulators, fp32 FMA with each half's scale into register
-//                 sums; at a segment's end the sets add their sums, then the tile write or the split-K hand-over
-//   warps 8..23   dequant: lop3 magic-number conversion, (q - zero) exact in f16, tcgen05.st
-//   warps 24..27  tcgen05.mma kind::f16 issuers (A = weights from tensor memory, B = activations from
-//                 shared memory); issuer w takes the 128-k halves h with h % 4 == w, each into its own
-//                 accumulator of a ring, so no two issuers ever share an accumulator
-// Tensor memory: NSLOT slab slots of two accumulators of MT columns (ring, 256 columns) + 4 stages of 64 columns
-// of converted weights (one 128-k half each).
+// Structure (persistent; the K slabs of the tiles are dealt to the CTAs, see W4HybridIter):
+//   warp 0        TMA: packed weights [128 rows x 128 B] per slab into the raw ring, the slab's scale (and zero) rows
+//   warp 1        bulk copies: prepared activations
+//   warps 2, 3    tcgen05.mma kind::f16 issuers (A = weights from tensor memory, B = activations from shared memory):
+//                 issuer w takes the slabs i with i % 2 == w, each of the two halves into its own accumulator
+//   warps 4..11   drain: tcgen05.ld of a half's accumulator, fp32 FMA with the half's scale into register sums; set e
+//                 (four warps, one per 32 rows) takes the slabs of parity e and the sets add their sums at a segment's
+//                 end; then the tile write or the split-K hand-over
+//   warps 12..19  dequant: set s (four warps, one per 32 rows) converts the slabs of parity s
+//   warps 20..23  split-K hand-overs
+// Tensor memory: NS slots of two accumulators of MT columns + WS stages of 128 columns of converted weights.
 //
 // Every wait is bounded: after a number of failed mbarrier.try_wait attempts (each suspends the thread
 // for a few microseconds) derived from the caller's limit, the wait stores its role code in a CTA-wide
@@ -48,61 +46,66 @@
 
 namespace qg {
 
+constexpr int W4G_FIRST_MMA_WARP = 2;
+constexpr int W4G_MMA_WARPS = 2;
 constexpr int W4G_FIRST_EPI_WARP = 4;
-constexpr int W4G_FIRST_DQ_WARP = 8;
-constexpr int W4G_DQ_WARPS = 16;
-constexpr int W4G_FIRST_MMA_WARP = W4G_FIRST_DQ_WARP + W4G_DQ_WARPS;  // 24
-constexpr int W4G_MMA_WARPS = 4;
-constexpr int W4G_FIRST_EPI2_WARP = W4G_FIRST_MMA_WARP + W4G_MMA_WARPS;  // 28: second set of drain warps
-constexpr int W4G_THREADS = (W4G_FIRST_EPI2_WARP + 4) * 32;             // 1024
-constexpr int W4G_WH = 4;          // stages of converted weights, one 128-k half (64 columns) each
-constexpr int W4G_HALF_COLS = 64;
-constexpr int W4G_RS = 8;          // raw (packed weight) ring, 16 KB per stage
-constexpr int W4G_SS = 16;         // scale ring, 512 B per stage
-constexpr int W4G_SC_BYTES = 512;  // up to two rows of 128 halves
+constexpr int W4G_EPI_WARPS = 8;
+constexpr int W4G_FIRST_DQ_WARP = W4G_FIRST_EPI_WARP + W4G_EPI_WARPS;  // 12
+constexpr int W4G_DQ_SETS = 2;      // sets of four dequant warps
+constexpr int W4G_FIN_WARP = W4G_FIRST_DQ_WARP + 4 * W4G_DQ_SETS;  // 20..23: split-K hand-overs
+constexpr int W4G_THREADS = (W4G_FIN_WARP + 4) * 32;               // 768: at most 80 registers per thread
+constexpr int W4G_SLAB_COLS = 128;  // tensor-memory columns of a converted slab
+constexpr int W4G_SC_BYTES = 512;   // a slab's scales: up to two rows of 128 halves
+constexpr int W4G_BARS = 8;         // barriers of a ring (whatever the number of data stages behind it), indexed by slab % 8
+constexpr int W4G_Z_BYTES = 2048;   // the zero point's operand: 128 rows x 8 k of f16 (k 8 .. 15 are one shared tile of zeros)
 
 // Byte offsets of the barriers (8 bytes each) and control words from the start of the barrier block.
-constexpr int W4G_RAW_FULL = 0;       // [8]
-constexpr int W4G_RAW_EMPTY = 64;     // [8]
-constexpr int W4G_A_FULL = 128;       // [<= 8]
-constexpr int W4G_A_EMPTY = 192;      // [<= 8]
-constexpr int W4G_W_FULL = 256;       // [4]
-constexpr int W4G_W_EMPTY = 288;      // [4]
-constexpr int W4G_ACC_FULL = 320;     // [<= 8] one per slab slot: both halves' issuers commit to it
-constexpr int W4G_ACC_EMPTY = 448;    // [<= 8]
-constexpr int W4G_SC_FULL = 576;      // [16]
-constexpr int W4G_SC_EMPTY = 704;     // [16]
-constexpr int W4G_DRAIN = 832;
-constexpr int W4G_TMEM_SLOT = 840;
-constexpr int W4G_CTL = 848;          // u32 abort word (0, or the role code of the first wait that gave up), u32 max tries
-constexpr int W4G_EPI_CTRL = 856;     // u32[2], alternating by segment: bit 0 abort, bit 1 last contributor
-constexpr int W4G_PART_FULL = 864;    // SMALL form, in the cluster's first CTA: the other CTAs' sums have arrived
+constexpr int W4G_RAW_FULL = 0;       // [8] a slab's packed weights (and scale rows) have landed
+constexpr int W4G_RAW_EMPTY = 64;     // [8] its set has them in registers
+constexpr int W4G_A_FULL = 128;       // [8] its activations have landed
+constexpr int W4G_W_FULL = 192;       // [8] its converted weights are in tensor memory
+constexpr int W4G_DONE = 256;         // [8] its MMAs have completed
+constexpr int W4G_ACC_EMPTY = 320;    // [<= 4] an accumulator slot has been drained
+constexpr int W4G_W_FULL0 = 352;      // [8] halves as steps (64 tokens): the first half's converted weights,
+constexpr int W4G_DONE0 = 416;        // [8]   and its MMAs
+constexpr int W4G_PART_READY = 480;   // [2] the CTA's (at most two) partial tiles: its sums are in the scratch buffer
+constexpr int W4G_DRAIN = 496;
+constexpr int W4G_PART_FULL = 504;    // SMALL form, in the cluster's first CTA: the other CTAs' sums have arrived
+constexpr int W4G_TMEM_SLOT = 512;
+constexpr int W4G_CTL = 520;          // u32 abort word (0, or the role code of the first wait that gave up), u32 max tries
+constexpr int W4G_FIN_WORD = 528;     // u32[2], one per partial tile: its arrival number
 constexpr int W4G_SMALL_MAX_SLABS = 4;  // SMALL form: slabs per CTA (stages 4.. of the raw ring receive the other CTAs' sums)
 
-template <int MT>
+// Bytes of one prepared activation half: MT rows x 128 k of f16 (two 128-byte-swizzled blocks of 64 k), then the MT x 16
+// sum columns as 8-row x 16-byte core matrices, padded to the 1024 bytes from which the swizzle counts.
+__host__ __device__ constexpr int w4g_half_bytes(int mt) { return (mt * 256 + mt * 32 + 1023) / 1024 * 1024; }
+
+template <int MT, bool ZT = false>
 struct W4GCfg {
   static_assert(MT == 16 || MT == 32 || MT == 64, "token tile");
-  static constexpr int AS = (MT == 16) ? 8 : (MT == 32 ? 4 : 2);  // activation ring (even: an issuer meets every phase of its stages)
-  static constexpr int NSLOT = 128 / MT;           // slab slots of two accumulators each (8, 4 or 2)
-  // How the two drain sets share the work: on alternate slabs, all tokens each (their sums meet at a segment's
-  // end), or - 64 tokens would not fit a thread's registers - every slab, 32 tokens each (nothing to exchange).
-  static constexpr bool SPLIT_TOKENS = MT == 64;
-  static constexpr int DT = SPLIT_TOKENS ? 32 : MT;  // tokens one drain thread accumulates
-  static constexpr int A_KB_BYTES = MT * 128;      // one 64-wide K block of activations
-  static constexpr int A_BYTES = 4 * A_KB_BYTES;   // one 256-wide slab
+  // Rings, in slabs.  64 KB of raw (packed) weights in flight per SM already stream at full speed.
+  static constexpr int RS = (MT == 16) ? 8 : 4;           // raw weights, 16 KB each
+  static constexpr int AS = (MT == 16) ? 4 : (MT == 32 ? 6 : 3);  // activations
+  static constexpr int WS = (MT <= 32) ? 3 : 2;           // converted weights (tensor memory)
+  static constexpr int NS = (MT == 16) ? 4 : 2;           // accumulator slots of two halves (even: a slot belongs to one set)
+  static constexpr int SS = (RS == 8) ? 32 : 16;          // scale rows (see the note at the weight producer)
+  static constexpr int A_HALF = w4g_half_bytes(MT);
+  static constexpr int A_BYTES = 2 * A_HALF;              // one slab
   static constexpr int TMEM_COLS = 512;
-  static constexpr int BAR_BYTES = 1024;
-  static constexpr int XBUF_BYTES = SPLIT_TOKENS ? 0 : MT * W4_BN * 4;  // the second drain set's sums of one segment
-  static constexpr int SMEM_BYTES =
-      W4G_RS * W4_RAW_PACKED + AS * A_BYTES + W4G_SS * W4G_SC_BYTES + W4G_RS * W4G_SC_BYTES + XBUF_BYTES + BAR_BYTES + 1024;
-  static constexpr int A_PER = AS / 2;                // activation stages one issuer meets
-  static constexpr int S_PER = NSLOT / 2;             // slab slots one issuer meets (those of its slab parity)
-  static_assert(A_PER == 4 || A_PER == 2 || A_PER == 1, "activation ring depth");
-  static_assert(S_PER == 4 || S_PER == 2 || S_PER == 1, "accumulator ring depth");
+  static constexpr int BAR_BYTES = 576;
+  // 64 tokens: tensor memory holds two slabs of converted weights only, so the hand-over to the MMAs and back is by
+  // halves - otherwise both sets convert while the tensor pipe idles and then both wait for it.
+  static constexpr bool HALVES = MT == 64;
+  static constexpr int XBUF_BYTES = MT * W4_BN * 4;       // the second drain set's sums of one segment
+  static constexpr int Z_STAGES = ZT ? 2 * WS : 1;        // a zeros tensor changes the operand tile with every half
+  static constexpr int SMEM_BYTES = RS * W4_RAW_PACKED + AS * A_BYTES + SS * W4G_SC_BYTES + (ZT ? RS * W4G_SC_BYTES : 0) +
+                                    (Z_STAGES + 1) * W4G_Z_BYTES + XBUF_BYTES + BAR_BYTES + 1024;
+  static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
+  static_assert(NS * 2 * MT + WS * W4G_SLAB_COLS <= 512 && (RS & (RS - 1)) == 0 && NS % 2 == 0 && AS < W4G_BARS, "layout");
 };
 
-// Debug hook for the bounded-wait test: when non-zero, the MMA issuers do not signal the accumulator of
-// the last 128-k half of the launch, so the drain warps' wait for it runs out.  Nothing else is affected:
+// Debug hook for the bounded-wait test: when non-zero, the MMA issuers do not signal the completion of
+// the last slab of the launch, so the drain warps' wait for it runs out.  Nothing else is affected:
 // every copy lands, every other barrier completes, the kernel frees its tensor memory and returns.
 struct W4GDebug {
   int withhold_last_commit;  // 1: as described above (two-launch form); 2: the single-launch form's cluster signal
@@ -181,10 +184,26 @@ __device__ __forceinline__ void w4g_fma2(float& d0, float& d1, uint32_t a0, uint
 // Named barrier of the eight drain warps.
 __device__ __forceinline__ void w4g_epi_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// Parity of the n-th visit (n = 4 * c + u, u < 4) of a ring position that is met every `PER` iterations.
-template <int PER>
-__device__ __forceinline__ uint32_t w4g_visit_parity(uint32_t c, int u) {
-  return (PER == 4) ? (c & 1u) : (uint32_t)((u / PER) & 1);
+
+// D = A * B + D * 2^-4, A from tensor memory (see the header comment: the step from the high to the low nibble words).
+__device__ __forceinline__ void w4g_mma_ts_shift4(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, 4;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc)
+      : "memory");
+}
+// Matrix descriptor of an unswizzled operand of 16 k: core matrices of 8 rows x 16 bytes, the two k halves of a row group
+// `k_stride` bytes apart, row groups `row_stride` bytes apart.
+__device__ __forceinline__ uint64_t w4g_desc_k16(uint32_t saddr, uint32_t k_stride, uint32_t row_stride) {
+  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(k_stride >> 4) << 16) |
+         (static_cast<uint64_t>(row_stride >> 4) << 32) | (static_cast<uint64_t>(1) << 46);
+}
+// Untiled bulk copy global -> shared memory.
+__device__ __forceinline__ void w4g_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 
 // The segments of a CTA: those of its stream-K range, then its whole tiles (first_dp, first_dp + stride, ...).
@@ -203,34 +222,166 @@ struct W4HybridIter {
   }
 };
 
+
+// ---- prepared activations ---------------------------------------------------------------------------------------
+// A 32-k chunk of a row becomes two groups of 16 f16 values: those whose weights the conversion finds in the low nibbles
+// of the bytes it masks, then those in the high ones.  Word w of a packed 16-byte chunk holds elements 8 w .. 8 w + 7:
+// low 8 w + {0, 4, 2, 6}, high 8 w + {1, 5, 3, 7}.
+// v: the eight values of word w as four f16x2 words (0 1)(2 3)(4 5)(6 7) -> lo, hi: two f16x2 words each.
+__device__ __forceinline__ void w4g_split_word(const uint4& v, uint2& lo, uint2& hi) {
+  lo = make_uint2(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.y, v.w, 0x5410));
+  hi = make_uint2(__byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x7632));
+}
+__device__ __forceinline__ uint4 w4g_to_f16(uint4 v, bool is_bf16) {
+  if (is_bf16) {
+    v.x = w4_bf16x2_to_f16x2(v.x);
+    v.y = w4_bf16x2_to_f16x2(v.y);
+    v.z = w4_bf16x2_to_f16x2(v.z);
+    v.w = w4_bf16x2_to_f16x2(v.w);
+  }
+  return v;
+}
+__device__ __forceinline__ float w4g_sum8(const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    s += f.x + f.y;
+  }
+  return s;
+}
+// The half's sum S as f16 parts p0 * 2^7 + p1 + p2: p0 takes the leading 11 bits (scaled, because S may exceed f16's
+// range), p1 and p2 the next 22; the remainder is below 2^-33 |S| or below f16's own granularity 2^-24, whichever is larger.
+__device__ __forceinline__ uint2 w4g_sum_parts(float S) {
+  const __half p0 = __float2half_rn(S * 0.0078125f);
+  const float r0 = S - __half2float(p0) * 128.0f;
+  const __half p1 = __float2half_rn(r0);
+  const __half p2 = __float2half_rn(r0 - __half2float(p1));
+  return make_uint2((uint32_t)__half_as_ushort(p0) | ((uint32_t)__half_as_ushort(p1) << 16), (uint32_t)__half_as_ushort(p2));
+}
+// The weights that face them: -zero in units of 2^-24, the first one times 2^7 (0 <= zero <= 15: exact in f16).
+__device__ __forceinline__ uint2 w4g_zero_weights(float zero) {
+  const uint32_t a = __half_as_ushort(__float2half_rn(-zero * 7.62939453125e-6f));     // 2^-17
+  const uint32_t b = __half_as_ushort(__float2half_rn(-zero * 5.9604644775390625e-8f));  // 2^-24
+  return make_uint2(a | (b << 16), b);
+}
+// Byte offset of 16-byte piece j (0..15) of row r inside a half's image: 64-k block j / 8, 128-byte swizzle.
+template <int MT>
+__device__ __forceinline__ uint32_t w4g_a_offset(int r, int j) {
+  return (uint32_t)((j >> 3) * (MT * 128) + r * 128 + (((j & 7) ^ (r & 7)) << 4));
+}
+__device__ __forceinline__ uint32_t w4g_core_offset(int r) { return (uint32_t)((r >> 3) * 256 + (r & 7) * 16); }
+
+// One 32-k chunk (chunk c of four) of row r: four 16-byte loads already in v -> the half's image at dst (global or shared
+// memory).  Four consecutive lanes hold the four chunks of a row's half; the first one writes the sum columns.
+template <int MT>
+__device__ __forceinline__ void w4g_emit_chunk(uint8_t* dst, int r, int c, const uint4 (&v)[4]) {
+  uint2 lo[4], hi[4];
+  float s = 0.f;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    w4g_split_word(v[w], lo[w], hi[w]);
+    s += w4g_sum8(v[w]);
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 0)) = make_uint4(lo[0].x, lo[0].y, lo[1].x, lo[1].y);
+  *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 1)) = make_uint4(lo[2].x, lo[2].y, lo[3].x, lo[3].y);
+  *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 2)) = make_uint4(hi[0].x, hi[0].y, hi[1].x, hi[1].y);
+  *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 3)) = make_uint4(hi[2].x, hi[2].y, hi[3].x, hi[3].y);
+  if (c == 0) {
+    const uint2 p = w4g_sum_parts(s);
+    *reinterpret_cast<uint4*>(dst + MT * 256 + w4g_core_offset(r)) = make_uint4(p.x, p.y, 0u, 0u);
+    *reinterpret_cast<uint4*>(dst + MT * 256 + w4g_core_offset(r) + 128) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+// Pre-pass: activations [batch, M, K] (f16 or bf16) -> [batch][token tile][half] images (rows beyond M and k beyond K are
+// zero).  One thread per 32-k chunk.  Block 0 also zeroes the split-K arrival counters, so every call starts from clean
+// counters whatever an earlier (possibly aborted) call left in the scratch.
+template <int MT>
+__global__ void __launch_bounds__(128)
+w4g_prepare_activations(const uint4* __restrict__ in, uint8_t* __restrict__ out, int batch, int M, int K, int m_tiles,
+                        int halves, int is_bf16, uint32_t* __restrict__ counters, int n_counters) {
+  pdl_launch_dependents();  // the GEMM kernel behind may set up and start streaming weights meanwhile
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = (int)(i & 3);
+  const int r = (int)((i >> 2) % MT);
+  const long long blk = (i >> 2) / MT;  // (b * m_tiles + tile) * halves + half
+  const int half = (int)(blk % halves);
+  const long long bt = blk / halves;
+  const int tile = (int)(bt % m_tiles);
+  const long long b = bt / m_tiles;
+  pdl_wait();  // the kernel in front (another call's GEMM, which lets its dependents start early) is done
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < n_counters; k += blockDim.x) counters[k] = 0u;
+  if (b >= batch) return;  // whole groups of four lanes; the grid is a multiple of MT * 4 threads, so whole warps too
+  const int m = tile * MT + r, k0 = half * 128 + c * 32;
+  uint4 v[4];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) v[w] = make_uint4(0u, 0u, 0u, 0u);
+  if (m < M && k0 < K) {  // K is a multiple of 32
+    const uint4* src = in + ((size_t)b * M + m) * (size_t)(K / 8) + k0 / 8;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) v[w] = src[w];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) v[w] = w4g_to_f16(v[w], is_bf16 != 0);
+  }
+  w4g_emit_chunk<MT>(out + (size_t)blk * w4g_half_bytes(MT), r, c, v);
+}
+
+// Sixteen packed bytes (32 weights) -> eight f16x2 words of low values (units of 2^-24), eight of high values (units of
+// 2^-20), K order as in w4g_split_word.  Sequential layout: five integer instructions per eight weights.  Interleaved
+// layout (nibbles 0 2 4 6 | 1 3 5 7): eight, into the same words, so that both layouts give the same sums bit for bit.
+template <bool INTERLEAVED>
+__device__ __forceinline__ void w4g_convert(const uint4& v, uint32_t (&o)[16]) {
+  const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+  if constexpr (!INTERLEAVED) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t y = x[w] >> 8;
+      o[2 * w] = x[w] & 0x000f000fu;
+      o[2 * w + 1] = y & 0x000f000fu;
+      o[8 + 2 * w] = x[w] & 0x00f000f0u;
+      o[8 + 2 * w + 1] = y & 0x00f000f0u;
+    }
+  } else {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t ev = __byte_perm(x[w], 0u, 0x4140), od = __byte_perm(x[w], 0u, 0x4342);  // (0 2 | 4 6), (1 3 | 5 7)
+      o[2 * w] = ev & 0x000f000fu;
+      o[2 * w + 1] = (ev >> 4) & 0x000f000fu;
+      o[8 + 2 * w] = (od << 4) & 0x00f000f0u;
+      o[8 + 2 * w + 1] = od & 0x00f000f0u;
+    }
+  }
+}
+
 // GATHER = true is the gathered form (several destination buffers, see W4A16Params::c_dst); it is a separate
-// instantiation because the destination loop in the store path costs the plain kernel 8 % through register
-// allocation alone.
+// instantiation because the destination loop in the store path costs the plain kernel registers.
 // ZT = true: one integer zero point per (group, output feature) instead of the scalar one - the zeros tensor
 // [K/g, N] f16 of zero mode "quantized" (tilelang/quantize/lop3.py:325-358: (q - qz) * s with the subtraction
 // exact).  The weight producer fetches the slab's zero rows (through tmZ, laid out like the scale rows) into a ring
-// that shares the packed weights' stages and barriers, and a dequant thread builds its row's two magic constants
-// from the zero it reads there: five more instructions per 128-k half.
+// that shares the packed weights' stages and barriers, and a dequant thread writes its row of the half's zero operand.
 // SMALL = true (16-token tile): the single-launch form for problems of a few slabs per CTA.  The kernel is launched in
 // clusters of C = KS / (slabs per CTA) CTAs, one tile per cluster, CTA r taking the r-th K range; there is no pre-pass
 // and no scratch memory:
-//  - the drain warps first fetch the CTA's own piece of the activations straight from the caller's tensor, convert
-//    and reorder it as the pre-pass would, and write it into the activation stages in the layout the MMA descriptor
-//    expects (128-byte swizzle: 16-byte chunk j of row r of a 64-k block at chunk position j ^ (r & 7));
+//  - the drain warps first fetch the CTA's own piece of the activations straight from the caller's tensor and write the
+//    stage images the pre-pass would have written;
 //  - at the end CTAs 1 .. C-1 write their sums through distributed shared memory into the unused upper half of the
 //    first CTA's raw ring, and the first CTA adds them in rank order and writes the tile - no counters, no partial
 //    sums in global memory, the same fixed summation order on every run.
 template <int MT, bool OUT_BF16, bool GATHER = false, bool ZT = false, bool SMALL = false>
 __global__ void __launch_bounds__(W4G_THREADS, 1)
 w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
-                const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmA, const W4A16Params p,
-                const W4GDebug dbg) {
-  using Cfg = W4GCfg<MT>;
-  constexpr int RS = W4G_RS;
+                const __grid_constant__ CUtensorMap tmZ, const W4A16Params p, const W4GDebug dbg) {
+  using Cfg = W4GCfg<MT, ZT>;
+  constexpr int RS = Cfg::RS;
   constexpr int AS = Cfg::AS;
-  constexpr int NSLOT = Cfg::NSLOT;
-  constexpr int SS = W4G_SS;
-  static_assert(RS == 8 && SS == 16 && AS <= 8 && NSLOT <= 8, "barrier block layout");
+  constexpr int NS = Cfg::NS;
+  constexpr int WS = Cfg::WS;
+  static_assert(RS <= 8 && NS <= 4, "barrier block layout");
   static_assert(!SMALL || (MT == 16 && !GATHER && !ZT), "the single-launch form: 16-token tile, one destination, scalar zero");
   // The next call's pre-pass (a programmatic dependent) may become resident now; it waits for this whole grid before
   // it touches anything, and the GEMM kernel behind it only reads weights and scales until that pre-pass is done.
@@ -239,75 +390,65 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* raw_base = smem;
-  uint8_t* a_base = smem + RS * W4_RAW_PACKED;
-  uint8_t* sc_base = a_base + AS * Cfg::A_BYTES;
-  uint8_t* z_base = sc_base + SS * W4G_SC_BYTES;  // zero rows, one 512-byte stage per raw stage (ZT only)
-  float* xbuf = reinterpret_cast<float*>(z_base + RS * W4G_SC_BYTES);
-  uint8_t* bar_block = z_base + RS * W4G_SC_BYTES + Cfg::XBUF_BYTES;
+  uint8_t* a_base = raw_base + RS * W4_RAW_PACKED;
+  uint8_t* zop_base = a_base + AS * Cfg::A_BYTES;        // the zero point's operand tile(s)
+  uint8_t* sc_base = zop_base + (Cfg::Z_STAGES + 1) * W4G_Z_BYTES;
+  uint8_t* z_base = sc_base + Cfg::SS * W4G_SC_BYTES;     // zero rows, one 512-byte stage per raw stage (ZT only)
+  float* xbuf = reinterpret_cast<float*>(z_base + (ZT ? RS * W4G_SC_BYTES : 0));
+  uint8_t* bar_block = reinterpret_cast<uint8_t*>(xbuf) + Cfg::XBUF_BYTES;
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(bar_block + W4G_RAW_FULL);
-  uint64_t* raw_empty = reinterpret_cast<uint64_t*>(bar_block + W4G_RAW_EMPTY);
   uint64_t* a_full = reinterpret_cast<uint64_t*>(bar_block + W4G_A_FULL);
-  uint64_t* a_empty = reinterpret_cast<uint64_t*>(bar_block + W4G_A_EMPTY);
-  uint64_t* w_full = reinterpret_cast<uint64_t*>(bar_block + W4G_W_FULL);
-  uint64_t* w_empty = reinterpret_cast<uint64_t*>(bar_block + W4G_W_EMPTY);
-  uint64_t* acc_full = reinterpret_cast<uint64_t*>(bar_block + W4G_ACC_FULL);
-  uint64_t* acc_empty = reinterpret_cast<uint64_t*>(bar_block + W4G_ACC_EMPTY);
-  uint64_t* sc_full = reinterpret_cast<uint64_t*>(bar_block + W4G_SC_FULL);
-  uint64_t* sc_empty = reinterpret_cast<uint64_t*>(bar_block + W4G_SC_EMPTY);
   uint64_t* drain = reinterpret_cast<uint64_t*>(bar_block + W4G_DRAIN);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_block + W4G_TMEM_SLOT);
   volatile uint32_t* ctl_words = reinterpret_cast<uint32_t*>(bar_block + W4G_CTL);  // [0] abort word, [1] max tries
-  volatile uint32_t* epi_ctrl = reinterpret_cast<uint32_t*>(bar_block + W4G_EPI_CTRL);
 
   // a warp index the compiler can prove uniform, so that everything derived from it may live in uniform registers
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
-  // One thread per barrier slot sets it up (the block is a dense array of 8-byte slots; a serial loop over the
-  // hundred of them costs about a microsecond of every launch).
-  if (threadIdx.x <= W4G_DRAIN / 8) {
+  // One thread per barrier slot sets it up (the block is a dense array of 8-byte slots).
+  if (threadIdx.x <= W4G_PART_FULL / 8) {
     const int off = 8 * (int)threadIdx.x;
-    const int drain_warps = Cfg::SPLIT_TOKENS ? 8 : 4;  // drain warps that read one slab: one set, or both
-    int count = 0;                                       // 0: unused slot
+    int count = 0;                                          // 0: unused slot
     if (off < W4G_RAW_EMPTY) count = 1;
-    else if (off < W4G_A_FULL) count = W4G_DQ_WARPS / 2;   // the eight dequant warps of the set that took the slab
-    else if (off < W4G_A_EMPTY) count = (off - W4G_A_FULL) / 8 < AS ? 1 : 0;
-    else if (off < W4G_W_FULL) count = (off - W4G_A_EMPTY) / 8 < AS ? 2 : 0;  // the issuers of the slab's two halves
-    else if (off < W4G_W_EMPTY) count = 4;                 // the four dequant warps (one per 32 rows) of that half
-    else if (off < W4G_ACC_FULL) count = 1;
-    else if (off < W4G_ACC_EMPTY) count = (off - W4G_ACC_FULL) / 8 < NSLOT ? 2 : 0;  // the issuers of the two halves
-    else if (off < W4G_SC_FULL) count = (off - W4G_ACC_EMPTY) / 8 < NSLOT ? drain_warps : 0;
-    else if (off < W4G_SC_EMPTY) count = 1;
-    else if (off < W4G_DRAIN) count = drain_warps;
-    else count = W4G_MMA_WARPS;
+    else if (off < W4G_A_FULL) count = 4;      // the four dequant warps of the slab's set
+    else if (off < W4G_W_FULL) count = 1;
+    else if (off < W4G_DONE) count = 4;
+    else if (off < W4G_ACC_EMPTY) count = 1;
+    else if (off < W4G_W_FULL0) count = 4;     // the four drain warps of the slab's set
+    else if (off < W4G_DONE0) count = 4;
+    else if (off < W4G_PART_READY) count = 1;
+    else if (off < W4G_DRAIN) count = 4;       // the four warps of drain set 0
+    else if (off < W4G_PART_FULL) count = W4G_MMA_WARPS;
+    else if (SMALL) count = max((int)cluster_nctarank() - 1, 1);
     if (count > 0) mbar_init(reinterpret_cast<uint64_t*>(bar_block + off), (uint32_t)count);
     fence_barrier_init();
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 64) {
     ctl_words[0] = 0;
     // a failed try_wait has suspended the thread for roughly 2 us or longer
     ctl_words[1] = (uint32_t)(p.wait_limit_ns >> 11) + 2u;
-    epi_ctrl[0] = epi_ctrl[1] = 0;
     tma_prefetch_desc(&tmW);
-    tma_prefetch_desc(&tmA);
     if (p.has_scales) tma_prefetch_desc(&tmS);
     if (ZT) tma_prefetch_desc(&tmZ);
-    if constexpr (SMALL) {
-      const uint32_t others = cluster_nctarank() - 1u;
-      mbar_init(reinterpret_cast<uint64_t*>(bar_block + W4G_PART_FULL), others > 0u ? others : 1u);
-      fence_barrier_init();
-    }
   }
-  if (warp == 2) {
+  if (warp == W4G_FIRST_MMA_WARP + 1) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
+  // the zero point's operand: k = 0 .. 2 face the parts of the activation sums, all other k are zero
+  for (int i = (int)threadIdx.x - 128; i >= 0 && i < (Cfg::Z_STAGES + 1) * 128; i += W4G_THREADS - 128) {
+    uint2 w = make_uint2(0u, 0u);
+    if (i < 128 && !ZT) w = w4g_zero_weights((float)p.zero);
+    *reinterpret_cast<uint4*>(zop_base + (i >> 7) * W4G_Z_BYTES + (i & 127) * 16) = make_uint4(w.x, w.y, 0u, 0u);
+  }
+  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   if constexpr (SMALL) cluster_sync_all();  // the first CTA's barrier exists before any other CTA of the cluster signals it
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_w = tmem_base + NSLOT * 2 * MT;  // converted weights behind the accumulator ring
+  const uint32_t tmem_w = tmem_base + NS * 2 * MT;  // converted weights behind the accumulator ring
   const uint32_t bar0 = smem_u32(bar_block);
   const uint32_t ctl = bar0 + W4G_CTL;
 
@@ -327,58 +468,93 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const int n_sk = (int)(item1 - item0);
   const int n_slabs = SMALL ? n_sk : n_sk + p.dp_rounds * p.KS;  // this CTA's slabs, numbered 0.. in processing order
 
-  if (warp <= 2) {
-    // ------------------------------------------------------------------ TMA producers
-    // warp 0: packed weights, warp 1: activations, warp 2: scales
-    if (lane == 0 && (warp != 2 || p.has_scales) && !(SMALL && warp == 1)) {
-      if (warp == 1) pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
-      uint64_t* full = warp == 0 ? raw_full : (warp == 1 ? a_full : sc_full);
-      const uint32_t empty0 = bar0 + (warp == 0 ? W4G_RAW_EMPTY : (warp == 1 ? W4G_A_EMPTY : W4G_SC_EMPTY));
-      const int depth = warp == 0 ? RS : (warp == 1 ? AS : SS);
-      const uint32_t sc_tx = (uint32_t)p.scale_rows * 256u;
+  // 64 tokens: a drain thread keeps 64 sums, more than the 80 registers the block is launched with; the warp groups that
+  // need few give theirs up (48 + 2 x 104 + 2 x 80 + 64 = 6 x 80).
+  if constexpr (MT == 64) {
+    if (warp < W4G_FIRST_EPI_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else if (warp >= W4G_FIN_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    else if (warp < W4G_FIRST_DQ_WARP) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+  }
+  if (warp < 2) {
+    // ------------------------------------------------------------------ producers
+    // One thread each.  A thread of this kernel gets to issue an instruction only every ten cycles or so, so what a
+    // producer does per slab is kept to a few dozen instructions (a slab's HBM time is 700 cycles).
+    if (lane == 0 && !(SMALL && warp == 1)) {
       int tile = n_sk > 0 ? (int)(item0 / p.KS) : p.sk_tiles + cta;
       int ks = n_sk > 0 ? (int)(item0 - (long long)tile * p.KS) : 0;
       int b, n0, m0;
       w4_tile_coords(p, tile, MT, b, n0, m0);
-      int st = 0;
-      uint32_t phase = 0, issued_mask = 0, parity_mask = 0, fail = 0;
-      for (int i = 0; i < n_slabs; ++i) {
-        w4g_wait<0, ST_TIMEOUT_PRODUCER>(empty0 + 8 * st, phase ^ 1u, ctl, fail);
-        if (fail) break;
-        if (warp == 0) {
-          mbar_arrive_expect_tx(&full[st], ZT ? W4_RAW_PACKED + sc_tx : (uint32_t)W4_RAW_PACKED);
-          tma_load_3d(raw_base + st * W4_RAW_PACKED, &tmW, &full[st], ks * (W4_SLAB_K / 2), n0, b);
-          if (ZT) {  // the zero rows of the slab's two halves, addressed like its scale rows
-            const int zrow = (p.scale_rows == 2) ? 2 * ks : (ks * W4_SLAB_K) / p.group;
-            tma_load_3d(z_base + st * W4G_SC_BYTES, &tmZ, &full[st], n0, zrow, b);
-          }
-        } else if (warp == 1) {
-          uint8_t* dstA = a_base + st * Cfg::A_BYTES;
-          mbar_arrive_expect_tx(&full[st], Cfg::A_BYTES);
-#pragma unroll
-          for (int kb = 0; kb < 4; ++kb)
-            tma_load_3d(dstA + kb * Cfg::A_KB_BYTES, &tmA, &full[st], ks * W4_SLAB_K + kb * 64, m0, b);
-        } else {
+      uint32_t fail = 0;
+      uint32_t issued_mask = 0, parity_mask = 0;
+      int left = n_sk > 0 ? min(n_sk, p.KS - ks) : p.KS;  // slabs up to the next change of tile
+      int i = 0;
+      if (warp == 0) {
+        // Packed weights, and with them - on the same barrier - the slab's scale rows, into a ring of their own that is SS
+        // slabs deep.  Loading slab L means that slab L - RS is in registers, so (its set having stored its previous slab,
+        // L - RS - 2) the MMAs up to slab L - RS - 2 - WS have completed, for which the drain warps have left the slot
+        // NS slabs further back: a scale slot is rewritten only after it has been read, without a barrier, as long as
+        // SS >= RS + WS + NS + 3.  A drain warp reads a scale only after the slab's MMAs, i.e. after this barrier.
+        static_assert(Cfg::SS >= RS + WS + NS + 3, "scale ring");
+        const uint32_t row_tx = (uint32_t)p.scale_rows * 256u;
+        const uint32_t tx = W4_RAW_PACKED + (p.has_scales ? row_tx : 0u) + (ZT ? row_tx : 0u);
+        const int spg = p.scale_rows == 2 ? 1 : (p.group + W4_SLAB_K - 1) / W4_SLAB_K;  // slabs per scale row (pair)
+        const int row_step = p.scale_rows == 2 ? 2 : 1;
+        int srow = (ks / spg) * row_step, in_group = ks % spg;
+        int st = 0;
+        uint32_t phase = 0;
+        while (i < n_slabs) {
+          w4g_wait<W4G_RAW_EMPTY, ST_TIMEOUT_PRODUCER>(bar0 + 8 * st, phase ^ 1u, ctl, fail);
+          if (fail) break;
+          mbar_arrive_expect_tx(&raw_full[st], tx);
+          tma_load_3d(raw_base + st * W4_RAW_PACKED, &tmW, &raw_full[st], ks * (W4_SLAB_K / 2), n0, b);
           // scale rows of the slab: two when the groups are 128 wide, else the one row of the slab's group
-          const int srow = (p.scale_rows == 2) ? 2 * ks : (ks * W4_SLAB_K) / p.group;
-          mbar_arrive_expect_tx(&full[st], sc_tx);
-          tma_load_3d(sc_base + st * W4G_SC_BYTES, &tmS, &full[st], n0, srow, b);
+          if (p.has_scales) tma_load_3d(sc_base + (i % Cfg::SS) * W4G_SC_BYTES, &tmS, &raw_full[st], n0, srow, b);
+          if (ZT) tma_load_3d(z_base + st * W4G_SC_BYTES, &tmZ, &raw_full[st], n0, srow, b);
+          issued_mask |= 1u << st;
+          parity_mask = (parity_mask & ~(1u << st)) | (phase << st);
+          if (++st == RS) { st = 0; phase ^= 1u; }
+          ++i;
+          ++ks;
+          if (++in_group == spg) { in_group = 0; srow += row_step; }
+          if (--left == 0) {  // the tile, or this CTA's share of it, is done
+            tile = i == n_sk ? p.sk_tiles + cta : tile + (i < n_sk ? 1 : G);
+            ks = srow = in_group = 0;
+            left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
+            w4_tile_coords(p, tile, MT, b, n0, m0);
+          }
         }
-        issued_mask |= 1u << st;
-        parity_mask = (parity_mask & ~(1u << st)) | (phase << st);
-        if (++st == depth) { st = 0; phase ^= 1u; }
-        if (i + 1 == n_sk) {  // the stream-K range is done: on to this CTA's first whole tile
-          ks = 0;
-          tile = p.sk_tiles + cta;
-          w4_tile_coords(p, tile, MT, b, n0, m0);
-        } else if (++ks == p.KS) {
-          ks = 0;
-          tile += (i + 1 < n_sk) ? 1 : G;
-          w4_tile_coords(p, tile, MT, b, n0, m0);
+      } else {
+        pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
+        const uint32_t a0 = smem_u32(a_base);
+        const uint8_t* base = reinterpret_cast<const uint8_t*>(p.A_raw);
+        auto tile_src = [&](int k) {
+          return base + (((size_t)b * p.m_tiles + (size_t)(m0 / MT)) * (size_t)p.KS + (size_t)k) * Cfg::A_BYTES;
+        };
+        const uint8_t* src = tile_src(ks);
+        int st = 0;
+        while (i < n_slabs) {
+          if (i >= AS)  // the slab that used this stage has been multiplied
+            w4g_wait<W4G_DONE, ST_TIMEOUT_PRODUCER>(bar0 + 8 * ((i - AS) % W4G_BARS), (uint32_t)((i - AS) / W4G_BARS) & 1u, ctl, fail);
+          if (fail) break;
+          uint64_t* bar = &a_full[i % W4G_BARS];
+          mbar_arrive_expect_tx(bar, Cfg::A_BYTES);
+          w4g_bulk_load(a0 + st * Cfg::A_BYTES, src, Cfg::A_BYTES, smem_u32(bar));
+          issued_mask |= 1u << (i % W4G_BARS);
+          parity_mask = (parity_mask & ~(1u << (i % W4G_BARS))) | (((uint32_t)(i / W4G_BARS) & 1u) << (i % W4G_BARS));
+          if (++st == AS) st = 0;
+          ++i;
+          src += Cfg::A_BYTES;
+          if (--left == 0) {
+            tile = i == n_sk ? p.sk_tiles + cta : tile + (i < n_sk ? 1 : G);
+            left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
+            w4_tile_coords(p, tile, MT, b, n0, m0);
+            src = tile_src(0);
+          }
         }
       }
       if (fail) {  // wait (bounded) for the copies still in flight before the CTA may exit
-        for (int s = 0; s < depth; ++s) {
+        uint64_t* full = warp == 0 ? raw_full : a_full;
+        for (int s = 0; s < 8; ++s) {
           if (!(issued_mask & (1u << s))) continue;
           const uint64_t t0 = global_timer_ns();
           while (!mbar_try_wait(&full[s], (parity_mask >> s) & 1u)) {
@@ -390,58 +566,73 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
       }
     }
-  } else if (warp >= W4G_FIRST_MMA_WARP && warp < W4G_FIRST_EPI2_WARP) {
+  } else if (warp < W4G_FIRST_EPI_WARP) {
     // ------------------------------------------------------------------ MMA issuers (warp-convergent)
-    // Iteration n = 4 * c + u of issuer w handles half h = w + 4 * n of slab (w / 2) + 2 n: weight stage w
-    // (parity n & 1 = u & 1), activation stage (w / 2) + 2 * (u % A_PER), slab slot (w / 2) + 2 * (u % S_PER),
-    // accumulator w & 1 of that slot.
+    // Issuer w takes the slabs i with i % 2 == w: weight stage i % WS, activation stage i % AS, accumulator slot i % NS.
     const int w = warp - W4G_FIRST_MMA_WARP;
     constexpr uint32_t idesc = make_idesc(ACC_F32, FMT_F16, FMT_F16, 0, 0, W4_BN, MT);
-    const int half = w & 1;
-    const int n_half = 2 * n_slabs;
-    const uint32_t tW = tmem_w + w * W4G_HALF_COLS;
     // K-major activation descriptor: the high word is constant, the low word holds the start address >> 4
-    const uint64_t desc0 = make_desc_kmajor(smem_u32(a_base) + (w >> 1) * Cfg::A_BYTES + half * 2 * Cfg::A_KB_BYTES);
+    const uint64_t desc0 = make_desc_kmajor(smem_u32(a_base));
     const uint32_t desc_hi = (uint32_t)(desc0 >> 32);
     const uint32_t desc_lo0 = (uint32_t)desc0;
-    const uint32_t d0 = tmem_base + (w >> 1) * 2 * MT + half * MT;
-    const uint32_t bw = bar0 + 8 * w;         // this issuer's weight stage
-    const uint32_t ba = bar0 + 8 * (w >> 1);  // this issuer's activation stages and slab slots
-    const int withhold_h = (dbg.withhold_last_commit && cta == G - 1) ? n_half - 1 : -1;
+    const uint64_t sdesc0 = w4g_desc_k16(smem_u32(a_base) + MT * 256, 128, 256);
+    const uint32_t zop0 = smem_u32(zop_base);
+    const int withhold_i = (dbg.withhold_last_commit == 1 && cta == G - 1) ? n_slabs - 1 : -1;
+    const bool has_zero = ZT || p.zero != 0;
     uint32_t fail = 0;
-    int h = w;
-    static_assert(Cfg::A_PER == Cfg::S_PER, "one unrolled step = one (activation stage, accumulator slot) pair");
-    for (uint32_t c = 0; h < n_half; ++c) {
-      // the four steps of an outer iteration, unrolled with compile-time stage indices
-      auto step = [&](auto u_) {
-        constexpr int u = decltype(u_)::value;
-        if (h >= n_half) return;
-        constexpr int ai = u % Cfg::A_PER;  // which of this issuer's activation stages
-        constexpr int si = u % Cfg::S_PER;  // which of this issuer's accumulator slots
-        w4g_wait<W4G_ACC_EMPTY + 16 * si, ST_TIMEOUT_MMA>(ba, w4g_visit_parity<Cfg::S_PER>(c, u) ^ 1u, ctl, fail);
-        w4g_wait<W4G_A_FULL + 16 * ai, ST_TIMEOUT_MMA>(ba, w4g_visit_parity<Cfg::A_PER>(c, u), ctl, fail);
-        w4g_wait<W4G_W_FULL, ST_TIMEOUT_MMA>(bw, (uint32_t)(u & 1), ctl, fail);
-        tc_fence_after_sync();
-        const uint32_t d = d0 + (2 * si) * 2 * MT;
-        const uint32_t lo = desc_lo0 + (uint32_t)((2 * ai * Cfg::A_BYTES) >> 4);
-        if (w4g_elect_one()) {
+    int as = w % AS, ws = w % WS;
+    for (int i = w; i < n_slabs; i += W4G_MMA_WARPS) {
+      const int slot = i % NS;
+      const uint32_t bi = bar0 + 8 * (i % W4G_BARS), par = (uint32_t)(i / W4G_BARS) & 1u;
+      w4g_wait<W4G_ACC_EMPTY, ST_TIMEOUT_MMA>(bar0 + 8 * slot, ((uint32_t)(i / NS) & 1u) ^ 1u, ctl, fail);
+      w4g_wait<W4G_A_FULL, ST_TIMEOUT_MMA>(bi, par, ctl, fail);
+      const uint32_t d = tmem_base + slot * (2 * MT);
+      const uint32_t tW = tmem_w + ws * W4G_SLAB_COLS;
+      const uint32_t a_off = (uint32_t)((as * Cfg::A_BYTES) >> 4);
+      auto issue_half = [&](auto half_) {
+        constexpr int half = decltype(half_)::value;
+        // chunk c of the half: tensor-memory columns 16 c .. 16 c + 7 low words, + 8 .. + 15 high words
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {  // 16 k per MMA: 8 columns of weights, 32 bytes of activations
-            const uint32_t off = (uint32_t)(((j >> 2) * Cfg::A_KB_BYTES + (j & 3) * 32) >> 4);
-            umma_f16_ts(d, tW + j * 8, ((uint64_t)desc_hi << 32) | (uint64_t)(lo + off), idesc, j != 0 ? 1u : 0u);
-          }
-          w4g_commit(bw + W4G_W_EMPTY);
-          w4g_commit(ba + W4G_A_EMPTY + 16 * ai);
-          if (h != withhold_h) w4g_commit(ba + W4G_ACC_FULL + 16 * si);
+        for (int j = 0; j < 8; ++j) {
+          const int k16 = j < 4 ? 2 * j + 1 : 2 * (j - 4);  // K steps 1 3 5 7 (high), then 0 2 4 6 (low)
+          const uint32_t off = (uint32_t)((half * Cfg::A_HALF + (k16 >> 2) * (MT * 128) + (k16 & 3) * 32) >> 4);
+          const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(desc_lo0 + a_off + off);
+          const uint32_t ta = tW + half * (W4G_SLAB_COLS / 2) + k16 * 8;
+          if (j == 4) w4g_mma_ts_shift4(d + half * MT, ta, bd, idesc);
+          else umma_f16_ts(d + half * MT, ta, bd, idesc, j != 0 ? 1u : 0u);
         }
-        h += W4G_MMA_WARPS;
+        if (has_zero) {
+          const int zs = ZT ? 2 * ws + half : 0;
+          umma_f16_ss(d + half * MT, w4g_desc_k16(zop0 + zs * W4G_Z_BYTES, (uint32_t)(Cfg::Z_STAGES - zs) * W4G_Z_BYTES, 128),
+                      sdesc0 + a_off + ((half * Cfg::A_HALF) >> 4), idesc, 1u);
+        }
       };
-      step(std::integral_constant<int, 0>{});
-      step(std::integral_constant<int, 1>{});
-      step(std::integral_constant<int, 2>{});
-      step(std::integral_constant<int, 3>{});
-      fail = __any_sync(0xffffffffu, fail != 0) ? 1u : 0u;
-      if (fail) break;
+      constexpr std::integral_constant<int, 0> H0{};
+      constexpr std::integral_constant<int, 1> H1{};
+      if constexpr (Cfg::HALVES) {
+        w4g_wait<W4G_W_FULL0, ST_TIMEOUT_MMA>(bi, par, ctl, fail);
+        tc_fence_after_sync();
+        if (w4g_elect_one()) {
+          issue_half(H0);
+          w4g_commit(bi + W4G_DONE0);
+        }
+      }
+      w4g_wait<W4G_W_FULL, ST_TIMEOUT_MMA>(bi, par, ctl, fail);
+      tc_fence_after_sync();
+      if (w4g_elect_one()) {
+        if constexpr (!Cfg::HALVES) issue_half(H0);
+        issue_half(H1);
+        if (i != withhold_i) w4g_commit(bi + W4G_DONE);
+      }
+      as += W4G_MMA_WARPS;
+      if (as >= AS) as -= AS;
+      ws += W4G_MMA_WARPS;
+      if (ws >= WS) ws -= WS;
+      // `fail` is looked at rarely: what is issued after a wait that gave up stays inside this CTA's memories
+      if ((i & 6) == 6) {
+        fail = __any_sync(0xffffffffu, fail != 0) ? 1u : 0u;
+        if (fail) break;
+      }
     }
     // everything this warp issued has completed before the CTA frees its tensor memory
     if (w4g_elect_one()) w4g_commit(bar0 + W4G_DRAIN);
@@ -451,12 +642,9 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         if (global_timer_ns() - t0 > p.wait_limit_ns) break;
       }
     }
-  } else if ((warp >= W4G_FIRST_EPI_WARP && warp < W4G_FIRST_DQ_WARP) || warp >= W4G_FIRST_EPI2_WARP) {
+  } else if (warp < W4G_FIRST_DQ_WARP) {
     // ------------------------------------------------------------------ drain / epilogue
-    // Set e (warps 4..7: 0, warps 28..31: 1) drains the CTA-local slabs i with i % 2 == e: slab slot i % NSLOT
-    // (parity (i / NSLOT) & 1), scale stage i % 16 (parity (i / 16) & 1).  Both sets walk the same segments and
-    // meet at every segment end, where set 1 hands its sums to set 0 through shared memory.
-    const int e = warp >= W4G_FIRST_EPI2_WARP ? 1 : 0;
+    const int e = (warp - W4G_FIRST_EPI_WARP) >> 2;  // drain set
     const int q = warp & 3;
     const int nl = q * 32 + lane;  // weight row inside the tile == TMEM lane
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
@@ -464,6 +652,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t sc_row1 = p.scale_rows == 2 ? 256u : 0u;  // the second half's scale row inside a stage
     const bool scaled = p.has_scales != 0;
     const bool lead = lane == 0;
+    constexpr int DT = MT;  // tokens a drain thread accumulates
     if constexpr (!SMALL) pdl_wait();  // the arrival counters are zeroed by the pre-pass kernel in front of this one
     if constexpr (SMALL) {
       // this CTA's piece of the activations: rows m0 .. m0 + 15 (zero beyond M), k [256 * ks_first, 256 * (ks_first + per))
@@ -472,52 +661,44 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       int bb, nn0, mm0;
       w4_tile_coords(p, tile_s, MT, bb, nn0, mm0);
       const int tid = (e * 4 + q) * 32 + lane;  // 0 .. 255
-      const int chunks_per_row = per * 32;       // 16-byte chunks (eight k) per row in this CTA's K range
+      const int units = MT * per * 8;           // 32-k chunks of this CTA: (half, row, chunk), a multiple of 128
       const uint4* src = reinterpret_cast<const uint4*>(p.A_raw) + ((size_t)bb * p.M) * (size_t)(p.K / 8);
-      const int row_chunks = p.K / 8;  // chunks in a whole row of A: the last slab of a short K is partly outside
-      constexpr int PER_THREAD = MT * W4G_SMALL_MAX_SLABS * 32 / 256;  // at most eight chunks per thread
+      constexpr int PER_THREAD = MT * W4G_SMALL_MAX_SLABS * 8 / 256;  // at most two chunks per thread
       const uint4* ptr[PER_THREAD];
-      uint32_t dst_off[PER_THREAD];  // byte offset in the activation stages, or ~0 for a chunk this thread does not have
 #pragma unroll
       for (int u = 0; u < PER_THREAD; ++u) {
-        const int c = tid + 256 * u;
-        const int r = c / chunks_per_row, kc = c - r * chunks_per_row;
-        const int slab = kc >> 5, j = kc & 31;  // chunk j of the slab: 64-k block j / 8, chunk j % 8 of the row there
-        dst_off[u] = c < MT * chunks_per_row
-                         ? (uint32_t)(slab * Cfg::A_BYTES + (j >> 3) * Cfg::A_KB_BYTES + r * 128 + (((j & 7) ^ (r & 7)) << 4))
-                         : 0xffffffffu;
-        const bool inside = c < MT * chunks_per_row && mm0 + r < p.M && ks_first * 32 + kc < row_chunks;
-        ptr[u] = inside ? src + (size_t)(mm0 + r) * (size_t)row_chunks + (size_t)ks_first * 32 + kc : nullptr;
+        const int i = tid + 256 * u;
+        const int c = i & 3, r = (i >> 2) % MT, hl = (i >> 2) / MT;
+        const int k0 = ks_first * W4_SLAB_K + hl * 128 + c * 32;
+        ptr[u] = (i < units && mm0 + r < p.M && k0 < p.K) ? src + (size_t)(mm0 + r) * (size_t)(p.K / 8) + k0 / 8 : nullptr;
       }
       pdl_wait();  // whatever is in front of this launch has finished: the activations may be read, the output written
-      uint4 v[PER_THREAD];
+      uint4 v[PER_THREAD][4];
 #pragma unroll
       for (int u = 0; u < PER_THREAD; ++u)  // all loads first, so that their latencies overlap
-        v[u] = ptr[u] != nullptr ? __ldcg(ptr[u]) : make_uint4(0u, 0u, 0u, 0u);  // L2 is the point of coherence
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          v[u][k] = ptr[u] != nullptr ? __ldcg(ptr[u] + k) : make_uint4(0u, 0u, 0u, 0u);  // L2 is the point of coherence
 #pragma unroll
       for (int u = 0; u < PER_THREAD; ++u) {
-        if (dst_off[u] != 0xffffffffu) {
-          uint4 w = v[u];
-          if (p.a_is_bf16) {
-            w.x = w4_bf16x2_to_f16x2(w.x);
-            w.y = w4_bf16x2_to_f16x2(w.y);
-            w.z = w4_bf16x2_to_f16x2(w.z);
-            w.w = w4_bf16x2_to_f16x2(w.w);
-          }
-          if (p.a_permute) w = w4_permute_act(w);
-          *reinterpret_cast<uint4*>(a_base + dst_off[u]) = w;
+        const int i = tid + 256 * u;
+        if (i < units) {  // warp-uniform: units is a multiple of 128
+          const int c = i & 3, r = (i >> 2) % MT, hl = (i >> 2) / MT;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[u][k] = w4g_to_f16(v[u][k], p.a_is_bf16 != 0);
+          w4g_emit_chunk<MT>(a_base + hl * Cfg::A_HALF, r, c, v[u]);
         }
       }
       fence_proxy_async_smem();  // the MMAs read these stages through the async proxy
       w4g_epi_bar();
       if (tid == 0)
-        for (int sidx = 0; sidx < per; ++sidx) mbar_arrive(&a_full[sidx]);
+        for (int sl = 0; sl < per; ++sl) mbar_arrive(&a_full[sl]);
     }
     W4HybridIter seg{W4SegIter{item0, item1, p.KS}, p.sk_tiles + cta, SMALL ? 0 : p.dp_rounds, G, p.KS};
     int tile, ks0, ks1;
     uint32_t i_seg0 = 0;  // CTA-local index of the segment's first slab
     uint32_t fail = 0;
-    int seg_idx = 0;
+    int n_partial = 0;
     while (seg.next(tile, ks0, ks1)) {
       int b, n0, m0;
       w4_tile_coords(p, tile, MT, b, n0, m0);
@@ -526,33 +707,29 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       const bool full_tile = (ks0 == 0 && ks1 == p.KS);
       const int my_slot = (ks1 < p.KS) ? 2 * cta + 1 : 2 * cta;
       const uint32_t i_end = i_seg0 + (uint32_t)(ks1 - ks0);
-      constexpr int DT = Cfg::DT;
-      constexpr bool SPLIT_TOKENS = Cfg::SPLIT_TOKENS;
-      const int tok0 = SPLIT_TOKENS ? 32 * e : 0;  // first token (inside the tile) of this thread's sums
       float psum[DT];
 #pragma unroll
       for (int m = 0; m < DT; ++m) psum[m] = 0.f;
-      for (uint32_t i = SPLIT_TOKENS ? i_seg0 : i_seg0 + ((i_seg0 ^ (uint32_t)e) & 1u); i < i_end; i += SPLIT_TOKENS ? 1 : 2) {
-        float s0 = 1.0f, s1 = 1.0f;
-        if (scaled) {
-          const uint32_t ss = i % SS;
-          w4g_wait<W4G_SC_FULL, ST_TIMEOUT_EPILOGUE>(bar0 + 8 * ss, (i / SS) & 1u, ctl, fail);
-          uint16_t h0, h1;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sc_addr0 + ss * W4G_SC_BYTES));
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sc_addr0 + ss * W4G_SC_BYTES + sc_row1));
-          s0 = __half2float(__ushort_as_half(h0));
-          s1 = __half2float(__ushort_as_half(h1));
-          __syncwarp();
-          if (lead) w4g_arrive<W4G_SC_EMPTY>(bar0 + 8 * ss);
-        }
-        const uint32_t slot = i % NSLOT;
+      for (uint32_t i = i_seg0 + ((i_seg0 ^ (uint32_t)e) & 1u); i < i_end; i += 2) {
+        const uint32_t slot = i % NS;
         const uint32_t bs = bar0 + 8 * slot;
-        w4g_wait<W4G_ACC_FULL, ST_TIMEOUT_EPILOGUE>(bs, (i / NSLOT) & 1u, ctl, fail);
+        w4g_wait<W4G_DONE, ST_TIMEOUT_EPILOGUE>(bar0 + 8 * (i % W4G_BARS), (i / W4G_BARS) & 1u, ctl, fail);
         tc_fence_after_sync();
-        const uint32_t ta = tmem_base + lane_addr + slot * (2 * MT) + tok0;
+        const uint32_t ta = tmem_base + lane_addr + slot * (2 * MT);
+        uint32_t r[32];  // two pieces of 16 columns (16 tokens: the two halves)
         if constexpr (MT == 16) {
-          uint32_t r[32];  // columns 0..15: first half's accumulator, 16..31: second half's
           tmem_ld_32x32b_x32(ta, r);
+        }
+        float s0 = 16777216.0f, s1 = 16777216.0f;  // 2^24: the converted weights are in units of 2^-24
+        if (scaled) {
+          uint16_t h0, h1;
+          const uint32_t sa = sc_addr0 + (i % Cfg::SS) * W4G_SC_BYTES;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sa));
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sa + sc_row1));
+          s0 *= __half2float(__ushort_as_half(h0));
+          s1 *= __half2float(__ushort_as_half(h1));
+        }
+        if constexpr (MT == 16) {
           tmem_ld_wait();
           tc_fence_before_sync();
           __syncwarp();
@@ -564,35 +741,28 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           }
         } else {
 #pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {  // 16 columns at a time: half c4 / 2, this thread's tokens 16 * (c4 % 2) ..
-            uint32_t r[16];
-            tmem_ld_32x32b_x16(ta + (c4 >> 1) * MT + 16 * (c4 & 1), r);
+          for (int c = 0; c < 2 * MT / 16; ++c) {  // 16 columns at a time: the first half's tokens, then the second's
+            uint32_t q16[16];
+            tmem_ld_32x32b_x16(ta + 16 * c, q16);
             tmem_ld_wait();
-            if (c4 == 3) {
+            if (c == 2 * MT / 16 - 1) {
               tc_fence_before_sync();
               __syncwarp();
               if (lead) w4g_arrive<W4G_ACC_EMPTY>(bs);
             }
-            const float s = (c4 >> 1) ? s1 : s0;
+            const int t0 = 16 * (c % (MT / 16));
+            const float sc = c < MT / 16 ? s0 : s1;
 #pragma unroll
-            if constexpr (MT == 64) {  // the paired form costs this tile registers it does not have (spills)
-              for (int m = 0; m < 16; ++m) psum[16 * (c4 & 1) + m] = fmaf(__uint_as_float(r[m]), s, psum[16 * (c4 & 1) + m]);
-            } else {
-              for (int m = 0; m < 16; m += 2)
-                w4g_fma2(psum[16 * (c4 & 1) + m], psum[16 * (c4 & 1) + m + 1], r[m], r[m + 1], s);
-            }
+            for (int m = 0; m < 16; m += 2) w4g_fma2(psum[t0 + m], psum[t0 + m + 1], q16[m], q16[m + 1], sc);
           }
         }
       }
       i_seg0 = i_end;
-      fail = __any_sync(0xffffffffu, fail != 0) ? 1u : 0u;
-      // Segment end.  With slab-alternating sets, set 1 hands over its sums (set 0 has read them before it reaches
-      // the second barrier below, which set 1 passes before its next hand-over) and set 0 adds them and writes the
-      // tile or its split-K partial; with token-split sets each set writes its own tokens.
-      const int par = seg_idx & 1;
-      ++seg_idx;
+      // Segment end.  Set 1 hands over its sums through shared memory; set 0 adds them and writes the tile, or its partial
+      // sums to the scratch buffer, where the split-K warp takes over.  (A wait that gave up does not change the course of
+      // events here: all waits of the CTA then give up quickly, and the status word says that C is unspecified.)
       float* xb = xbuf + nl;
-      if (!SPLIT_TOKENS && e == 1) {
+      if (e == 1) {
 #pragma unroll
         for (int j = 0; j < DT; ++j) xb[j * W4_BN] = psum[j];
       }
@@ -607,7 +777,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
         float* landing = reinterpret_cast<float*>(raw_base + W4G_SMALL_MAX_SLABS * W4_RAW_PACKED);  // [rank - 1][token][row]
         if (crank != 0) {
-          if (e == 0 && !fail) {
+          if (e == 0 && __all_sync(0xffffffffu, fail == 0)) {
             const uint32_t dst = mapa_u32(smem_u32(landing + (size_t)(crank - 1) * (MT * W4_BN) + nl), 0);
 #pragma unroll
             for (int j = 0; j < DT; ++j)
@@ -650,176 +820,181 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
         break;
       }
-      const long long first_item = (long long)tile * p.KS;
-      int b_first = 0, b_last = 0;
-      if (!full_tile) {
-        b_first = w4_owner(T, G, first_item);
-        b_last = w4_owner(T, G, first_item + p.KS - 1);
-      }
-      if ((SPLIT_TOKENS || e == 0) && !fail) {
-        if (!SPLIT_TOKENS) {
+      if (e == 0) {
 #pragma unroll
-          for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
-        }
+        for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
         if (full_tile) {
           if (n < p.N) {
 #pragma unroll
             for (int j = 0; j < DT; ++j) {
-              const int m = m0 + tok0 + j;
+              const int m = m0 + j;
               if (m < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m, n, psum[j]);
             }
           }
         } else {
-          float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + (size_t)tok0 * W4_BN + nl;
+          float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + nl;
 #pragma unroll
           for (int j = 0; j < DT; ++j) dst[j * W4_BN] = psum[j];
+          __syncwarp();
+          if (lead) w4g_arrive<W4G_PART_READY>(bar0 + 8 * n_partial);
+          ++n_partial;
+        }
+      }
+      w4g_epi_bar();  // set 0 has read the exchange buffer
+    }
+  } else if (warp >= W4G_FIN_WARP) {
+    // ------------------------------------------------------------------ split-K hand-over
+    // A tile that several CTAs share: each one's partial sums go to the scratch buffer and a counter tells the last
+    // contributor (never by waiting), which adds them in a fixed order and writes the tile.  This chain of global-memory
+    // round trips (fence, atomic, loads: 7 000 cycles when the drain warps ran it, with the pipeline standing still behind
+    // them) is these four warps' alone; each of them adds a quarter of the tokens.
+    const int fw = warp - W4G_FIN_WARP;
+    volatile uint32_t* fin_word = reinterpret_cast<uint32_t*>(bar_block + W4G_FIN_WORD);
+    if constexpr (!SMALL) {
+      pdl_wait();  // the arrival counters are zeroed by the pre-pass kernel in front of this one
+      W4SegIter seg{item0, item1, p.KS};
+      int tile, ks0, ks1;
+      int n_partial = 0;
+      uint32_t fail = 0;
+      while (seg.next(tile, ks0, ks1)) {
+        if (ks0 == 0 && ks1 == p.KS) continue;
+        w4g_wait<W4G_PART_READY, ST_TIMEOUT_EPILOGUE>(bar0 + 8 * n_partial, 0u, ctl, fail);
+        const long long first_item = (long long)tile * p.KS;
+        const int b_first = w4_owner(T, G, first_item), b_last = w4_owner(T, G, first_item + p.KS - 1);
+        if (fw == 0 && lane == 0) {
           __threadfence();
+          fin_word[n_partial] = atomicAdd(p.ws_counters + b_first, 1u);
         }
-      }
-      // The eight drain warps decide together whether to go on: one thread reads the abort word once and
-      // publishes it (with the split-K outcome) in a control word that alternates between two slots, so a fast
-      // warp's next write cannot overtake a slow warp's read.
-      w4g_epi_bar();
-      if (warp == W4G_FIRST_EPI_WARP && lane == 0) {
-        uint32_t ctrl = (ctl_words[0] || fail) ? 1u : 0u;
-        if (!ctrl && !full_tile) {
-          // split tile: count arrivals; the last contributor adds all partials in a fixed order
-          const uint32_t old = atomicAdd(p.ws_counters + b_first, 1u);
-          if (old == (uint32_t)(b_last - b_first)) ctrl |= 2u;
-        }
-        epi_ctrl[par] = ctrl;
-      }
-      w4g_epi_bar();
-      const uint32_t ctrl = epi_ctrl[par];
-      if (ctrl & 1u) break;
-      const bool is_last = (ctrl & 2u) != 0;
-      if (is_last && (Cfg::SPLIT_TOKENS || e == 0)) {
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        const bool last = fin_word[n_partial] == (uint32_t)(b_last - b_first);
+        ++n_partial;
+        if (!last) continue;
         __threadfence();
-        if (n < p.N) {
-          const int rows = min(Cfg::SPLIT_TOKENS ? 32 * e + 32 : MT, p.M - m0);
+        int b, n0, m0;
+        w4_tile_coords(p, tile, MT, b, n0, m0);
+        uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
+        const int n = n0 + 4 * lane;  // four rows of the tile per lane
+        const int rows = min(MT / 4 * (fw + 1), p.M - m0);
+        constexpr int RU = 4;
 #pragma unroll 1
-          for (int mb = Cfg::SPLIT_TOKENS ? 32 * e : 0; mb < rows; mb += 16) {
-            float sum[16];
+        for (int mb = MT / 4 * fw; mb < rows; mb += RU) {
+          float4 sum[RU];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) sum[u] = 0.0f;
+          for (int u = 0; u < RU; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-            for (int c = b_first; c <= b_last; ++c) {  // fixed order: results do not depend on arrival order
-              const long long c_end = w4_range_begin(T, G, c + 1);
-              const int pslot = (c_end >= first_item + p.KS) ? 2 * c : 2 * c + 1;
-              const float* src = p.ws_partials + (size_t)pslot * (MT * W4_BN) + (size_t)mb * W4_BN + nl;
-              float v[16];
+          for (int c = b_first; c <= b_last; ++c) {  // fixed order: results do not depend on arrival order
+            const long long c_end = w4_range_begin(T, G, c + 1);
+            const int pslot = (c_end >= first_item + p.KS) ? 2 * c : 2 * c + 1;
+            const float4* src = reinterpret_cast<const float4*>(p.ws_partials + (size_t)pslot * (MT * W4_BN) + (size_t)mb * W4_BN) + lane;
+            float4 v[RU];
 #pragma unroll
-              for (int u = 0; u < 16; ++u) v[u] = (mb + u < rows) ? __ldcg(src + u * W4_BN) : 0.0f;
+            for (int u = 0; u < RU; ++u) v[u] = __ldcg(src + u * (W4_BN / 4));
 #pragma unroll
-              for (int u = 0; u < 16; ++u) sum[u] += v[u];
+            for (int u = 0; u < RU; ++u) {
+              sum[u].x += v[u].x;
+              sum[u].y += v[u].y;
+              sum[u].z += v[u].z;
+              sum[u].w += v[u].w;
             }
+          }
+          if (n < p.N) {  // N is a multiple of 8
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-              if (mb + u < rows)
-                w4_store_out<OUT_BF16, GATHER>(p, Cout, m0 + mb + u, n, sum[u]);
-            }
+            for (int u = 0; u < RU; ++u)
+              if (mb + u < rows) w4_store_out4<OUT_BF16, GATHER>(p, Cout, m0 + mb + u, n, sum[u]);
           }
         }
       }
     }
-  } else if (warp >= W4G_FIRST_DQ_WARP && warp < W4G_FIRST_MMA_WARP) {
+  } else {
     // ------------------------------------------------------------------ dequant
-    // Two sets of eight warps take alternate slabs: set g = wd / 8 converts slabs g, g + 2, ...  Inside a set,
-    // warp (q, hf) owns TMEM lanes 32 q .. 32 q + 31 (the quadrant it may touch) and the 128-k half hf of the
-    // slab = the packed 16-byte chunks 4 hf .. 4 hf + 3 of a row = the 64 columns of weight stage 2 g + hf.
-    // Iteration n = 4 * c + u of a set handles slab 2 n + g: raw stage 2 u + g (its c-th fill, parity c & 1),
-    // weight stage 2 g + hf (its n-th use, parity n & 1 = u & 1).
-    const int wd = warp - W4G_FIRST_DQ_WARP;
-    const int g = wd >> 3;
+    // Set s (four warps, one per 32 rows = tensor-memory lanes 32 q .. 32 q + 31, the quadrant a warp may touch) converts
+    // the slabs i with i % 2 == s into weight stage i % WS, which is free once the MMAs of slab i - WS have completed.
+    // Whole slabs, because a hand-over costs a warp as much time as converting a quarter of one.
+    const int sset = (warp - W4G_FIRST_DQ_WARP) >> 2;
     const int q = warp & 3;
-    const int hf = (wd >> 2) & 1;
     const int row = q * 32 + lane;
-    const int sw = row & 7;
-    const uint32_t rawr = smem_u32(raw_base) + g * W4_RAW_PACKED + row * 128;  // this thread's row in raw stage g
-    // quarter-warps read 8 rows x 8 distinct chunks (128-byte swizzle)
-    const uint32_t ch0 = rawr + (((4 * hf + 0) ^ sw) << 4), ch1 = rawr + (((4 * hf + 1) ^ sw) << 4);
-    const uint32_t ch2 = rawr + (((4 * hf + 2) ^ sw) << 4), ch3 = rawr + (((4 * hf + 3) ^ sw) << 4);
-    const uint32_t zero = (uint32_t)p.zero;
-    const uint32_t sub_lo_c = (0x6400u + zero) * 0x00010001u;                     // (1024 + zero) x2
-    const uint32_t sub_hi_c = ((0x5400u + (zero << 4)) | 0x8000u) * 0x00010001u;  // -(64 + zero) x2
-    // this row's zero point of the half: stage g of the zero ring, second row for the second half of 128-wide groups
-    const uint32_t z_addr = smem_u32(z_base) + g * W4G_SC_BYTES + 2 * row + ((p.scale_rows == 2 && hf) ? 256u : 0u);
-    const uint32_t st_addr = tmem_w + ((uint32_t)(q * 32) << 16) + (2 * g + hf) * W4G_HALF_COLS;
-    const uint32_t bg = bar0 + 8 * g;             // raw stages g, g + 2, g + 4, g + 6
-    const uint32_t bws = bar0 + 8 * (2 * g + hf);  // weight stage 2 g + hf
+    const uint32_t rawr = smem_u32(raw_base) + row * 128;
+    const uint32_t sw = (uint32_t)(row & 7) << 4;  // 128-byte swizzle: quarter-warps read 8 rows x 8 distinct chunks
+    const uint32_t st_addr = tmem_w + ((uint32_t)(q * 32) << 16);
+    // ZT: this row's zero points of the slab's halves (128-wide groups: two rows), and where their operands go
+    const uint32_t z_addr = smem_u32(z_base) + 2 * row;
+    const uint32_t z_row1 = p.scale_rows == 2 ? 256u : 0u;
+    uint8_t* zop = zop_base + row * 16;
     const bool lead = lane == 0;
-    const int n_mine = (n_slabs - g + 1) >> 1;  // slabs g, g + 2, ... below n_slabs
+    // one loop per weight layout: a branch around the conversion inside it costs a register move per converted word
+    auto convert_slabs = [&](auto il_) {
     uint32_t fail = 0;
-    for (int nb = 0; nb < n_mine; nb += 4) {
-      const uint32_t rphase = (uint32_t)(nb >> 2) & 1u;
-      auto step = [&](auto u_) {
-        constexpr int u = decltype(u_)::value;
-        if (nb + u >= n_mine) return;
-        w4g_wait<W4G_RAW_FULL + 16 * u, ST_TIMEOUT_DEQUANT>(bg, rphase, ctl, fail);
-        uint32_t sub_lo = sub_lo_c, sub_hi = sub_hi_c;
+    int ws = sset % WS;
+#pragma unroll 1
+    for (int i = sset; i < n_slabs; i += W4G_DQ_SETS) {
+      const int rs = i % RS;
+      const uint32_t rb = rawr + (uint32_t)rs * W4_RAW_PACKED;
+      w4g_wait<W4G_RAW_FULL, ST_TIMEOUT_DEQUANT>(bar0 + 8 * rs, (uint32_t)(i / RS) & 1u, ctl, fail);
+      uint4 v[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = w4g_lds128<0>(rb + ((uint32_t)(c << 4) ^ sw));
+      uint2 zw[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+      if constexpr (ZT) {
+        uint16_t z0, z1;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(z0) : "r"(z_addr + rs * W4G_SC_BYTES));
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(z1) : "r"(z_addr + rs * W4G_SC_BYTES + z_row1));
+        zw[0] = w4g_zero_weights(__half2float(__ushort_as_half(z0)));
+        zw[1] = w4g_zero_weights(__half2float(__ushort_as_half(z1)));
+      }
+      const uint32_t bp = bar0 + 8 * ((i - WS) % W4G_BARS), ppar = (uint32_t)((i - WS) / W4G_BARS) & 1u;
+      if (i >= WS) {
+        if constexpr (Cfg::HALVES) w4g_wait<W4G_DONE0, ST_TIMEOUT_DEQUANT>(bp, ppar, ctl, fail);
+        else w4g_wait<W4G_DONE, ST_TIMEOUT_DEQUANT>(bp, ppar, ctl, fail);
+      }
+      tc_fence_after_sync();
+      const uint32_t ta = st_addr + ws * W4G_SLAB_COLS;
+      auto store_zero = [&](int half) {
         if constexpr (ZT) {
-          // integer zero z as f16: 1024 + z and 64 + z are exact f16 sums
-          uint16_t zh;
-          asm volatile("ld.shared.u16 %0, [%1+%2];" : "=h"(zh) : "r"(z_addr), "n"(2 * u * W4G_SC_BYTES));
-          uint32_t z2;
-          asm("mov.b32 %0, {%1, %1};" : "=r"(z2) : "h"(zh));
-          asm("add.rn.f16x2 %0, %1, %2;" : "=r"(sub_lo) : "r"(0x64006400u), "r"(z2));
-          asm("add.rn.f16x2 %0, %1, %2;" : "=r"(sub_hi) : "r"(0x54005400u), "r"(z2));
-          sub_hi ^= 0x80008000u;
+          *reinterpret_cast<uint2*>(zop + (2 * ws + half) * W4G_Z_BYTES) = zw[half];
+          fence_proxy_async_smem();
         }
-        const uint4 v0 = w4g_lds128<2 * u * W4_RAW_PACKED>(ch0);
-        const uint4 v1 = w4g_lds128<2 * u * W4_RAW_PACKED>(ch1);
-        const uint4 v2 = w4g_lds128<2 * u * W4_RAW_PACKED>(ch2);
-        const uint4 v3 = w4g_lds128<2 * u * W4_RAW_PACKED>(ch3);
-        // four batches of 32 weights (16 columns) each, so that few registers are live at a time
-        uint32_t o[16];
-        w4_dequant8(v0.x, sub_lo, sub_hi, 0u, false, o + 0);
-        w4_dequant8(v0.y, sub_lo, sub_hi, 0u, false, o + 4);
-        w4_dequant8(v0.z, sub_lo, sub_hi, 0u, false, o + 8);
-        w4_dequant8(v0.w, sub_lo, sub_hi, 0u, false, o + 12);
-        w4g_wait<W4G_W_EMPTY, ST_TIMEOUT_DEQUANT>(bws, (uint32_t)((u & 1) ^ 1), ctl, fail);
-        tc_fence_after_sync();
-        tmem_st_32x32b_x16(st_addr, o);
-        uint32_t o1[16];
-        w4_dequant8(v1.x, sub_lo, sub_hi, 0u, false, o1 + 0);
-        w4_dequant8(v1.y, sub_lo, sub_hi, 0u, false, o1 + 4);
-        w4_dequant8(v1.z, sub_lo, sub_hi, 0u, false, o1 + 8);
-        w4_dequant8(v1.w, sub_lo, sub_hi, 0u, false, o1 + 12);
-        tmem_st_32x32b_x16(st_addr + 16, o1);
-        uint32_t o2[16];
-        w4_dequant8(v2.x, sub_lo, sub_hi, 0u, false, o2 + 0);
-        w4_dequant8(v2.y, sub_lo, sub_hi, 0u, false, o2 + 4);
-        w4_dequant8(v2.z, sub_lo, sub_hi, 0u, false, o2 + 8);
-        w4_dequant8(v2.w, sub_lo, sub_hi, 0u, false, o2 + 12);
-        tmem_st_32x32b_x16(st_addr + 32, o2);
-        uint32_t o3[16];
-        w4_dequant8(v3.x, sub_lo, sub_hi, 0u, false, o3 + 0);
-        // the last of the four loads has delivered: the packed bytes are in registers, hand the raw stage back
-        __syncwarp();
-        if (lead) w4g_arrive<W4G_RAW_EMPTY + 16 * u>(bg);
-        w4_dequant8(v3.y, sub_lo, sub_hi, 0u, false, o3 + 4);
-        w4_dequant8(v3.z, sub_lo, sub_hi, 0u, false, o3 + 8);
-        w4_dequant8(v3.w, sub_lo, sub_hi, 0u, false, o3 + 12);
-        tmem_st_32x32b_x16(st_addr + 48, o3);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lead) w4g_arrive<W4G_W_FULL>(bws);
       };
-      step(std::integral_constant<int, 0>{});
-      step(std::integral_constant<int, 1>{});
-      step(std::integral_constant<int, 2>{});
-      step(std::integral_constant<int, 3>{});
-      fail = __any_sync(0xffffffffu, fail != 0) ? 1u : 0u;
-      if (fail) break;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if (Cfg::HALVES && c == 4) {
+          store_zero(0);
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lead) w4g_arrive<W4G_W_FULL0>(bar0 + 8 * (i % W4G_BARS));
+          if (i >= WS) w4g_wait<W4G_DONE, ST_TIMEOUT_DEQUANT>(bp, ppar, ctl, fail);
+          tc_fence_after_sync();
+        }
+        uint32_t o[16];
+        w4g_convert<decltype(il_)::value>(v[c], o);
+        tmem_st_32x32b_x16(ta + 16 * c, o);
+      }
+      // the loads have delivered: hand the raw stage back
+      __syncwarp();
+      if (lead) w4g_arrive<W4G_RAW_EMPTY>(bar0 + 8 * rs);
+      if (!Cfg::HALVES) store_zero(0);
+      store_zero(1);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lead) w4g_arrive<W4G_W_FULL>(bar0 + 8 * (i % W4G_BARS));
+      ws += W4G_DQ_SETS;
+      if (ws >= WS) ws -= WS;
+      if ((i & 6) == 6) {
+        fail = __any_sync(0xffffffffu, fail != 0) ? 1u : 0u;
+        if (fail) break;
+      }
     }
+    };
+    if (p.w_interleaved == 0) convert_slabs(std::integral_constant<bool, false>{});
+    else convert_slabs(std::integral_constant<bool, true>{});
   }
 
   // ------------------------------------------------------------------ teardown
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (SMALL) cluster_sync_all();  // no CTA of the cluster leaves while another may still reach into it
-  if (warp == 2) {
+  if (warp == W4G_FIRST_MMA_WARP + 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
     if (lane == 0 && ctl_words[0] != 0 && p.status != nullptr) atomicMax(p.status, ctl_words[0]);
