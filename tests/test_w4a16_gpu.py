@@ -491,3 +491,39 @@ def test_single_launch_form_gives_up_cleanly_when_a_cluster_signal_is_missing():
     C = q.w4a16_gemm(Ad, Pd, Sd, 8, 128, status=status)
     _close(C, ref)
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("M,K,N,zeros", [
+    (3, 1024, 256, None),       # one launch, K over a cluster
+    (16, 8192, 264, None),      # tiles shared by several CTAs
+    (1, 512, 128 * 160, None),  # whole tiles
+    (33, 1024, 128 * 150, None), (64, 4096, 144, "tensor"), (20, 2048, 272, "tensor"),
+])
+@pytest.mark.parametrize("fmt", ["sequential", "interleaved"])
+def test_non_finite_activations(M, K, N, zeros, fmt):
+    """An infinite activation gives +inf, -inf or (where q == zero) NaN per output feature, and leaves the other rows alone."""
+    q = _q()
+    A, packed, scales = oc.make_w4a16_inputs(M, K, N, "bfloat16", 128, seed=M + N)
+    clean = A.clone()
+    A[0, K // 2 + 5] = float("inf")
+    A[0, 7] = 1.0e38  # beyond f16: the operator's 16-bit activations make it an infinity
+    if M > 2:
+        A[M - 1, K - 1] = float("-inf")
+        A[M // 2, 3] = float("nan")
+    kw = {}
+    if zeros == "tensor":
+        kw["zeros_mode"] = "quantized"
+        z = torch.randint(0, 16, scales.shape, generator=torch.Generator().manual_seed(1)).to(torch.float16)
+    else:
+        z = 8
+    W = (oc.dequant_weight_zeros_ref(packed, scales, z, 128, "quantized") if zeros == "tensor"
+         else oc.dequant_weight_ref(packed, scales, 8, 128)).double()
+    B = oc.interleave_int4_f16_ref(packed) if fmt == "interleaved" else packed
+    if fmt == "interleaved":
+        kw["weight_layout"] = "interleaved"
+    call = lambda a: q.w4a16_gemm(a.cuda(), B.cuda(), scales.cuda(), z.cuda() if zeros else z, 128, out_dtype="float16", **kw).cpu()
+    C, C0 = call(A), call(clean)
+    rows = sorted({0} | ({M - 1, M // 2} if M > 2 else set()))
+    torch.testing.assert_close(C[rows].double(), A[rows].half().double() @ W.t(), equal_nan=True)  # +-inf and NaN only
+    other = [m for m in range(M) if m not in rows]
+    assert torch.equal(C[other], C0[other])

@@ -922,7 +922,11 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
   p.A_raw = nullptr;
-  p.a_is_bf16 = 0;
+  p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
+  p.A_src = A;
+  p.W_src = B_packed;
+  p.S_src = static_cast<const uint16_t*>(scales);
+  p.Z_src = static_cast<const uint16_t*>(zeros);
   p.w_interleaved = weight_format == QGEMM_W4_SEQUENTIAL ? 0 : 1;
   int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   if (p.total_items < grid) grid = p.total_items;
@@ -968,7 +972,6 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
       static const int small_waves = getenv("QGEMM_W4_SMALL_WAVES") ? atoi(getenv("QGEMM_W4_SMALL_WAVES")) : 1;
       if (cluster > 0 && num_tiles * cluster <= (int64_t)small_waves * sms) {
         p.A_raw = A;
-        p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
         return launch_w4g_small(bf, tmW, tmS, p, (int)(num_tiles * cluster), cluster, s);
       }
     }

@@ -358,6 +358,52 @@ __device__ __forceinline__ void w4g_convert(const uint4& v, uint32_t (&o)[16]) {
   }
 }
 
+// Output (b, m, n) once more, straight from its definition, when its sum came out NaN.  Subtracting zero * sum(A) turns an
+// infinite activation into inf - inf for every output feature, where (q - zero) * inf is +inf, -inf or, for q == zero,
+// NaN; an activation that is not finite makes the sum above NaN in every case, so NaN is what to look for.  One compare
+// per output on the ordinary path; the loop here is slow and runs for rows that hold an infinity or a NaN only.
+template <bool OUT_BF16, bool GATHER>
+__device__ __forceinline__ void w4g_redo_output(const W4A16Params& p, int b, int m, int n) {
+  const uint16_t* a = reinterpret_cast<const uint16_t*>(p.A_src) + ((size_t)b * p.M + m) * (size_t)p.K;
+  const uint8_t* w = p.W_src + ((size_t)b * p.N + n) * (size_t)(p.K / 2);
+  const int group = min(p.group, p.K), groups = p.K / group;
+  float sum = 0.f;
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    const size_t at = ((size_t)b * groups + g) * (size_t)p.N + n;
+    const float zero = p.Z_src != nullptr ? __half2float(__ushort_as_half(p.Z_src[at])) : (float)p.zero;
+    const float scale = p.has_scales ? __half2float(__ushort_as_half(p.S_src[at])) : 1.0f;
+    float part = 0.f;
+#pragma unroll 1
+    for (int k = g * group; k < (g + 1) * group; ++k) {
+      // interleaved layout: a word's nibbles are elements 0 2 4 6 1 3 5 7
+      const int e = k & 7, nib = p.w_interleaved ? (k - e) + (e >> 1) + 4 * (e & 1) : k;
+      const int q = (w[nib >> 1] >> (4 * (nib & 1))) & 15;
+      const uint32_t raw = a[k];
+      const uint32_t h = p.a_is_bf16 ? (w4_bf16x2_to_f16x2(raw) & 0xffffu) : raw;
+      part += __half2float(__ushort_as_half((uint16_t)h)) * ((float)q - zero);
+    }
+    sum += scale * part;
+    if (sum != sum) break;
+  }
+  w4_store_out<OUT_BF16, GATHER>(p, reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N, m, n, sum);
+}
+
+// The sums of tokens m0 .. m0 + MT - 1 (those below M) of output feature n.
+template <int MT, bool OUT_BF16, bool GATHER>
+__device__ __forceinline__ void w4g_store_checked(const W4A16Params& p, int b, int m0, int n, const float (&sum)[MT]) {
+  uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
+  uint64_t redo = 0;
+#pragma unroll
+  for (int j = 0; j < MT; ++j) {
+    const int m = m0 + j;
+    if (m < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m, n, sum[j]);
+    if (sum[j] != sum[j] && m < p.M) redo |= 1ull << j;
+  }
+#pragma unroll 1
+  for (; redo != 0; redo &= redo - 1) w4g_redo_output<OUT_BF16, GATHER>(p, b, m0 + __ffsll((long long)redo) - 1, n);
+}
+
 // GATHER = true is the gathered form (several destination buffers, see W4A16Params::c_dst); it is a separate
 // instantiation because the destination loop in the store path costs the plain kernel registers.
 // ZT = true: one integer zero point per (group, output feature) instead of the scalar one - the zeros tensor
@@ -375,7 +421,7 @@ __device__ __forceinline__ void w4g_convert(const uint4& v, uint32_t (&o)[16]) {
 template <int MT, bool OUT_BF16, bool GATHER = false, bool ZT = false, bool SMALL = false>
 __global__ void __launch_bounds__(W4G_THREADS, 1)
 w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
-                const __grid_constant__ CUtensorMap tmZ, const W4A16Params p, const W4GDebug dbg) {
+                const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ W4A16Params p, const W4GDebug dbg) {
   using Cfg = W4GCfg<MT, ZT>;
   constexpr int RS = Cfg::RS;
   constexpr int AS = Cfg::AS;
@@ -703,7 +749,6 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       int b, n0, m0;
       w4_tile_coords(p, tile, MT, b, n0, m0);
       const int n = n0 + nl;
-      uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
       const bool full_tile = (ks0 == 0 && ks1 == p.KS);
       const int my_slot = (ks1 < p.KS) ? 2 * cta + 1 : 2 * cta;
       const uint32_t i_end = i_seg0 + (uint32_t)(ks1 - ks0);
@@ -811,11 +856,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
               for (int j = 0; j < DT; ++j) psum[j] += src[j * W4_BN];
             }
-#pragma unroll
-            for (int j = 0; j < DT; ++j) {
-              const int m = m0 + j;
-              if (m < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m, n, psum[j]);
-            }
+            w4g_store_checked<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
           }
         }
         break;
@@ -824,13 +865,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
         if (full_tile) {
-          if (n < p.N) {
-#pragma unroll
-            for (int j = 0; j < DT; ++j) {
-              const int m = m0 + j;
-              if (m < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m, n, psum[j]);
-            }
-          }
+          if (n < p.N) w4g_store_checked<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
         } else {
           float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + nl;
 #pragma unroll
@@ -901,6 +936,19 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
             for (int u = 0; u < RU; ++u)
               if (mb + u < rows) w4_store_out4<OUT_BF16, GATHER>(p, Cout, m0 + mb + u, n, sum[u]);
+            uint32_t redo = 0;
+#pragma unroll
+            for (int u = 0; u < RU; ++u) {
+              const float one[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (one[i] != one[i] && mb + u < rows) redo |= 1u << (4 * u + i);
+            }
+#pragma unroll 1
+            for (; redo != 0; redo &= redo - 1) {
+              const int bit = __ffs(redo) - 1;
+              w4g_redo_output<OUT_BF16, GATHER>(p, b, m0 + mb + (bit >> 2), n + (bit & 3));
+            }
           }
         }
       }
