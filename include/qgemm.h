@@ -119,7 +119,8 @@ int qgemm_w8a8_grouped_zeroed(const int8_t* A, const int8_t* B, const float* sca
                               int b_layout, uint32_t* status, void* stream);
 
 /* Bytes of scratch memory qgemm_w4a16 needs for this problem on the current device (split-K partial
- * sums and arrival counters, the prepared activations and, from 1792 tokens on, the weights as f16: 2*N*K).
+ * sums and arrival counters, the prepared activations).  Above 64 tokens a smaller buffer with room for 128-token tiles
+ * (qgemm_w4a16_counter_bytes() + SMs * 128 KB + 2*batch*M*K) is accepted too; no tile is cut along K then, which is slower.
  * The buffer needs no initialisation: every call zeroes the qgemm_w4a16_counter_bytes() bytes of arrival
  * counters at its start, on the stream, and writes everything else before reading it.  Two launches
  * that may overlap on the device must not share a scratch buffer. */
@@ -182,13 +183,10 @@ int qgemm_w4a16_batched(const void* A, const uint8_t* B_packed, const void* scal
  *                QGEMM_ZERO_RESCALE    W = q * s - |z|      (one f16 FMA; needs the zeros tensor)
  *                QGEMM_ZERO_QUANTIZED  W = (q - qz) * s     with integer qz given as fp16 values (unpack
  *                                      packed qzeros on the host first)
- * A zeros tensor of mode QGEMM_ZERO_QUANTIZED (integer zero points 0..15) is taken in flight by the streaming kernel
- * when M <= 64 and the groups are 128 wide, a multiple of 256 or the whole K: no dequantised copy of the weights,
- * (q - qz) exact, and a scratch buffer of qgemm_w4a16_ex_workspace_bytes(..., has_zeros_tensor = 0) suffices.
- * Otherwise a zeros tensor makes the operator dequantise the weights once into the scratch buffer
- * (f16 [batch, N, K]) and multiply with the f16 tensor-core GEMM, whatever the token count; that scratch size comes
- * from qgemm_w4a16_ex_workspace_bytes(..., has_zeros_tensor = 1).  Without a zeros tensor the same kernels as
- * qgemm_w4a16 run.
+ * A zeros tensor is taken in flight whatever its mode: by the streaming kernel (mode QGEMM_ZERO_QUANTIZED, integer zero
+ * points 0..15, M <= 64, groups 128 wide, a multiple of 256 or the whole K), otherwise by the wide tiles, with the
+ * roundings written above.  No dequantised copy of the weights is made; has_zeros_tensor below no longer changes the
+ * scratch size.
  */
 #define QGEMM_W4_SEQUENTIAL 0
 #define QGEMM_W4_INTERLEAVED_F16 1
@@ -215,7 +213,7 @@ int qgemm_w4a16_ex(const void* A, const uint8_t* B_packed, const void* scales, c
  * examples/shmem/shmem_mm_test_put_nbi.py:69-74; there is no gathered dequantize-GEMM in the reference.
  *
  * C_dst is a HOST array of n_dst (1..8) device pointers.  ldc and col0 must be multiples of 8, and from the
- * token count at which the weights are dequantised once (1024) N must be a multiple of 64.  Everything else as
+ * 1792 tokens on N must be a multiple of 64 (unless it is no multiple of 16).  Everything else as
  * qgemm_w4a16 (batch 1, scalar zero point, sequential nibbles); the workspace size is qgemm_w4a16_workspace_bytes.
  * The call returns when the kernels are queued; a destination buffer is complete on its GPU once EVERY rank's
  * call has finished, which the ranks establish among themselves (a stream-ordered barrier, for example a small

@@ -527,3 +527,48 @@ def test_non_finite_activations(M, K, N, zeros, fmt):
     torch.testing.assert_close(C[rows].double(), A[rows].half().double() @ W.t(), equal_nan=True)  # +-inf and NaN only
     other = [m for m in range(M) if m not in rows]
     assert torch.equal(C[other], C0[other])
+
+
+@pytest.mark.parametrize("M,K,N,group,zeros", [
+    (65, 256, 8, 128, None),        # one tile of 80 tokens, one slab
+    (128, 4096, 136, 32, None),     # K cut over CTAs, two accumulators
+    (129, 1056, 272, 32, "rescale"),    # K not a multiple of 64
+    (256, 8192, 128, 64, None),     # the tallest tile, cut along K
+    (257, 512, 128 * 75, 128, None),    # two token tiles, whole tiles and a cut remainder
+    (17, 2048, 144, 64, "quantized"), (9, 512, 2064, 128, "original"), (1, 1024, 16, 32, "rescale"),
+    (700, 768, 1040, 768, "original"),
+])
+@pytest.mark.parametrize("dt", ["float16", "bfloat16"])
+def test_wide_tiles(M, K, N, group, zeros, dt):
+    """The wide tiles at the edges of their token tiles, K slabs and cuts; once more with the scratch of 128-token tiles
+    (no tile is split then).  Sums of f16 x f16 products in fp32 against float64: the output's rounding and 2^-24 per
+    addition of at most K terms, of the sum of magnitudes."""
+    q = _q()
+    from tilelang_ascend_b200 import _lib
+    A, packed, scales = oc.make_w4a16_inputs(M, K, N, dt, group, seed=M + N)
+    if zeros is None:
+        z, W = 7, oc.dequant_weight_ref(packed, scales, 7, group)
+    else:
+        z = torch.randint(0, 16, scales.shape, generator=torch.Generator().manual_seed(M)).to(torch.float16)
+        W = oc.dequant_weight_zeros_ref(packed, scales, z, group, zeros)
+    A64, W64 = A.half().double(), W.double()
+    ref = A64 @ W64.t()
+    bound = (2.0 ** -11 if dt == "float16" else 2.0 ** -8) * ref.abs() + K * 2.0 ** -24 * (A64.abs() @ W64.abs().t()) + 1e-6
+    Ac, P, S = A.cuda(), packed.cuda(), scales.cuda()
+    Z = z.cuda() if zeros else None
+    C = q.w4a16_gemm(Ac, P, S, Z if zeros else 7, group, zeros_mode=zeros or "original")
+    assert bool(((C.cpu().double() - ref).abs() <= bound).all())
+    lib = _lib.load()
+    mode = {None: 0, "original": 0, "rescale": 1, "quantized": 2}[zeros]
+    code = q.ops._ABI_DT[Ac.dtype]
+    small = lib.qgemm_w4a16_call_workspace_bytes(1, M, N, K, group, 1, 1 if zeros else 0, mode)
+    if M > 64:
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        small = min(small, lib.qgemm_w4a16_counter_bytes() + sms * 2 * 128 * 128 * 4 + M * K * 2)
+    ws = torch.empty(small, dtype=torch.uint8, device="cuda")
+    C2 = torch.full((M, N), float("nan"), dtype=Ac.dtype, device="cuda")
+    args = (Ac.data_ptr(), P.data_ptr(), S.data_ptr(), Z.data_ptr() if zeros else 0, 7, mode, 0, group, C2.data_ptr(), ws.data_ptr())
+    call = lambda size: lib.qgemm_w4a16_ex(*args, size, 1, M, N, K, code, code, 0, torch.cuda.current_stream().cuda_stream)
+    assert call(small - 1) != 0  # refused
+    assert call(small) == 0, _lib.last_error()
+    assert bool(((C2.cpu().double() - ref).abs() <= bound).all())

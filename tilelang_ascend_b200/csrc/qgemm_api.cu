@@ -2,6 +2,7 @@
 // The exported functions are declared and documented in include/qgemm.h.
 #include "../../include/qgemm.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -12,6 +13,7 @@
 #include "w4a16.cuh"
 #include "w4a16_decode.cuh"
 #include "w4a16_gs.cuh"
+#include "w4a16_wide.cuh"
 #include "act_quant.cuh"
 #include "w4a8.cuh"
 #include "w8a8.cuh"
@@ -61,13 +63,11 @@ int set_smem_w8() {
   if (set_smem(qg::w8a8_gemm_kernel<BN, false, true>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w8a8_gemm_kernel<BN, true, false>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w8a8_gemm_kernel<BN, true, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w8a8_gemm_kernel<BN, true, false, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w8a8_gemm_kernel<BN, true, true, true>, C::SMEM_BYTES)) return -1;
   if (BN == 256) {  // the two-CTA K split
-    if (set_smem(qg::w8a8_gemm_kernel<256, false, false, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, false, true, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, false, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, false, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, true, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, true>, C::SMEM_BYTES)) return -1;
   }
   return 0;
 }
@@ -112,6 +112,13 @@ int set_smem_w4g() {
 }
 
 // Once per device, with that device current.
+int set_smem_w4w() {
+  if (set_smem(qg::w4a16_wide_kernel<false, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a16_wide_kernel<true, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a16_wide_kernel<false, true>, qg::W4WideCfg<true>::SMEM_BYTES)) return -1;
+  return set_smem(qg::w4a16_wide_kernel<true, true>, qg::W4WideCfg<true>::SMEM_BYTES);
+}
+
 int ensure_device(int* sm_count) {
   int dev = 0;
   CUDA_OK(cudaGetDevice(&dev));
@@ -134,9 +141,10 @@ int ensure_device(int* sm_count) {
       g_encode = reinterpret_cast<EncodeTiledFn>(fn);
     }
     if (set_smem_w8<128>() || set_smem_w8<256>()) return -1;
-    if (set_smem_w4<16>() || set_smem_w4<32>() || set_smem_w4<64>() || set_smem_w4<128>()) return -1;
+    if (set_smem_w4<16>()) return -1;
     if (set_smem_w4g<16>() || set_smem_w4g<32>() || set_smem_w4g<64>()) return -1;
     if (set_smem_w4i8<16>() || set_smem_w4i8<32>() || set_smem_w4i8<64>() || set_smem_w4i8<128>()) return -1;
+    if (set_smem_w4w()) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
     st.ready.store(true, std::memory_order_release);
@@ -201,9 +209,7 @@ int w8_group_m(int64_t m_tiles, int64_t k_bytes) {
 template <int BN, bool NK, bool BF>
 int launch_w8(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p, int grid,
               cudaStream_t s) {
-  qg::W8Dst dst;
-  for (int d = 0; d < 8; ++d) dst.m[d] = tmC;
-  qg::w8a8_gemm_kernel<BN, NK, BF><<<grid, qg::W8_THREADS, qg::W8Cfg<BN>::SMEM_BYTES, s>>>(tmA, tmB, dst, p);
+  qg::w8a8_gemm_kernel<BN, NK, BF><<<grid, qg::W8_THREADS, qg::W8Cfg<BN>::SMEM_BYTES, s>>>(tmA, tmB, tmC, p);
   CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -212,8 +218,6 @@ int launch_w8(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap&
 template <bool NK, bool BF>
 int launch_w8_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p,
                      int tiles, cudaStream_t s) {
-  qg::W8Dst dst;
-  for (int d = 0; d < 8; ++d) dst.m[d] = tmC;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * tiles));
   cfg.blockDim = dim3((unsigned)qg::W8_THREADS);
@@ -226,15 +230,14 @@ int launch_w8_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, false, true>, tmA, tmB, dst, p));
+  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, true>, tmA, tmB, tmC, p));
   return 0;
 }
 
-template <int MT>
 int launch_w4(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap& tmA,
               const qg::W4A16Params& p, int grid, cudaStream_t s) {
-  if (bf) return launch_pdl(qg::w4a16_gemm_kernel<MT, true>, grid, qg::W4_THREADS, qg::W4Cfg<MT>::SMEM_BYTES, s, tmW, tmS, tmA, p);
-  return launch_pdl(qg::w4a16_gemm_kernel<MT, false>, grid, qg::W4_THREADS, qg::W4Cfg<MT>::SMEM_BYTES, s, tmW, tmS, tmA, p);
+  if (bf) return launch_pdl(qg::w4a16_gemm_kernel<16, true>, grid, qg::W4_THREADS, qg::W4Cfg<16>::SMEM_BYTES, s, tmW, tmS, tmA, p);
+  return launch_pdl(qg::w4a16_gemm_kernel<16, false>, grid, qg::W4_THREADS, qg::W4Cfg<16>::SMEM_BYTES, s, tmW, tmS, tmA, p);
 }
 constexpr int64_t kW4MaxGrid = 1024;
 constexpr int64_t kW4CounterBytes = kW4MaxGrid * 4;
@@ -550,8 +553,6 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
 
   qg::W8A8Params p;
   p.tma_store = tma_store ? 1 : 0;
-  p.n_dst = 0;
-  p.col0 = 0;
   p.scale_b = scale_b;
   p.scale_a = scale_a;
   p.C = C;
@@ -646,59 +647,99 @@ int qgemm_w8a8_grouped_zeroed(const int8_t* A, const int8_t* B, const float* sca
 
 int64_t qgemm_w4a16_counter_bytes(void) { return kW4CounterBytes; }
 
-// Token counts from this on (and N a multiple of 16) dequantise the whole weight matrix to f16 once and run
-// the f16 tensor-core GEMM on it: the in-flight conversion is repeated for every 128-token tile and at some point
-// costs more than writing and re-reading 2 bytes per weight.  Measured sweep on K=8192, N=28672 (in-flight against
-// dequantise-once, us): 512 tokens 230 / 366, 1024: 445 / 526, 1536: 685 / 710, 2048: 927 / 877 - the paths cross
-// near 1800.  QGEMM_W4_GEMM_MIN_M overrides the threshold (0 = never).
-int64_t w4_gemm_min_m() {
-  static int64_t v = -1;
-  if (v < 0) {
-    v = 1792;
-    if (const char* e = getenv("QGEMM_W4_GEMM_MIN_M")) v = atoll(e) > 0 ? atoll(e) : (1ll << 62);
-    if (v <= 16) v = 17;  // the small-token kernels keep their range
+// Wide tiles (w4a16_wide.cuh): the tile's tokens and the cut of the work.  Of the cuts into equal tiles (48 .. 256 tokens,
+// a multiple of 16, fewer when there are fewer tokens) and of three ways to deal T tiles to G CTAs the one with the
+// smallest estimated time: whole tiles only; whole rounds of G tiles and each tile of the remainder cut into S equal K
+// ranges for S CTAs; or the remainder (with one whole round, when it is small) cut evenly over all CTAs.  The estimate is
+// fitted to a sweep of tile heights and cuts over K = 1024 .. 8192, N = 1024 .. 14336, 80 .. 2048 tokens (us): a slab
+// 0.95, from about 96 tokens on 0.5 + 0.0048 per token; a tile's end 2 + 0.015 per token; the sum of a tile that S CTAs
+// share 2 + S (0.3 + 0.011 per token), or 2 where whole tiles follow behind which it runs; the even cut, where a CTA can
+// hold two partial tiles, 3 + 0.06 per token, or 6.  So large problems take the tallest tiles, problems of fewer tiles
+// than SMs shorter ones (512 x 2048 x 4096: 128 tiles of 128 tokens 16.4 us, 64 tiles of 256 cut in two 25.5 us), and a
+// cut along K is for few tiles of long K (128 x 8192 x 2048: 32 tiles of 64 tokens cut in four 23.3 us, whole 38.6 us).
+struct W4WidePlan {
+  int mt = 0, sk_tiles = 0, sk_grid = 1;
+};
+static W4WidePlan w4_wide_plan(int64_t M, int64_t weight_tiles, int64_t KS, int64_t G) {
+  W4WidePlan best;
+  double best_time = 0.0;
+  if (M <= 0 || weight_tiles <= 0 || KS <= 0) return best;  // a size query about an empty problem
+  for (int64_t t = (M + qg::W4W_MAX_MT - 1) / qg::W4W_MAX_MT;; ++t) {
+    const int64_t mt = ((M + t - 1) / t + 15) / 16 * 16;
+    const int64_t tiles = weight_tiles * ((M + mt - 1) / mt), rounds = tiles / G, r = tiles % G;
+    const double slab = std::max(0.95, 0.5 + 0.0048 * (double)mt), end = 2.0 + 0.015 * (double)mt;
+    auto consider = [&](double slabs, double extra, int64_t sk_tiles, int64_t sk_grid) {
+      const double time = slabs * slab + end + extra;
+      if (best.mt != 0 && time >= best_time) return;
+      best_time = time;
+      best.mt = (int)mt;
+      best.sk_tiles = (int)sk_tiles;
+      best.sk_grid = (int)sk_grid;
+    };
+    consider((double)((rounds + (r != 0 ? 1 : 0)) * KS), 0.0, 0, 1);
+    if (r != 0) {
+      for (int64_t S = 2; S <= 8 && S * r <= G && S <= KS; S += 2)
+        consider((double)(rounds * KS + (KS + S - 1) / S), rounds != 0 ? 2.0 : 2.0 + (double)S * (0.3 + 0.011 * (double)mt), r, r * S);
+      const int64_t sk = r + (rounds != 0 && 2 * r < G ? G : 0);
+      if (sk * KS >= G) consider((double)(tiles * KS) / (double)G, rounds != 0 ? 6.0 : 3.0 + 0.06 * (double)mt, sk, G);
+    }
+    if (mt <= 48 || tiles > 4 * G) break;  // more tiles than that only convert the weights more often
   }
-  return v;
+  return best;
 }
-bool w4_use_f16_gemm(int64_t M, int64_t N) { return M >= w4_gemm_min_m() && (N % 16) == 0; }
+static int64_t w4_wide_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  int sms = 0;
+  if (ensure_device(&sms)) return -1;
+  const int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
+  const int mt = w4_wide_plan(M, batch * ((N + 127) / 128), (K + 255) / 256, grid).mt;
+  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + batch * M * K * 2;
+}
 
-static int64_t w4_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, bool dequant_once) {
+// Which of the W4A16 kernels takes a call: the group-sum kernel (w4a16_gs.cuh) up to 64 tokens where it can (wide scale
+// groups, scalar zero point or a zeros tensor of mode "quantized"); scale groups of 32 / 64 up to 16 tokens the
+// register-operand decode kernel (up to 8) and w4a16.cuh; everything else the wide tiles.  Groups of 64, K = 8192, N =
+// 28672: at 16 tokens 46.9 us (w4a16.cuh) against 54.2 (wide), at 24 56.6 against 53.7; K = N = 4096 at 24: 16.1
+// against 12.1, at 64: 23.9 against 15.6.
+enum W4Route { W4_GROUP_SUM, W4_NARROW_GROUPS, W4_WIDE };
+static W4Route w4_route(int64_t M, int64_t K, int64_t group, bool has_scales, bool zeros_tensor, int zero_mode) {
+  const bool gs = w4_gs_shape_ok(M, has_scales, group, K);
+  if (zeros_tensor) return gs && zero_mode == QGEMM_ZERO_QUANTIZED ? W4_GROUP_SUM : W4_WIDE;
+  if (gs) return W4_GROUP_SUM;
+  return M <= 16 ? W4_NARROW_GROUPS : W4_WIDE;
+}
+
+// Scratch of the kernels for few tokens: the arrival counters first (fixed place whatever the tile height), then two
+// partial slots of [MT][128] fp32 per CTA, then the prepared activations - plain f16 [M, K] in the kernel's K order, or
+// the group-sum kernel's stage images (token tiles padded).
+static int64_t w4_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
   if (ensure_device(&sms)) return -1;
   const int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   // sized for whichever small-token kernel the scale groups will select (the group-sum kernel's tile is the taller)
-  const int mt = M <= 64 ? w4_pick_mt(M, true) : w4_pick_mt(M, false);
-  // prepared activations: plain f16 [M, K], or the group-sum kernel's stage images (token tiles padded)
+  const int mt = M <= 64 ? w4_pick_mt(M, true) : 128;
   int64_t a_bytes = batch * M * K * 2;
   if (M <= 64) {
     const int64_t images = batch * ((K + 255) / 256) * 2 * (int64_t)qg::w4g_half_bytes(mt);
     if (images > a_bytes) a_bytes = images;
   }
-  // the arrival counters first (fixed place whatever the tile height), then two partial slots of
-  // [MT][128] fp32 per CTA, then the f16 copy of the activations in the kernel's K order
-  // ... and, for the large-token path, the dequantised f16 weights
-  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + a_bytes +
-         ((dequant_once || w4_use_f16_gemm(M, N)) ? batch * N * K * 2 : 0);
+  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + a_bytes;
 }
 
 int64_t qgemm_w4a16_batched_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
-  return w4_workspace_bytes(batch, M, N, K, false);
+  const int64_t few = w4_workspace_bytes(batch, M, N, K);
+  return few < 0 ? -1 : std::max(few, w4_wide_workspace_bytes(batch, M, N, K));
 }
 
 int64_t qgemm_w4a16_ex_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int has_zeros_tensor) {
-  return w4_workspace_bytes(batch, M, N, K, has_zeros_tensor != 0);
-}
-
-// Whether a zeros tensor is taken in flight by the group-sum kernel (see w4a16_impl).
-static bool w4_zeros_inflight(int64_t M, int64_t N, int64_t K, int64_t group, int zero_mode) {
-  static const int on = getenv("QGEMM_W4_ZEROS_INFLIGHT") ? atoi(getenv("QGEMM_W4_ZEROS_INFLIGHT")) : 1;
-  return on && zero_mode == QGEMM_ZERO_QUANTIZED && !w4_use_f16_gemm(M, N) && w4_gs_shape_ok(M, true, group, K);
+  (void)has_zeros_tensor;  // zero points are taken in flight
+  return qgemm_w4a16_batched_workspace_bytes(batch, M, N, K);
 }
 
 int64_t qgemm_w4a16_call_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int64_t group, int has_scales,
                                          int has_zeros_tensor, int zero_mode) {
-  const bool zeros = has_scales && has_zeros_tensor;
-  return w4_workspace_bytes(batch, M, N, K, zeros && !w4_zeros_inflight(M, N, K, group, zero_mode));
+  if (w4_route(M, K, group, has_scales != 0, has_scales && has_zeros_tensor, zero_mode) == W4_WIDE)
+    return w4_wide_workspace_bytes(batch, M, N, K);
+  return w4_workspace_bytes(batch, M, N, K);
 }
 
 int64_t qgemm_w4a16_workspace_bytes(int64_t M, int64_t N, int64_t K) {
@@ -712,78 +753,6 @@ struct GatherDst {
   int n;
   int64_t ldc, col0;
 };
-
-// C[b] = A16[b] (f16 [M, K]) x W16[b]^T (f16 [N, K]), fp32 accumulation, f16 / bf16 out: the tile pipeline of
-// the W8A8 kernel on 2-byte elements (K counted in bytes).
-static int w4_f16_gemm(const void* A16, const void* W16, void* C, int64_t batch, int64_t M, int64_t N, int64_t K,
-                       bool bf, uint32_t* status, cudaStream_t s, int sms, const GatherDst* gd) {
-  const int64_t Kb = K * 2;
-  CUtensorMap tmA, tmB, tmC;
-  {
-    const uint64_t dims[3] = {(uint64_t)Kb, (uint64_t)M, (uint64_t)batch};
-    const uint64_t str[2] = {(uint64_t)Kb, (uint64_t)M * (uint64_t)Kb};
-    const uint32_t box[3] = {128, 128, 1};
-    if (encode_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, A16, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-  }
-  const int64_t m_tiles = (M + 127) / 128;
-  const int BN = (N > 128 && batch * m_tiles * ((N + 255) / 256) >= sms) ? 256 : 128;
-  {
-    const uint64_t dims[3] = {(uint64_t)Kb, (uint64_t)N, (uint64_t)batch};
-    const uint64_t str[2] = {(uint64_t)Kb, (uint64_t)N * (uint64_t)Kb};
-    const uint32_t box[3] = {128, (uint32_t)BN, 1};
-    if (encode_map(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, W16, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-  }
-  qg::W8Dst dst;
-  if (gd == nullptr) {
-    const uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)batch};
-    const uint64_t str[2] = {(uint64_t)N * 2, (uint64_t)M * (uint64_t)N * 2};
-    const uint32_t box[3] = {64, 32, 1};
-    if (encode_map(&tmC, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, C, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
-    for (int d = 0; d < 8; ++d) dst.m[d] = tmC;
-  } else {
-    // one map per destination over its whole [M, ldc] buffer; a tile lands at column col0 + n.  The 64-column
-    // store boxes must not reach into the next rank's columns, hence N % 64 == 0 (checked by the caller).
-    for (int d = 0; d < 8; ++d) {
-      const uint64_t dims[3] = {(uint64_t)gd->ldc, (uint64_t)M, 1};
-      const uint64_t str[2] = {(uint64_t)gd->ldc * 2, (uint64_t)M * (uint64_t)gd->ldc * 2};
-      const uint32_t box[3] = {64, 32, 1};
-      if (encode_map(&dst.m[d], CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, gd->dst[d < gd->n ? d : 0], dims, str, box,
-                     CU_TENSOR_MAP_SWIZZLE_128B))
-        return -1;
-    }
-  }
-  qg::W8A8Params p;
-  memset(&p, 0, sizeof(p));
-  p.n_dst = gd ? gd->n : 0;
-  p.col0 = gd ? (int)gd->col0 : 0;
-  p.C = C;
-  p.batch = (int)batch;
-  p.M = (int)M;
-  p.N = (int)N;
-  p.K = (int)Kb;
-  p.m_tiles = (int)m_tiles;
-  p.group_m = w8_group_m(m_tiles, Kb);
-  p.n_tiles = (int)((N + BN - 1) / BN);
-  p.bn = BN;
-  const int64_t num_tiles = batch * p.m_tiles * p.n_tiles;
-  if (num_tiles > 0x7fffffff) return fail("qgemm_w4a16: too many tiles");
-  p.num_tiles = (int)num_tiles;
-  p.k_blocks = (int)((Kb + 127) / 128);
-  p.status = status;
-  p.wait_limit_ns = g_wait_limit_ns;
-  p.tma_store = 1;
-  p.split_from = p.num_items = p.num_tiles;
-  const int grid = (int)(num_tiles < sms ? num_tiles : sms);
-  if (BN == 256) {
-    if (bf) qg::w8a8_gemm_kernel<256, true, true, true><<<grid, qg::W8_THREADS, qg::W8Cfg<256>::SMEM_BYTES, s>>>(tmA, tmB, dst, p);
-    else qg::w8a8_gemm_kernel<256, true, false, true><<<grid, qg::W8_THREADS, qg::W8Cfg<256>::SMEM_BYTES, s>>>(tmA, tmB, dst, p);
-  } else {
-    if (bf) qg::w8a8_gemm_kernel<128, true, true, true><<<grid, qg::W8_THREADS, qg::W8Cfg<128>::SMEM_BYTES, s>>>(tmA, tmB, dst, p);
-    else qg::w8a8_gemm_kernel<128, true, false, true><<<grid, qg::W8_THREADS, qg::W8Cfg<128>::SMEM_BYTES, s>>>(tmA, tmB, dst, p);
-  }
-  CUDA_OK(cudaGetLastError());
-  return 0;
-}
 
 int qgemm_w4a16(const void* A, const uint8_t* B_packed, const void* scales, int zero, int64_t group, void* C,
                 void* workspace, int64_t workspace_bytes, int64_t M, int64_t N, int64_t K, int a_dtype,
@@ -845,20 +814,22 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
     zero = 0;
     group = K;
   }
-  // A zeros tensor of mode "quantized" (integer zero points) is taken in flight by the group-sum kernel wherever that
-  // kernel applies; the other zero modes, whose f16 roundings per weight the group-sum form cannot reproduce, and all
-  // other shapes go through the whole-matrix dequantisation.  QGEMM_W4_ZEROS_INFLIGHT=0 sends every zeros tensor there.
-  const bool zeros_inflight = zeros != nullptr && gd == nullptr && w4_zeros_inflight(M, N, K, group, zero_mode);
-  const bool dequant_once = (zeros != nullptr && !zeros_inflight) || w4_use_f16_gemm(M, N);
-  // a zeros tensor that is taken in flight needs no room for dequantised weights
-  const int64_t need = w4_workspace_bytes(batch, M, N, K, zeros != nullptr && !zeros_inflight);
+  const W4Route route = w4_route(M, K, group, scales != nullptr, zeros != nullptr, zero_mode);
+  const bool use_gs = route == W4_GROUP_SUM, wide = route == W4_WIDE;
+  int64_t need = w4_workspace_bytes(batch, M, N, K);
   if (need < 0) return -1;
+  const int64_t wide_need = wide ? w4_wide_workspace_bytes(batch, M, N, K) : 0;
+  // a workspace too small for the wide tiles' partial sums will do if it has room for 128 tokens': no tile is split then
+  if (wide) need = std::min(need, wide_need);
+  const bool wide_unsplit = wide && workspace_bytes < wide_need;
   if (workspace == nullptr || workspace_bytes < need) return fail("qgemm_w4a16: workspace of %lld bytes needed (got %lld)", (long long)need, (long long)workspace_bytes);
 
   int sms = 0;
   if (ensure_device(&sms)) return -1;
-  const bool use_gs = !dequant_once && w4_gs_shape_ok(M, scales != nullptr, group, K);
-  int mt = w4_pick_mt(M, use_gs);
+  const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
+  W4WidePlan plan;
+  if (wide) plan = w4_wide_plan(M, batch * ((N + 127) / 128), (K + 255) / 256, grid_max);
+  int mt = wide ? plan.mt : w4_pick_mt(M, use_gs);
   if (gd != nullptr && mt < 16) mt = 16;  // the register-operand decode kernel writes one destination only
 
   CUtensorMap tmW, tmS, tmZ, tmA;
@@ -878,12 +849,11 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
     const uint64_t str[2] = {(uint64_t)N * 2, (uint64_t)(K / group) * (uint64_t)N * 2};
     const uint32_t box[3] = {128, (uint32_t)scale_rows, 1};
     if (encode_map(&tmS, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, scales, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return -1;
-    if (zeros_inflight &&
+    if (zeros != nullptr &&
         encode_map(&tmZ, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, zeros, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE))
       return -1;
   }
-  const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
-  uint8_t* a_prepared = static_cast<uint8_t*>(workspace) + kW4CounterBytes + grid_max * 2 * (int64_t)mt * 128 * 4;
+  uint8_t* a_prepared = static_cast<uint8_t*>(workspace) + kW4CounterBytes + (wide_unsplit ? 0 : grid_max * 2 * (int64_t)mt * 128 * 4);
   if (!use_gs) {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)M * (uint64_t)K * 2};
@@ -932,7 +902,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   if (p.total_items < grid) grid = p.total_items;
   // Small problems (a few slabs per CTA): prefer a slightly smaller grid that cuts every tile into equal K ranges,
   // one per CTA, over an even deal that leaves most CTAs with two partial tiles and so two split-K hand-overs.
-  if (p.total_items <= 8 * grid && p.total_items > grid) {
+  if (!wide && p.total_items <= 8 * grid && p.total_items > grid) {
     for (int64_t g2 = grid; g2 * 4 >= grid * 3; --g2) {
       if (p.total_items % g2 != 0) continue;
       const int64_t per = p.total_items / g2;
@@ -947,8 +917,12 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   // run beside the whole tiles' work and the launch ends with plain tile writes.  QGEMM_W4_HYBRID=0 cuts all tiles
   // stream-K fashion.
   p.sk_tiles = p.num_tiles;
+  p.sk_grid = 1;
   p.dp_rounds = 0;
-  {
+  if (wide) {
+    p.sk_tiles = wide_unsplit ? 0 : plan.sk_tiles;
+    p.sk_grid = plan.sk_grid;
+  } else {
     static const int hybrid = getenv("QGEMM_W4_HYBRID") ? atoi(getenv("QGEMM_W4_HYBRID")) : 1;
     const int64_t rounds = num_tiles / grid, r = num_tiles % grid;
     if (hybrid && use_gs && rounds >= 1) {
@@ -965,7 +939,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   // 8.8 / 9.8 us; with more clusters than SMs (several waves) it loses.  QGEMM_W4_SMALL=0 keeps the two-launch form.
   {
     static const int small_on = getenv("QGEMM_W4_SMALL") ? atoi(getenv("QGEMM_W4_SMALL")) : 1;
-    if (small_on && use_gs && mt == 16 && gd == nullptr && !zeros_inflight && g_w4g_withhold_commit != 1) {
+    if (small_on && use_gs && mt == 16 && gd == nullptr && zeros == nullptr && g_w4g_withhold_commit != 1) {
       int cluster = 0;
       for (int c = 1; c <= 4; c *= 2)  // clusters of eight were measured slower than the two-launch form (15.3 / 11.3 us)
         if (p.KS % c == 0 && p.KS / c <= qg::W4G_SMALL_MAX_SLABS) { cluster = c; break; }
@@ -977,7 +951,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
     }
   }
   if (use_gs) {
-    const CUtensorMap* tz = zeros_inflight ? &tmZ : nullptr;
+    const CUtensorMap* tz = zeros != nullptr ? &tmZ : nullptr;
     const bool a_bf = a_dtype == QGEMM_DT_BF16;
     p.A_raw = a_prepared;
     if (mt == 16) return launch_w4g_prepare<16>(A, a_prepared, p, a_bf, s) || launch_w4g<16>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
@@ -998,19 +972,15 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
                    p.ws_counters, (int)(kW4CounterBytes / 4)))
       return -1;
   }
-  if (dequant_once) {
-    uint8_t* w16 = a_prepared + batch * M * K * 2;
-    const int64_t geff = group > K ? K : group;
-    const long long n_chunks = (long long)batch * N * (K / 32);
-    const long long blocks = (n_chunks + 255) / 256;
-    if (blocks > 0x7fffffffll) return fail("qgemm_w4a16: weight tensor too large");
-    qg::w4a16_dequant_weights<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const uint4*>(B_packed),
-                                                             static_cast<const __half*>(scales),
-                                                             static_cast<const __half*>(zeros), zero_mode,
-                                                             reinterpret_cast<uint4*>(w16), n_chunks, (int)(K / 32),
-                                                             (int)N, (int)K, (int)geff, zero);
-    CUDA_OK(cudaGetLastError());
-    return w4_f16_gemm(a_prepared, w16, C, batch, M, N, K, bf, status, s, sms, gd);
+  if (wide) {
+    const CUtensorMap& tz = zeros != nullptr ? tmZ : tmS;
+    constexpr int smem = qg::W4WideCfg<false>::SMEM_BYTES, smem_zt = qg::W4WideCfg<true>::SMEM_BYTES;
+    if (zeros != nullptr) {
+      if (bf) return launch_pdl(qg::w4a16_wide_kernel<true, true>, (int)grid, qg::W4W_THREADS, smem_zt, s, tmW, tmS, tz, tmA, p, mt, zero_mode);
+      return launch_pdl(qg::w4a16_wide_kernel<false, true>, (int)grid, qg::W4W_THREADS, smem_zt, s, tmW, tmS, tz, tmA, p, mt, zero_mode);
+    }
+    if (bf) return launch_pdl(qg::w4a16_wide_kernel<true, false>, (int)grid, qg::W4W_THREADS, smem, s, tmW, tmS, tz, tmA, p, mt, 0);
+    return launch_pdl(qg::w4a16_wide_kernel<false, false>, (int)grid, qg::W4W_THREADS, smem, s, tmW, tmS, tz, tmA, p, mt, 0);
   }
   if (gd == nullptr && w4_use_decode(M) && mt <= 16 && M <= w4_decode_max_m()) {
     if (scales == nullptr) return launch_w4d<0>(bf, mt, tmW, tmS, tmA, p, (int)grid, s);
@@ -1018,12 +988,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
     if (group == 64) return launch_w4d<2>(bf, mt, tmW, tmS, tmA, p, (int)grid, s);
     return launch_w4d<1>(bf, mt, tmW, tmS, tmA, p, (int)grid, s);
   }
-  switch (mt) {
-    case 16: return launch_w4<16>(bf, tmW, tmS, tmA, p, (int)grid, s);
-    case 32: return launch_w4<32>(bf, tmW, tmS, tmA, p, (int)grid, s);
-    case 64: return launch_w4<64>(bf, tmW, tmS, tmA, p, (int)grid, s);
-    default: return launch_w4<128>(bf, tmW, tmS, tmA, p, (int)grid, s);
-  }
+  return launch_w4(bf, tmW, tmS, tmA, p, (int)grid, s);
 }
 
 int qgemm_w4a16_gather(const void* A, const uint8_t* B_packed, const void* scales, int zero, int64_t group,
@@ -1036,8 +1001,8 @@ int qgemm_w4a16_gather(const void* A, const uint8_t* B_packed, const void* scale
   if (ldc <= 0 || ldc > (1ll << 30) || col0 < 0 || N <= 0 || col0 + N > ldc)
     return fail("qgemm_w4a16_gather: columns [%lld, %lld) do not fit in rows of %lld", (long long)col0, (long long)(col0 + N), (long long)ldc);
   if (ldc % 8 != 0 || col0 % 8 != 0) return fail("qgemm_w4a16_gather: ldc and col0 must be multiples of 8 (got %lld, %lld)", (long long)ldc, (long long)col0);
-  if (w4_use_f16_gemm(M, N) && N % 64 != 0)
-    return fail("qgemm_w4a16_gather: from %lld tokens on N must be a multiple of 64 (got %lld)", (long long)w4_gemm_min_m(), (long long)N);
+  if (M >= 1792 && N % 16 == 0 && N % 64 != 0)
+    return fail("qgemm_w4a16_gather: from 1792 tokens on N must be a multiple of 64 (got %lld)", (long long)N);
   GatherDst gd{C_dst, n_dst, ldc, col0};
   return w4a16_impl(A, B_packed, scales, zero, group, nullptr, workspace, workspace_bytes, 1, M, N, K, a_dtype, out_dtype,
                     status, stream, nullptr, QGEMM_ZERO_ORIGINAL, QGEMM_W4_SEQUENTIAL, &gd);

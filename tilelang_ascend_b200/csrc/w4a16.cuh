@@ -1,4 +1,5 @@
-// W4A16 dequantize-GEMM for sm_100a:
+// W4A16 dequantize-GEMM for sm_100a, scale groups of 32 / 64 at up to 16 tokens (w4_route in qgemm_api.cu), and what the
+// other W4A16 kernels share with it:
 //   C[m, n] = cast( sum_k float(A[m, k]) * float(W[n, k]) ),  W[n, k] = half(q[n, k] - zero) * s[k / g, n]
 // with q packed two per byte along K, low nibble first, in B_packed[N, K/2].
 //
@@ -44,6 +45,7 @@ struct W4A16Params {
   // Group-sum kernel only: tiles 0 .. sk_tiles - 1 are cut stream-K fashion over all CTAs, then CTA c takes dp_rounds
   // whole tiles sk_tiles + c + j * grid.  The other kernels deal all (tile, slab) items evenly (total_items).
   int sk_tiles, dp_rounds;
+  int sk_grid;  // wide tiles only: the first sk_tiles tiles are cut over this many CTAs
   // Group-sum kernel: the prepared activations (stage images) or, in its single-launch form (no pre-pass), the caller's
   // activations [batch, M, K] and whether they are bf16; and whether the weight layout is the interleaved one.
   const void* A_raw;
@@ -184,6 +186,18 @@ __device__ __forceinline__ void w4_dequant8(uint32_t x, uint32_t sub_lo, uint32_
   }
 }
 
+// Two raw nibble values -> weights under a zero point z2 and scale s2 (each twice), zero_mode 0 / 2: (q - z) * s, two
+// roundings as the reference's sub.f16x2 + fma (tilelang/quantize/lop3.py:135-175, 325-358); 1: q * s - |z|, one.
+__device__ __forceinline__ void w4_apply_zero(uint32_t& o, uint32_t s2, uint32_t z2, int zero_mode) {
+  if (zero_mode == 1) {
+    const uint32_t nz = z2 | 0x80008000u;  // -|z|, as the reference forms it (lop3.py:247)
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(o) : "r"(o), "r"(s2), "r"(nz));
+  } else {
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(o) : "r"(o), "r"(z2));
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(o) : "r"(o), "r"(s2));
+  }
+}
+
 __device__ __forceinline__ uint32_t w4_bf16x2_to_f16x2(uint32_t w) {
   const float lo = __uint_as_float(w << 16);
   const float hi = __uint_as_float(w & 0xffff0000u);
@@ -198,64 +212,6 @@ __device__ __forceinline__ uint4 w4_permute_act(uint4 v) {
   o.z = __byte_perm(v.y, v.w, 0x5410);
   o.w = __byte_perm(v.y, v.w, 0x7632);
   return o;
-}
-
-// Whole-matrix dequantisation for the large-token path: packed [rows, K/2] + scales [K/group, N] per problem
-// -> f16 [rows, K] with every group of eight K values in the order 0,4,1,5,2,6,3,7 (what w4_dequant8 emits and
-// what w4a16_prepare_activations gives the activations), same values as the GEMM kernels' in-flight
-// conversion.  One 16-byte packed chunk (32 weights -> 64 bytes) per thread, consecutive threads along K.
-__global__ void __launch_bounds__(256)
-w4a16_dequant_weights(const uint4* __restrict__ packed, const __half* __restrict__ scales,
-                      const __half* __restrict__ zeros, int zero_mode, uint4* __restrict__ out, long long n_chunks,
-                      int chunks_per_row, int N, int K, int group, int zero) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_chunks) return;
-  const long long row = i / chunks_per_row;  // batch * N + n
-  const int k0 = (int)(i - row * chunks_per_row) * 32;
-  const uint4 v = __ldcs(packed + i);
-  const uint32_t z = (uint32_t)zero;
-  const uint32_t sub_lo = (0x6400u + z) * 0x00010001u;
-  const uint32_t sub_hi = ((0x5400u + (z << 4)) | 0x8000u) * 0x00010001u;
-  uint32_t s2 = 0x3C003C00u;
-  const bool scaled = scales != nullptr;
-  if (scaled) {
-    const long long b = row / N;
-    const int n = (int)(row - b * N);
-    const int g = k0 / group;  // a 32-wide chunk never straddles a group (group is a multiple of 32)
-    s2 = (uint32_t)__half_as_ushort(scales[(b * (K / group) + g) * (long long)N + n]) * 0x00010001u;
-  }
-  uint32_t o[16];
-  if (zeros == nullptr) {
-    w4_dequant8(v.x, sub_lo, sub_hi, s2, scaled, o + 0);
-    w4_dequant8(v.y, sub_lo, sub_hi, s2, scaled, o + 4);
-    w4_dequant8(v.z, sub_lo, sub_hi, s2, scaled, o + 8);
-    w4_dequant8(v.w, sub_lo, sub_hi, s2, scaled, o + 12);
-  } else {
-    // Per-(group, column) zero points (tilelang/quantize/lop3.py:135-175, 232-270, 325-358).  The raw nibble
-    // values come out exact; then mode 0 / 2 ("original" / "quantized"): (q - z) * s, two roundings as the
-    // reference's sub.f16x2 + fma; mode 1 ("rescale"): fma(q, s, -|z|), one rounding.
-    const long long b = row / N;
-    const int n = (int)(row - b * N);
-    const uint32_t z2 = (uint32_t)__half_as_ushort(zeros[(b * (K / group) + k0 / group) * (long long)N + n]) * 0x00010001u;
-    const uint32_t raw_lo = 0x6400u * 0x00010001u, raw_hi = (0x5400u | 0x8000u) * 0x00010001u;
-    w4_dequant8(v.x, raw_lo, raw_hi, s2, false, o + 0);
-    w4_dequant8(v.y, raw_lo, raw_hi, s2, false, o + 4);
-    w4_dequant8(v.z, raw_lo, raw_hi, s2, false, o + 8);
-    w4_dequant8(v.w, raw_lo, raw_hi, s2, false, o + 12);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      if (zero_mode == 1) {
-        const uint32_t nz = z2 | 0x80008000u;  // -|z|, as the reference forms it (lop3.py:247)
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(o[j]) : "r"(o[j]), "r"(s2), "r"(nz));
-      } else {
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(o[j]) : "r"(o[j]), "r"(z2));
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(o[j]) : "r"(o[j]), "r"(s2));
-      }
-    }
-  }
-  uint4* dst = out + i * 4;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) __stcs(dst + j, make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]));
 }
 
 // Pre-pass: activations [M, K] (f16 or bf16) -> f16 with every group of eight K values reordered to

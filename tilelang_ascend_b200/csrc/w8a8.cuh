@@ -38,14 +38,6 @@ struct W8A8Params {
   // twice as many SMs busy for about half as long.  num_items = num_tiles when nothing is split.
   int split_from, num_items;
   int tma_store;  // C is written with tiled bulk stores from a shared-memory staging tile (needs bn % 64 == 0)
-  // Gathered form: n_dst > 0 destinations (tensor maps in the kernel's W8Dst argument, one [M, ldc] buffer per
-  // rank) receive every tile at column col0 + n instead of the single C.
-  int n_dst, col0;
-};
-
-// Output tensor maps of the gathered form (unused entries are copies of the first).
-struct W8Dst {
-  CUtensorMap m[8];
 };
 
 // One output tile's coordinates: batch index of B / scale_b, batch index of A / C / scale_a, first row, valid rows.
@@ -146,10 +138,6 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
   }
 }
 
-// F16 = true runs the same pipeline on f16 operands (kind::f16, fp32 accumulators, no scales): one MMA K step
-// is 32 bytes for both element types, so with K counted in bytes (p.K, p.k_blocks) nothing else changes.  It
-// serves the large-token W4A16 path, whose weights are dequantised to f16 once and then multiplied here.
-//
 // SPLITK = true is the form for grids that would leave more than half of the SMs idle (fewer 128 x 256 tiles than
 // half the SM count): the kernel is launched in clusters of two CTAs, one tile per cluster; each CTA accumulates
 // one half of the K range in its own tensor memory; then each CTA writes its int32 accumulators of the OTHER CTA's
@@ -159,13 +147,11 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
 // converts and stores half a tile.  The counterpart in the
 // reference is the K split of examples/gemm_splitk/example_tilelang_gemm_splitk.py:15-48, whose partial tiles meet
 // in global memory through atomic adds (src/tl_templates/ascend/common.h:249-259).
-template <int BN, bool B_NK, bool OUT_BF16, bool F16 = false, bool SPLITK = false>
+template <int BN, bool B_NK, bool OUT_BF16, bool SPLITK = false>
 __global__ void __launch_bounds__(W8_THREADS, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ W8Dst tmCs, const W8A8Params p) {
+                 const __grid_constant__ CUtensorMap tmC, const W8A8Params p) {
   using Cfg = W8Cfg<BN>;
-  static_assert(!(SPLITK && F16), "the split form adds int32 partial sums");
-  const CUtensorMap& tmC = tmCs.m[0];
   constexpr int STAGES = Cfg::STAGES;
 
   extern __shared__ uint8_t smem_raw[];
@@ -272,8 +258,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       bool ok = true;
       for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride, ++it) {
         const uint32_t bn = (uint32_t)((tile < p.split_from) ? p.bn : (p.bn >> 1));
-        const uint32_t idesc = F16 ? make_idesc(ACC_F32, FMT_F16, FMT_F16, 0, B_NK ? 0 : 1, W8_BM, bn)
-                                   : make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, W8_BM, bn);
+        const uint32_t idesc = make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, W8_BM, bn);
         const int buf = it & 1;
         const uint32_t tphase = (it >> 1) & 1;
         if (!mbar_wait(&tempty[buf], tphase ^ 1u, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
@@ -295,8 +280,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               // [K rows][128 B of N]: 32 K rows per MMA = 4096 B; the next 128 columns are one box (16 KB) further.
               bdesc = make_desc_mnmajor(sB + k * (W8_UMMA_K * 128), W8_BK * 128);
             }
-            if constexpr (F16) umma_f16_ss(d, adesc, bdesc, idesc, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
-            else umma_i8_ss(d, adesc, bdesc, idesc, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+            umma_i8_ss(d, adesc, bdesc, idesc, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -334,7 +318,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const bool row_ok = q * 32 + lane < t.rows;
       float sa = 1.0f;
       if (p.sa_mode != 0 && row_ok) sa = __ldg(p.scale_a + (p.sa_mode == 2 ? (size_t)t.bA * p.M : 0) + m);
-      if (!F16 && p.C != nullptr) {
+      if (p.C != nullptr) {
         const float* sbp = p.scale_b + (p.sb_mode == 2 ? (size_t)t.bB * p.N : 0);
         __syncwarp();  // the previous tile's reads of sb_s are done
         for (int c = lane; c < t.bn; c += 32) {
@@ -441,17 +425,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const int col = 8 * j + 2 * e;
-                  float f0, f1;
-                  if constexpr (F16) {
-                    f0 = __uint_as_float(r[h][col]);
-                    f1 = __uint_as_float(r[h][col + 1]);
-                  } else {
-                    f0 = __int2float_rn((int)r[h][col]);
-                    f1 = __int2float_rn((int)r[h][col + 1]);
-                    if (p.sa_mode != 0) { f0 = __fmul_rn(f0, sa); f1 = __fmul_rn(f1, sa); }
-                    f0 = __fmul_rn(f0, sc[2 * e]);
-                    f1 = __fmul_rn(f1, sc[2 * e + 1]);
-                  }
+                  float f0 = __int2float_rn((int)r[h][col]), f1 = __int2float_rn((int)r[h][col + 1]);
+                  if (p.sa_mode != 0) { f0 = __fmul_rn(f0, sa); f1 = __fmul_rn(f1, sa); }
+                  f0 = __fmul_rn(f0, sc[2 * e]);
+                  f1 = __fmul_rn(f1, sc[2 * e + 1]);
                   o[e] = pack_out2<OUT_BF16>(f0, f1);
                 }
                 *reinterpret_cast<uint4*>(my_stage + lane * 128 + (((h * 4 + j) ^ (lane & 7)) << 4)) =
@@ -471,17 +448,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
                     const int col = 8 * j + 2 * e;
-                    float f0, f1;
-                    if constexpr (F16) {
-                      f0 = __uint_as_float(r[h][col]);
-                      f1 = __uint_as_float(r[h][col + 1]);
-                    } else {
-                      f0 = __int2float_rn((int)r[h][col]);
-                      f1 = __int2float_rn((int)r[h][col + 1]);
-                      if (p.sa_mode != 0) { f0 = __fmul_rn(f0, sa); f1 = __fmul_rn(f1, sa); }
-                      f0 = __fmul_rn(f0, sc[2 * e]);
-                      f1 = __fmul_rn(f1, sc[2 * e + 1]);
-                    }
+                    float f0 = __int2float_rn((int)r[h][col]), f1 = __int2float_rn((int)r[h][col + 1]);
+                    if (p.sa_mode != 0) { f0 = __fmul_rn(f0, sa); f1 = __fmul_rn(f1, sa); }
+                    f0 = __fmul_rn(f0, sc[2 * e]);
+                    f1 = __fmul_rn(f1, sc[2 * e + 1]);
                     o[e] = pack_out2<OUT_BF16>(f0, f1);
                   }
                   *reinterpret_cast<uint4*>(cbase + 8 * j) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -494,12 +464,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           fence_proxy_async_smem();  // this thread's staging writes are visible to the bulk-copy engine
           __syncwarp();
           if (lane == 0) {
-            if (p.n_dst == 0) {
-              tma_store_3d_hint(&tmC, my_stage, t.n0 + c2 * 32, t.m0 + q * 32, t.bA, pol_out);
-            } else {
-              for (int d = 0; d < p.n_dst; ++d)
-                tma_store_3d_hint(&tmCs.m[d], my_stage, p.col0 + t.n0 + c2 * 32, t.m0 + q * 32, 0, pol_out);
-            }
+            tma_store_3d_hint(&tmC, my_stage, t.n0 + c2 * 32, t.m0 + q * 32, t.bA, pol_out);
             bulk_commit_group();
           }
         }
