@@ -251,44 +251,46 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      bool ok = true;
-      for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride, ++it) {
-        const uint32_t bn = (uint32_t)((tile < p.split_from) ? p.bn : (p.bn >> 1));
-        const uint32_t idesc = make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, W8_BM, bn);
-        const int buf = it & 1;
-        const uint32_t tphase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty[buf], tphase ^ 1u, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
+    // The warp runs converged and one hardware-elected lane issues, which lets the compiler keep the descriptors in uniform
+    // registers.  The stage descriptors differ by their start address only.
+    constexpr uint32_t K_STEP = (B_NK ? W8_UMMA_K : W8_UMMA_K * 128) >> 4;  // B's start address from one MMA to the next
+    // K-major: 128 bytes of K per row.  [K rows][128 B of N]: 32 K rows per MMA = 4096 B; the next 128 columns are one
+    // box (16 KB) further.
+    const uint64_t b_desc = B_NK ? make_desc_kmajor(0) : make_desc_mnmajor(0, W8_BK * 128);
+    const uint64_t a_desc = make_desc_kmajor(0);
+    const uint32_t smem0 = smem_u32(smem);
+    int stage = 0;
+    uint32_t phase = 0;
+    int it = 0;
+    bool ok = true;
+    for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride, ++it) {
+      const uint32_t bn = (uint32_t)((tile < p.split_from) ? p.bn : (p.bn >> 1));
+      const uint32_t idesc = make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, W8_BM, bn);
+      const int buf = it & 1;
+      const uint32_t tphase = (it >> 1) & 1;
+      if (!mbar_wait_warp(&tempty[buf], tphase ^ 1u, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t d = tmem_base + buf * BN;
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if (!mbar_wait_warp(&full[stage], phase, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d = tmem_base + buf * BN;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(&full[stage], phase, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t sA = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-          const uint32_t sB = sA + Cfg::A_BYTES;
-          const uint64_t a0 = make_desc_kmajor(sA);
+        if (elect_one_sync()) {
+          const uint32_t sA = smem0 + stage * Cfg::STAGE_BYTES;
+          const uint64_t adesc = a_desc | (uint64_t)((sA & 0x3FFFFu) >> 4);
+          const uint64_t bdesc = b_desc | (uint64_t)(((sA + Cfg::A_BYTES) & 0x3FFFFu) >> 4);
 #pragma unroll
-          for (int k = 0; k < W8_BK / W8_UMMA_K; ++k) {
-            const uint64_t adesc = a0 + (uint64_t)((k * W8_UMMA_K) >> 4);
-            uint64_t bdesc;
-            if constexpr (B_NK) {
-              bdesc = make_desc_kmajor(sB) + (uint64_t)((k * W8_UMMA_K) >> 4);
-            } else {
-              // [K rows][128 B of N]: 32 K rows per MMA = 4096 B; the next 128 columns are one box (16 KB) further.
-              bdesc = make_desc_mnmajor(sB + k * (W8_UMMA_K * 128), W8_BK * 128);
-            }
-            umma_i8_ss(d, adesc, bdesc, idesc, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < W8_BK / W8_UMMA_K; ++k)
+            umma_i8_ss(d, adesc + (uint64_t)(k * (W8_UMMA_K >> 4)), bdesc + (uint64_t)(k * K_STEP), idesc,
+                       ((kb - kb_begin) | k) != 0 ? 1u : 0u);
           umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&tfull[buf]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
-      if (!ok) {
-        umma_commit(drain);
+      if (ok && elect_one_sync()) umma_commit(&tfull[buf]);  // the elected lane is the same one every time
+    }
+    if (!ok) {
+      if (elect_one_sync()) umma_commit(drain);
+      if (lane == 0) {
         const uint64_t t0 = global_timer_ns();
         while (!mbar_try_wait(drain, 0)) {
           if (global_timer_ns() - t0 > p.wait_limit_ns) break;
