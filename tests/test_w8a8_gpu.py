@@ -238,3 +238,61 @@ def test_empty_inputs_give_empty_outputs():
     P = torch.zeros(64, 64, dtype=torch.uint8, device="cuda")
     C4 = q.w4a16_gemm(torch.zeros(0, 128, dtype=torch.float16, device="cuda"), P, None)
     assert C4.shape == (0, 64)
+
+
+@pytest.mark.parametrize("batch,M,K,N", [
+    (0, 1, 16, 16),          # one CTA, one ragged block
+    (0, 16, 1024, 144),      # K over eight CTAs: shares of four tokens
+    (0, 33, 1040, 4112),     # shares that are no multiple of 16, ragged K and N
+    (0, 64, 2064, 14336),    # a cluster of two
+    (3, 17, 512, 8192),      # one or two CTAs per tile, batched
+    (40, 64, 128, 1024),     # more tiles than CTAs fit at once
+    (0, 129, 1024, 1040), (0, 512, 256, 1024), (2, 300, 272, 256),  # several token tiles
+    (0, 192, 4112, 2064),
+])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+@pytest.mark.parametrize("odt", ["float16", "bfloat16"])
+def test_few_tokens_exact(batch, M, K, N, layout, odt):
+    """The few-token form at the edges of its token tiles and K cuts: bit-exact (an exact integer sum, then one fp32
+    multiplication per scale), with every form of the scales."""
+    q = _q()
+    A, B, sa, sb = oc.make_w8a8_inputs(batch, M, K, N, seed=M + K)
+    Bd = (B if layout == "KN" else B.transpose(-1, -2).contiguous()).cuda()
+    for a, b in ((sa, sb), (None, sb), (sa.reshape(-1)[:M].contiguous(), sb.reshape(-1)[:N].contiguous()),
+                 (None, sb.reshape(-1)[:1].contiguous())):
+        ref = oc.quant_matmul_ref(A, B, b, odt, scale_a=a)
+        C = q.quant_matmul(A.cuda(), Bd, b.cuda(), scale_a=None if a is None else a.cuda(), out_dtype=odt, b_layout=layout)
+        _cmp(C, ref)
+
+
+def test_few_tokens_behind_the_quantiser():
+    """The quantiser lets the product behind it start early: a chain in which each step reads what the step in front has
+    just written - the activations and, [N, K], the weights - gives what the same chain gives with the device drained
+    between the steps."""
+    q = _q()
+    g = torch.Generator().manual_seed(3)
+    X = [torch.randn((48, 2048), generator=g).to(torch.bfloat16).cuda() for _ in range(4)]
+    W = [torch.randn((2048, 2048), generator=g).to(torch.bfloat16).cuda() for _ in range(4)]
+
+    def chain(sync):
+        x = X[0]
+        for i in range(12):
+            b, sb = q.act_quant(W[i % 4])
+            if sync:
+                torch.cuda.synchronize()
+            a, sa = q.act_quant(x)
+            if sync:
+                torch.cuda.synchronize()
+            x = q.quant_matmul(a, b, sb.view(-1), scale_a=sa.view(-1), out_dtype="bfloat16", b_layout="NK") * 0.02
+            if sync:
+                torch.cuda.synchronize()
+            y = q.quant_matmul(a, q.act_quant(W[(i + 1) % 4])[0], sb.view(-1), scale_a=sa.view(-1), out_dtype="bfloat16",
+                               b_layout="NK")
+            if sync:
+                torch.cuda.synchronize()
+            x = x + y * 0.01
+        return x
+
+    ref = chain(True)
+    for _ in range(5):
+        assert torch.equal(chain(False), ref)

@@ -306,6 +306,11 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld_32x32b_x4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Registers -> tensor memory: thread i of the warp writes 32 consecutive 32-bit columns of lane (base lane + i).
@@ -411,6 +416,23 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack_out2(float lo, float hi) {
   return BF16 ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
+}
+
+
+// 16-bit values of four tokens m .. m + 3 and this lane's feature n, as two words (m, m + 1) and (m + 2, m + 3): four
+// neighbouring lanes exchange them, so that each holds four consecutive features of one token.  On return m is this lane's
+// token and n its first feature; a warp's 8-byte stores then cover 64 contiguous bytes of four rows, a quarter of the
+// instructions of storing value by value.  Every lane of the warp takes part.
+__device__ __forceinline__ uint2 transpose_tokens4(int lane, uint32_t w01, uint32_t w23, int& m, int& n) {
+  const bool odd = lane & 1, upper = lane & 2;
+  const uint32_t o01 = __shfl_xor_sync(0xffffffffu, w01, 1), o23 = __shfl_xor_sync(0xffffffffu, w23, 1);
+  // token m + (lane & 1) (and the same of the second pair), features n & ~1, n | 1
+  const uint32_t a = odd ? __byte_perm(o01, w01, 0x7632) : __byte_perm(w01, o01, 0x5410);
+  const uint32_t b = odd ? __byte_perm(o23, w23, 0x7632) : __byte_perm(w23, o23, 0x5410);
+  const uint32_t other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 2);
+  m += (upper ? 2 : 0) + (odd ? 1 : 0);
+  n &= ~3;
+  return upper ? make_uint2(other, b) : make_uint2(a, other);
 }
 
 }  // namespace qg

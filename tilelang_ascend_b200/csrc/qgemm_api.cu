@@ -17,6 +17,7 @@
 #include "act_quant.cuh"
 #include "w4a8.cuh"
 #include "w8a8.cuh"
+#include "w8a8_rows.cuh"
 
 namespace {
 
@@ -112,6 +113,12 @@ int set_smem_w4g() {
 }
 
 // Once per device, with that device current.
+int set_smem_w8r() {
+  if (set_smem(qg::w8a8_rows_kernel<false, false>, qg::W8R_SMEM_BYTES)) return -1;
+  if (set_smem(qg::w8a8_rows_kernel<false, true>, qg::W8R_SMEM_BYTES)) return -1;
+  if (set_smem(qg::w8a8_rows_kernel<true, false>, qg::W8R_SMEM_BYTES)) return -1;
+  return set_smem(qg::w8a8_rows_kernel<true, true>, qg::W8R_SMEM_BYTES);
+}
 int set_smem_w4w() {
   if (set_smem(qg::w4a16_wide_kernel<false, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
   if (set_smem(qg::w4a16_wide_kernel<true, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
@@ -144,7 +151,7 @@ int ensure_device(int* sm_count) {
     if (set_smem_w4<16>()) return -1;
     if (set_smem_w4g<16>() || set_smem_w4g<32>() || set_smem_w4g<64>()) return -1;
     if (set_smem_w4i8<16>() || set_smem_w4i8<32>() || set_smem_w4i8<64>() || set_smem_w4i8<128>()) return -1;
-    if (set_smem_w4w()) return -1;
+    if (set_smem_w8r() || set_smem_w4w()) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
     st.ready.store(true, std::memory_order_release);
@@ -231,6 +238,27 @@ int launch_w8_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, true>, tmA, tmB, tmC, p));
+  return 0;
+}
+
+// Few-token form: clusters of S CTAs, a programmatic dependent of whatever is in front of it on the stream.
+template <bool NK, bool BF>
+int launch_w8_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const qg::W8RowsParams& p, int grid, int S, cudaStream_t s) {
+  static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(qg::W8_THREADS);
+  cfg.dynamicSmemBytes = (size_t)qg::W8R_SMEM_BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_rows_kernel<NK, BF>, tmA, tmB, p));
   return 0;
 }
 
@@ -508,6 +536,50 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   if (ensure_device(&sms)) return -1;
 
   CUtensorMap tmA, tmB;
+  // Few tokens (w8a8_rows.cuh), and what would leave most SMs idle: up to 128 tokens; up to 32 tiles of 128 x 128; 192 tokens
+  // from K = 4096 on.  us, this form against the other, [N, K] weights, K x N: 16 tokens 4096 x 14336 14.3 / 22.6, 8192 x 8192
+  // 15.4 / 26.6, 1024 x 1024 4.5 / 8.2; 128 tokens 17.8 / 20.5, 19.7 / 26.7, 6.6 / 8.2; 192 tokens 20.5 / 22.6, 22.1 / 26.7
+  // and, K = 1024 .. 2048, 10.8 / 10.3 and 9.9 / 9.4; 256 tokens 22.4 / 22.7, 2048 x 4096 11.6 / 10.3, 1024 x 1024 6.8 / 8.2
+  // (16 tiles; 512 tokens, 32 tiles: 7.2 / 8.2).
+  const int64_t rows_m_tiles = (M + qg::W8R_MAX_MT - 1) / qg::W8R_MAX_MT, rows_n_tiles = (N + 127) / 128;
+  const bool rows_shape = M <= 128 || batch * rows_m_tiles * rows_n_tiles <= 32 || (M <= 192 && K >= 4096);
+  if (rows_shape && meta == nullptr && acc_out == nullptr) {
+    const int64_t n_tiles = rows_n_tiles, m_tiles = rows_m_tiles, k_blocks = (K + 127) / 128, tiles = batch * n_tiles * m_tiles;
+    if (tiles > 0x7fffffff / qg::W8R_MAX_SPLIT) return fail("qgemm_w8a8: too many tiles");
+    // K is cut until two CTAs per SM are at work, each with two 128-k blocks at least
+    int S = 1;
+    while (S < qg::W8R_MAX_SPLIT && tiles * 2 * S <= 2 * sms && k_blocks >= 4 * S) S *= 2;
+    const int unit = S == 8 ? 32 : 16;
+    qg::W8RowsParams p;
+    p.scale_b = scale_b;
+    p.scale_a = scale_a;
+    p.C = C;
+    p.M = (int)M;
+    p.N = (int)N;
+    p.sb_mode = (scale_b_len == 1) ? 0 : ((scale_b_len == N) ? 1 : 2);
+    p.sa_mode = (scale_a == nullptr) ? 0 : ((scale_a_len == M) ? 1 : 2);
+    p.n_tiles = (int)n_tiles;
+    p.k_blocks = (int)k_blocks;
+    p.m_tiles = (int)m_tiles;
+    p.mt = (int)(((M + m_tiles - 1) / m_tiles + unit - 1) / unit * unit);
+    p.tmem_cols = p.mt <= 32 ? 32 : (p.mt <= 64 ? 64 : 128);
+    p.status = status;
+    p.wait_limit_ns = g_wait_limit_ns;
+    const uint64_t dims_a[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batch};
+    const uint64_t str_a[2] = {(uint64_t)K, (uint64_t)M * (uint64_t)K};
+    const uint32_t box_a[3] = {128, (uint32_t)p.mt, 1};
+    if (encode_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, A, dims_a, str_a, box_a, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    const bool nk = b_layout == QGEMM_B_NK;
+    const uint64_t dims_b[3] = {(uint64_t)(nk ? K : N), (uint64_t)(nk ? N : K), (uint64_t)batch};
+    const uint64_t str_b[2] = {(uint64_t)(nk ? K : N), (uint64_t)N * (uint64_t)K};
+    const uint32_t box_b[3] = {128, 128, 1};
+    if (encode_map(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, B, dims_b, str_b, box_b, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    const int grid = (int)(tiles * S);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const bool bf = out_dtype == QGEMM_DT_BF16;
+    if (nk) return bf ? launch_w8_rows<true, true>(tmA, tmB, p, grid, S, s) : launch_w8_rows<true, false>(tmA, tmB, p, grid, S, s);
+    return bf ? launch_w8_rows<false, true>(tmA, tmB, p, grid, S, s) : launch_w8_rows<false, false>(tmA, tmB, p, grid, S, s);
+  }
   {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batchA};
     const uint64_t str[2] = {(uint64_t)K, (uint64_t)M * (uint64_t)K};

@@ -51,20 +51,12 @@ struct W4WideCfg {
   static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
 };
 
-// 16-bit outputs of four tokens m .. m + 3 and this lane's output feature n, as two f16x2 / bf16x2 words (m, m + 1) and
-// (m + 2, m + 3): four neighbouring lanes exchange them, so that each stores four consecutive features of one token (a
-// warp's store instruction covers 64 contiguous bytes of four rows, a quarter of the instructions of storing values one
-// by one while the accumulator waits).  Every lane takes part; N, ldc and col0 are multiples of 8.
+// 16-bit outputs of four tokens m .. m + 3 and this lane's output feature n (see transpose_tokens4; N, ldc and col0 are
+// multiples of 8).
 __device__ __forceinline__ void w4w_store_tokens4(const W4A16Params& p, uint16_t* Cout, int m, int n, int lane, uint32_t w01,
                                                   uint32_t w23) {
-  const bool odd = lane & 1, upper = lane & 2;
-  const uint32_t o01 = __shfl_xor_sync(0xffffffffu, w01, 1), o23 = __shfl_xor_sync(0xffffffffu, w23, 1);
-  // token m + (lane & 1) (and the same of the second pair), features n & ~1, n | 1
-  const uint32_t a = odd ? __byte_perm(o01, w01, 0x7632) : __byte_perm(w01, o01, 0x5410);
-  const uint32_t b = odd ? __byte_perm(o23, w23, 0x7632) : __byte_perm(w23, o23, 0x5410);
-  const uint32_t other = __shfl_xor_sync(0xffffffffu, upper ? a : b, 2);
-  const uint2 v = upper ? make_uint2(other, b) : make_uint2(a, other);
-  const int row = m + (upper ? 2 : 0) + (odd ? 1 : 0), col = n & ~3;
+  int row = m, col = n;
+  const uint2 v = transpose_tokens4(lane, w01, w23, row, col);
   if (row >= p.M || col >= p.N) return;
   if (p.n_dst == 0) {
     *reinterpret_cast<uint2*>(Cout + (size_t)row * p.N + col) = v;
