@@ -572,3 +572,25 @@ def test_wide_tiles(M, K, N, group, zeros, dt):
     assert call(small - 1) != 0  # refused
     assert call(small) == 0, _lib.last_error()
     assert bool(((C2.cpu().double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("K", [96, 160, 192, 224])
+@pytest.mark.parametrize("M,mode", [(70, None), (1800, None), (5, "original"), (33, "rescale"), (70, "quantized")])
+def test_one_group_shorter_than_a_slab(K, M, mode):
+    """One group of the whole K, K below a slab of 256 and no divisor of it, on the wide tiles: only the scale rows that
+    were fetched may be read.  A call before it leaves NaN in the places where further rows would be."""
+    q = _q()
+    N, g = 272, torch.Generator().manual_seed(K + M)
+    junk = [t.cuda() for t in oc.make_w4a16_inputs(70, 256, 148 * 128, "float16", 32, seed=1)]
+    nan = torch.full_like(junk[2], float("nan"))
+    q.w4a16_gemm(junk[0], junk[1], nan, nan, 32, zeros_mode="original")
+    q.w4a16_gemm(junk[0], junk[1], nan, 8, 32)
+    A, P, S = oc.make_w4a16_inputs(M, K, N, "float16", K, seed=K)
+    if mode is None:
+        W, zeros = oc.dequant_weight_ref(P, S, 8, K), 8
+        C = q.w4a16_gemm(A.cuda(), P.cuda(), S.cuda(), 8, K)
+    else:
+        zeros = torch.randint(0, 16, (1, N), generator=g).half()
+        W = oc.dequant_weight_zeros_ref(P, S, zeros, K, mode)
+        C = q.w4a16_gemm(A.cuda(), P.cuda(), S.cuda(), zeros.cuda(), K, zeros_mode=mode)
+    _close(C, (A.float() @ W.float().t()).half())

@@ -913,10 +913,13 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
     const uint32_t box[3] = {128, 128, 1};
     if (encode_map(&tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, B_packed, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   }
+  // One group for a K below a slab: to the other kernels that is one scale row for the whole slab, whatever K is (256 / K rows
+  // are fewer than the K / 32 that a slab's chunks would be dealt to, and those beyond are never fetched).
+  const int64_t row_k = !use_gs && group >= K && group < 256 ? 256 : group;
   // the group-sum kernel fetches the scale rows of a slab's two 128-k halves: two rows for groups of 128, else one
   int scale_rows = 1;
   if (scales != nullptr) {
-    scale_rows = use_gs ? (group == 128 ? 2 : 1) : (group < 256 ? (int)(256 / group) : 1);
+    scale_rows = use_gs ? (group == 128 ? 2 : 1) : (row_k < 256 ? (int)(256 / row_k) : 1);
     const uint64_t dims[3] = {(uint64_t)N, (uint64_t)(K / group), (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)N * 2, (uint64_t)(K / group) * (uint64_t)N * 2};
     const uint32_t box[3] = {128, (uint32_t)scale_rows, 1};
@@ -949,7 +952,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.M = (int)M;
   p.N = (int)N;
   p.K = (int)K;
-  p.group = (int)(group > (1 << 30) ? (1 << 30) : group);
+  p.group = (int)(row_k > (1 << 30) ? (1 << 30) : row_k);
   p.zero = zero;
   p.has_scales = scales != nullptr;
   p.m_tiles = (int)((M + mt - 1) / mt);
