@@ -278,7 +278,7 @@ int qgemm_peer_signal_wait(void* const* flag_slots, int n, const uint32_t* local
  */
 #define QGEMM_W4A16_NOALLOC_MAX_M 32
 #define QGEMM_W4A16_NOALLOC_MAX_K 16384
-#define QGEMM_W4A16_NOALLOC_SCRATCH_MB 6.4
+#define QGEMM_W4A16_NOALLOC_SCRATCH_MB 6.3
 int qgemm_w4a16_noalloc(const void* A, const uint8_t* B_packed, const void* scales, int zero, int64_t group,
                         void* C, int64_t M, int64_t N, int64_t K, int a_dtype, int out_dtype, uint32_t* status,
                         void* stream);

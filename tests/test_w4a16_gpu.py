@@ -594,3 +594,40 @@ def test_one_group_shorter_than_a_slab(K, M, mode):
         W = oc.dequant_weight_zeros_ref(P, S, zeros, K, mode)
         C = q.w4a16_gemm(A.cuda(), P.cuda(), S.cuda(), zeros.cuda(), K, zeros_mode=mode)
     _close(C, (A.float() @ W.float().t()).half())
+
+
+def _float64_ref(A, packed, scales, zeros, group):
+    """C and the sum of the terms' magnitudes in float64: sum over k of a * (q - zero) * s, zeros an int or [K/g, N]."""
+    qv = oc.unpack_uint4(packed).double()  # [N, K]
+    z = zeros if isinstance(zeros, int) else zeros.double().t().repeat_interleave(group, 1)
+    W = (qv - z) * scales.double().t().repeat_interleave(group, 1)
+    A = A.half().double()
+    return A @ W.t(), A.abs() @ W.abs().t()
+
+
+@pytest.mark.parametrize("M,K,group,zeros,dt", [
+    (1, 1024, 128, 8, "float16"), (16, 1024, 1024, 3, "bfloat16"),  # the single-launch form
+    (5, 8192, 128, 8, "float16"), (24, 1024, 256, 15, "float16"), (64, 1024, 128, 8, "bfloat16"),  # pre-pass, three tile heights
+    (16, 1024, 128, None, "float16"), (24, 1024, 1024, None, "bfloat16"), (40, 2048, 128, None, "float16"),  # zero tensors
+])
+def test_large_activations_at_the_zero_point(M, K, group, zeros, dt):
+    """Large activations that face weights at the zero point contribute nothing, so they must not cost the other terms
+    precision: (q - zero) is formed exactly before anything is multiplied.  Bar: the rounding of the output (8 or 11 bits)
+    and of an fp32 sum of K terms, K * 2^-24 of the sum of the terms' magnitudes."""
+    q = _q()
+    N = 264 if zeros is not None else 272
+    g = torch.Generator().manual_seed(M + K)
+    A = (torch.randn((M, K), generator=g) * 0.02).to(getattr(torch, dt))
+    A[:, 5::64] = torch.tensor([60000.0, -31000.0]).repeat(K // 128).to(A.dtype)
+    nib = torch.randint(0, 16, (N, K), generator=g)
+    z = torch.full((K // group, N), zeros) if zeros is not None else torch.randint(0, 16, (K // group, N), generator=g)
+    nib[:, 5::64] = z.t().repeat_interleave(group, 1)[:, 5::64]
+    packed = (nib[:, 0::2] | (nib[:, 1::2] << 4)).to(torch.uint8)
+    scales = (torch.rand((K // group, N), generator=g) * 0.02 + 0.005).half()
+    zt = zeros if zeros is not None else z.half()
+    ref, mag = _float64_ref(A, packed, scales, zt, group)
+    C = q.w4a16_gemm(A.cuda(), packed.cuda(), scales.cuda(), zt if zeros is not None else zt.cuda(), group,
+                     zeros_mode="original" if zeros is not None else "quantized")
+    bound = ref.abs() * 2.0 ** (-11 if dt == "float16" else -8) + mag * (K * 2.0 ** -24) + 1e-7
+    err = (C.cpu().double() - ref).abs()
+    assert (err <= bound).all(), (err / bound).max().item()

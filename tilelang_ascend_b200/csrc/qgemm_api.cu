@@ -968,10 +968,6 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.wait_limit_ns = g_wait_limit_ns;
   p.A_raw = nullptr;
   p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
-  p.A_src = A;
-  p.W_src = B_packed;
-  p.S_src = static_cast<const uint16_t*>(scales);
-  p.Z_src = static_cast<const uint16_t*>(zeros);
   p.w_interleaved = weight_format == QGEMM_W4_SEQUENTIAL ? 0 : 1;
   int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   if (p.total_items < grid) grid = p.total_items;
@@ -1285,7 +1281,7 @@ constexpr int64_t kStaticMaxM = QGEMM_W4A16_NOALLOC_MAX_M;
 constexpr int64_t kStaticMaxK = QGEMM_W4A16_NOALLOC_MAX_K;
 constexpr int64_t kStaticMaxSms = 160;
 constexpr int64_t kStaticScratchBytes =
-    kW4CounterBytes + kStaticMaxSms * 2 * kStaticMaxM * 128 * 4 + (kStaticMaxK / 128) * qg::w4g_half_bytes(kStaticMaxM);  // about 6.4 MB
+    kW4CounterBytes + kStaticMaxSms * 2 * kStaticMaxM * 128 * 4 + (kStaticMaxK / 128) * qg::w4g_half_bytes(kStaticMaxM);  // about 6.3 MB
 
 static __device__ __align__(256) unsigned char g_w4a16_static_scratch[kStaticScratchBytes];
 

@@ -50,10 +50,6 @@ struct W4A16Params {
   // activations [batch, M, K] and whether they are bf16; and whether the weight layout is the interleaved one.
   const void* A_raw;
   int a_is_bf16, w_interleaved;
-  // Group-sum kernel: the caller's tensors, read only where a sum came out NaN (see w4g_store_checked).
-  const void* A_src;
-  const uint8_t* W_src;
-  const uint16_t *S_src, *Z_src;
   int scale_rows;       // scale rows fetched per slab (256 / group, at least 1)
   long long total_items;
   uint32_t* status;

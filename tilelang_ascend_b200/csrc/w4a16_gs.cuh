@@ -7,15 +7,16 @@
 //
 // What bounds these shapes is not memory but the number of instructions and hand-overs an SM spends per 16 KB slab of
 // packed weights (a slab's HBM time is about 700 cycles per SM), so the kernel is built to spend few:
-//  - Conversion in five integer instructions per eight weights, no arithmetic at all.  A nibble q in bits 0..3 of an f16
-//    word IS the number q * 2^-24 (a subnormal), one in bits 4..7 is q * 2^-20, and the tensor core takes subnormals at
-//    full precision; so masking is converting: x & 0x000f000f, x & 0x00f000f0, and the same of x >> 8.  The MMAs of a
-//    128-k half first sum the "high" words (16 times too large), then the "low" ones, the first of which scales what has
-//    been accumulated by 2^-4 (tcgen05.mma's scale-input-d): exact, as is the factor 2^24 that the group scale carries.
-//  - The zero point enters as one more MMA per half: a constant weight column -zero against the activations' sum over the
-//    half, which the pre-pass provides as three f16 parts (about 33 bits, see w4g_sum_parts).
-//  - Activations are laid out by the pre-pass in the exact image of a shared-memory stage (swizzle, K order, sum
-//    columns), so that a stage is one untiled bulk copy.
+//  - Conversion in nine instructions per eight weights: masking a nibble and setting an exponent around it in one lop3, so
+//    that q in the low bits of 1024 is 1024 + q and q above the low four bits of 64 is 64 + q, and one f16 subtraction of
+//    1024 + zero or 64 + zero: (q - zero), exactly.  (Leaving the zero point to the end - masked nibbles as subnormals, five
+//    instructions, and one more MMA that takes zero * sum(A) off the accumulator - is no faster: 16 x 4096 x 4096 9.4 us
+//    against 8.5, 32 of them in one call 73.4 / 71.3, 1, 32 and 64 tokens of 8192 x 28672 25.2 / 24.9, 31.4 / 29.8 and
+//    40.8 / 40.5; only raw nibbles, 64 tokens, 38.0 / 39.5.  And a large
+//    activation at a weight equal to zero then costs all other terms of the half their low bits: 18 to 400 times the
+//    bound of test_large_activations_at_the_zero_point; an infinite one makes the difference NaN.)
+//  - Activations are laid out by the pre-pass in the exact image of a shared-memory stage (swizzle, K order), so that a
+//    stage is one untiled bulk copy.
 //  - All hand-overs are by whole slabs; one commit per slab signals one barrier that the weight stage, the activation
 //    stage and the accumulators share; the group scales arrive with the packed bytes and need no barrier of their own.
 //
@@ -57,7 +58,6 @@ constexpr int W4G_THREADS = (W4G_FIN_WARP + 4) * 32;               // 768: at mo
 constexpr int W4G_SLAB_COLS = 128;  // tensor-memory columns of a converted slab
 constexpr int W4G_SC_BYTES = 512;   // a slab's scales: up to two rows of 128 halves
 constexpr int W4G_BARS = 8;         // barriers of a ring (whatever the number of data stages behind it), indexed by slab % 8
-constexpr int W4G_Z_BYTES = 2048;   // the zero point's operand: 128 rows x 8 k of f16 (k 8 .. 15 are one shared tile of zeros)
 
 // Byte offsets of the barriers (8 bytes each) and control words from the start of the barrier block.
 constexpr int W4G_RAW_FULL = 0;       // [8] a slab's packed weights (and scale rows) have landed
@@ -76,9 +76,8 @@ constexpr int W4G_CTL = 520;          // u32 abort word (0, or the role code of 
 constexpr int W4G_FIN_WORD = 528;     // u32[2], one per partial tile: its arrival number
 constexpr int W4G_SMALL_MAX_SLABS = 4;  // SMALL form: slabs per CTA (stages 4.. of the raw ring receive the other CTAs' sums)
 
-// Bytes of one prepared activation half: MT rows x 128 k of f16 (two 128-byte-swizzled blocks of 64 k), then the MT x 16
-// sum columns as 8-row x 16-byte core matrices, padded to the 1024 bytes from which the swizzle counts.
-__host__ __device__ constexpr int w4g_half_bytes(int mt) { return (mt * 256 + mt * 32 + 1023) / 1024 * 1024; }
+// Bytes of one prepared activation half: MT rows x 128 k of f16 (two 128-byte-swizzled blocks of 64 k).
+__host__ __device__ constexpr int w4g_half_bytes(int mt) { return mt * 256; }
 
 template <int MT, bool ZT = false>
 struct W4GCfg {
@@ -97,9 +96,8 @@ struct W4GCfg {
   // halves - otherwise both sets convert while the tensor pipe idles and then both wait for it.
   static constexpr bool HALVES = MT == 64;
   static constexpr int XBUF_BYTES = MT * W4_BN * 4;       // the second drain set's sums of one segment
-  static constexpr int Z_STAGES = ZT ? 2 * WS : 1;        // a zeros tensor changes the operand tile with every half
   static constexpr int SMEM_BYTES = RS * W4_RAW_PACKED + AS * A_BYTES + SS * W4G_SC_BYTES + (ZT ? RS * W4G_SC_BYTES : 0) +
-                                    (Z_STAGES + 1) * W4G_Z_BYTES + XBUF_BYTES + BAR_BYTES + 1024;
+                                    XBUF_BYTES + BAR_BYTES + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
   static_assert(NS * 2 * MT + WS * W4G_SLAB_COLS <= 512 && (RS & (RS - 1)) == 0 && NS % 2 == 0 && AS < W4G_BARS, "layout");
 };
@@ -184,21 +182,6 @@ __device__ __forceinline__ void w4g_fma2(float& d0, float& d1, uint32_t a0, uint
 // Named barrier of the eight drain warps.
 __device__ __forceinline__ void w4g_epi_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-
-// D = A * B + D * 2^-4, A from tensor memory (see the header comment: the step from the high to the low nibble words).
-__device__ __forceinline__ void w4g_mma_ts_shift4(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, 4;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc)
-      : "memory");
-}
-// Matrix descriptor of an unswizzled operand of 16 k: core matrices of 8 rows x 16 bytes, the two k halves of a row group
-// `k_stride` bytes apart, row groups `row_stride` bytes apart.
-__device__ __forceinline__ uint64_t w4g_desc_k16(uint32_t saddr, uint32_t k_stride, uint32_t row_stride) {
-  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(k_stride >> 4) << 16) |
-         (static_cast<uint64_t>(row_stride >> 4) << 32) | (static_cast<uint64_t>(1) << 46);
-}
 // Untiled bulk copy global -> shared memory.
 __device__ __forceinline__ void w4g_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -241,60 +224,23 @@ __device__ __forceinline__ uint4 w4g_to_f16(uint4 v, bool is_bf16) {
   }
   return v;
 }
-__device__ __forceinline__ float w4g_sum8(const uint4& v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-    s += f.x + f.y;
-  }
-  return s;
-}
-// The half's sum S as f16 parts p0 * 2^7 + p1 + p2: p0 takes the leading 11 bits (scaled, because S may exceed f16's
-// range), p1 and p2 the next 22; the remainder is below 2^-33 |S| or below f16's own granularity 2^-24, whichever is larger.
-__device__ __forceinline__ uint2 w4g_sum_parts(float S) {
-  const __half p0 = __float2half_rn(S * 0.0078125f);
-  const float r0 = S - __half2float(p0) * 128.0f;
-  const __half p1 = __float2half_rn(r0);
-  const __half p2 = __float2half_rn(r0 - __half2float(p1));
-  return make_uint2((uint32_t)__half_as_ushort(p0) | ((uint32_t)__half_as_ushort(p1) << 16), (uint32_t)__half_as_ushort(p2));
-}
-// The weights that face them: -zero in units of 2^-24, the first one times 2^7 (0 <= zero <= 15: exact in f16).
-__device__ __forceinline__ uint2 w4g_zero_weights(float zero) {
-  const uint32_t a = __half_as_ushort(__float2half_rn(-zero * 7.62939453125e-6f));     // 2^-17
-  const uint32_t b = __half_as_ushort(__float2half_rn(-zero * 5.9604644775390625e-8f));  // 2^-24
-  return make_uint2(a | (b << 16), b);
-}
 // Byte offset of 16-byte piece j (0..15) of row r inside a half's image: 64-k block j / 8, 128-byte swizzle.
 template <int MT>
 __device__ __forceinline__ uint32_t w4g_a_offset(int r, int j) {
   return (uint32_t)((j >> 3) * (MT * 128) + r * 128 + (((j & 7) ^ (r & 7)) << 4));
 }
-__device__ __forceinline__ uint32_t w4g_core_offset(int r) { return (uint32_t)((r >> 3) * 256 + (r & 7) * 16); }
 
 // One 32-k chunk (chunk c of four) of row r: four 16-byte loads already in v -> the half's image at dst (global or shared
-// memory).  Four consecutive lanes hold the four chunks of a row's half; the first one writes the sum columns.
+// memory).
 template <int MT>
 __device__ __forceinline__ void w4g_emit_chunk(uint8_t* dst, int r, int c, const uint4 (&v)[4]) {
   uint2 lo[4], hi[4];
-  float s = 0.f;
 #pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    w4g_split_word(v[w], lo[w], hi[w]);
-    s += w4g_sum8(v[w]);
-  }
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  for (int w = 0; w < 4; ++w) w4g_split_word(v[w], lo[w], hi[w]);
   *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 0)) = make_uint4(lo[0].x, lo[0].y, lo[1].x, lo[1].y);
   *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 1)) = make_uint4(lo[2].x, lo[2].y, lo[3].x, lo[3].y);
   *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 2)) = make_uint4(hi[0].x, hi[0].y, hi[1].x, hi[1].y);
   *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 3)) = make_uint4(hi[2].x, hi[2].y, hi[3].x, hi[3].y);
-  if (c == 0) {
-    const uint2 p = w4g_sum_parts(s);
-    *reinterpret_cast<uint4*>(dst + MT * 256 + w4g_core_offset(r)) = make_uint4(p.x, p.y, 0u, 0u);
-    *reinterpret_cast<uint4*>(dst + MT * 256 + w4g_core_offset(r) + 128) = make_uint4(0u, 0u, 0u, 0u);
-  }
 }
 
 // Pre-pass: activations [batch, M, K] (f16 or bf16) -> [batch][token tile][half] images (rows beyond M and k beyond K are
@@ -316,7 +262,7 @@ w4g_prepare_activations(const uint4* __restrict__ in, uint8_t* __restrict__ out,
   pdl_wait();  // the kernel in front (another call's GEMM, which lets its dependents start early) is done
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < n_counters; k += blockDim.x) counters[k] = 0u;
-  if (b >= batch) return;  // whole groups of four lanes; the grid is a multiple of MT * 4 threads, so whole warps too
+  if (b >= batch) return;
   const int m = tile * MT + r, k0 = half * 128 + c * 32;
   uint4 v[4];
 #pragma unroll
@@ -331,77 +277,60 @@ w4g_prepare_activations(const uint4* __restrict__ in, uint8_t* __restrict__ out,
   w4g_emit_chunk<MT>(out + (size_t)blk * w4g_half_bytes(MT), r, c, v);
 }
 
-// Sixteen packed bytes (32 weights) -> eight f16x2 words of low values (units of 2^-24), eight of high values (units of
-// 2^-20), K order as in w4g_split_word.  Sequential layout: five integer instructions per eight weights.  Interleaved
-// layout (nibbles 0 2 4 6 | 1 3 5 7): eight, into the same words, so that both layouts give the same sums bit for bit.
+// Sixteen packed bytes (32 weights) -> eight f16x2 words of the low nibbles' q - zero, then eight of the high ones', K order
+// as in w4g_split_word.  lo_sub = 1024 + zero, hi_sub = 64 + zero (both f16x2): every sum and difference here is exact.
+// Interleaved layout (nibbles 0 2 4 6 | 1 3 5 7): three more instructions per eight weights, the same words, so that both
+// layouts give the same sums bit for bit.
+__device__ __forceinline__ uint32_t w4g_lo2(uint32_t x, uint32_t lo_sub) {
+  uint32_t o;
+  asm("lop3.b32 %0, %1, 0x000f000f, 0x64006400, 0xea;" : "=r"(o) : "r"(x));
+  asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(o) : "r"(lo_sub));
+  return o;
+}
+__device__ __forceinline__ uint32_t w4g_hi2(uint32_t x, uint32_t hi_sub) {
+  uint32_t o;
+  asm("lop3.b32 %0, %1, 0x00f000f0, 0x54005400, 0xea;" : "=r"(o) : "r"(x));
+  asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(o) : "r"(hi_sub));
+  return o;
+}
 template <bool INTERLEAVED>
-__device__ __forceinline__ void w4g_convert(const uint4& v, uint32_t (&o)[16]) {
+__device__ __forceinline__ void w4g_convert(const uint4& v, uint32_t lo_sub, uint32_t hi_sub, uint32_t (&o)[16]) {
   const uint32_t x[4] = {v.x, v.y, v.z, v.w};
   if constexpr (!INTERLEAVED) {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const uint32_t y = x[w] >> 8;
-      o[2 * w] = x[w] & 0x000f000fu;
-      o[2 * w + 1] = y & 0x000f000fu;
-      o[8 + 2 * w] = x[w] & 0x00f000f0u;
-      o[8 + 2 * w + 1] = y & 0x00f000f0u;
+      o[2 * w] = w4g_lo2(x[w], lo_sub);
+      o[2 * w + 1] = w4g_lo2(y, lo_sub);
+      o[8 + 2 * w] = w4g_hi2(x[w], hi_sub);
+      o[8 + 2 * w + 1] = w4g_hi2(y, hi_sub);
     }
   } else {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const uint32_t ev = __byte_perm(x[w], 0u, 0x4140), od = __byte_perm(x[w], 0u, 0x4342);  // (0 2 | 4 6), (1 3 | 5 7)
-      o[2 * w] = ev & 0x000f000fu;
-      o[2 * w + 1] = (ev >> 4) & 0x000f000fu;
-      o[8 + 2 * w] = (od << 4) & 0x00f000f0u;
-      o[8 + 2 * w + 1] = od & 0x00f000f0u;
+      o[2 * w] = w4g_lo2(ev, lo_sub);
+      o[2 * w + 1] = w4g_lo2(ev >> 4, lo_sub);
+      o[8 + 2 * w] = w4g_hi2(od << 4, hi_sub);
+      o[8 + 2 * w + 1] = w4g_hi2(od, hi_sub);
     }
   }
 }
-
-// Output (b, m, n) once more, straight from its definition, when its sum came out NaN.  Subtracting zero * sum(A) turns an
-// infinite activation into inf - inf for every output feature, where (q - zero) * inf is +inf, -inf or, for q == zero,
-// NaN; an activation that is not finite makes the sum above NaN in every case, so NaN is what to look for.  One compare
-// per output on the ordinary path; the loop here is slow and runs for rows that hold an infinity or a NaN only.
-template <bool OUT_BF16, bool GATHER>
-__device__ __forceinline__ void w4g_redo_output(const W4A16Params& p, int b, int m, int n) {
-  const uint16_t* a = reinterpret_cast<const uint16_t*>(p.A_src) + ((size_t)b * p.M + m) * (size_t)p.K;
-  const uint8_t* w = p.W_src + ((size_t)b * p.N + n) * (size_t)(p.K / 2);
-  const int group = min(p.group, p.K), groups = p.K / group;
-  float sum = 0.f;
-#pragma unroll 1
-  for (int g = 0; g < groups; ++g) {
-    const size_t at = ((size_t)b * groups + g) * (size_t)p.N + n;
-    const float zero = p.Z_src != nullptr ? __half2float(__ushort_as_half(p.Z_src[at])) : (float)p.zero;
-    const float scale = p.has_scales ? __half2float(__ushort_as_half(p.S_src[at])) : 1.0f;
-    float part = 0.f;
-#pragma unroll 1
-    for (int k = g * group; k < (g + 1) * group; ++k) {
-      // interleaved layout: a word's nibbles are elements 0 2 4 6 1 3 5 7
-      const int e = k & 7, nib = p.w_interleaved ? (k - e) + (e >> 1) + 4 * (e & 1) : k;
-      const int q = (w[nib >> 1] >> (4 * (nib & 1))) & 15;
-      const uint32_t raw = a[k];
-      const uint32_t h = p.a_is_bf16 ? (w4_bf16x2_to_f16x2(raw) & 0xffffu) : raw;
-      part += __half2float(__ushort_as_half((uint16_t)h)) * ((float)q - zero);
-    }
-    sum += scale * part;
-    if (sum != sum) break;
-  }
-  w4_store_out<OUT_BF16, GATHER>(p, reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N, m, n, sum);
+// What w4g_convert takes for a zero point z, an integer as f16 in both halves of z2: 1024 + z and 64 + z.
+__device__ __forceinline__ uint2 w4g_zero_subs(uint32_t z2) {
+  uint2 s;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(s.x) : "r"(0x64006400u), "r"(z2));
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(s.y) : "r"(0x54005400u), "r"(z2));
+  return s;
 }
 
 // The sums of tokens m0 .. m0 + MT - 1 (those below M) of output feature n.
 template <int MT, bool OUT_BF16, bool GATHER>
-__device__ __forceinline__ void w4g_store_checked(const W4A16Params& p, int b, int m0, int n, const float (&sum)[MT]) {
+__device__ __forceinline__ void w4g_store_tile(const W4A16Params& p, int b, int m0, int n, const float (&sum)[MT]) {
   uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
-  uint64_t redo = 0;
 #pragma unroll
-  for (int j = 0; j < MT; ++j) {
-    const int m = m0 + j;
-    if (m < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m, n, sum[j]);
-    if (sum[j] != sum[j] && m < p.M) redo |= 1ull << j;
-  }
-#pragma unroll 1
-  for (; redo != 0; redo &= redo - 1) w4g_redo_output<OUT_BF16, GATHER>(p, b, m0 + __ffsll((long long)redo) - 1, n);
+  for (int j = 0; j < MT; ++j)
+    if (m0 + j < p.M) w4_store_out<OUT_BF16, GATHER>(p, Cout, m0 + j, n, sum[j]);
 }
 
 // GATHER = true is the gathered form (several destination buffers, see W4A16Params::c_dst); it is a separate
@@ -409,7 +338,7 @@ __device__ __forceinline__ void w4g_store_checked(const W4A16Params& p, int b, i
 // ZT = true: one integer zero point per (group, output feature) instead of the scalar one - the zeros tensor
 // [K/g, N] f16 of zero mode "quantized" (tilelang/quantize/lop3.py:325-358: (q - qz) * s with the subtraction
 // exact).  The weight producer fetches the slab's zero rows (through tmZ, laid out like the scale rows) into a ring
-// that shares the packed weights' stages and barriers, and a dequant thread writes its row of the half's zero operand.
+// that shares the packed weights' stages and barriers, and a dequant thread takes its row's zero point from there.
 // SMALL = true (16-token tile): the single-launch form for problems of a few slabs per CTA.  The kernel is launched in
 // clusters of C = KS / (slabs per CTA) CTAs, one tile per cluster, CTA r taking the r-th K range; there is no pre-pass
 // and no scratch memory:
@@ -437,8 +366,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* raw_base = smem;
   uint8_t* a_base = raw_base + RS * W4_RAW_PACKED;
-  uint8_t* zop_base = a_base + AS * Cfg::A_BYTES;        // the zero point's operand tile(s)
-  uint8_t* sc_base = zop_base + (Cfg::Z_STAGES + 1) * W4G_Z_BYTES;
+  uint8_t* sc_base = a_base + AS * Cfg::A_BYTES;
   uint8_t* z_base = sc_base + Cfg::SS * W4G_SC_BYTES;     // zero rows, one 512-byte stage per raw stage (ZT only)
   float* xbuf = reinterpret_cast<float*>(z_base + (ZT ? RS * W4G_SC_BYTES : 0));
   uint8_t* bar_block = reinterpret_cast<uint8_t*>(xbuf) + Cfg::XBUF_BYTES;
@@ -482,13 +410,6 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
   }
-  // the zero point's operand: k = 0 .. 2 face the parts of the activation sums, all other k are zero
-  for (int i = (int)threadIdx.x - 128; i >= 0 && i < (Cfg::Z_STAGES + 1) * 128; i += W4G_THREADS - 128) {
-    uint2 w = make_uint2(0u, 0u);
-    if (i < 128 && !ZT) w = w4g_zero_weights((float)p.zero);
-    *reinterpret_cast<uint4*>(zop_base + (i >> 7) * W4G_Z_BYTES + (i & 127) * 16) = make_uint4(w.x, w.y, 0u, 0u);
-  }
-  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -621,10 +542,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint64_t desc0 = make_desc_kmajor(smem_u32(a_base));
     const uint32_t desc_hi = (uint32_t)(desc0 >> 32);
     const uint32_t desc_lo0 = (uint32_t)desc0;
-    const uint64_t sdesc0 = w4g_desc_k16(smem_u32(a_base) + MT * 256, 128, 256);
-    const uint32_t zop0 = smem_u32(zop_base);
     const int withhold_i = (dbg.withhold_last_commit == 1 && cta == G - 1) ? n_slabs - 1 : -1;
-    const bool has_zero = ZT || p.zero != 0;
     uint32_t fail = 0;
     int as = w % AS, ws = w % WS;
     for (int i = w; i < n_slabs; i += W4G_MMA_WARPS) {
@@ -637,20 +555,11 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       const uint32_t a_off = (uint32_t)((as * Cfg::A_BYTES) >> 4);
       auto issue_half = [&](auto half_) {
         constexpr int half = decltype(half_)::value;
-        // chunk c of the half: tensor-memory columns 16 c .. 16 c + 7 low words, + 8 .. + 15 high words
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int k16 = j < 4 ? 2 * j + 1 : 2 * (j - 4);  // K steps 1 3 5 7 (high), then 0 2 4 6 (low)
+        for (int k16 = 0; k16 < 8; ++k16) {
           const uint32_t off = (uint32_t)((half * Cfg::A_HALF + (k16 >> 2) * (MT * 128) + (k16 & 3) * 32) >> 4);
           const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(desc_lo0 + a_off + off);
-          const uint32_t ta = tW + half * (W4G_SLAB_COLS / 2) + k16 * 8;
-          if (j == 4) w4g_mma_ts_shift4(d + half * MT, ta, bd, idesc);
-          else umma_f16_ts(d + half * MT, ta, bd, idesc, j != 0 ? 1u : 0u);
-        }
-        if (has_zero) {
-          const int zs = ZT ? 2 * ws + half : 0;
-          umma_f16_ss(d + half * MT, w4g_desc_k16(zop0 + zs * W4G_Z_BYTES, (uint32_t)(Cfg::Z_STAGES - zs) * W4G_Z_BYTES, 128),
-                      sdesc0 + a_off + ((half * Cfg::A_HALF) >> 4), idesc, 1u);
+          umma_f16_ts(d + half * MT, tW + half * (W4G_SLAB_COLS / 2) + k16 * 8, bd, idesc, k16 != 0 ? 1u : 0u);
         }
       };
       constexpr std::integral_constant<int, 0> H0{};
@@ -765,14 +674,14 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         if constexpr (MT == 16) {
           tmem_ld_32x32b_x32(ta, r);
         }
-        float s0 = 16777216.0f, s1 = 16777216.0f;  // 2^24: the converted weights are in units of 2^-24
+        float s0 = 1.0f, s1 = 1.0f;
         if (scaled) {
           uint16_t h0, h1;
           const uint32_t sa = sc_addr0 + (i % Cfg::SS) * W4G_SC_BYTES;
           asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sa));
           asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sa + sc_row1));
-          s0 *= __half2float(__ushort_as_half(h0));
-          s1 *= __half2float(__ushort_as_half(h1));
+          s0 = __half2float(__ushort_as_half(h0));
+          s1 = __half2float(__ushort_as_half(h1));
         }
         if constexpr (MT == 16) {
           tmem_ld_wait();
@@ -856,7 +765,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
               for (int j = 0; j < DT; ++j) psum[j] += src[j * W4_BN];
             }
-            w4g_store_checked<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
+            w4g_store_tile<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
           }
         }
         break;
@@ -865,7 +774,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
         if (full_tile) {
-          if (n < p.N) w4g_store_checked<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
+          if (n < p.N) w4g_store_tile<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
         } else {
           float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + nl;
 #pragma unroll
@@ -936,19 +845,6 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
             for (int u = 0; u < RU; ++u)
               if (mb + u < rows) w4_store_out4<OUT_BF16, GATHER>(p, Cout, m0 + mb + u, n, sum[u]);
-            uint32_t redo = 0;
-#pragma unroll
-            for (int u = 0; u < RU; ++u) {
-              const float one[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (one[i] != one[i] && mb + u < rows) redo |= 1u << (4 * u + i);
-            }
-#pragma unroll 1
-            for (; redo != 0; redo &= redo - 1) {
-              const int bit = __ffs(redo) - 1;
-              w4g_redo_output<OUT_BF16, GATHER>(p, b, m0 + mb + (bit >> 2), n + (bit & 3));
-            }
           }
         }
       }
@@ -964,10 +860,10 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t rawr = smem_u32(raw_base) + row * 128;
     const uint32_t sw = (uint32_t)(row & 7) << 4;  // 128-byte swizzle: quarter-warps read 8 rows x 8 distinct chunks
     const uint32_t st_addr = tmem_w + ((uint32_t)(q * 32) << 16);
-    // ZT: this row's zero points of the slab's halves (128-wide groups: two rows), and where their operands go
+    // ZT: this row's zero points of the slab's halves (128-wide groups: two rows)
     const uint32_t z_addr = smem_u32(z_base) + 2 * row;
     const uint32_t z_row1 = p.scale_rows == 2 ? 256u : 0u;
-    uint8_t* zop = zop_base + row * 16;
+    const uint2 scalar_sub = make_uint2((0x6400u + (uint32_t)p.zero) * 0x00010001u, (0x5400u + ((uint32_t)p.zero << 4)) * 0x00010001u);
     const bool lead = lane == 0;
     // one loop per weight layout: a branch around the conversion inside it costs a register move per converted word
     auto convert_slabs = [&](auto il_) {
@@ -981,13 +877,13 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       uint4 v[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) v[c] = w4g_lds128<0>(rb + ((uint32_t)(c << 4) ^ sw));
-      uint2 zw[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
+      uint2 sub[2] = {scalar_sub, scalar_sub};
       if constexpr (ZT) {
         uint16_t z0, z1;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(z0) : "r"(z_addr + rs * W4G_SC_BYTES));
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(z1) : "r"(z_addr + rs * W4G_SC_BYTES + z_row1));
-        zw[0] = w4g_zero_weights(__half2float(__ushort_as_half(z0)));
-        zw[1] = w4g_zero_weights(__half2float(__ushort_as_half(z1)));
+        sub[0] = w4g_zero_subs((uint32_t)z0 * 0x00010001u);
+        sub[1] = w4g_zero_subs((uint32_t)z1 * 0x00010001u);
       }
       const uint32_t bp = bar0 + 8 * ((i - WS) % W4G_BARS), ppar = (uint32_t)((i - WS) / W4G_BARS) & 1u;
       if (i >= WS) {
@@ -996,16 +892,9 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
       tc_fence_after_sync();
       const uint32_t ta = st_addr + ws * W4G_SLAB_COLS;
-      auto store_zero = [&](int half) {
-        if constexpr (ZT) {
-          *reinterpret_cast<uint2*>(zop + (2 * ws + half) * W4G_Z_BYTES) = zw[half];
-          fence_proxy_async_smem();
-        }
-      };
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         if (Cfg::HALVES && c == 4) {
-          store_zero(0);
           tmem_st_wait();
           tc_fence_before_sync();
           __syncwarp();
@@ -1014,14 +903,12 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           tc_fence_after_sync();
         }
         uint32_t o[16];
-        w4g_convert<decltype(il_)::value>(v[c], o);
+        w4g_convert<decltype(il_)::value>(v[c], sub[c >> 2].x, sub[c >> 2].y, o);
         tmem_st_32x32b_x16(ta + 16 * c, o);
       }
       // the loads have delivered: hand the raw stage back
       __syncwarp();
       if (lead) w4g_arrive<W4G_RAW_EMPTY>(bar0 + 8 * rs);
-      if (!Cfg::HALVES) store_zero(0);
-      store_zero(1);
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
