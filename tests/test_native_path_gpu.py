@@ -82,3 +82,23 @@ def test_runs_on_the_current_stream_and_rejects_as_before():
     with pytest.raises(ValueError, match="device mismatch"):
         q.quant_matmul(A, B, sb.cpu())
     assert q.quant_matmul(A[:0], B, sb).shape == (0, 64)
+
+
+def test_function_transforms_are_refused_in_torch_words():
+    """Under vmap and jvp the arguments are wrappers without storage: every operator raises, as on the Python path, and the
+    process goes on (the exception is met while the interpreter lock is released)."""
+    A, B, sa, sb = [t.cuda() for t in oc.make_w8a8_inputs(2, 16, 64, 32, seed=9)]
+    X = torch.randn((2, 16, 64), device="cuda").half()
+    P = torch.zeros((32, 32), dtype=torch.uint8, device="cuda")
+    W, C = torch.empty((32, 64), dtype=torch.int8, device="cuda"), torch.empty((16, 32), dtype=torch.int32, device="cuda")
+    meta = q.build_block_metadata((16,), 128, "cuda")
+    calls = [(lambda a: q.quant_matmul(a, B[0], sb[0]), A), (q.act_quant, X), (lambda x: q.w4a16_gemm(x, P), X),
+             (lambda a: q.w4a8_gemm_cv(16, 32, 64)(a, P, W, C), A), (lambda x: q.w4a8_gemm_act_quant(16, 32, 64)(x, P, W, C), X),
+             (lambda a: q.grouped_quant_matmul(a, B[:1], meta, sb[0]), A)]
+    for call, arg in calls:
+        with pytest.raises(RuntimeError):
+            torch.vmap(call)(arg)
+    for call in (q.act_quant, lambda x: q.w4a16_gemm(x, P)):
+        with pytest.raises(RuntimeError):
+            torch.func.jvp(call, (X[0],), (X[1],))
+    assert q.quant_matmul(A[0], B[0], sb[0]).shape == (16, 32)

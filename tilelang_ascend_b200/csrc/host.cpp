@@ -75,8 +75,14 @@ int64_t as_int(PyObject* o) {  // -1 on anything that is not a non-negative int
   return (overflow || v < 0) ? -1 : v;
 }
 
-// C++ exceptions (out of memory, ...) must not cross into the interpreter: the Python path then meets the same
-// condition and raises it in torch's own words.
+// The library call runs without the interpreter lock; a scope, so that an exception takes the lock back before it is caught.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
+// C++ exceptions (out of memory, a tensor without storage under vmap or jvp, ...) must not cross into the interpreter: the
+// Python path then meets the same condition and raises it in torch's own words.
 #define QHOST_TRY try {
 #define QHOST_CATCH                     \
   }                                     \
@@ -146,11 +152,12 @@ PyObject* h_w8a8(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor C = empty_cuda(batched ? at::IntArrayRef(shape, 3) : at::IntArrayRef(shape + 1, 2), out, dev);
   void* st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = api.w8a8(static_cast<const int8_t*>(A->const_data_ptr()), static_cast<const int8_t*>(B->const_data_ptr()),
-                static_cast<const float*>(sb->const_data_ptr()), sa ? static_cast<const float*>(sa->const_data_ptr()) : nullptr,
-                C.mutable_data_ptr(), nullptr, batch, M, N, K, sb_len, sa_len, abi_dt(out), nk ? QGEMM_B_NK : QGEMM_B_KN, nullptr, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil unlocked;
+    rc = api.w8a8(static_cast<const int8_t*>(A->const_data_ptr()), static_cast<const int8_t*>(B->const_data_ptr()),
+                  static_cast<const float*>(sb->const_data_ptr()), sa ? static_cast<const float*>(sa->const_data_ptr()) : nullptr,
+                  C.mutable_data_ptr(), nullptr, batch, M, N, K, sb_len, sa_len, abi_dt(out), nk ? QGEMM_B_NK : QGEMM_B_KN, nullptr, st);
+  }
   if (rc != 0) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(C));
   QHOST_CATCH
@@ -177,10 +184,11 @@ PyObject* h_act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   void* st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   const int dt = abi_dt(x->scalar_type()), rs = args[1] == Py_True ? 1 : 0;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = api.act_quant(x->const_data_ptr(), static_cast<int8_t*>(y.mutable_data_ptr()), static_cast<float*>(s.mutable_data_ptr()), M,
-                     N, dt, rs, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil unlocked;
+    rc = api.act_quant(x->const_data_ptr(), static_cast<int8_t*>(y.mutable_data_ptr()), static_cast<float*>(s.mutable_data_ptr()), M,
+                       N, dt, rs, st);
+  }
   if (rc != 0) Py_RETURN_NONE;
   PyObject* py = THPVariable_Wrap(std::move(y));
   PyObject* ps = THPVariable_Wrap(std::move(s));
@@ -264,11 +272,12 @@ PyObject* h_w4a16(PyObject*, PyObject* const* args, Py_ssize_t n) {
   // scratch of this call: handed back to the stream-ordered caching allocator when the call returns
   const at::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate((size_t)(need > 0 ? need : 16));
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = api.w4a16(A->const_data_ptr(), static_cast<const uint8_t*>(B->const_data_ptr()), sc ? sc->const_data_ptr() : nullptr,
-                 zt ? zt->const_data_ptr() : nullptr, zero, (int)zero_mode, (int)layout, group, C.mutable_data_ptr(), ws.get(), need,
-                 batch, M, N, K, abi_dt(A->scalar_type()), abi_dt(out), nullptr, stream.stream());
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil unlocked;
+    rc = api.w4a16(A->const_data_ptr(), static_cast<const uint8_t*>(B->const_data_ptr()), sc ? sc->const_data_ptr() : nullptr,
+                   zt ? zt->const_data_ptr() : nullptr, zero, (int)zero_mode, (int)layout, group, C.mutable_data_ptr(), ws.get(), need,
+                   batch, M, N, K, abi_dt(A->scalar_type()), abi_dt(out), nullptr, stream.stream());
+  }
   if (rc != 0) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(C));
   QHOST_CATCH
@@ -296,19 +305,21 @@ PyObject* h_w4a8_common(PyObject* const* args, bool quant) {
   int8_t* w = static_cast<int8_t*>(W->data_ptr());
   int rc;
   if (!quant) {
-    Py_BEGIN_ALLOW_THREADS
-    rc = api.w4a8(static_cast<const int8_t*>(A->const_data_ptr()), b, w, C->data_ptr(), M, N, K, 1, QGEMM_DT_I32, nullptr, st);
-    Py_END_ALLOW_THREADS
+    {
+    WithoutGil unlocked;
+      rc = api.w4a8(static_cast<const int8_t*>(A->const_data_ptr()), b, w, C->data_ptr(), M, N, K, 1, QGEMM_DT_I32, nullptr, st);
+    }
     if (rc != 0) Py_RETURN_NONE;
     Py_RETURN_TRUE;
   }
   if (args[7] != Py_True && args[7] != Py_False) Py_RETURN_NONE;
   at::Tensor s = empty_cuda({M}, at::kFloat, dev);
   const int rs = args[7] == Py_True ? 1 : 0, dt = abi_dt(A->scalar_type());
-  Py_BEGIN_ALLOW_THREADS
-  rc = api.w4a8_aq(A->const_data_ptr(), dt, b, w, static_cast<int32_t*>(C->data_ptr()), static_cast<float*>(s.mutable_data_ptr()), rs,
-                   M, N, K, 1, nullptr, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil unlocked;
+    rc = api.w4a8_aq(A->const_data_ptr(), dt, b, w, static_cast<int32_t*>(C->data_ptr()), static_cast<float*>(s.mutable_data_ptr()), rs,
+                     M, N, K, 1, nullptr, st);
+  }
   if (rc != 0) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(s));
 }
@@ -363,12 +374,13 @@ PyObject* h_grouped(PyObject*, PyObject* const* args, Py_ssize_t n) {
   void* st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   const auto fn = given ? api.w8a8_grouped : api.w8a8_grouped_zeroed;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = fn(static_cast<const int8_t*>(A->const_data_ptr()), static_cast<const int8_t*>(B->const_data_ptr()),
-          static_cast<const float*>(sb->const_data_ptr()), sa ? static_cast<const float*>(sa->const_data_ptr()) : nullptr,
-          C.data_ptr(), nullptr, static_cast<const int32_t*>(meta->const_data_ptr()), blocks, G, M, N, K, sb_len, sa_len,
-          abi_dt(out), nk ? QGEMM_B_NK : QGEMM_B_KN, nullptr, st);
-  Py_END_ALLOW_THREADS
+  {
+    WithoutGil unlocked;
+    rc = fn(static_cast<const int8_t*>(A->const_data_ptr()), static_cast<const int8_t*>(B->const_data_ptr()),
+            static_cast<const float*>(sb->const_data_ptr()), sa ? static_cast<const float*>(sa->const_data_ptr()) : nullptr,
+            C.data_ptr(), nullptr, static_cast<const int32_t*>(meta->const_data_ptr()), blocks, G, M, N, K, sb_len, sa_len,
+            abi_dt(out), nk ? QGEMM_B_NK : QGEMM_B_KN, nullptr, st);
+  }
   if (rc != 0) Py_RETURN_NONE;
   if (given) {
     Py_INCREF(args[7]);
