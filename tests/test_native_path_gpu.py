@@ -102,3 +102,17 @@ def test_function_transforms_are_refused_in_torch_words():
         with pytest.raises(RuntimeError):
             torch.func.jvp(call, (X[0],), (X[1],))
     assert q.quant_matmul(A[0], B[0], sb[0]).shape == (16, 32)
+
+
+def test_integral_floats_in_a_factory():
+    """A factory takes its shape by value, so 16.0 is 16; and a shape that does not fit is refused either way."""
+    A, P, S = [t.cuda() for t in oc.make_w4a16_inputs(16, 512, 256, "float16", 128, seed=8)]
+    want = q.w4a16_gemm(A, P, S)
+    assert torch.equal(q.dequant_gemm_fp16_wrapper(16.0, 256.0, 512.0, 128, 256, 64)(A, P, S), want)
+    with pytest.raises(ValueError, match="shape mismatch"):
+        q.dequant_gemm_fp16_wrapper(17.0, 256, 512, 128, 256, 64)(A, P, S)
+    y, s = q.act_quant_kernel_int8_optimized(512.0)(A)
+    y0, s0 = q.act_quant(A)
+    assert torch.equal(y, y0) and torch.equal(s, s0.view(-1))
+    with pytest.raises(ValueError, match="shape"):
+        q.act_quant_kernel_int8_optimized(256.0)(A)

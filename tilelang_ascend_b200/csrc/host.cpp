@@ -75,6 +75,15 @@ int64_t as_int(PyObject* o) {  // -1 on anything that is not a non-negative int
   return (overflow || v < 0) ? -1 : v;
 }
 
+// An int of any sign (-1: any size will do) into v; false, with no Python error set, for anything else - an integral float
+// in a factory's shape, say, which the Python path compares by value.
+bool plain_int(PyObject* o, int64_t* v) {
+  if (!PyLong_CheckExact(o)) return false;
+  int overflow = 0;
+  *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return overflow == 0;
+}
+
 // The library call runs without the interpreter lock; a scope, so that an exception takes the lock back before it is caught.
 struct WithoutGil {
   PyThreadState* state = PyEval_SaveThread();
@@ -136,7 +145,8 @@ PyObject* h_w8a8(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int64_t batch = batched ? A->size(0) : 1, M = A->size(-2), K = A->size(-1);
   const int64_t N = nk ? B->size(-2) : B->size(-1);
   if ((nk ? B->size(-1) : B->size(-2)) != K || (batched && B->size(0) != batch)) Py_RETURN_NONE;
-  const long want_batch = PyLong_AsLong(args[6]);
+  int64_t want_batch;
+  if (!plain_int(args[6], &want_batch)) Py_RETURN_NONE;
   if (want_batch >= 0) {  // a factory's static shape; its scale rule (what the scale length may be) is the caller's
     if ((want_batch > 0) != batched || (batched && batch != want_batch) || M != as_int(args[7]) || N != as_int(args[8]) ||
         K != as_int(args[9]))
@@ -170,7 +180,8 @@ PyObject* h_act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Tensor* x = plain(args[0], at::kBFloat16);
   if (x == nullptr) x = plain(args[0], at::kHalf);
   if (x == nullptr || (args[1] != Py_True && args[1] != Py_False)) Py_RETURN_NONE;
-  const long want_n = PyLong_AsLong(args[2]);
+  int64_t want_n;
+  if (!plain_int(args[2], &want_n)) Py_RETURN_NONE;
   const int64_t nd = x->dim();
   if (nd != 2 && nd != 3) Py_RETURN_NONE;
   const int64_t N = x->size(-1);
@@ -225,9 +236,9 @@ PyObject* h_w4a16(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const bool batched = nd == 3;
   const int64_t batch = batched ? A->size(0) : 1, M = A->size(-2), K = A->size(-1), N = B->size(-2);
   if (K % 2 != 0 || B->size(-1) != K / 2 || (batched && B->size(0) != batch)) Py_RETURN_NONE;
-  const long want_m = PyLong_AsLong(args[8]);
+  int64_t want_m, zero_mode, layout;
+  if (!plain_int(args[8], &want_m) || !plain_int(args[6], &zero_mode) || !plain_int(args[7], &layout)) Py_RETURN_NONE;
   if (want_m >= 0 && (batched || M != want_m || N != as_int(args[9]) || K != as_int(args[10]))) Py_RETURN_NONE;
-  const long zero_mode = PyLong_AsLong(args[6]), layout = PyLong_AsLong(args[7]);
   if (zero_mode < 0 || layout < 0) Py_RETURN_NONE;
   int64_t group = K;
   int zero = 0;
@@ -354,8 +365,10 @@ PyObject* h_grouped(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (A->dim() != 2 || B->dim() != 3 || meta->dim() != 2 || meta->size(1) != 3) Py_RETURN_NONE;
   const int64_t M = A->size(0), K = A->size(1), G = B->size(0), N = nk ? B->size(1) : B->size(2), blocks = meta->size(0);
   if ((nk ? B->size(2) : B->size(1)) != K || blocks == 0 || M * N == 0) Py_RETURN_NONE;
-  if (PyLong_AsLong(args[8]) >= 0 &&
-      (M != as_int(args[8]) || K != as_int(args[9]) || G != as_int(args[10]) || blocks != as_int(args[11])))
+  int64_t want_rows;
+  if (!plain_int(args[8], &want_rows)) Py_RETURN_NONE;
+  if (want_rows >= 0 &&
+      (M != want_rows || K != as_int(args[9]) || G != as_int(args[10]) || blocks != as_int(args[11])))
     Py_RETURN_NONE;
   const int64_t sb_len = sb->numel(), sa_len = sa ? sa->numel() : 0;
   if ((sb_len != 1 && sb_len != N && sb_len != G * N) || (sa != nullptr && sa_len != M)) Py_RETURN_NONE;
