@@ -103,3 +103,42 @@ def test_group_quantiser_matches_reference_vector(golden):
     assert torch.equal(q.to(torch.int32), torch.clamp(centred + 8, 0, 15))
     z = qz.unpack_qzeros(qz.pack_int4(torch.tensor([[1, 15, 8, 0]])), 4)
     assert torch.equal(z, torch.tensor([[1, 15, 8, 0]], dtype=torch.float16))
+
+
+def test_extension_belongs_to_one_interpreter_and_torch(monkeypatch, tmp_path):
+    """Another torch: another file, so that the old one is neither loaded nor taken for up to date."""
+    from tilelang_ascend_b200 import build
+    build.build()
+    here = build.host_lib()
+    assert os.path.isfile(here) and not build.needs_build()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.host_lib() != here and build.needs_build()
+
+
+def test_failed_compile_leaves_the_old_file(monkeypatch, tmp_path):
+    from tilelang_ascend_b200 import build
+    target = tmp_path / "x.so"
+    target.write_bytes(b"old")
+
+    def half_written(cmd, verbose):
+        open(cmd[cmd.index("-o") + 1], "wb").write(b"ne")
+        assert target.read_bytes() == b"old"
+        raise RuntimeError("build failed")
+    monkeypatch.setattr(build, "_run", half_written)
+    with pytest.raises(RuntimeError):
+        build._compile(["cc"], str(target), False)
+    assert target.read_bytes() == b"old" and os.listdir(tmp_path) == ["x.so"]
+
+
+def test_operators_do_without_the_extension(monkeypatch, tmp_path):
+    """An extension that is missing or does not load: one warning, and every operator declines to its Python path."""
+    from tilelang_ascend_b200 import _lib, build
+    broken = tmp_path / "broken.so"
+    broken.write_bytes(b"not a library")
+    for path in (tmp_path / "missing.so", broken):
+        monkeypatch.setattr(_lib, "_host", None)
+        _lib.load()
+        monkeypatch.setattr(build, "host_lib", lambda p=path: str(p))
+        with pytest.warns(RuntimeWarning, match="native call path"):
+            host = _lib.host()
+        assert host is _lib.host() and host.w8a8(1, 2) is None and host.grouped() is None
