@@ -20,6 +20,8 @@ def _dirty(nbytes):
     (300, [(0, 5, 100), (7, 105, 50), (1, 290, 10), (1, 4000, 10)]),      # holes at both ends, entries outside the tensors
     (40000, [(0, 128 * i, 127) for i in range(300)]),                     # more rows than one pass of the grid, one row each open
     (1, [(0, 0, 0)]),                                                     # nothing covered
+    (20011, [(1, 19000, 100)]),                                           # two tiles, rows to clear for every SM
+    (5000, [(i % 2, 5 * i, 3) for i in range(1000)] + [(0, 4999, 1)]),    # a long table of short blocks
 ])
 def test_grouped_clears_uncovered_rows(total, blocks):
     K, N, G = 32, 48, 2

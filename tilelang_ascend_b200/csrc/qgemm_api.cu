@@ -649,7 +649,9 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.k_blocks = (int)((K + 127) / 128);
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
-  const int grid = (int)(num_tiles < sms ? num_tiles : sms);
+  // with rows that no block can cover, a CTA per SM to clear them, whatever the number of tiles
+  const bool sure_to_clear = p.zero_uncovered && M > num_blocks * qg::W8_BM;
+  const int grid = (int)(num_tiles < sms && !sure_to_clear ? num_tiles : sms);
   // Tail split: when the last round of the persistent grid would run R < grid/2 tiles, those tiles are issued
   // as 2R half-width items instead ([K, N] layout, 256-column tiles).
   p.split_from = p.num_items = p.num_tiles;

@@ -106,34 +106,41 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
 }
 
 // Grouped form, rows of C that no table entry covers: set to zero by the four epilogue warps before their first tile
-// (they would otherwise wait for it), CTA c looking after every grid-th block of 128 rows.  A clear of the whole output in front
-// of the launch cost a pass over C (33 MB for 8192 x 2048: 10 us of 125) although normally every row is covered.
+// (they would otherwise wait for it), CTA c looking after every grid-th block of 128 rows; a launch that is sure to have such
+// rows has a CTA on every SM, with or without a tile (w8a8_impl).  A clear of the whole output in front of the launch cost a
+// pass over C (33 MB for 8192 x 2048: 8 us of 137) although normally every row is covered.  us, in the kernel / cleared in
+// front: 4096 x 2048 with one open block of 32 19.2 / 24.5; 65536 x 256 with one block of 100 rows 11.2 / 15.4 (cleared by
+// the two CTAs that have a tile: 935); 131072 x 1024 with 300 blocks of 20 rows 123 / 159.
 __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4, int lane) {
-  // a warp takes 32 rows at a time, one per lane, and walks the table once for them
+  // a warp takes 32 rows at a time and walks the table once for them, an entry per lane: which of the rows it covers
   for (long long base = (long long)blockIdx.x * 128 + warp4 * 32; base < p.M; base += (long long)gridDim.x * 128) {
-    const int row = (int)base + lane;
-    bool covered = row >= p.M;
-    for (int i = 0; i < p.num_blocks; i += 32) {
-      int first = 0, rows = 0;
-      if (i + lane < p.num_blocks) {
-        const int g = __ldg(p.meta + 3 * (i + lane));
-        first = __ldg(p.meta + 3 * (i + lane) + 1);
-        rows = min(__ldg(p.meta + 3 * (i + lane) + 2), W8_BM);
-        if (g < 0 || g >= p.groups || first < 0 || first >= p.M) rows = 0;  // as in w8_tile
+    const int row0 = (int)base, n_here = min(32, p.M - row0);
+    const uint32_t all_rows = n_here == 32 ? 0xffffffffu : (1u << n_here) - 1u;
+    uint32_t open_rows = all_rows;
+    for (int i = lane; open_rows != 0 && i - lane < p.num_blocks; i += 32) {
+      uint32_t mine = 0;
+      if (i < p.num_blocks) {
+        const int g = __ldg(p.meta + 3 * i), first = __ldg(p.meta + 3 * i + 1);
+        const int rows = min(__ldg(p.meta + 3 * i + 2), W8_BM);
+        if (g >= 0 && g < p.groups && first >= 0 && first < p.M && rows > 0) {  // as in w8_tile
+          const int lo = max(first - row0, 0), hi = min(first - row0 + rows, 32);
+          if (lo < hi) mine = (hi - lo == 32 ? 0xffffffffu : (1u << (hi - lo)) - 1u) << lo;
+        }
       }
-      const int n_here = min(32, p.num_blocks - i);
-      for (int j = 0; j < n_here; ++j) {
-        const int f = __shfl_sync(0xffffffffu, first, j), r = __shfl_sync(0xffffffffu, rows, j);
-        covered = covered || (row >= f && row - f < r);
-      }
-      if (__all_sync(0xffffffffu, covered)) break;
+      open_rows &= ~__reduce_or_sync(0xffffffffu, mine);
     }
-    uint32_t open_rows = __ballot_sync(0xffffffffu, !covered);
+    uint4* const dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + (size_t)base * (size_t)p.N);
+    const int row_pieces = p.N / 8;  // N is a multiple of 16
+    if (open_rows == all_rows) {
+      const long long pieces = (long long)n_here * row_pieces;
+#pragma unroll 8
+      for (long long c = lane; c < pieces; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
     while (open_rows) {
       const int r = __ffs(open_rows) - 1;
       open_rows &= open_rows - 1;
-      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + ((size_t)base + r) * (size_t)p.N);
-      for (int c = lane; c < p.N / 8; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);  // N is a multiple of 16
+      for (int c = lane; c < row_pieces; c += 32) dst[(size_t)r * row_pieces + c] = make_uint4(0u, 0u, 0u, 0u);
     }
   }
 }
