@@ -141,6 +141,19 @@ __device__ __forceinline__ bool elect_one_sync() {
 // Both are no-ops when the launch carries no such dependency.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A value that the kernel in front may still have been writing when this one started, after pdl_wait(): an ordinary load.
+// (__ldg and const __restrict__ pointers promise that nobody writes the data while the kernel lives.  __ldcg would do, but
+// goes around L1: 1.6 us of 21 for 24 tokens x 4096 x 14336 of the few-token W8A8 kernel, whose warps read a scale per token.)
+__device__ __forceinline__ float ld_written(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_written(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 
 // ----------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {

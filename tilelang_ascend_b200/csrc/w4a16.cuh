@@ -222,7 +222,7 @@ w4a16_prepare_activations(const uint4* __restrict__ in, uint4* __restrict__ out,
     for (int c = threadIdx.x; c < n_counters; c += blockDim.x) counters[c] = 0u;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_chunks) return;
-  uint4 v = in[i];
+  uint4 v = ld_written(in + i);
   if (is_bf16) {
     v.x = w4_bf16x2_to_f16x2(v.x);
     v.y = w4_bf16x2_to_f16x2(v.y);

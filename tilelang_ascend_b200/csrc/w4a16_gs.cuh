@@ -270,7 +270,7 @@ w4g_prepare_activations(const uint4* __restrict__ in, uint8_t* __restrict__ out,
   if (m < M && k0 < K) {  // K is a multiple of 32
     const uint4* src = in + ((size_t)b * M + m) * (size_t)(K / 8) + k0 / 8;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) v[w] = src[w];
+    for (int w = 0; w < 4; ++w) v[w] = ld_written(src + w);
 #pragma unroll
     for (int w = 0; w < 4; ++w) v[w] = w4g_to_f16(v[w], is_bf16 != 0);
   }

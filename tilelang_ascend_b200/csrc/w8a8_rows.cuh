@@ -187,7 +187,7 @@ w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   };
   const int n = n0 + nl;
   float sb = 0.f;
-  if (warp >= 2 && n < p.N) sb = __ldg(p.scale_b + (p.sb_mode == 0 ? 0 : (p.sb_mode == 2 ? (size_t)b * p.N : 0) + n));
+  if (warp >= 2 && n < p.N) sb = ld_written(p.scale_b + (p.sb_mode == 0 ? 0 : (p.sb_mode == 2 ? (size_t)b * p.N : 0) + n));
   const float* sap = p.scale_a + (p.sa_mode == 2 ? (size_t)b * p.M : 0);
   auto finish = [&](auto piece) {
     constexpr int CH = decltype(piece)::value;
@@ -203,7 +203,7 @@ w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       float sa[CH];
       if (p.sa_mode != 0) {
 #pragma unroll
-        for (int j = 0; j < CH; ++j) sa[j] = m + j < p.M ? __ldg(sap + m + j) : 0.f;
+        for (int j = 0; j < CH; ++j) sa[j] = m + j < p.M ? ld_written(sap + m + j) : 0.f;
       }
       tmem_ld_wait();
 #pragma unroll 1
