@@ -212,8 +212,7 @@ int qgemm_w4a16_ex(const void* A, const uint8_t* B_packed, const void* scales, c
  * counterpart in the reference is the put of src/tl_templates/ascend/common.h:358-408 as used by
  * examples/shmem/shmem_mm_test_put_nbi.py:69-74; there is no gathered dequantize-GEMM in the reference.
  *
- * C_dst is a HOST array of n_dst (1..8) device pointers.  ldc and col0 must be multiples of 8, and from the
- * 1792 tokens on N must be a multiple of 64 (unless it is no multiple of 16).  Everything else as
+ * C_dst is a HOST array of n_dst (1..8) device pointers.  ldc and col0 must be multiples of 8.  Everything else as
  * qgemm_w4a16 (batch 1, scalar zero point, sequential nibbles); the workspace size is qgemm_w4a16_workspace_bytes.
  * The call returns when the kernels are queued; a destination buffer is complete on its GPU once EVERY rank's
  * call has finished, which the ranks establish among themselves (a stream-ordered barrier, for example a small

@@ -631,3 +631,28 @@ def test_large_activations_at_the_zero_point(M, K, group, zeros, dt):
     bound = ref.abs() * 2.0 ** (-11 if dt == "float16" else -8) + mag * (K * 2.0 ** -24) + 1e-7
     err = (C.cpu().double() - ref).abs()
     assert (err <= bound).all(), (err / bound).max().item()
+
+
+@pytest.mark.parametrize("M,K,N,n_dst", [
+    (16, 1024, 264, 2), (33, 2048, 128, 8),            # group-sum kernel: whole tiles and tiles cut along K
+    (100, 512, 272, 3), (128, 8192, 256, 2),           # wide tiles: whole ones; a few of long K, cut
+    (300, 1024, 128 * 75, 2), (1800, 256, 272, 1),     # whole tiles and a cut remainder; many tokens, N no multiple of 64
+])
+@pytest.mark.parametrize("dt", ["float16", "bfloat16"])
+def test_gathered_form_writes_every_destination(M, K, N, n_dst, dt):
+    """The gathered form with buffers of this GPU as destinations: the plain call's bits in columns [col0, col0 + N) of each,
+    nothing beside them."""
+    from tilelang_ascend_b200.ops import w4a16_gemm_gather
+    q = _q()
+    A, P, S = [t.cuda() for t in oc.make_w4a16_inputs(M, K, N, dt, 128, seed=M + N)]
+    want = q.w4a16_gemm(A, P, S, 8, 128)
+    ldc, col0 = N + 24, 8
+    dst = [torch.full((M, ldc), 7.0, dtype=A.dtype, device="cuda") for _ in range(n_dst)]
+    w4a16_gemm_gather(A, P, S, 8, 128, [d.data_ptr() for d in dst], ldc, col0)
+    for d in dst:
+        # (16 tokens: the plain call may be the single launch, which adds the K ranges in another order)
+        if M <= 16:
+            torch.testing.assert_close(d[:, col0:col0 + N].float(), want.float(), rtol=2e-3, atol=2e-3)
+        else:
+            assert torch.equal(d[:, col0:col0 + N], want)
+        assert bool((d[:, :col0] == 7).all()) and bool((d[:, col0 + N:] == 7).all())

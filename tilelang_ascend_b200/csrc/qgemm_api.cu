@@ -1074,8 +1074,6 @@ int qgemm_w4a16_gather(const void* A, const uint8_t* B_packed, const void* scale
   if (ldc <= 0 || ldc > (1ll << 30) || col0 < 0 || N <= 0 || col0 + N > ldc)
     return fail("qgemm_w4a16_gather: columns [%lld, %lld) do not fit in rows of %lld", (long long)col0, (long long)(col0 + N), (long long)ldc);
   if (ldc % 8 != 0 || col0 % 8 != 0) return fail("qgemm_w4a16_gather: ldc and col0 must be multiples of 8 (got %lld, %lld)", (long long)ldc, (long long)col0);
-  if (M >= 1792 && N % 16 == 0 && N % 64 != 0)
-    return fail("qgemm_w4a16_gather: from 1792 tokens on N must be a multiple of 64 (got %lld)", (long long)N);
   GatherDst gd{C_dst, n_dst, ldc, col0};
   return w4a16_impl(A, B_packed, scales, zero, group, nullptr, workspace, workspace_bytes, 1, M, N, K, a_dtype, out_dtype,
                     status, stream, nullptr, QGEMM_ZERO_ORIGINAL, QGEMM_W4_SEQUENTIAL, &gd);
