@@ -172,37 +172,18 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uin
       ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-// L2 eviction priorities for bulk copies.  A GEMM's operand tiles are read again by other CTAs (evict last), its
-// output is written once and never read by the kernel (evict first): without the hints the 117 MB of output of a
-// 4096 x 14336 GEMM pushed operand tiles out of L2 and DRAM reads were 2.5 x the operands' size.
+// L2 eviction priority for bulk stores.  A GEMM's output is written once and never read by the kernel: without the hint
+// the 117 MB of output of a 4096 x 14336 GEMM pushed operand tiles out of L2 and DRAM reads were 2.5 x the operands' size.
+// The tiled store goes shared memory -> global (bulk async-group completion); boxes are clipped at the tensor's bounds.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
-__device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z,
-                                                 uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
-      "[%0], [%1, {%3, %4, %5}], [%2], %6;"
-      ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "l"(policy)
-      : "memory");
-}
 __device__ __forceinline__ void tma_store_3d_hint(const CUtensorMap* m, const void* src, int x, int y, int z,
                                                   uint64_t policy) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group.L2::cache_hint [%0, {%2, %3, %4}], [%1], %5;"
                ::"l"(m), "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z), "l"(policy)
-               : "memory");
-}
-// Tiled store shared memory -> global (bulk async-group completion); boxes are clipped at the tensor's bounds.
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(m), "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -245,14 +226,6 @@ __device__ __forceinline__ void umma_i8_ss(uint32_t tmem_d, uint64_t adesc, uint
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: the A operand (M rows = lanes, K packed two 16-bit values per
 // 32-bit column, even k in the low half) is read from tensor memory.
@@ -273,28 +246,6 @@ __device__ __forceinline__ void umma_i8_ts(uint32_t tmem_d, uint32_t tmem_a, uin
       "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-
-// Warp-convergent forms: every lane executes the call with the same operands (so the compiler can keep
-// them in uniform registers) and only the lane with `leader != 0` issues the instruction.
-__device__ __forceinline__ void umma_f16_ts_elect(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
-                                                  uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_elect(uint32_t leader, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(smem_u32(bar)), "r"(leader)
-      : "memory");
-}
-// Ask the TMA unit to bring a tile into L2 only (no shared-memory destination, no completion signal).
-__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
 }
 
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives lane (base lane + i).

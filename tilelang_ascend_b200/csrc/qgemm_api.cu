@@ -112,7 +112,6 @@ int set_smem_w4g() {
   return 0;
 }
 
-// Once per device, with that device current.
 int set_smem_w8r() {
   if (set_smem(qg::w8a8_rows_kernel<false, false>, qg::W8R_SMEM_BYTES)) return -1;
   if (set_smem(qg::w8a8_rows_kernel<false, true>, qg::W8R_SMEM_BYTES)) return -1;
@@ -126,6 +125,7 @@ int set_smem_w4w() {
   return set_smem(qg::w4a16_wide_kernel<true, true>, qg::W4WideCfg<true>::SMEM_BYTES);
 }
 
+// The set-up of the current device, once per device.
 int ensure_device(int* sm_count) {
   int dev = 0;
   CUDA_OK(cudaGetDevice(&dev));
@@ -204,7 +204,7 @@ int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaSt
 // wave of CTAs shares few B tiles and the band's A rows (group_m x 128 x K bytes) stay in L2 while every B tile
 // streams through once per band.  As many row blocks as keep the band's A rows within 34 MB, at least 8: config 3
 // takes all 32 row blocks (16.8 MB, B read from DRAM once instead of four times: 172 -> 165 us; 16 or 24 row blocks:
-// 170 us), the f16 GEMM of 4096 x 8192 x 28672 takes 16 (33.5 MB: 1525 us; 8: 1570, 32: 1553).
+// 170 us).
 int w8_group_m(int64_t m_tiles, int64_t k_bytes) {
   static const int forced = getenv("QGEMM_W8_GROUP_M") ? atoi(getenv("QGEMM_W8_GROUP_M")) : 0;  // tuning override
   int64_t g = forced > 0 ? forced : (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1));
@@ -330,9 +330,8 @@ int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, co
 
 // The group-sum kernel (w4a16_gs.cuh) serves up to 64 tokens when the scale groups are 128 wide, a multiple of
 // 256 or the whole K (or there are no scales); it is faster than the register-operand decode kernel at every
-// token count (K=8192, N=28672: 36 against 40 us at one token, 37 against 42 us at eight).  Groups of 32 / 64 keep
-// the decode kernel (M <= 8) and the per-weight-scale tcgen05 kernel.  QGEMM_W4_GS=0 disables the group-sum kernel,
-// QGEMM_W4_GS_MIN_M raises the token count from which it is used.
+// token count (K=8192, N=28672: 25 against 40 us at one token).  Groups of 32 / 64: see w4_route.  QGEMM_W4_GS=0 disables
+// the group-sum kernel, QGEMM_W4_GS_MIN_M raises the token count from which it is used.
 int w4_gs_min_m() {
   static const int v = getenv("QGEMM_W4_GS_MIN_M") ? atoi(getenv("QGEMM_W4_GS_MIN_M")) : 1;
   return v;
@@ -355,8 +354,8 @@ int launch_w4d(bool bf, int mt, const CUtensorMap& tmW, const CUtensorMap& tmS, 
   if (mt == 16) return launch_w4d_nb<FLUSH, 2>(bf, tmW, tmS, tmA, p, grid, s);
   return launch_w4d_nb<FLUSH, 1>(bf, tmW, tmS, tmA, p, grid, s);
 }
-// Token counts up to this use the register-operand streaming kernel (w4a16_decode.cuh); above it the
-// tcgen05 kernel (w4a16.cuh).
+// Narrow scale groups: token counts up to this use the register-operand streaming kernel (w4a16_decode.cuh), above it
+// the tcgen05 kernel (w4a16.cuh).
 int w4_decode_max_m() {
   static int v = -1;
   if (v < 0) {
@@ -366,12 +365,10 @@ int w4_decode_max_m() {
   return v;
 }
 bool w4_use_decode(int64_t M) { return M <= w4_decode_max_m(); }
-// Token-tile height: 8 for the decode kernel, 16..128 for the tcgen05 kernel.
-// Token-tile height: 16 / 32 for the group-sum kernel, 8 for the decode kernel, 16..128 for the tcgen05 kernel.
+// Token-tile height: 16, 32 or 64 for the group-sum kernel, 8 or 16 for the decode kernel, 16 for w4a16.cuh's.
 int w4_pick_mt(int64_t M, bool gs) {
   if (gs) return M <= 16 ? 16 : (M <= 32 ? 32 : 64);
-  if (w4_use_decode(M)) return M <= 8 ? 8 : 16;
-  return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+  return w4_use_decode(M) && M <= 8 ? 8 : 16;
 }
 
 __global__ void unpack_int4_kernel(const uint8_t* __restrict__ packed, int8_t* __restrict__ out, long long n_bytes,

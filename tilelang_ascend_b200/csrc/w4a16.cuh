@@ -4,7 +4,7 @@
 // with q packed two per byte along K, low nibble first, in B_packed[N, K/2].
 //
 // The weight rows are the MMA "M" dimension (128 per tile, one TMEM lane per weight row) and the
-// tokens are the MMA "N" dimension (MT = 16..128 per tile), so the memory-bound decode shapes stream
+// tokens are the MMA "N" dimension (MT = 16 per tile), so the memory-bound decode shapes stream
 // the packed weights once at full tile height whatever the token count is.
 //
 // The dequantised weights never touch shared memory: each dequant thread owns one weight row, turns
@@ -77,26 +77,23 @@ template <int MT>
 struct W4Cfg {
   // Ring depths: a slot of the activation ring is recycled only after its item's MMAs have completed,
   // so that ring must cover the load latency plus the dequant and MMA time of the items in between.
-  static constexpr int RAW_STAGES = (MT == 16) ? 8 : (MT == 32 ? 7 : (MT == 64 ? 5 : 4));
-  static constexpr int A_STAGES = (MT == 16) ? 9 : (MT == 32 ? 6 : (MT == 64 ? 4 : 2));
+  static_assert(MT == 16, "token tile");
+  static constexpr int RAW_STAGES = 8;
+  static constexpr int A_STAGES = 9;
   // One warp can issue a tcgen05.mma only every ~49 cycles (measured), far longer than a 16-token MMA runs,
   // so MMAW warps issue the K steps of a slab in parallel, each into its own accumulator; the epilogue adds
   // the MMAW accumulators in a fixed order.
-  static constexpr int MMAW = (MT <= 32) ? 4 : (MT == 64 ? 2 : 1);
-  // Two accumulator sets: the epilogue of a segment overlaps the next segment's MMAs.  (One set was measured for
-  // the 128-token tile in three forms that need the room - two issuers, two blocks of tokens per converted slab,
-  // two blocks of weight rows per activation stage: 290 us each at 512 tokens, N=28672, against 228 us; a tile is
-  // only 32 slabs long, and draining and refilling the pipeline at every segment end costs more than any of them
-  // saves.)
+  static constexpr int MMAW = 4;
+  // Two accumulator sets: the epilogue of a segment overlaps the next segment's MMAs.
   static constexpr int ACC_BUFS = 2;
-  static constexpr int W_STAGES = (MT == 16) ? 3 : 2;
+  static constexpr int W_STAGES = 3;
   static constexpr int A_KB_BYTES = MT * 128;          // one 64-wide K block of activations
   static constexpr int A_BYTES = 4 * A_KB_BYTES;       // one 256-wide slab
   static constexpr int ACC_COLS = ACC_BUFS * MMAW * MT;  // ACC_BUFS sets of MMAW accumulators
   static constexpr int TMEM_COLS = 512;
   static constexpr int BAR_BYTES = 512;
   static constexpr int SMEM_BYTES = RAW_STAGES * W4_RAW_BYTES + A_STAGES * A_BYTES + BAR_BYTES + 1024;
-  static constexpr int CH = (MT < 32) ? 16 : 32;  // accumulator columns per TMEM load
+  static constexpr int CH = 16;  // accumulator columns per TMEM load
   static_assert(ACC_COLS + W_STAGES * W4_W_COLS <= 512, "tensor memory budget");
 };
 
@@ -492,8 +489,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             // issuer a wrote its accumulator in this segment only if one of the segment's slabs was its turn
             if (!ROUND_ROBIN_E || ((a - first_turn + Cfg::MMAW) % Cfg::MMAW) < seg_len) {
               uint32_t r2[CH];
-              if constexpr (CH == 16) tmem_ld_32x32b_x16(taddr + a * MT + c * CH, r2);
-              else tmem_ld_32x32b_x32(taddr + a * MT + c * CH, r2);
+              tmem_ld_32x32b_x16(taddr + a * MT + c * CH, r2);
               tmem_ld_wait();
 #pragma unroll
               for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));

@@ -233,8 +233,7 @@ def release_workspaces():
 
 
 def _w4a16_workspace(lib, batch, M, N, K, device, stream_handle, group, has_scales, zeros_tensor=False, zero_mode=0):
-    """Scratch buffer of one call (split-K partial sums + arrival counters + prepared activations, and from 1024
-    tokens on, or with a zeros tensor, the f16 copy of the weights).
+    """Scratch buffer of one call (split-K partial sums + arrival counters + prepared activations).
 
     It needs no initialisation: the call zeroes its arrival counters itself, on its stream.  It is allocated per
     call from torch's caching allocator, so no launch ever sees a buffer that another call may still be using or
