@@ -21,8 +21,7 @@ def _free_port():
 
 def _worker(rank, world, port, q):
     try:
-        os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), NCCL_NVLS_ENABLE="0",
-                          QGEMM_W4_GEMM_MIN_M="64")  # the dequantise-once path already at 64 tokens (small shapes)
+        os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), NCCL_NVLS_ENABLE="0")
         import torch.distributed as dist
         from oracle import qgemm_oracle as oc
         from tilelang_ascend_b200.dist import ColumnShardedW4A16
@@ -34,7 +33,7 @@ def _worker(rank, world, port, q):
         peer = ColumnShardedW4A16(P, S, 8, 128, peer_stores=True).to("cuda")
         coll = ColumnShardedW4A16(P, S, 8, 128, peer_stores=False).to("cuda")
         ok, msg = True, ""
-        for M, dt in [(1, "float16"), (16, "bfloat16"), (40, "float16"), (70, "bfloat16"), (16, "float16")]:
+        for M, dt in [(1, "float16"), (16, "bfloat16"), (40, "float16"), (70, "bfloat16"), (300, "float16"), (16, "float16")]:
             A, _, _ = oc.make_w4a16_inputs(M, K, N, dt, 128, seed=100 + M)
             ref = oc.dequant_gemm_fp16_ref(A, P, dt, S, 8, 128)
             for rep in range(3):  # both buffer generations, and a generation's second use

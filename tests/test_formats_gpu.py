@@ -57,9 +57,8 @@ def test_zero_modes_exact_dequantisation_and_gemm(mode, M, K, N, group):
                                             (64, 1024, 264 + 8, 1024, "bfloat16"), (16, 8192, 4096, 128, "float16")])
 def test_integer_zeros_in_flight_up_to_64_tokens(M, K, N, group, dt):
     """Zero mode "quantized" with up to 64 tokens and groups of 128, a multiple of 256 or the whole K stays on the
-    streaming kernel (no dequantised copy of the weights): one-hot rows read (q - qz) * s back bit for bit, results
-    match the oracle, the interleaved layout gives the same bits, and the whole-matrix path agrees within the
-    operator's tolerance."""
+    streaming kernel: one-hot rows read (q - qz) * s back bit for bit, results match the oracle, the interleaved layout
+    gives the same bits, and the wide tiles (65 tokens) agree within the operator's tolerance."""
     g = torch.Generator().manual_seed(M + K + N)
     A, P, S = oc.make_w4a16_inputs(M, K, N, dt, group, seed=K + M)
     zeros = torch.randint(0, 16, (K // group, N), generator=g).to(torch.float16)

@@ -239,47 +239,40 @@ def test_rejects_bad_arguments():
     assert torch.equal(q.w4a16_gemm(A, P).cpu(), torch.zeros(4, 16, dtype=torch.float16))
 
 
-def test_dequantise_once_path_small_shapes():
-    """Above QGEMM_W4_GEMM_MIN_M tokens (default 1792) the weights are dequantised to f16 once and multiplied by
-    the f16 tensor-core GEMM.  The threshold is read once per process, so a child process with a low threshold
-    runs that path on small ragged shapes: scaled / unscaled, every group size, f16 / bf16, batched."""
-    import os
-    import subprocess
-    import sys
-    code = r"""
-import torch
-from oracle import qgemm_oracle as oc
-import tilelang_ascend_b200 as q
-def close(C, ref): torch.testing.assert_close(C.cpu().float(), ref.float(), rtol=1e-2, atol=1e-2)
-for M, K, N, dt, group in [(17, 256, 128, "float16", 128), (40, 512, 272, "bfloat16", 64), (200, 1024, 528, "float16", 32),
-                           (130, 768, 2320, "bfloat16", 256), (300, 512, 144, "float16", 512), (129, 2048, 1024, "bfloat16", 128)]:
+@pytest.mark.parametrize("M,K,N,dt,group", [
+    (17, 256, 128, "float16", 128), (40, 512, 272, "bfloat16", 64), (200, 1024, 528, "float16", 32),
+    (130, 768, 2320, "bfloat16", 256), (300, 512, 144, "float16", 512), (129, 2048, 1024, "bfloat16", 128)])
+def test_small_ragged_shapes_scaled_and_unscaled(M, K, N, dt, group):
+    """Every group size on small ragged shapes (up to 64 tokens with wide groups the group-sum kernel, otherwise wide
+    tiles, whole or cut along K), with scales and with the raw nibble values."""
+    q = _q()
     A, P, S = oc.make_w4a16_inputs(M, K, N, dt, group, seed=M + K)
-    C = q.w4a16_gemm(A.cuda(), P.cuda(), S.cuda(), 8, group)
-    close(C, oc.dequant_gemm_fp16_ref(A, P, dt, S, 8, group))
-    C0 = q.w4a16_gemm(A.cuda(), P.cuda(), None)
-    close(C0, oc.dequant_gemm_fp16_ref(A, P, dt))
-# exact dequantisation: unit activations read back half(q - zero) * s bit for bit
-K, N, group = 256, 144, 64
-_, P, S = oc.make_w4a16_inputs(1, K, N, "float16", group, seed=3)
-eye = torch.eye(K, dtype=torch.float16)
-W = q.w4a16_gemm(eye.cuda(), P.cuda(), S.cuda(), 8, group)   # [K, N] = dequantised weights, transposed
-assert torch.equal(W.cpu().t().contiguous(), oc.dequant_weight_ref(P, S, 8, group).half())
-# batched
-ins = [oc.make_w4a16_inputs(48, 512, 272, "float16", 128, seed=s) for s in range(3)]
-A, P, S = [torch.stack([x[i] for x in ins]).cuda() for i in range(3)]
-C = q.w4a16_gemm(A, P, S, 8, 128)
-for b in range(3): close(C[b], oc.dequant_gemm_fp16_ref(ins[b][0], ins[b][1], "float16", ins[b][2], 8, 128))
-print("dequantise-once ok")
-"""
-    env = dict(os.environ, QGEMM_W4_GEMM_MIN_M="17")
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0 and "dequantise-once ok" in r.stdout, r.stdout + r.stderr
+    _close(q.w4a16_gemm(A.cuda(), P.cuda(), S.cuda(), 8, group), oc.dequant_gemm_fp16_ref(A, P, dt, S, 8, group))
+    _close(q.w4a16_gemm(A.cuda(), P.cuda(), None), oc.dequant_gemm_fp16_ref(A, P, dt))
+
+
+def test_wide_tiles_read_dequantised_weights_back_exactly():
+    """Unit activations, 256 tokens: half(q - zero) * s bit for bit with groups of 64."""
+    q = _q()
+    K, N, group = 256, 144, 64
+    _, P, S = oc.make_w4a16_inputs(1, K, N, "float16", group, seed=3)
+    W = q.w4a16_gemm(torch.eye(K, dtype=torch.float16).cuda(), P.cuda(), S.cuda(), 8, group)  # [K, N], transposed
+    assert torch.equal(W.cpu().t().contiguous(), oc.dequant_weight_ref(P, S, 8, group).half())
+
+
+@pytest.mark.parametrize("M", [48, 100])
+def test_batched_ragged(M):
+    q = _q()
+    ins = [oc.make_w4a16_inputs(M, 512, 272, "float16", 128, seed=s) for s in range(3)]
+    A, P, S = [torch.stack([x[i] for x in ins]).cuda() for i in range(3)]
+    C = q.w4a16_gemm(A, P, S, 8, 128)
+    for b in range(3):
+        _close(C[b], oc.dequant_gemm_fp16_ref(ins[b][0], ins[b][1], "float16", ins[b][2], 8, 128))
 
 
 def test_config5_prefill_m4096_band_and_linearity():
-    """Config 5 at 4096 tokens goes through the dequantise-once path at full size: bands of output columns
-    against the oracle, and f(2A) == 2 f(A) over the whole output."""
+    """Config 5 at 4096 tokens, on wide tiles of 256 tokens: bands of output columns against the oracle, and f(2A) == 2 f(A)
+    over the whole output."""
     q = _q()
     A, packed, scales = oc.make_config_inputs("cfg5", M=4096)
     Ad, Pd, Sd = A.cuda(), packed.cuda(), scales.cuda()

@@ -166,7 +166,9 @@ def test_config3_full_size_properties():
     assert torch.equal(acc1 + acc2, acc)
 
 
-SPLITK_SHAPES = [(0, 256, 4096, 1024), (2, 200, 4224, 528), (0, 130, 7168, 272), (3, 256, 4608, 1024)]
+# the last two have too many tokens and tiles for the few-token form, so that they are split with and without accumulators
+SPLITK_SHAPES = [(0, 256, 4096, 1024), (2, 200, 4224, 528), (0, 130, 7168, 272), (3, 256, 4608, 1024),
+                 (0, 200, 4112, 2064), (2, 300, 4096, 1040)]
 
 
 @pytest.mark.parametrize("batch,M,K,N", SPLITK_SHAPES)
@@ -179,13 +181,15 @@ def test_k_split_over_cta_pairs_is_exact(batch, M, K, N):
     ref, acc_ref = oc.quant_matmul_ref(A, B, sb, "bfloat16", scale_a=sa, return_acc=True)
     C, acc = q.quant_matmul(A.cuda(), B.cuda(), sb.cuda(), scale_a=sa.cuda(), out_dtype="bfloat16", return_accumulators=True)
     assert torch.equal(acc.cpu(), acc_ref) and torch.equal(C.cpu(), ref)
+    assert torch.equal(q.quant_matmul(A.cuda(), B.cuda(), sb.cuda(), scale_a=sa.cuda(), out_dtype="bfloat16").cpu(), ref)
     acc2 = q.quant_matmul(A.cuda(), B.transpose(-1, -2).contiguous().cuda(), None, out_dtype=torch.int32, b_layout="NK")
     assert torch.equal(acc2.cpu(), acc_ref)
 
 
 def test_k_split_and_unsplit_kernels_give_the_same_bits():
     """The same shapes with the K split switched off (QGEMM_W8_SPLITK=0 is read once per process, hence a child
-    process): identical outputs, which also shows that the shapes above really take the split path's place."""
+    process): the accumulators keep all of them off the few-token form, so that unsplit tiles take the split ones'
+    place, with identical results."""
     import os
     import subprocess
     import sys
@@ -195,9 +199,9 @@ from oracle import qgemm_oracle as oc
 import tilelang_ascend_b200 as q
 for batch, M, K, N in %r:
     A, B, sa, sb = oc.make_w8a8_inputs(batch, M, K, N, seed=M + K)
-    ref = oc.quant_matmul_ref(A, B, sb, "bfloat16", scale_a=sa)
-    C = q.quant_matmul(A.cuda(), B.cuda(), sb.cuda(), scale_a=sa.cuda(), out_dtype="bfloat16")
-    assert torch.equal(C.cpu(), ref), (batch, M, K, N)
+    ref, acc_ref = oc.quant_matmul_ref(A, B, sb, "bfloat16", scale_a=sa, return_acc=True)
+    C, acc = q.quant_matmul(A.cuda(), B.cuda(), sb.cuda(), scale_a=sa.cuda(), out_dtype="bfloat16", return_accumulators=True)
+    assert torch.equal(C.cpu(), ref) and torch.equal(acc.cpu(), acc_ref), (batch, M, K, N)
 print("unsplit ok")
 """ % (SPLITK_SHAPES,)
     env = dict(os.environ, QGEMM_W8_SPLITK="0")
