@@ -39,7 +39,7 @@ CFG2 = dict(M=16, K=4096, N=4096, group=128)
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed ncu
 # summary under profiles/.
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 293437952  # profiles/w4a16_gs_cfg2_headline.md (284.0 MB read + 9.5 MB written)
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 288777472  # profiles/w4a16_gs_cfg2_headline.md (281.1 MB read + 7.7 MB written)
 
 
 def w4a16_bytes(M, K, N, group, out_bytes=2, a_bytes=2):
@@ -297,7 +297,7 @@ def run_ours(args):
                        "multi_gpu": "replicas only for this config; sharded configs are under suite"},
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": NCU_TRAFFIC_BYTES_PER_LAUNCH,
-                         "kernel": "w4a16_gs_kernel<16,f16>, batch 32 (time includes its w4a16_prepare_activations pre-pass)",
+                         "kernel": "w4a16_gs_kernel<16,f16>, batch 32 (time includes its w4g_prepare_activations pre-pass)",
                          "us_per_launch": round(launch_us, 3),
                          "algorithmic_bytes_per_launch": bytes_step, "peak_source": peaks_src + " (copy)"},
             "per_layer_launch": per_layer,
