@@ -106,15 +106,21 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
 }
 
 // Grouped form, rows of C that no table entry covers: set to zero by the four epilogue warps before their first tile
-// (they would otherwise wait for it), CTA c looking after every grid-th block of 128 rows; a launch that is sure to have such
-// rows has a CTA on every SM, with or without a tile (w8a8_impl).  A clear of the whole output in front of the launch cost a
-// pass over C (33 MB for 8192 x 2048: 8 us of 137) although normally every row is covered.  us, in the kernel / cleared in
-// front: 4096 x 2048 with one open block of 32 19.2 / 24.5; 65536 x 256 with one block of 100 rows 11.2 / 15.4 (cleared by
-// the two CTAs that have a tile: 935); 131072 x 1024 with 300 blocks of 20 rows 123 / 159.
+// (they would otherwise wait for it), dealt to all CTAs; a launch that is sure to have such rows has a CTA on every SM,
+// with or without a tile (w8a8_impl).  A clear of the whole output in front of the launch cost a pass over C (33 MB for
+// 8192 x 2048: 8 us of 137) although normally every row is covered.  us, in the kernel / cleared in front: 4096 x 2048 with
+// one open block of 32 19.0 / 24.2; 8192 x 1024, 16 blocks of 64 there could be 9.3 / 12.2; 65536 x 256 with one block of 100
+// rows 12.2 / 15.5 (cleared by the two CTAs that have a tile: 935); 131072 x 1024 with 300 blocks of 20 rows 111 / 139.  (128 rows
+// per CTA at a time, whatever M: 1055 x 2528 with three blocks 18.6 us instead of 9.8 cleared in front.)
 __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4, int lane) {
-  // a warp takes 32 rows at a time and walks the table once for them, an entry per lane: which of the rows it covers
-  for (long long base = (long long)blockIdx.x * 128 + warp4 * 32; base < p.M; base += (long long)gridDim.x * 128) {
-    const int row0 = (int)base, n_here = min(32, p.M - row0);
+  // A warp walks the table once per 32 rows, an entry per lane: which of the rows it covers.  Where there are not 128 rows
+  // for every CTA the four warps take the same 32 rows, or 8, and share the columns.
+  const bool own = p.M >= 128 * (long long)gridDim.x;
+  const int chunk = own || p.M >= 32 * (long long)gridDim.x ? 32 : 8, step = own ? 4 * chunk : chunk;
+  const int thread = own ? lane : warp4 * 32 + lane, threads = own ? 32 : 128;
+  const int row_pieces = p.N / 8;  // N is a multiple of 16
+  for (long long base = (long long)blockIdx.x * step + (own ? warp4 * 32 : 0); base < p.M; base += (long long)gridDim.x * step) {
+    const int row0 = (int)base, n_here = min(chunk, p.M - row0);
     const uint32_t all_rows = n_here == 32 ? 0xffffffffu : (1u << n_here) - 1u;
     uint32_t open_rows = all_rows;
     for (int i = lane; open_rows != 0 && i - lane < p.num_blocks; i += 32) {
@@ -130,17 +136,16 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
       open_rows &= ~__reduce_or_sync(0xffffffffu, mine);
     }
     uint4* const dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C) + (size_t)base * (size_t)p.N);
-    const int row_pieces = p.N / 8;  // N is a multiple of 16
     if (open_rows == all_rows) {
       const long long pieces = (long long)n_here * row_pieces;
-#pragma unroll 8
-      for (long long c = lane; c < pieces; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 4
+      for (long long c = thread; c < pieces; c += threads) dst[c] = make_uint4(0u, 0u, 0u, 0u);
       continue;
     }
     while (open_rows) {
       const int r = __ffs(open_rows) - 1;
       open_rows &= open_rows - 1;
-      for (int c = lane; c < row_pieces; c += 32) dst[(size_t)r * row_pieces + c] = make_uint4(0u, 0u, 0u, 0u);
+      for (int c = thread; c < row_pieces; c += threads) dst[(size_t)r * row_pieces + c] = make_uint4(0u, 0u, 0u, 0u);
     }
   }
 }
