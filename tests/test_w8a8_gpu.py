@@ -166,7 +166,7 @@ def test_config3_full_size_properties():
     assert torch.equal(acc1 + acc2, acc)
 
 
-# the last two have too many tokens and tiles for the few-token form, so that they are split with and without accumulators
+# (with accumulators; without them the few-token form takes these shapes)
 SPLITK_SHAPES = [(0, 256, 4096, 1024), (2, 200, 4224, 528), (0, 130, 7168, 272), (3, 256, 4608, 1024),
                  (0, 200, 4112, 2064), (2, 300, 4096, 1040)]
 
@@ -253,6 +253,8 @@ def test_empty_inputs_give_empty_outputs():
     (40, 64, 128, 1024),     # more tiles than CTAs fit at once
     (0, 129, 1024, 1040), (0, 512, 256, 1024), (2, 300, 272, 256),  # several token tiles
     (0, 192, 4112, 2064),
+    (0, 300, 4112, 272), (2, 260, 2064, 256), (0, 500, 1040, 528),  # ... with K cut over eight or four CTAs
+    (0, 112, 1152, 1040), (0, 128, 512, 4112), (3, 96, 2048, 8192),   # on either side of the choice of the form
 ])
 @pytest.mark.parametrize("layout", ["KN", "NK"])
 @pytest.mark.parametrize("odt", ["float16", "bfloat16"])

@@ -500,6 +500,32 @@ int qgemm_init(void) {
   return ensure_device(&sms);
 }
 
+// Over how many CTAs the few-token form (w8a8_rows.cuh) cuts the K of its `tiles` tiles; 0: w8a8.cuh is the faster one.
+// The cut.  A CTA per SM, at least two 128-k blocks each; a second one per SM, or clusters of eight on more than half of the
+// SMs (they rarely find eight SMs close together), from eight blocks each on.  us, cut so / two CTAs per SM whatever their K: 32
+// tokens 1024 x 8192 6.1 / 7.3, 2048 x 2048 4.9 / 6.6, 64 tokens 4096 x 4096 8.3 / 10.0.
+// The choice.  Per tile this form pays for its tokens (8.4 ns each, not shared when K is not cut) and saves the k blocks that
+// other CTAs of the cluster take.  So up to 48 tokens always; up to 64 unless nothing is cut, K is long and there are more
+// tiles than SMs; above that when the cut saves enough blocks.  us, this form / w8a8.cuh: 32 tokens 1024 x 8192 6.1 / 7.3, 128
+// tokens 512 x 14336 7.9 / 6.0, 1024 x 1024 7.0 / 7.1, 2048 x 2048 7.9 / 8.9, 4096 x 14336 18.3 / 20.3, 10 x 96 x 2048 x 3072
+// 18.0 / 16.7.  Over 1739 shapes (1 .. 10 problems of 16 .. 512 tokens, K and N 128 .. 14336, weights from DRAM) the choice is
+// within 1 % of the better one in the mean and 5 % behind w8a8.cuh at worst ([N, K] weights).
+static int w8_rows_split(int64_t tiles, int64_t k_blocks, int64_t tokens, int sms) {
+  int S = 1;
+  while (S < qg::W8R_MAX_SPLIT) {
+    const int n = 2 * S;
+    const int64_t ctas = tiles * n;
+    const bool fits = k_blocks >= 2 * n && ctas <= (n == qg::W8R_MAX_SPLIT ? sms / 2 : sms);
+    if (!fits && !(k_blocks >= 8 * n && ctas <= 2 * sms)) break;
+    S = n;
+  }
+  const int64_t saved = k_blocks - (k_blocks + S - 1) / S, ctas = tiles * S;
+  if (tokens <= 48) return S;
+  if (tokens <= 64) return saved >= 4 || k_blocks <= 12 || tiles <= sms ? S : 0;
+  if (ctas > sms) return saved >= 16 ? S : 0;
+  return saved >= (tokens <= 96 ? 7 : 9) || (saved >= 6 && 2 * ctas <= sms) ? S : 0;
+}
+
 // Plain / batched form: meta == nullptr.  Grouped form: A and C are single [M, K] / [M, N] stacks, B holds
 // `batch` (= groups) matrices and `meta` lists num_blocks row blocks (group, first row, valid rows).
 static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
@@ -533,19 +559,11 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   if (ensure_device(&sms)) return -1;
 
   CUtensorMap tmA, tmB;
-  // Few tokens (w8a8_rows.cuh), and what would leave most SMs idle: up to 128 tokens; up to 32 tiles of 128 x 128; 192 tokens
-  // from K = 4096 on.  us, this form against the other, [N, K] weights, K x N: 16 tokens 4096 x 14336 14.3 / 22.6, 8192 x 8192
-  // 15.4 / 26.6, 1024 x 1024 4.5 / 8.2; 128 tokens 17.8 / 20.5, 19.7 / 26.7, 6.6 / 8.2; 192 tokens 20.5 / 22.6, 22.1 / 26.7
-  // and, K = 1024 .. 2048, 10.8 / 10.3 and 9.9 / 9.4; 256 tokens 22.4 / 22.7, 2048 x 4096 11.6 / 10.3, 1024 x 1024 6.8 / 8.2
-  // (16 tiles; 512 tokens, 32 tiles: 7.2 / 8.2).
-  const int64_t rows_m_tiles = (M + qg::W8R_MAX_MT - 1) / qg::W8R_MAX_MT, rows_n_tiles = (N + 127) / 128;
-  const bool rows_shape = M <= 128 || batch * rows_m_tiles * rows_n_tiles <= 32 || (M <= 192 && K >= 4096);
-  if (rows_shape && meta == nullptr && acc_out == nullptr) {
-    const int64_t n_tiles = rows_n_tiles, m_tiles = rows_m_tiles, k_blocks = (K + 127) / 128, tiles = batch * n_tiles * m_tiles;
+  const int64_t k_blocks = (K + 127) / 128, n_tiles128 = (N + 127) / 128, row_tiles = (M + qg::W8R_MAX_MT - 1) / qg::W8R_MAX_MT;
+  const int S = meta == nullptr && acc_out == nullptr ? w8_rows_split(batch * n_tiles128 * row_tiles, k_blocks, (M + row_tiles - 1) / row_tiles, sms) : 0;
+  if (S > 0) {
+    const int64_t n_tiles = n_tiles128, m_tiles = row_tiles, tiles = batch * n_tiles * m_tiles;
     if (tiles > 0x7fffffff / qg::W8R_MAX_SPLIT) return fail("qgemm_w8a8: too many tiles");
-    // K is cut until two CTAs per SM are at work, each with two 128-k blocks at least
-    int S = 1;
-    while (S < qg::W8R_MAX_SPLIT && tiles * 2 * S <= 2 * sms && k_blocks >= 4 * S) S *= 2;
     const int unit = S == 8 ? 32 : 16;
     qg::W8RowsParams p;
     p.scale_b = scale_b;
