@@ -791,8 +791,8 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     // A tile that several CTAs share: each one's partial sums go to the scratch buffer and a counter tells the last
     // contributor (never by waiting), which adds them in a fixed order and writes the tile.  This chain of global-memory
     // round trips (fence, atomic, loads: 7 000 cycles when the drain warps ran it, with the pipeline standing still behind
-    // them) is these four warps' alone; they take four tokens in turn, two contributors' at a time (35 x 5888 x 768, 23
-    // contributors to a tile: 45.9 -> 27.6 us; a quarter of the tokens each, one contributor at a time and a 64-bit division
+    // them) is these four warps' alone; they take four tokens in turn, two contributors' at a time (20 x 7168 x 480, 28
+    // contributors to a tile: 26.7 -> 16.7 us; a quarter of the tokens each, one contributor at a time and a 64-bit division
     // for every one of them was what it replaced).
     const int fw = warp - W4G_FIN_WARP;
     volatile uint32_t* fin_word = reinterpret_cast<uint32_t*>(bar_block + W4G_FIN_WORD);
@@ -821,7 +821,9 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
         const int n = n0 + 4 * lane;  // four rows of the tile per lane
         const int rows = min(MT, p.M - m0);
-        constexpr int RU = 4, CU = 2;  // four tokens of two contributors in flight
+        // four tokens of two contributors in flight; of one with 64 tokens, where the second one's values spilled (64 x 8192 x
+        // 28672 48.9 -> 51.1 us)
+        constexpr int RU = 4, CU = MT == 64 ? 1 : 2;
         // every contributor but the last one stops short of the tile's end: its partial tile is its second one (slot 2 c + 1)
         auto part = [&](int c, int m) {
           return reinterpret_cast<const float4*>(p.ws_partials + (size_t)(c == b_last ? 2 * c : 2 * c + 1) * (MT * W4_BN) +
