@@ -746,6 +746,9 @@ int64_t qgemm_w4a16_counter_bytes(void) { return kW4CounterBytes; }
 // hold two partial tiles, 3 + 0.06 per token, or 6.  So large problems take the tallest tiles, problems of fewer tiles
 // than SMs shorter ones (512 x 2048 x 4096: 128 tiles of 128 tokens 16.4 us, 64 tiles of 256 cut in two 25.5 us), and a
 // cut along K is for few tiles of long K (128 x 8192 x 2048: 32 tiles of 64 tokens cut in four 23.3 us, whole 38.6 us).
+// Beside whole rounds, and below K = 8192, a remainder is cut in two only: with four or more shares the sums, of tall tiles with
+// one accumulator, set the pace (1040 x 1024 x 8192: 41 us, whole tiles 27; 1700 x 4096 x 3072 53 / 43; but 4096 x 8192 x 28672
+// in four 1641, in two 1652).
 struct W4WidePlan {
   int mt = 0, sk_tiles = 0, sk_grid = 1;
 };
@@ -767,7 +770,7 @@ static W4WidePlan w4_wide_plan(int64_t M, int64_t weight_tiles, int64_t KS, int6
     };
     consider((double)((rounds + (r != 0 ? 1 : 0)) * KS), 0.0, 0, 1);
     if (r != 0) {
-      for (int64_t S = 2; S <= 8 && S * r <= G && S <= KS; S += 2)
+      for (int64_t S = 2; S <= (rounds != 0 && KS < 32 ? 2 : 8) && S * r <= G && S <= KS; S += 2)
         consider((double)(rounds * KS + (KS + S - 1) / S), rounds != 0 ? 2.0 : 2.0 + (double)S * (0.3 + 0.011 * (double)mt), r, r * S);
       const int64_t sk = r + (rounds != 0 && 2 * r < G ? G : 0);
       if (sk * KS >= G) consider((double)(tiles * KS) / (double)G, rounds != 0 ? 6.0 : 3.0 + 0.06 * (double)mt, sk, G);
