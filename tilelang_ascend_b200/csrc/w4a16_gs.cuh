@@ -821,8 +821,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
         const int n = n0 + 4 * lane;  // four rows of the tile per lane
         const int rows = min(MT, p.M - m0);
-        // four tokens of two contributors in flight; of one with 64 tokens, where the second one's values spilled (64 x 8192 x
-        // 28672 48.9 -> 51.1 us)
+        // four tokens of two contributors in flight; of one with 64 tokens, where the second one's would spill
         constexpr int RU = 4, CU = MT == 64 ? 1 : 2;
         // every contributor but the last one stops short of the tile's end: its partial tile is its second one (slot 2 c + 1)
         auto part = [&](int c, int m) {
