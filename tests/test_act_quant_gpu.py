@@ -124,3 +124,29 @@ def test_fused_quantiser_rejects_more_than_128_tokens():
     with pytest.raises(q.QGemmError, match="M <= 128"):
         kernel(torch.zeros((M, K), dtype=torch.bfloat16, device="cuda"), torch.zeros((N, K // 2), dtype=torch.uint8, device="cuda"),
                torch.empty((N, K), dtype=torch.int8, device="cuda"), torch.empty((M, N), dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("M,K,layers", [(1, 2048, 24), (24, 4096, 12), (40, 16384 + 256, 4)])
+def test_chain_of_quantisers_and_few_token_gemms(M, K, layers):
+    """Quantiser and few-token W8A8 kernel are programmatic dependents of each other: a chain in which each call reads what the
+    one in front has just written is bit-identical to the same chain with the device drained between the calls."""
+    g = torch.Generator().manual_seed(M + K)
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    W = torch.randint(-128, 128, (K, K), dtype=torch.int8, generator=g).cuda()
+    scale = (torch.rand(K, generator=g) * 2e-4).cuda()
+
+    def chain(drain):
+        h = x
+        for _ in range(layers):
+            a, sa = q.act_quant(h)
+            if drain:
+                torch.cuda.synchronize()
+            h = q.quant_matmul(a, W, scale, scale_a=sa.view(-1), out_dtype="bfloat16")
+            if drain:
+                torch.cuda.synchronize()
+        return h
+
+    want = chain(True)
+    for _ in range(3):
+        assert torch.equal(chain(False), want)
+    assert torch.isfinite(want.float()).all() and want.float().abs().max() > 0

@@ -123,6 +123,7 @@ template <int TPR, int KEEP>
 __global__ void __launch_bounds__(AQ_THREADS, KEEP == 4 ? AQ_MIN_BLOCKS : 1) act_quant_kernel(const ActQuantParams p) {
   // A W8A8 kernel behind this one may set up meanwhile; it waits for this whole grid before it reads anything.
   pdl_launch_dependents();
+  pdl_wait();  // a programmatic dependent itself: the kernel in front may have written X, and may still read Y and S
   constexpr int ROWS = AQ_THREADS / TPR;
   constexpr int WPR = TPR / 32;  // warps per row
   __shared__ float red[AQ_THREADS / 32];
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(AQ_THREADS, KEEP == 4 ? AQ_MIN_BLOCKS : 1) act
         m2 = aq_absmax8(keep[i], bf16, m2);
       }
     }
-    for (int c = t + KEEP * TPR; c < chunks; c += TPR) m2 = aq_absmax8(__ldg(x + c), bf16, m2);
+    for (int c = t + KEEP * TPR; c < chunks; c += TPR) m2 = aq_absmax8(ld_written(x + c), bf16, m2);
   }
   float m = aq_pair_max(m2, bf16);
 #pragma unroll
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(AQ_THREADS, KEEP == 4 ? AQ_MIN_BLOCKS : 1) act
     const int c = t + i * TPR;
     if (c < chunks) __stcs(y + c, aq_quant8(keep[i], bf16, scale, rcp));
   }
-  for (int c = t + KEEP * TPR; c < chunks; c += TPR) __stcs(y + c, aq_quant8(__ldg(x + c), bf16, scale, rcp));
+  for (int c = t + KEEP * TPR; c < chunks; c += TPR) __stcs(y + c, aq_quant8(ld_written(x + c), bf16, scale, rcp));
 }
 
 }  // namespace qg

@@ -1237,17 +1237,15 @@ int qgemm_act_quant(const void* X, int8_t* Y, float* S, int64_t M, int64_t N, in
   const int64_t grid = (M + rows_per_block - 1) / rows_per_block;
   if (grid > 0x7fffffffll) return fail("qgemm_act_quant: too many rows (%lld)", (long long)M);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // A programmatic dependent: behind the few-token W8A8 kernel it is resident when that kernel ends.
   switch (tpr) {
-    case 32: qg::act_quant_kernel<32, 4><<<(unsigned)grid, qg::AQ_THREADS, 0, st>>>(p); break;
-    case 64: qg::act_quant_kernel<64, 4><<<(unsigned)grid, qg::AQ_THREADS, 0, st>>>(p); break;
-    case 128: qg::act_quant_kernel<128, 4><<<(unsigned)grid, qg::AQ_THREADS, 0, st>>>(p); break;
+    case 32: return launch_pdl(qg::act_quant_kernel<32, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 64: return launch_pdl(qg::act_quant_kernel<64, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 128: return launch_pdl(qg::act_quant_kernel<128, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
     default:
-      if (keep8) qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS><<<(unsigned)grid, qg::AQ_THREADS, 0, st>>>(p);
-      else qg::act_quant_kernel<256, 4><<<(unsigned)grid, qg::AQ_THREADS, 0, st>>>(p);
-      break;
+      if (keep8) return launch_pdl(qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS>, (int)grid, qg::AQ_THREADS, 0, st, p);
+      return launch_pdl(qg::act_quant_kernel<256, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
   }
-  CUDA_OK(cudaGetLastError());
-  return 0;
 }
 
 int qgemm_w4a8(const int8_t* A, const uint8_t* qB, int8_t* workspace, void* C, int64_t M, int64_t N, int64_t K,
