@@ -133,7 +133,7 @@ def test_chain_of_quantisers_and_few_token_gemms(M, K, layers):
     g = torch.Generator().manual_seed(M + K)
     x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
     W = torch.randint(-128, 128, (K, K), dtype=torch.int8, generator=g).cuda()
-    scale = (torch.rand(K, generator=g) * 2e-4).cuda()
+    scale = (torch.rand(K, generator=g) / (0.577 * 74 * K ** 0.5)).cuda()  # a layer keeps its input's magnitude
 
     def chain(drain):
         h = x
@@ -149,4 +149,4 @@ def test_chain_of_quantisers_and_few_token_gemms(M, K, layers):
     want = chain(True)
     for _ in range(3):
         assert torch.equal(chain(False), want)
-    assert torch.isfinite(want.float()).all() and want.float().abs().max() > 0
+    assert torch.isfinite(want.float()).all() and want.float().abs().max() > 0.1
