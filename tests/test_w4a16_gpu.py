@@ -649,3 +649,20 @@ def test_gathered_form_writes_every_destination(M, K, N, n_dst, dt):
         else:
             assert torch.equal(d[:, col0:col0 + N], want)
         assert bool((d[:, :col0] == 7).all()) and bool((d[:, col0 + N:] == 7).all())
+
+
+@pytest.mark.parametrize("M", [17, 31, 32, 33, 48, 49, 63, 64])
+@pytest.mark.parametrize("K,N", [(512, 40), (2304, 1008), (4096, 20480)])
+def test_each_token_gets_its_own_sums(M, K, N):
+    """The drain sets share a tile's tokens: with one-hot activations token m reads weight column k(m) back, (q - 8) * s rounded
+    once, bit for bit, whether its tile is whole or cut along K over several CTAs."""
+    q = _q()
+    _, packed, scales = oc.make_w4a16_inputs(M, K, N, "float16", 128, seed=M)
+    k = (torch.arange(M) * 2654435761) % K
+    A = torch.zeros(M, K, dtype=torch.float16)
+    A[torch.arange(M), k] = 1.0
+    C = q.w4a16_gemm(A.cuda(), packed.cuda(), scales.cuda(), 8, 128)
+    byte = packed[:, k // 2].to(torch.int32)
+    nibble = torch.where(k % 2 == 0, byte & 15, byte >> 4)              # [N, M]
+    want = ((nibble - 8).float() * scales[k // 128].float().T).T.half()  # the product of two f16 values is exact in fp32
+    assert torch.equal(C.cpu(), want)

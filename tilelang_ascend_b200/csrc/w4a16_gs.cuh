@@ -25,9 +25,10 @@
 //   warp 1        bulk copies: prepared activations
 //   warps 2, 3    tcgen05.mma kind::f16 issuers (A = weights from tensor memory, B = activations from shared memory):
 //                 issuer w takes the slabs i with i % 2 == w, each of the two halves into its own accumulator
-//   warps 4..11   drain: tcgen05.ld of a half's accumulator, fp32 FMA with the half's scale into register sums; set e
-//                 (four warps, one per 32 rows) takes the slabs of parity e and the sets add their sums at a segment's
-//                 end; then the tile write or the split-K hand-over
+//   warps 4..11   drain: tcgen05.ld of a half's accumulator, fp32 FMA with the half's scale into register sums, in two sets of
+//                 four warps (one per 32 rows); then the tile write or the split-K hand-over.  16 tokens: set e takes the
+//                 slabs of parity e and the sets add their sums at a segment's end.  32 and 64 tokens: set e takes half of
+//                 the tokens of every slab
 //   warps 12..19  dequant: set s (four warps, one per 32 rows) converts the slabs of parity s
 //   warps 20..23  split-K hand-overs
 // Tensor memory: NS slots of two accumulators of MT columns + WS stages of 128 columns of converted weights.
@@ -84,7 +85,7 @@ struct W4GCfg {
   static_assert(MT == 16 || MT == 32 || MT == 64, "token tile");
   // Rings, in slabs.  64 KB of raw (packed) weights in flight per SM already stream at full speed.
   static constexpr int RS = (MT == 16) ? 8 : 4;           // raw weights, 16 KB each
-  static constexpr int AS = (MT == 16) ? 4 : (MT == 32 ? 6 : 3);  // activations
+  static constexpr int AS = (MT == 16) ? 4 : (MT == 32 ? 7 : 4);  // activations
   static constexpr int WS = (MT <= 32) ? 3 : 2;           // converted weights (tensor memory)
   static constexpr int NS = (MT == 16) ? 4 : 2;           // accumulator slots of two halves (even: a slot belongs to one set)
   static constexpr int SS = (RS == 8) ? 32 : 16;          // scale rows (see the note at the weight producer)
@@ -95,7 +96,14 @@ struct W4GCfg {
   // 64 tokens: tensor memory holds two slabs of converted weights only, so the hand-over to the MMAs and back is by
   // halves - otherwise both sets convert while the tensor pipe idles and then both wait for it.
   static constexpr bool HALVES = MT == 64;
-  static constexpr int XBUF_BYTES = MT * W4_BN * 4;       // the second drain set's sums of one segment
+  // Above 16 tokens each drain set takes half of the tokens of every slab, so that a thread has one load of a half's sums to
+  // wait for instead of a chain of them (64 tokens, 8192 x 28672: 41.2 -> 36.9 us; back to back for seconds, where the power
+  // limit sets the clock, 48.3 -> 45.1; 48 tokens, 8192 x 8192, zeros tensor 22.4 -> 19.4).  Giving accumulators and converted
+  // weights back half by half, in rings of 3 + 5 or 4 + 4 halves, was slower: 51.1 and 47.7.
+  static constexpr bool BY_TOKENS = MT > 16;
+  static constexpr int DT = BY_TOKENS ? MT / 2 : MT;      // tokens a drain thread accumulates
+  static constexpr int DRAIN_WARPS = BY_TOKENS ? W4G_EPI_WARPS : W4G_EPI_WARPS / 2;  // that read a slab's accumulators
+  static constexpr int XBUF_BYTES = BY_TOKENS ? 0 : MT * W4_BN * 4;  // the second drain set's sums of one segment
   static constexpr int SMEM_BYTES = RS * W4_RAW_PACKED + AS * A_BYTES + SS * W4G_SC_BYTES + (ZT ? RS * W4G_SC_BYTES : 0) +
                                     XBUF_BYTES + BAR_BYTES + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
@@ -389,10 +397,10 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     else if (off < W4G_W_FULL) count = 1;
     else if (off < W4G_DONE) count = 4;
     else if (off < W4G_ACC_EMPTY) count = 1;
-    else if (off < W4G_W_FULL0) count = 4;     // the four drain warps of the slab's set
+    else if (off < W4G_W_FULL0) count = Cfg::DRAIN_WARPS;
     else if (off < W4G_DONE0) count = 4;
     else if (off < W4G_PART_READY) count = 1;
-    else if (off < W4G_DRAIN) count = 4;       // the four warps of drain set 0
+    else if (off < W4G_DRAIN) count = Cfg::DRAIN_WARPS;
     else if (off < W4G_PART_FULL) count = W4G_MMA_WARPS;
     else if (SMALL) count = max((int)cluster_nctarank() - 1, 1);
     if (count > 0) mbar_init(reinterpret_cast<uint64_t*>(bar_block + off), (uint32_t)count);
@@ -435,12 +443,13 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const int n_sk = (int)(item1 - item0);
   const int n_slabs = SMALL ? n_sk : n_sk + p.dp_rounds * p.KS;  // this CTA's slabs, numbered 0.. in processing order
 
-  // 64 tokens: a drain thread keeps 64 sums, more than the 80 registers the block is launched with; the warp groups that
-  // need few give theirs up (48 + 2 x 104 + 2 x 80 + 64 = 6 x 80).
+  // 64 tokens: a drain thread holds 32 sums and 32 values on their way into them, a hand-over thread two contributors' values,
+  // more than the 80 registers the block is launched with; the producers and issuers give theirs up (48 + 2 x 88 + 2 x 80 + 96 =
+  // 6 x 80).
   if constexpr (MT == 64) {
     if (warp < W4G_FIRST_EPI_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-    else if (warp >= W4G_FIN_WARP) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    else if (warp < W4G_FIRST_DQ_WARP) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    else if (warp >= W4G_FIN_WARP) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+    else if (warp < W4G_FIRST_DQ_WARP) asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
   }
   if (warp < 2) {
     // ------------------------------------------------------------------ producers
@@ -607,7 +616,8 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t sc_row1 = p.scale_rows == 2 ? 256u : 0u;  // the second half's scale row inside a stage
     const bool scaled = p.has_scales != 0;
     const bool lead = lane == 0;
-    constexpr int DT = MT;  // tokens a drain thread accumulates
+    constexpr int DT = Cfg::DT;
+    const int t_first = Cfg::BY_TOKENS ? e * DT : 0;  // first of this set's tokens
     if constexpr (!SMALL) pdl_wait();  // the arrival counters are zeroed by the pre-pass kernel in front of this one
     if constexpr (SMALL) {
       // this CTA's piece of the activations: rows m0 .. m0 + 15 (zero beyond M), k [256 * ks_first, 256 * (ks_first + per))
@@ -664,63 +674,74 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       float psum[DT];
 #pragma unroll
       for (int m = 0; m < DT; ++m) psum[m] = 0.f;
-      for (uint32_t i = i_seg0 + ((i_seg0 ^ (uint32_t)e) & 1u); i < i_end; i += 2) {
+      for (uint32_t i = Cfg::BY_TOKENS ? i_seg0 : i_seg0 + ((i_seg0 ^ (uint32_t)e) & 1u); i < i_end; i += Cfg::BY_TOKENS ? 1 : 2) {
         const uint32_t slot = i % NS;
         const uint32_t bs = bar0 + 8 * slot;
-        w4g_wait<W4G_DONE, ST_TIMEOUT_EPILOGUE>(bar0 + 8 * (i % W4G_BARS), (i / W4G_BARS) & 1u, ctl, fail);
-        tc_fence_after_sync();
-        const uint32_t ta = tmem_base + lane_addr + slot * (2 * MT);
-        uint32_t r[32];  // two pieces of 16 columns (16 tokens: the two halves)
-        if constexpr (MT == 16) {
-          tmem_ld_32x32b_x32(ta, r);
-        }
+        const uint32_t bd = bar0 + 8 * (i % W4G_BARS), dpar = (i / W4G_BARS) & 1u;
+        const uint32_t ta = tmem_base + lane_addr + slot * (2 * MT) + t_first;
         float s0 = 1.0f, s1 = 1.0f;
-        if (scaled) {
-          uint16_t h0, h1;
-          const uint32_t sa = sc_addr0 + (i % Cfg::SS) * W4G_SC_BYTES;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sa));
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sa + sc_row1));
-          s0 = __half2float(__ushort_as_half(h0));
-          s1 = __half2float(__ushort_as_half(h1));
-        }
-        if constexpr (MT == 16) {
+        auto load_scales = [&]() {  // after the slab's MMAs, see the note at the weight producer
+          if (scaled) {
+            uint16_t h0, h1;
+            const uint32_t sa = sc_addr0 + (i % Cfg::SS) * W4G_SC_BYTES;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sa));
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sa + sc_row1));
+            s0 = __half2float(__ushort_as_half(h0));
+            s1 = __half2float(__ushort_as_half(h1));
+          }
+        };
+        auto release = [&]() {  // the accumulators are in registers
           tmem_ld_wait();
           tc_fence_before_sync();
           __syncwarp();
           if (lead) w4g_arrive<W4G_ACC_EMPTY>(bs);
+        };
+        if constexpr (DT == 16) {
+          w4g_wait<W4G_DONE, ST_TIMEOUT_EPILOGUE>(bd, dpar, ctl, fail);
+          tc_fence_after_sync();
+          uint32_t r[32];  // the two halves
+          if constexpr (MT == 16) {
+            tmem_ld_32x32b_x32(ta, r);
+          } else {
+            tmem_ld_32x32b_x16(ta, reinterpret_cast<uint32_t(&)[16]>(r[0]));
+            tmem_ld_32x32b_x16(ta + MT, reinterpret_cast<uint32_t(&)[16]>(r[16]));
+          }
+          load_scales();
+          release();
 #pragma unroll
           for (int m = 0; m < 16; m += 2) {
             w4g_fma2(psum[m], psum[m + 1], r[m], r[m + 1], s0);
             w4g_fma2(psum[m], psum[m + 1], r[16 + m], r[17 + m], s1);
           }
-        } else {
+        } else {  // the first half's sums while the second half's MMAs run
+          uint32_t r[32];
+          w4g_wait<W4G_DONE0, ST_TIMEOUT_EPILOGUE>(bd, dpar, ctl, fail);
+          tc_fence_after_sync();
+          tmem_ld_32x32b_x32(ta, r);
+          load_scales();
+          tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < 2 * MT / 16; ++c) {  // 16 columns at a time: the first half's tokens, then the second's
-            uint32_t q16[16];
-            tmem_ld_32x32b_x16(ta + 16 * c, q16);
-            tmem_ld_wait();
-            if (c == 2 * MT / 16 - 1) {
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lead) w4g_arrive<W4G_ACC_EMPTY>(bs);
-            }
-            const int t0 = 16 * (c % (MT / 16));
-            const float sc = c < MT / 16 ? s0 : s1;
+          for (int m = 0; m < 32; m += 2) w4g_fma2(psum[m], psum[m + 1], r[m], r[m + 1], s0);
+          w4g_wait<W4G_DONE, ST_TIMEOUT_EPILOGUE>(bd, dpar, ctl, fail);
+          tc_fence_after_sync();
+          tmem_ld_32x32b_x32(ta + MT, r);
+          release();
 #pragma unroll
-            for (int m = 0; m < 16; m += 2) w4g_fma2(psum[t0 + m], psum[t0 + m + 1], q16[m], q16[m + 1], sc);
-          }
+          for (int m = 0; m < 32; m += 2) w4g_fma2(psum[m], psum[m + 1], r[m], r[m + 1], s1);
         }
       }
       i_seg0 = i_end;
-      // Segment end.  Set 1 hands over its sums through shared memory; set 0 adds them and writes the tile, or its partial
-      // sums to the scratch buffer, where the split-K warp takes over.  (A wait that gave up does not change the course of
-      // events here: all waits of the CTA then give up quickly, and the status word says that C is unspecified.)
+      // Segment end.  16 tokens: set 1 hands over its sums through shared memory, set 0 adds them.  The tile is written, or the
+      // partial sums to the scratch buffer, where the split-K warps take over.  (A wait that gave up does not change the course
+      // of events here: all waits of the CTA then give up quickly, and the status word says that C is unspecified.)
       float* xb = xbuf + nl;
-      if (e == 1) {
+      if constexpr (!Cfg::BY_TOKENS) {
+        if (e == 1) {
 #pragma unroll
-        for (int j = 0; j < DT; ++j) xb[j * W4_BN] = psum[j];
+          for (int j = 0; j < DT; ++j) xb[j * W4_BN] = psum[j];
+        }
+        w4g_epi_bar();
       }
-      w4g_epi_bar();
       if constexpr (SMALL) {
         // One segment per CTA.  Set 0 holds the CTA's sums; CTAs 1 .. C-1 of the cluster write theirs into the first
         // CTA's landing area (the raw ring's stages 4 .. 7, never filled in this form) and signal it; the first CTA
@@ -770,13 +791,15 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
         break;
       }
-      if (e == 0) {
+      if (Cfg::BY_TOKENS || e == 0) {
+        if constexpr (!Cfg::BY_TOKENS) {
 #pragma unroll
-        for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
+          for (int j = 0; j < DT; ++j) psum[j] += xb[j * W4_BN];
+        }
         if (full_tile) {
-          if (n < p.N) w4g_store_tile<MT, OUT_BF16, GATHER>(p, b, m0, n, psum);
+          if (n < p.N) w4g_store_tile<DT, OUT_BF16, GATHER>(p, b, m0 + t_first, n, psum);
         } else {
-          float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + nl;
+          float* dst = p.ws_partials + (size_t)my_slot * (MT * W4_BN) + (size_t)t_first * W4_BN + nl;
 #pragma unroll
           for (int j = 0; j < DT; ++j) dst[j * W4_BN] = psum[j];
           __syncwarp();
@@ -784,7 +807,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           ++n_partial;
         }
       }
-      w4g_epi_bar();  // set 0 has read the exchange buffer
+      if constexpr (!Cfg::BY_TOKENS) w4g_epi_bar();  // set 0 has read the exchange buffer
     }
   } else if (warp >= W4G_FIN_WARP) {
     // ------------------------------------------------------------------ split-K hand-over
@@ -821,8 +844,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
         const int n = n0 + 4 * lane;  // four rows of the tile per lane
         const int rows = min(MT, p.M - m0);
-        // four tokens of two contributors in flight; of one with 64 tokens, where the second one's would spill
-        constexpr int RU = 4, CU = MT == 64 ? 1 : 2;
+        constexpr int RU = 4, CU = 2;  // four tokens of two contributors in flight
         // every contributor but the last one stops short of the tile's end: its partial tile is its second one (slot 2 c + 1)
         auto part = [&](int c, int m) {
           return reinterpret_cast<const float4*>(p.ws_partials + (size_t)(c == b_last ? 2 * c : 2 * c + 1) * (MT * W4_BN) +
