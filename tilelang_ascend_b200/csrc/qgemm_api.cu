@@ -247,7 +247,7 @@ int launch_w8_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const qg::W8R
   static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(qg::W8_THREADS);
+  cfg.blockDim = dim3(qg::W8R_THREADS);
   cfg.dynamicSmemBytes = (size_t)qg::W8R_SMEM_BYTES;
   cfg.stream = s;
   cudaLaunchAttribute attr[2] = {};

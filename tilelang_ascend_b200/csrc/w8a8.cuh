@@ -4,7 +4,8 @@
 // Persistent, warp-specialised kernel. One CTA per SM walks a list of 128 x BN output tiles:
 //   warp 0      TMA producer: A tile [128 x 128 B] and B tile into a multistage shared-memory ring
 //   warp 1      tcgen05.mma kind::i8 issuer; int32 accumulators live in tensor memory, double buffered
-//   warps 2..5  epilogue: tcgen05.ld -> cvt.rn.f32.s32 -> fp32 scale(s) -> cvt.rn f16/bf16 -> 16-byte stores
+//   warps 2..9  epilogue: tcgen05.ld -> cvt.rn.f32.s32 -> fp32 scale(s) -> cvt.rn f16/bf16 -> staging tile -> bulk store; two
+//               warps per 32 rows, each with half of the columns
 // B is consumed in the operator's own [K, N] row-major layout as an MN-major operand (no transpose
 // pass), or in [N, K] layout as a K-major operand.
 #pragma once
@@ -48,7 +49,8 @@ struct W8Tile {
 constexpr int W8_BM = 128;      // tile rows (= MMA M, one TMEM lane per row)
 constexpr int W8_BK = 128;      // K bytes per pipeline stage (one 128-byte swizzle atom)
 constexpr int W8_UMMA_K = 32;   // K per tcgen05.mma for 8-bit operands
-constexpr int W8_THREADS = 192;
+constexpr int W8_EPI_WARPS = 8;
+constexpr int W8_THREADS = (2 + W8_EPI_WARPS) * 32;
 
 template <int BN>
 struct W8Cfg {
@@ -58,9 +60,10 @@ struct W8Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int BAR_BYTES = 256;
-  static constexpr int SCALE_BYTES = 4 * BN * 4;  // each epilogue warp's copy of the tile's column scales
-  static constexpr int OUT_BYTES = 4 * 4096;      // each epilogue warp's staging tile: 32 rows x 64 outputs
+  static constexpr int SCALE_BYTES = W8_EPI_WARPS * 32 * 4;  // each epilogue warp's scales of 32 columns
+  static constexpr int OUT_BYTES = W8_EPI_WARPS * 4096;      // each epilogue warp's staging tile: 32 rows x 64 outputs
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + BAR_BYTES + SCALE_BYTES + 1024;  // + alignment slack
+  static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
 };
 
 __device__ __forceinline__ void w8_decode_tile(const W8A8Params& p, int tile, int& b, int& m_blk, int& n_blk) {
@@ -105,7 +108,7 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
   return t;
 }
 
-// Grouped form, rows of C that no table entry covers: set to zero by the four epilogue warps before their first tile
+// Grouped form, rows of C that no table entry covers: set to zero by four of the epilogue warps before their first tile
 // (they would otherwise wait for it), dealt to all CTAs; a launch that is sure to have such rows has a CTA on every SM,
 // with or without a tile (w8a8_impl).  A clear of the whole output in front of the launch cost a pass over C (33 MB for
 // 8192 x 2048: 8 us of 137) although normally every row is covered.  us, in the kernel / cleared in front: 4096 x 2048 with
@@ -194,11 +197,11 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(stages_free, 4);
-    mbar_init(partial_full, 4);
+    mbar_init(stages_free, W8_EPI_WARPS);
+    mbar_init(partial_full, W8_EPI_WARPS);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
-      mbar_init(&tempty[i], 4);
+      mbar_init(&tempty[i], W8_EPI_WARPS);
     }
     if (p.tma_store) tma_prefetch_desc(&tmC);
     mbar_init(drain, 1);
@@ -311,15 +314,18 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     // ---------------------------------------------------------------- epilogue
-    // Each warp stages the tile's column scales in its own piece of shared memory BEFORE it waits for the
-    // accumulators (the loads hide behind the main loop), and keeps the next 32-column chunk's tcgen05.ld in
-    // flight while it converts and stores the current one.
-    const int q = warp & 3;  // TMEM lane quadrant this warp may read
+    // A warp keeps the next 32-column chunk's tcgen05.ld and column scales (a scale per lane, handed round through 128 bytes of
+    // shared memory) in flight while it converts and stores the current one.  With four warps a tile of 128 x 256 took 6 us
+    // from the end of its MMAs, more than its MMAs below K = 2048, and as much again at the end of every launch:
+    // 4096 x 1024 x 4096 29.0 -> 20.9 us, 3000 x 1024 x 1024 12.3 -> 10.3, 512 x 512 x 4096 8.2 -> 7.2, 4000 rows in 32 groups,
+    // K = 1024, N = 4096 52.7 -> 43.1; K = 4096 and more as before (the power limit).
+    const int q = warp & 3;         // TMEM lane quadrant this warp may read
+    const int e = (warp - 2) >> 2;  // which half of the columns
     const uint64_t pol_out = l2_policy_evict_first();  // the output is written once and not read here
-    float* sb_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES) + q * BN;
-    uint8_t* my_stage = out_stage + q * 4096;  // [32 rows][128 B], 16-byte piece j of row r at (j ^ (r & 7))
+    float* sb_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES) + (warp - 2) * 32;
+    uint8_t* my_stage = out_stage + (warp - 2) * 4096;  // [32 rows][128 B], 16-byte piece j of row r at (j ^ (r & 7))
     int it = 0;
-    if (p.zero_uncovered) w8_zero_uncovered(p, q, lane);
+    if (p.zero_uncovered && e == 0) w8_zero_uncovered(p, q, lane);
     // split form: the other CTA's accumulators travel through CTA 0's pipeline stages, one 16-byte piece per
     // (row, four columns): piece (col / 4, row) at ((col / 4) * 128 + row) * 16, so that a warp's 32 rows are
     // 512 contiguous bytes for the sender's stores and the receiver's loads alike
@@ -332,38 +338,37 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const bool row_ok = q * 32 + lane < t.rows;
       float sa = 1.0f;
       if (p.sa_mode != 0 && row_ok) sa = __ldg(p.scale_a + (p.sa_mode == 2 ? (size_t)t.bA * p.M : 0) + m);
-      if (p.C != nullptr) {
-        const float* sbp = p.scale_b + (p.sb_mode == 2 ? (size_t)t.bB * p.N : 0);
-        __syncwarp();  // the previous tile's reads of sb_s are done
-        for (int c = lane; c < t.bn; c += 32) {
-          const int n = t.n0 + c;
-          sb_s[c] = (p.sb_mode == 0) ? __ldg(sbp) : (n < p.N ? __ldg(sbp + n) : 0.f);
-        }
-        __syncwarp();
-      }
+      const float* sbp = p.scale_b + (p.sb_mode == 2 ? (size_t)t.bB * p.N : 0);
+      auto column_scale = [&](int c) {  // of this lane's column of chunk c
+        const int n = t.n0 + c * 32 + lane;
+        return p.C == nullptr ? 0.f : (p.sb_mode == 0 ? __ldg(sbp) : (n < p.N ? __ldg(sbp + n) : 0.f));
+      };
+      // This warp's chunks of 32 columns.  Split form: of the half of the tile that this CTA finishes.
+      const int own_chunks = (SPLITK ? t.bn >> 6 : t.bn >> 5) >> 1;
+      const int c_begin = (SPLITK ? crank * (t.bn >> 6) : 0) + e * own_chunks, chunks = c_begin + own_chunks;
+      float sb_next = column_scale(c_begin);
       if (!mbar_wait_warp(&tfull[buf], tphase, ctl, ST_TIMEOUT_EPILOGUE)) break;
       tc_fence_after_sync();
       // Split form: each CTA of the pair finishes ONE half of the tile's columns (CTA r: columns r * bn/2 ...): it sends
       // its accumulators of the other half into the peer's pipeline stages and receives the peer's for its own, so
       // that the exchange runs in both directions at once and each CTA converts and stores half a tile.
-      int c_begin = 0, c_end = t.bn >> 5;
       if constexpr (SPLITK) {
         const uint32_t taddr_s = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
         const uint32_t peer = (uint32_t)(crank ^ 1);
-        const int half_chunks = t.bn >> 6;  // 32-column chunks per half
+        const int peer_begin = (int)peer * (t.bn >> 6) + e * own_chunks;  // the chunks that this warp sends
         // this CTA's MMAs are done (tfull): the peer may write into its stages
         if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(stages_free), peer));
-        // ... and the peer's are done when its four epilogue warps have said so here
+        // ... and the peer's are done when its epilogue warps have said so here
         if (!mbar_wait_warp(stages_free, 0, ctl, ST_TIMEOUT_EPILOGUE)) break;
         const uint32_t dst_row = mapa_u32(part_row, peer);
 #pragma unroll 1
-        for (int c = 0; c < half_chunks; ++c) {
+        for (int c = 0; c < own_chunks; ++c) {
           uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr_s + ((int)peer * half_chunks + c) * 32, r);
+          tmem_ld_32x32b_x32(taddr_s + (peer_begin + c) * 32, r);
           tmem_ld_wait();
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj)
-            st_cluster_v4(dst_row + (uint32_t)((c * 8 + jj) * 128 * 16), r[4 * jj], r[4 * jj + 1], r[4 * jj + 2], r[4 * jj + 3]);
+            st_cluster_v4(dst_row + (uint32_t)(((e * own_chunks + c) * 8 + jj) * 128 * 16), r[4 * jj], r[4 * jj + 1], r[4 * jj + 2], r[4 * jj + 3]);
         }
         fence_acq_rel_cluster();
         __syncwarp();
@@ -384,12 +389,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
         if (!got) break;
         fence_acq_rel_cluster();
-        c_begin = crank * half_chunks;
-        c_end = c_begin + half_chunks;
       }
       const size_t row_off = ((size_t)t.bA * p.M + (row_ok ? m : 0)) * (size_t)p.N;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
-      const int chunks = c_end;
       // Whole row blocks go out as tiled bulk stores (coalesced, clipped at the tensor's edge); a partial
       // block of the grouped form must not touch the rows after it and uses per-row stores.
       const bool tma_out = p.tma_store != 0 && (p.meta == nullptr || t.rows == W8_BM);
@@ -405,6 +407,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int h = 0; h < 2; ++h) {
           const int c = c2 + h;
           if (c >= chunks) break;
+          __syncwarp();  // the previous chunk's reads of sb_s are done
+          sb_s[lane] = sb_next;
+          __syncwarp();
+          if (c + 1 < chunks) sb_next = column_scale(c + 1);
           tmem_ld_wait();                                                     // chunk c is in r[h]
           if (c + 1 < chunks) tmem_ld_32x32b_x32(taddr + (c + 1) * 32, r[h ^ 1]);  // chunk c + 1 in flight
           if constexpr (SPLITK) {  // add the other CTA's half of the K range (exact: int32)
@@ -413,7 +419,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               uint4 pv;
               asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                            : "=r"(pv.x), "=r"(pv.y), "=r"(pv.z), "=r"(pv.w)
-                           : "r"(part_row + (uint32_t)(((c - c_begin) * 8 + j) * 128 * 16)));
+                           : "r"(part_row + (uint32_t)(((c - crank * (t.bn >> 6)) * 8 + j) * 128 * 16)));
               r[h][4 * j] += pv.x;
               r[h][4 * j + 1] += pv.y;
               r[h][4 * j + 2] += pv.z;
@@ -430,7 +436,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           if (tma_out) {
             if (n < p.N) {
-              const float4* sv = reinterpret_cast<const float4*>(sb_s + c * 32);
+              const float4* sv = reinterpret_cast<const float4*>(sb_s);
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const float4 s_lo = sv[2 * j], s_hi = sv[2 * j + 1];
@@ -452,7 +458,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           } else if (row_ok && n < p.N) {
             if (p.C != nullptr) {
               uint16_t* cbase = reinterpret_cast<uint16_t*>(p.C) + row_off + n;
-              const float4* sv = reinterpret_cast<const float4*>(sb_s + c * 32);
+              const float4* sv = reinterpret_cast<const float4*>(sb_s);
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 if (n + 8 * j < p.N) {

@@ -24,6 +24,7 @@
 
 namespace qg {
 
+constexpr int W8R_THREADS = 192;
 constexpr int W8R_MAX_MT = 128;
 constexpr int W8R_MAX_SPLIT = 8;
 constexpr int W8R_RING_BYTES = 96 * 1024;  // two CTAs per SM
@@ -45,7 +46,7 @@ struct W8RowsParams {
 };
 
 template <bool B_NK, bool OUT_BF16>
-__global__ void __launch_bounds__(W8_THREADS, 2)
+__global__ void __launch_bounds__(W8R_THREADS, 2)
 w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const W8RowsParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
