@@ -302,3 +302,21 @@ def test_few_tokens_behind_the_quantiser():
     ref = chain(True)
     for _ in range(5):
         assert torch.equal(chain(False), ref)
+
+
+# Tiles of 256 x 256 made by two CTAs: one round of them and two, with the last one cut in half-width items; rows that end in the
+# first or in the second CTA's half of a tile, one row into it or with it; columns that end in either CTA's half of B; K with a
+# remainder of 16; several problems.
+@pytest.mark.parametrize("batch,M,K,N", [(0, 1300, 3072, 2064), (0, 1281, 3088, 2304), (0, 1409, 4096, 2192),
+                                         (0, 2200, 3072, 2320), (3, 520, 4112, 2048), (9, 256, 3072, 2320)])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_tiles_of_two_ctas_are_exact(batch, M, K, N, layout):
+    q = _q()
+    A, B, sa, sb = oc.make_w8a8_inputs(batch, M, K, N, seed=M + N)
+    odt = "bfloat16" if layout == "KN" else "float16"
+    ref, acc_ref = oc.quant_matmul_ref(A, B, sb, odt, scale_a=sa, return_acc=True)
+    Bd = (B if layout == "KN" else B.transpose(-1, -2).contiguous()).cuda()
+    C = q.quant_matmul(A.cuda(), Bd, sb.cuda(), scale_a=sa.cuda(), out_dtype=odt, b_layout=layout)
+    _cmp(C, ref)
+    acc = q.quant_matmul(A.cuda(), Bd, sb.cuda(), out_dtype="int32", b_layout=layout)
+    assert torch.equal(acc.cpu(), acc_ref)

@@ -64,11 +64,16 @@ int set_smem_w8() {
   if (set_smem(qg::w8a8_gemm_kernel<BN, false, true>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w8a8_gemm_kernel<BN, true, false>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w8a8_gemm_kernel<BN, true, true>, C::SMEM_BYTES)) return -1;
-  if (BN == 256) {  // the two-CTA K split
-    if (set_smem(qg::w8a8_gemm_kernel<256, false, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, false, true, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, true>, C::SMEM_BYTES)) return -1;
+  if constexpr (BN == 256) {  // the forms of two CTAs
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, false, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, true, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
+    constexpr int pair_bytes = qg::W8Cfg<256, qg::W8_PAIR>::SMEM_BYTES;
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, false, qg::W8_PAIR>, pair_bytes)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, false, true, qg::W8_PAIR>, pair_bytes)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, qg::W8_PAIR>, pair_bytes)) return -1;
+    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, qg::W8_PAIR>, pair_bytes)) return -1;
   }
   return 0;
 }
@@ -221,14 +226,14 @@ int launch_w8(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap&
   return 0;
 }
 
-// The K split: clusters of two CTAs, one 128 x 256 tile per cluster.
-template <bool NK, bool BF>
-int launch_w8_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p,
-                     int tiles, cudaStream_t s) {
+// The forms in which a cluster of two CTAs makes a tile: `clusters` of them.
+template <bool NK, bool BF, qg::W8Form FORM>
+int launch_w8_clusters(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p,
+                       int clusters, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * tiles));
+  cfg.gridDim = dim3((unsigned)(2 * clusters));
   cfg.blockDim = dim3((unsigned)qg::W8_THREADS);
-  cfg.dynamicSmemBytes = (size_t)qg::W8Cfg<256>::SMEM_BYTES;
+  cfg.dynamicSmemBytes = (size_t)qg::W8Cfg<256, FORM>::SMEM_BYTES;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -237,8 +242,14 @@ int launch_w8_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, true>, tmA, tmB, tmC, p));
+  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, FORM>, tmA, tmB, tmC, p));
   return 0;
+}
+template <qg::W8Form FORM>
+int launch_w8_clusters(bool nk, bool bf, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                       const qg::W8A8Params& p, int clusters, cudaStream_t s) {
+  if (nk) return bf ? launch_w8_clusters<true, true, FORM>(tmA, tmB, tmC, p, clusters, s) : launch_w8_clusters<true, false, FORM>(tmA, tmB, tmC, p, clusters, s);
+  return bf ? launch_w8_clusters<false, true, FORM>(tmA, tmB, tmC, p, clusters, s) : launch_w8_clusters<false, false, FORM>(tmA, tmB, tmC, p, clusters, s);
 }
 
 // Few-token form: clusters of S CTAs, a programmatic dependent of whatever is in front of it on the stream.
@@ -526,6 +537,25 @@ static int w8_rows_split(int64_t tiles, int64_t k_blocks, int64_t tokens, int sm
   return saved >= (tokens <= 96 ? 7 : 9) || (saved >= 6 && 2 * ctas <= sms) ? S : 0;
 }
 
+// Whether two CTAs per tile of 256 x 256 (PAIR of w8a8.cuh) are faster than one per tile of 128 x 256 or 128 x 128.  Counted in
+// rounds of 128 x 256 tiles over the SMs: a last round that is cut in half-width items counts 0.6, a round of 128 x 128 tiles
+// 0.55, a round of pairs 0.87; the pairs' longer start and hand-over of a tile count the less the longer K is.  From a sweep over
+// 400 shapes, K 512 .. 8192, 64 .. 3500 tiles of 128 x 256, both layouts (us, one / two CTAs per tile): 4096 x 4096 x 14336
+// 166 / 150, 4096 x 2048 x 4096 31.5 / 30.0, 1300 x 2048 x 8192 23.8 / 24.7 (2.6 rounds against 3), 512 x 8192 x 5120 36.2 / 28.9,
+// but 4096 x 1024 x 4096 19.6 / 22.4.  QGEMM_W8_PAIR=0 disables it.
+static bool w8_pair_pays(int64_t batch, int64_t M, int64_t N, int64_t k_blocks, bool kn, int64_t sms) {
+  static const int pair_on = getenv("QGEMM_W8_PAIR") ? atoi(getenv("QGEMM_W8_PAIR")) : 1;
+  if (!pair_on || N <= 128 || k_blocks < 16) return false;
+  auto rounds = [](int64_t tiles, int64_t workers, bool halves) {
+    const int64_t whole = tiles / workers, left = tiles % workers;
+    return (double)whole + (left == 0 ? 0.0 : (halves && whole != 0 && 2 * left <= workers ? 0.6 : 1.0));
+  };
+  const int64_t row_blocks = (M + 127) / 128, tiles256 = batch * row_blocks * ((N + 255) / 256);
+  const double one = tiles256 >= sms ? rounds(tiles256, sms, kn) : 0.55 * rounds(batch * row_blocks * ((N + 127) / 128), sms, false);
+  const double two = rounds(batch * ((M + 255) / 256) * ((N + 255) / 256), sms / 2, true);
+  return two * (0.87 + 1.3 / (double)k_blocks) + 2.4 / (double)k_blocks < one;
+}
+
 // Plain / batched form: meta == nullptr.  Grouped form: A and C are single [M, K] / [M, N] stacks, B holds
 // `batch` (= groups) matrices and `meta` lists num_blocks row blocks (group, first row, valid rows).
 static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, const float* scale_a, void* C,
@@ -601,8 +631,8 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
     const uint32_t box[3] = {128, 128, 1};
     if (encode_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, A, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   }
-  const int64_t m_tiles = meta ? num_blocks : (M + 127) / 128;
-  const int64_t tiles256 = batchA * m_tiles * ((N + 255) / 256);
+  const int64_t row_blocks = meta ? num_blocks : (M + 127) / 128;
+  const int64_t tiles256 = batchA * row_blocks * ((N + 255) / 256);
   // Fewer 256-wide tiles than half the SMs: split K over pairs of CTAs (one tile per pair, twice as many SMs at
   // work on full-width tiles) instead of falling back to 128-wide tiles - when K is long enough to pay for the
   // cluster launch and the exchange: on 2 x 512 x K x 2048, split against 128-wide tiles, K = 7168: 19.8 / 23.6 us,
@@ -610,7 +640,10 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   // QGEMM_W8_SPLITK=0 disables it.
   static const int splitk_on = getenv("QGEMM_W8_SPLITK") ? atoi(getenv("QGEMM_W8_SPLITK")) : 1;
   const bool use_splitk = splitk_on && meta == nullptr && N > 128 && 2 * tiles256 <= sms && (K + 127) / 128 >= 32;
-  const int BN = (N > 128 && (tiles256 >= sms || use_splitk)) ? 256 : 128;
+  // Otherwise two CTAs per tile of 256 x 256 where that is the faster one (w8_pair_pays).
+  const bool use_pair = meta == nullptr && !use_splitk && w8_pair_pays(batch, M, N, k_blocks, b_layout == QGEMM_B_KN, sms);
+  const int BN = (N > 128 && (tiles256 >= sms || use_splitk || use_pair)) ? 256 : 128;
+  const int64_t m_tiles = use_pair ? (M + 255) / 256 : row_blocks;  // of 128 rows, of 256 for two CTAs
   // Width actually computed per tile (a multiple of 32, at most BN).  Narrower tiles that fill the last
   // round of the persistent grid better were measured slower on B200 (224 instead of 256 columns on the
   // 4096 x 4096 x 14336 shape: 235 us against 231 us), so the full width is used.
@@ -623,7 +656,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   } else {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)K, (uint64_t)N * (uint64_t)K};
-    const uint32_t box[3] = {128, (uint32_t)BN, 1};
+    const uint32_t box[3] = {128, (uint32_t)(use_pair ? 128 : BN), 1};
     if (encode_map(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, B, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   }
 
@@ -655,7 +688,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.sb_mode = (scale_b_len == 1) ? 0 : ((scale_b_len == N) ? 1 : 2);
   p.sa_mode = (scale_a == nullptr) ? 0 : ((scale_a_len == M) ? 1 : 2);
   p.m_tiles = (int)m_tiles;
-  p.group_m = w8_group_m(m_tiles, K);
+  p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K) + 1) / 2 : w8_group_m(m_tiles, K);
   p.n_tiles = (int)((N + bn_eff - 1) / bn_eff);
   p.bn = bn_eff;
   const int64_t num_tiles = batchA * p.m_tiles * p.n_tiles;
@@ -666,14 +699,15 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.wait_limit_ns = g_wait_limit_ns;
   // with rows that no block can cover, a CTA per SM to clear them, whatever the number of tiles
   const bool sure_to_clear = p.zero_uncovered && M > num_blocks * qg::W8_BM;
-  const int grid = (int)(num_tiles < sms && !sure_to_clear ? num_tiles : sms);
+  const int workers = use_pair ? sms / 2 : sms;  // CTAs, or pairs of them
+  const int grid = (int)(num_tiles < workers && !sure_to_clear ? num_tiles : workers);
   // Tail split: when the last round of the persistent grid would run R < grid/2 tiles, those tiles are issued
   // as 2R half-width items instead ([K, N] layout, 256-column tiles).
   p.split_from = p.num_items = p.num_tiles;
   {
     static const int tail_split = getenv("QGEMM_W8_TAIL_SPLIT") ? atoi(getenv("QGEMM_W8_TAIL_SPLIT")) : 1;
     const int64_t R = num_tiles % grid;
-    if (tail_split && b_layout == QGEMM_B_KN && BN == 256 && num_tiles > grid && R > 0 && 2 * R <= grid) {
+    if (tail_split && (use_pair || b_layout == QGEMM_B_KN) && BN == 256 && num_tiles > grid && R > 0 && 2 * R <= grid) {
       p.split_from = (int)(num_tiles - R);
       p.num_items = (int)(num_tiles + R);
     }
@@ -681,10 +715,8 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool nk = b_layout == QGEMM_B_NK;
   const bool bf = out_dtype == QGEMM_DT_BF16;
-  if (use_splitk) {
-    if (nk) return bf ? launch_w8_splitk<true, true>(tmA, tmB, tmC, p, (int)num_tiles, s) : launch_w8_splitk<true, false>(tmA, tmB, tmC, p, (int)num_tiles, s);
-    return bf ? launch_w8_splitk<false, true>(tmA, tmB, tmC, p, (int)num_tiles, s) : launch_w8_splitk<false, false>(tmA, tmB, tmC, p, (int)num_tiles, s);
-  }
+  if (use_splitk) return launch_w8_clusters<qg::W8_SPLITK>(nk, bf, tmA, tmB, tmC, p, (int)num_tiles, s);
+  if (use_pair) return launch_w8_clusters<qg::W8_PAIR>(nk, bf, tmA, tmB, tmC, p, grid, s);
   if (BN == 256) {
     if (nk) return bf ? launch_w8<256, true, true>(tmA, tmB, tmC, p, grid, s) : launch_w8<256, true, false>(tmA, tmB, tmC, p, grid, s);
     return bf ? launch_w8<256, false, true>(tmA, tmB, tmC, p, grid, s) : launch_w8<256, false, false>(tmA, tmB, tmC, p, grid, s);

@@ -52,11 +52,15 @@ constexpr int W8_UMMA_K = 32;   // K per tcgen05.mma for 8-bit operands
 constexpr int W8_EPI_WARPS = 8;
 constexpr int W8_THREADS = (2 + W8_EPI_WARPS) * 32;
 
-template <int BN>
+// How the CTAs of a launch share the work: each by itself; two cut a tile's K (see SPLITK below); or two make one tile of 256 x
+// 256 with MMAs over both (see PAIR below).
+enum W8Form { W8_ALONE, W8_SPLITK, W8_PAIR };
+
+template <int BN, W8Form FORM = W8_ALONE>
 struct W8Cfg {
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
+  static constexpr int STAGES = (FORM == W8_PAIR || BN == 128) ? 6 : 4;
   static constexpr int A_BYTES = W8_BM * W8_BK;
-  static constexpr int B_BYTES = BN * W8_BK;
+  static constexpr int B_BYTES = (FORM == W8_PAIR ? BN / 2 : BN) * W8_BK;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int BAR_BYTES = 256;
@@ -79,7 +83,8 @@ __device__ __forceinline__ void w8_decode_tile(const W8A8Params& p, int tile, in
   n_blk = in_band / gsz;
 }
 
-__device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
+template <bool PAIR>
+__device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item, int crank) {
   int b, m_blk, n_blk;
   W8Tile t;
   if (item < p.split_from) {
@@ -94,7 +99,7 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item) {
   }
   if (p.meta == nullptr) {
     t.bB = t.bA = b;
-    t.m0 = m_blk * W8_BM;
+    t.m0 = PAIR ? (2 * m_blk + crank) * W8_BM : m_blk * W8_BM;  // PAIR: a row block is 256 rows, 128 for each CTA
     t.rows = min(W8_BM, p.M - t.m0);
   } else {
     t.bB = __ldg(p.meta + 3 * m_blk);
@@ -162,12 +167,21 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
 // converts and stores half a tile.  The counterpart in the
 // reference is the K split of examples/gemm_splitk/example_tilelang_gemm_splitk.py:15-48, whose partial tiles meet
 // in global memory through atomic adds (src/tl_templates/ascend/common.h:249-259).
-template <int BN, bool B_NK, bool OUT_BF16, bool SPLITK = false>
+//
+// PAIR: a cluster of two CTAs makes tiles of 256 x 256 with MMAs over both (tcgen05.mma.cta_group::2): CTA r holds rows 128 r ..
+// of A and of the accumulator, and loads half of the columns of B, which the tensor cores of both read.  A k block costs each
+// CTA 32 KB of loads instead of 48, so that six of them are in flight instead of four, and B crosses from L2 once for 256 rows.
+// The leader (rank 0) issues; all bytes are counted on its barriers; its commits signal both CTAs, and the epilogue warps of both
+// hand an accumulator back to it.  Traffic is what bounds these shapes, for what it costs in time and, at the power limit, in
+// clock: 4096 x 4096 x 14336 166 -> 150 us (back to back for seconds 190 -> 175; 3.2 POPS, cuBLASLt's plain int8 GEMM 3.0),
+// 16 x 512 x 7168 x 2048 [N, K] 101 -> 91.  Which shapes take it: w8_pair_pays in qgemm_api.cu.
+template <int BN, bool B_NK, bool OUT_BF16, W8Form FORM = W8_ALONE>
 __global__ void __launch_bounds__(W8_THREADS, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const W8A8Params p) {
-  using Cfg = W8Cfg<BN>;
+  using Cfg = W8Cfg<BN, FORM>;
   constexpr int STAGES = Cfg::STAGES;
+  constexpr bool SPLITK = FORM == W8_SPLITK, PAIR = FORM == W8_PAIR;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -186,9 +200,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   // split form: CTA `crank` of the pair takes the k blocks [kb_begin, kb_end) of tile (block index / 2)
-  const int crank = SPLITK ? (int)cluster_ctarank() : 0;
-  const int tile_first = SPLITK ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int tile_stride = SPLITK ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int crank = FORM != W8_ALONE ? (int)cluster_ctarank() : 0;
+  const int tile_first = FORM != W8_ALONE ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int tile_stride = FORM != W8_ALONE ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   const int kb_begin = SPLITK ? (crank ? p.k_blocks / 2 : 0) : 0;
   const int kb_end = SPLITK ? (crank ? p.k_blocks : p.k_blocks / 2) : p.k_blocks;
 
@@ -201,7 +215,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     mbar_init(partial_full, W8_EPI_WARPS);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
-      mbar_init(&tempty[i], W8_EPI_WARPS);
+      mbar_init(&tempty[i], (PAIR ? 2 : 1) * W8_EPI_WARPS);  // PAIR: both CTAs', on the leader's barrier
     }
     if (p.tma_store) tma_prefetch_desc(&tmC);
     mbar_init(drain, 1);
@@ -211,13 +225,18 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tma_prefetch_desc(&tmB);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  if constexpr (SPLITK) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
+  if constexpr (FORM != W8_ALONE) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
   const uint32_t tmem_base = *tmem_slot;
   const WaitCtl ctl{abort_flag, p.status, p.wait_limit_ns};
 
@@ -228,7 +247,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
       bool ok = true;
       for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride) {
-        const W8Tile t = w8_tile(p, tile);
+        const W8Tile t = w8_tile<PAIR>(p, tile, crank);
         const int m0 = t.m0, n0 = t.n0;
         const int b_boxes = B_NK ? 1 : (t.bn + 127) / 128;  // 128-column boxes of B actually needed
         const uint32_t tx = Cfg::A_BYTES + (B_NK ? (uint32_t)Cfg::B_BYTES : (uint32_t)(b_boxes * W8_BK * 128));
@@ -236,6 +255,19 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait(&empty[stage], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* sA = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sB = sA + Cfg::A_BYTES;
+          if constexpr (PAIR) {
+            // both CTAs' bytes are counted on the leader's barrier; columns: this CTA's half of the item's
+            const uint32_t bar = mapa_u32(smem_u32(&full[stage]), 0);
+            const int nh = n0 + crank * (t.bn >> 1);
+            if (crank == 0) mbar_arrive_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);
+            tma_load_3d_pair(sA, &tmA, bar, kb * W8_BK, m0, t.bA);
+            if constexpr (B_NK) tma_load_3d_pair(sB, &tmB, bar, kb * W8_BK, nh, t.bB);
+            else tma_load_3d_pair(sB, &tmB, bar, nh, kb * W8_BK, t.bB);
+            issued_mask |= 1u << stage;
+            parity_mask = (parity_mask & ~(1u << stage)) | (phase << stage);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            continue;
+          }
           mbar_arrive_expect_tx(&full[stage], tx);
           tma_load_3d(sA, &tmA, &full[stage], kb * W8_BK, m0, t.bA);
           if constexpr (B_NK) {
@@ -251,10 +283,15 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
       if (!ok) {
-        // Gave up: wait (bounded) until every bulk copy already issued has landed before the CTA may exit.
+        // Gave up: wait (bounded) until every bulk copy already issued has landed before the CTA may exit.  PAIR: the counts are
+        // the leader's; the second CTA, which leaves with it, waits for what a copy may take.
         for (int s = 0; s < STAGES; ++s) {
           if (!(issued_mask & (1u << s))) continue;
           const uint64_t t0 = global_timer_ns();
+          if (PAIR && crank != 0) {
+            while (global_timer_ns() - t0 < 50000ull) {}
+            continue;
+          }
           while (!mbar_try_wait(&full[s], (parity_mask >> s) & 1u)) {
             if (global_timer_ns() - t0 > p.wait_limit_ns) {
               if (p.status) atomicMax(p.status, (uint32_t)ST_TIMEOUT_DRAIN);
@@ -265,7 +302,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // -------------------------------------------------------------- MMA issuer
+    // -------------------------------------------------------------- MMA issuer (PAIR: the leader's, for both CTAs)
     // The warp runs converged and one hardware-elected lane issues, which lets the compiler keep the descriptors in uniform
     // registers.  The stage descriptors differ by their start address only.
     constexpr uint32_t K_STEP = (B_NK ? W8_UMMA_K : W8_UMMA_K * 128) >> 4;  // B's start address from one MMA to the next
@@ -278,9 +315,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint32_t phase = 0;
     int it = 0;
     bool ok = true;
-    for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride, ++it) {
+    for (int tile = PAIR && crank != 0 ? p.num_items : tile_first; ok && tile < p.num_items; tile += tile_stride, ++it) {
       const uint32_t bn = (uint32_t)((tile < p.split_from) ? p.bn : (p.bn >> 1));
-      const uint32_t idesc = make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, W8_BM, bn);
+      const uint32_t idesc = make_idesc(ACC_S32, FMT_S8, FMT_S8, 0, B_NK ? 0 : 1, PAIR ? 2 * W8_BM : W8_BM, bn);
       const int buf = it & 1;
       const uint32_t tphase = (it >> 1) & 1;
       if (!mbar_wait_warp(&tempty[buf], tphase ^ 1u, ctl, ST_TIMEOUT_MMA)) { ok = false; break; }
@@ -294,17 +331,26 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint64_t adesc = a_desc | (uint64_t)((sA & 0x3FFFFu) >> 4);
           const uint64_t bdesc = b_desc | (uint64_t)(((sA + Cfg::A_BYTES) & 0x3FFFFu) >> 4);
 #pragma unroll
-          for (int k = 0; k < W8_BK / W8_UMMA_K; ++k)
-            umma_i8_ss(d, adesc + (uint64_t)(k * (W8_UMMA_K >> 4)), bdesc + (uint64_t)(k * K_STEP), idesc,
-                       ((kb - kb_begin) | k) != 0 ? 1u : 0u);
-          umma_commit(&empty[stage]);
+          for (int k = 0; k < W8_BK / W8_UMMA_K; ++k) {
+            const uint64_t ad = adesc + (uint64_t)(k * (W8_UMMA_K >> 4)), bd = bdesc + (uint64_t)(k * K_STEP);
+            if constexpr (PAIR) umma_i8_ss_pair(d, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
+            else umma_i8_ss(d, ad, bd, idesc, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+          }
+          if constexpr (PAIR) umma_commit_pair(&empty[stage]);
+          else umma_commit(&empty[stage]);
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
-      if (ok && elect_one_sync()) umma_commit(&tfull[buf]);  // the elected lane is the same one every time
+      if (ok && elect_one_sync()) {  // the elected lane is the same one every time
+        if constexpr (PAIR) umma_commit_pair(&tfull[buf]);
+        else umma_commit(&tfull[buf]);
+      }
     }
     if (!ok) {
-      if (elect_one_sync()) umma_commit(drain);
+      if (elect_one_sync()) {
+        if constexpr (PAIR) umma_commit_pair(drain);
+        else umma_commit(drain);
+      }
       if (lane == 0) {
         const uint64_t t0 = global_timer_ns();
         while (!mbar_try_wait(drain, 0)) {
@@ -331,7 +377,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // 512 contiguous bytes for the sender's stores and the receiver's loads alike
     const uint32_t part_row = smem_u32(smem) + (uint32_t)(q * 32 + lane) * 16u;
     for (int tile = tile_first; tile < p.num_items; tile += tile_stride, ++it) {
-      const W8Tile t = w8_tile(p, tile);
+      const W8Tile t = w8_tile<PAIR>(p, tile, crank);
       const int buf = it & 1;
       const uint32_t tphase = (it >> 1) & 1;
       const int m = t.m0 + q * 32 + lane;
@@ -491,7 +537,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[buf]);
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[buf]), 0));
+        else mbar_arrive(&tempty[buf]);
+      }
     }
     if (lane == 0) bulk_wait_group_read0();  // the staging tile must outlive the last bulk store's read
   }
@@ -499,10 +548,11 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // ------------------------------------------------------------------ teardown
   tc_fence_before_sync();
   __syncthreads();
-  if constexpr (SPLITK) cluster_sync_all();  // neither CTA of the pair leaves while the other may still reach into it
+  if constexpr (FORM != W8_ALONE) cluster_sync_all();  // neither CTA of the pair leaves while the other may still reach into it
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+    else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
