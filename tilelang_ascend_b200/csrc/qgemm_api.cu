@@ -210,9 +210,13 @@ int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaSt
 // streams through once per band.  As many row blocks as keep the band's A rows within 34 MB, at least 8: config 3
 // takes all 32 row blocks (16.8 MB, B read from DRAM once instead of four times: 172 -> 165 us; 16 or 24 row blocks:
 // 170 us).
-int w8_group_m(int64_t m_tiles, int64_t k_bytes) {
+// Grouped form: 8 whatever K is.  A higher band holds row blocks of many groups, whose B tiles do not share anything, and comes
+// back to its A rows only after all of those (16 groups, 8192 x 7168 x 2048: 359 MB of DRAM reads for 294 MB of operands).  us, at
+// the power limit, bands of 34 MB / 8 / 16 row blocks: that shape 126.4 / 123.4 / 125.5; 32 groups, 8192 x 4096 x 4096 187 / 178 /
+// 180; 16 groups, 8192 x 1024 x 2048 27.9 / 26.7 / 27.5; four row blocks as eight.
+int w8_group_m(int64_t m_tiles, int64_t k_bytes, bool grouped) {
   static const int forced = getenv("QGEMM_W8_GROUP_M") ? atoi(getenv("QGEMM_W8_GROUP_M")) : 0;  // tuning override
-  int64_t g = forced > 0 ? forced : (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1));
+  int64_t g = forced > 0 ? forced : (grouped ? 8 : (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1)));
   if (g < 8) g = 8;
   if (g > m_tiles) g = m_tiles;
   return (int)(g > 0 ? g : 1);
@@ -688,7 +692,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.sb_mode = (scale_b_len == 1) ? 0 : ((scale_b_len == N) ? 1 : 2);
   p.sa_mode = (scale_a == nullptr) ? 0 : ((scale_a_len == M) ? 1 : 2);
   p.m_tiles = (int)m_tiles;
-  p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K) + 1) / 2 : w8_group_m(m_tiles, K);
+  p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K, false) + 1) / 2 : w8_group_m(m_tiles, K, meta != nullptr);
   p.n_tiles = (int)((N + bn_eff - 1) / bn_eff);
   p.bn = bn_eff;
   const int64_t num_tiles = batchA * p.m_tiles * p.n_tiles;
