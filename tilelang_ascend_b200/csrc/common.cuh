@@ -366,11 +366,25 @@ __device__ __forceinline__ void umma_i8_ss_pair(uint32_t tmem_d, uint64_t adesc,
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The M operand of both CTAs from their own tensor memory, at the same address in both.
+__device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Arrive on the barrier at this shared-memory offset of both CTAs once the pair's MMAs issued so far have completed.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_u32(bar)), "h"((uint16_t)3)
                : "memory");
+}
+// Arrive on the barrier at this shared-memory offset of the pair's leader.  For hand-overs of tensor memory, which the tcgen05
+// fences order; memory that the leader reads would need mbar_arrive_cluster, whose release at cluster scope waits for all of the
+// thread's earlier accesses (2 us a slab in w4a16_wide.cuh).
+__device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapa_u32(smem_u32(bar), 0)) : "memory");
 }
 // ----------------------------------------------------------------- descriptors
 // 64-bit shared-memory matrix descriptor (tcgen05): start address, leading / stride byte offsets

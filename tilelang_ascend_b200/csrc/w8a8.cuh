@@ -538,7 +538,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[buf]), 0));
+        if constexpr (PAIR) mbar_arrive_leader(&tempty[buf]);
         else mbar_arrive(&tempty[buf]);
       }
     }
