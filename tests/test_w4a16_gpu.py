@@ -666,3 +666,33 @@ def test_each_token_gets_its_own_sums(M, K, N):
     nibble = torch.where(k % 2 == 0, byte & 15, byte >> 4)              # [N, M]
     want = ((nibble - 8).float() * scales[k // 128].float().T).T.half()  # the product of two f16 values is exact in fp32
     assert torch.equal(C.cpu(), want)
+
+
+# Wide tiles made by two CTAs (256 weight rows): whole tiles and tiles cut along K; tokens that fill a tile or end in the first or
+# the second CTA's half of it; weight rows that end in either CTA's half; scale groups of 64 and 128; a zeros tensor.
+@pytest.mark.parametrize("M,K,N,group,zeros", [(500, 8192, 14344, 128, False), (1000, 2048, 20488, 128, False), (385, 8192, 9472, 128, False),
+                                               (800, 6144, 6016, 64, True), (2100, 4096, 4240, 128, False)])
+@pytest.mark.parametrize("dt", ["float16", "bfloat16"])
+def test_wide_tiles_of_two_ctas(M, K, N, group, zeros, dt):
+    """One-hot activations read columns of half(q - zero) * s (f16) back bit for bit, for every token and weight row; dense ones
+    agree with float64 within the fp32 sums' bound and the output's rounding."""
+    q = _q()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    P = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+    S = (torch.rand(K // group, N, generator=g, device="cuda") * 0.015 + 0.005).half()
+    Z = torch.randint(0, 16, (K // group, N), generator=g, device="cuda").half() if zeros else 8
+    nib = torch.stack([P & 15, P >> 4], dim=-1).view(N, K).half()
+    rep = lambda t: t.T.repeat_interleave(group, dim=1)  # noqa: E731
+    W = (nib - (rep(Z) if zeros else 8)) * rep(S)        # the difference is exact, the product rounds once
+    out = torch.float16 if dt == "float16" else torch.bfloat16
+    kw = dict(zeros_mode="quantized") if zeros else {}
+    k = (torch.arange(M, device="cuda") * 2654435761) % K
+    A = torch.zeros(M, K, dtype=out, device="cuda")
+    A[torch.arange(M, device="cuda"), k] = 1.0
+    assert torch.equal(q.w4a16_gemm(A, P, S, Z, group, **kw), W[:, k].T.to(out))
+    A = torch.randn(M, K, generator=g, device="cuda").to(out)
+    C = q.w4a16_gemm(A, P, S, Z, group, **kw).double()
+    a = A.half().double()
+    ref, mag = a @ W.double().T, a.abs() @ W.double().abs().T
+    eps = 2.0 ** -11 if dt == "float16" else 2.0 ** -8
+    assert ((C - ref).abs() <= eps * ref.abs() + K * 2.0 ** -24 * mag + 1e-7).all()

@@ -123,11 +123,12 @@ int set_smem_w8r() {
   if (set_smem(qg::w8a8_rows_kernel<true, false>, qg::W8R_SMEM_BYTES)) return -1;
   return set_smem(qg::w8a8_rows_kernel<true, true>, qg::W8R_SMEM_BYTES);
 }
+template <bool PAIR>
 int set_smem_w4w() {
-  if (set_smem(qg::w4a16_wide_kernel<false, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_wide_kernel<true, false>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_wide_kernel<false, true>, qg::W4WideCfg<true>::SMEM_BYTES)) return -1;
-  return set_smem(qg::w4a16_wide_kernel<true, true>, qg::W4WideCfg<true>::SMEM_BYTES);
+  if (set_smem(qg::w4a16_wide_kernel<false, false, PAIR>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a16_wide_kernel<true, false, PAIR>, qg::W4WideCfg<false>::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a16_wide_kernel<false, true, PAIR>, qg::W4WideCfg<true>::SMEM_BYTES)) return -1;
+  return set_smem(qg::w4a16_wide_kernel<true, true, PAIR>, qg::W4WideCfg<true>::SMEM_BYTES);
 }
 
 // The set-up of the current device, once per device.
@@ -156,7 +157,7 @@ int ensure_device(int* sm_count) {
     if (set_smem_w4<16>()) return -1;
     if (set_smem_w4g<16>() || set_smem_w4g<32>() || set_smem_w4g<64>()) return -1;
     if (set_smem_w4i8<16>() || set_smem_w4i8<32>() || set_smem_w4i8<64>() || set_smem_w4i8<128>()) return -1;
-    if (set_smem_w8r() || set_smem_w4w()) return -1;
+    if (set_smem_w8r() || set_smem_w4w<false>() || set_smem_w4w<true>()) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
     st.ready.store(true, std::memory_order_release);
@@ -305,6 +306,34 @@ int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CU
   }
   if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
   return launch_pdl(qg::w4a16_gs_kernel<MT, false>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+}
+
+// The wide tiles, `workers` CTAs or pairs of them; a programmatic dependent of the pre-pass.
+template <bool BF, bool ZT, bool PAIR>
+int launch_w4w(const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap& tmZ, const CUtensorMap& tmA,
+               const qg::W4A16Params& p, int mt, int zero_mode, int workers, cudaStream_t s) {
+  static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(PAIR ? 2 * workers : workers));
+  cfg.blockDim = dim3((unsigned)qg::W4W_THREADS);
+  cfg.dynamicSmemBytes = (size_t)qg::W4WideCfg<ZT>::SMEM_BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_wide_kernel<BF, ZT, PAIR>, tmW, tmS, tmZ, tmA, p, mt, zero_mode));
+  return 0;
+}
+template <bool PAIR>
+int launch_w4w(bool bf, bool zt, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap& tmZ, const CUtensorMap& tmA,
+               const qg::W4A16Params& p, int mt, int zero_mode, int workers, cudaStream_t s) {
+  if (zt) return bf ? launch_w4w<true, true, PAIR>(tmW, tmS, tmZ, tmA, p, mt, zero_mode, workers, s) : launch_w4w<false, true, PAIR>(tmW, tmS, tmZ, tmA, p, mt, zero_mode, workers, s);
+  return bf ? launch_w4w<true, false, PAIR>(tmW, tmS, tmZ, tmA, p, mt, 0, workers, s) : launch_w4w<false, false, PAIR>(tmW, tmS, tmZ, tmA, p, mt, 0, workers, s);
 }
 
 // The pre-pass of the group-sum kernel: activations -> stage images.
@@ -787,10 +816,11 @@ int64_t qgemm_w4a16_counter_bytes(void) { return kW4CounterBytes; }
 // in four 1641, in two 1652).
 struct W4WidePlan {
   int mt = 0, sk_tiles = 0, sk_grid = 1;
+  bool pair = false;
+  double time = 0.0;  // estimated
 };
-static W4WidePlan w4_wide_plan(int64_t M, int64_t weight_tiles, int64_t KS, int64_t G) {
+static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, int64_t G) {
   W4WidePlan best;
-  double best_time = 0.0;
   if (M <= 0 || weight_tiles <= 0 || KS <= 0) return best;  // a size query about an empty problem
   for (int64_t t = (M + qg::W4W_MAX_MT - 1) / qg::W4W_MAX_MT;; ++t) {
     const int64_t mt = ((M + t - 1) / t + 15) / 16 * 16;
@@ -798,8 +828,8 @@ static W4WidePlan w4_wide_plan(int64_t M, int64_t weight_tiles, int64_t KS, int6
     const double slab = std::max(0.95, 0.5 + 0.0048 * (double)mt), end = 2.0 + 0.015 * (double)mt;
     auto consider = [&](double slabs, double extra, int64_t sk_tiles, int64_t sk_grid) {
       const double time = slabs * slab + end + extra;
-      if (best.mt != 0 && time >= best_time) return;
-      best_time = time;
+      if (best.mt != 0 && time >= best.time) return;
+      best.time = time;
       best.mt = (int)mt;
       best.sk_tiles = (int)sk_tiles;
       best.sk_grid = (int)sk_grid;
@@ -815,11 +845,25 @@ static W4WidePlan w4_wide_plan(int64_t M, int64_t weight_tiles, int64_t KS, int6
   }
   return best;
 }
+// On G SMs: by single CTAs, or by pairs of them with tiles of 256 weight rows.  A pair halves what a CTA loads of the activations,
+// which counts from tiles of about 192 tokens on, and each hand-over between the two CTAs takes longer, which counts while there
+// are few of them: 0.93 of the time and 2.5 us.  us, one CTA / two, alone | back to back for seconds: 4096 x 8192 x 28672 1438 /
+// 1318 | 1648 / 1545, 500 x 8192 x 28672 177 / 167 | 208 / 198, 800 x 6144 x 6000 64.0 / 62.2 | 72.7 / 68.8, 700 x 3072 x 12288 46.4
+// / 46.9 | 53.5 / 52.0; not taken: 100 x 8192 x 28672 60.0 / 61.3 | 72.1 / 71.2, 256 x 8192 x 8192 41.7 / 43.9, 2000 x 1024 x 1024
+// 12.1 / 12.7.  QGEMM_W4_PAIR=0 disables pairs.
+static W4WidePlan w4_wide_plan(int64_t M, int64_t batch, int64_t N, int64_t KS, int64_t G) {
+  static const int pair_on = getenv("QGEMM_W4_PAIR") ? atoi(getenv("QGEMM_W4_PAIR")) : 1;
+  const W4WidePlan one = w4_wide_plan_for(M, batch * ((N + 127) / 128), KS, G);
+  if (!pair_on || G < 2 || one.mt == 0) return one;
+  W4WidePlan two = w4_wide_plan_for(M, batch * ((N + 255) / 256), KS, G / 2);
+  two.pair = true;
+  return two.mt >= 192 && 0.93 * two.time + 2.5 < one.time ? two : one;
+}
 static int64_t w4_wide_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
   if (ensure_device(&sms)) return -1;
   const int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
-  const int mt = w4_wide_plan(M, batch * ((N + 127) / 128), (K + 255) / 256, grid).mt;
+  const int mt = w4_wide_plan(M, batch, N, (K + 255) / 256, grid).mt;
   return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + batch * M * K * 2;
 }
 
@@ -956,7 +1000,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   if (ensure_device(&sms)) return -1;
   const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   W4WidePlan plan;
-  if (wide) plan = w4_wide_plan(M, batch * ((N + 127) / 128), (K + 255) / 256, grid_max);
+  if (wide) plan = w4_wide_plan(M, batch, N, (K + 255) / 256, grid_max);
   int mt = wide ? plan.mt : w4_pick_mt(M, use_gs);
   if (gd != nullptr && mt < 16) mt = 16;  // the register-operand decode kernel writes one destination only
 
@@ -988,7 +1032,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   if (!use_gs) {
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)K * 2, (uint64_t)M * (uint64_t)K * 2};
-    const uint32_t box[3] = {64, (uint32_t)mt, 1};
+    const uint32_t box[3] = {64, (uint32_t)(plan.pair ? mt / 2 : mt), 1};
     if (encode_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, a_prepared, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
   }
 
@@ -1012,7 +1056,8 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.zero = zero;
   p.has_scales = scales != nullptr;
   p.m_tiles = (int)((M + mt - 1) / mt);
-  p.n_tiles = (int)((N + 127) / 128);
+  const int tile_rows = plan.pair ? 256 : 128;  // weight rows
+  p.n_tiles = (int)((N + tile_rows - 1) / tile_rows);
   p.batch = (int)batch;
   const int64_t num_tiles = batch * (int64_t)p.m_tiles * p.n_tiles;
   if (num_tiles > 0x3fffffff) return fail("qgemm_w4a16: too many tiles");
@@ -1026,6 +1071,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
   p.w_interleaved = weight_format == QGEMM_W4_SEQUENTIAL ? 0 : 1;
   int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
+  if (plan.pair) grid /= 2;  // pairs of CTAs
   if (p.total_items < grid) grid = p.total_items;
   // Small problems (a few slabs per CTA): prefer a slightly smaller grid that cuts every tile into equal K ranges,
   // one per CTA, over an even deal that leaves most CTAs with two partial tiles and so two split-K hand-overs.
@@ -1101,13 +1147,8 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   }
   if (wide) {
     const CUtensorMap& tz = zeros != nullptr ? tmZ : tmS;
-    constexpr int smem = qg::W4WideCfg<false>::SMEM_BYTES, smem_zt = qg::W4WideCfg<true>::SMEM_BYTES;
-    if (zeros != nullptr) {
-      if (bf) return launch_pdl(qg::w4a16_wide_kernel<true, true>, (int)grid, qg::W4W_THREADS, smem_zt, s, tmW, tmS, tz, tmA, p, mt, zero_mode);
-      return launch_pdl(qg::w4a16_wide_kernel<false, true>, (int)grid, qg::W4W_THREADS, smem_zt, s, tmW, tmS, tz, tmA, p, mt, zero_mode);
-    }
-    if (bf) return launch_pdl(qg::w4a16_wide_kernel<true, false>, (int)grid, qg::W4W_THREADS, smem, s, tmW, tmS, tz, tmA, p, mt, 0);
-    return launch_pdl(qg::w4a16_wide_kernel<false, false>, (int)grid, qg::W4W_THREADS, smem, s, tmW, tmS, tz, tmA, p, mt, 0);
+    if (plan.pair) return launch_w4w<true>(bf, zeros != nullptr, tmW, tmS, tz, tmA, p, mt, zero_mode, (int)grid, s);
+    return launch_w4w<false>(bf, zeros != nullptr, tmW, tmS, tz, tmA, p, mt, zero_mode, (int)grid, s);
   }
   if (gd == nullptr && w4_use_decode(M) && mt <= 16 && M <= w4_decode_max_m()) {
     if (scales == nullptr) return launch_w4d<0>(bf, mt, tmW, tmS, tmA, p, (int)grid, s);

@@ -103,11 +103,12 @@ __device__ __forceinline__ long long w4_range_begin(long long T, int G, int b) {
 __device__ __forceinline__ int w4_owner(long long T, int G, long long i) { return (int)(((i + 1) * G - 1) / T); }
 
 // tile -> batch index, first weight row, first token
+template <int BN = W4_BN>
 __device__ __forceinline__ void w4_tile_coords(const W4A16Params& p, int tile, int mt, int& b, int& n0, int& m0) {
   const int per_batch = p.n_tiles * p.m_tiles;
   b = tile / per_batch;
   const int t = tile - b * per_batch;
-  n0 = (t / p.m_tiles) * 128;
+  n0 = (t / p.m_tiles) * BN;
   m0 = (t % p.m_tiles) * mt;
 }
 

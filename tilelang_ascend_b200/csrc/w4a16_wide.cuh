@@ -18,6 +18,7 @@
 //   warp 0        TMA: packed weights + scale (and zero) rows, one slab per stage
 //   warp 1        TMA: prepared activations, [tile tokens x 64 k] per stage
 //   warp 2        tcgen05.mma kind::f16 issuer (A = weights from tensor memory, B = activations from shared memory)
+//   (two CTAs may share a tile of 256 weight rows, see PAIR)
 //   warp 3        allocates tensor memory
 //   warps 4..11   epilogue: two sets of four warps take 16 tokens in turn; the accumulator is handed back as soon as it
 //                 has been read, the split-K sum runs beside the next tile's MMAs
@@ -69,7 +70,12 @@ __device__ __forceinline__ void w4w_store_tokens4(const W4A16Params& p, uint16_t
 }
 
 // ZT: zero points from a [K/group, N] f16 tensor in any of the three modes (w4_apply_zero).
-template <bool OUT_BF16, bool ZT>
+// PAIR: a cluster of two CTAs makes tiles of 256 weight rows with MMAs over both (tcgen05.mma.cta_group::2): each CTA converts its
+// own 128 rows into its own tensor memory, holds their accumulators, and loads half of the tile's tokens, which the tensor cores
+// of both read.  At 256 tokens one CTA by itself takes 36 KB from L2 per 64 k, whose MMAs last 512 cycles, more than the 64 bytes
+// a cycle that reach an SM; a pair 20 KB each.  The leader (rank 0) issues; converted weights, activations and free accumulators
+// of both CTAs are signalled on its barriers, its commits signal both.  Figures and the choice: w4_wide_plan in qgemm_api.cu.
+template <bool OUT_BF16, bool ZT, bool PAIR>
 __global__ void __launch_bounds__(W4W_THREADS, 1)
 w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
                   const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmA,
@@ -98,7 +104,9 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  const int a_bytes = mt * 128;                                     // one stage: mt tokens x 64 k
+  const int crank = PAIR ? (int)cluster_ctarank() : 0;
+  const int a_rows = PAIR ? mt / 2 : mt;                            // tokens that this CTA loads
+  const int a_bytes = a_rows * 128;                                 // one stage: their 64 k
   const int AS = min(W4W_MAX_AS, W4W_A_RING_BYTES / a_bytes);
   const int acc_bufs = mt <= W4W_ACC_COLS / 2 ? 2 : 1;
 
@@ -112,12 +120,12 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       mbar_init(&a_empty[s], 1);
     }
     for (int s = 0; s < WS; ++s) {
-      mbar_init(&w_full[s], W4W_DQ_WARPS / 2);
+      mbar_init(&w_full[s], (PAIR ? 2 : 1) * W4W_DQ_WARPS / 2);  // PAIR: both CTAs' warps, on the leader's barrier
       mbar_init(&w_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
-      mbar_init(&tempty[i], W4W_EPI_WARPS);
+      mbar_init(&tempty[i], (PAIR ? 2 : 1) * W4W_EPI_WARPS);
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
@@ -129,23 +137,37 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (ZT) tma_prefetch_desc(&tmZ);
   }
   if (warp == 3) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_slot, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_w = tmem_base + W4W_ACC_COLS;
   const WaitCtl ctl{abort_flag, p.status, p.wait_limit_ns, 0};
 
-  const int G = gridDim.x;
-  const int cta = blockIdx.x;
+  const int G = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;  // workers: CTAs, or pairs of them
+  const int cta = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int n_off = crank * W4_BN;                              // PAIR: a tile is 256 weight rows, 128 for each CTA
+  // where this CTA's partial sums and its tile's arrival counter are: each CTA of a pair has its own
+  auto partial_slot = [&](int worker, int second) { return PAIR ? 2 * (2 * worker + second) + crank : 2 * worker + second; };
+  auto counter = [&](int worker) { return p.ws_counters + (PAIR ? 2 * worker + crank : worker); };
+  auto arrive_leader = [&](uint64_t* bar) {  // on the leader's barrier
+    if constexpr (PAIR) mbar_arrive_leader(bar);
+    else mbar_arrive(bar);
+  };
   // the first sk_tiles tiles' slabs, dealt evenly to the first Gs CTAs as contiguous ranges
   const long long T = (long long)p.sk_tiles * p.KS;
   const int Gs = p.sk_grid;
   const long long item0 = cta < Gs ? w4_range_begin(T, Gs, cta) : T, item1 = cta < Gs ? w4_range_begin(T, Gs, cta + 1) : T;
-  const int whole = (p.num_tiles - p.sk_tiles - cta + G - 1) / G;  // this CTA's whole tiles
+  const int whole = (p.num_tiles - p.sk_tiles - cta + G - 1) / G;  // this worker's whole tiles
   W4HybridIter seg{W4SegIter{item0, item1, p.KS}, p.sk_tiles + cta, whole, G, p.KS};
   int tile, ks0, ks1;
 
@@ -160,15 +182,15 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const uint32_t tx = W4_RAW_PACKED + (p.has_scales ? row_tx : 0u) + (ZT ? row_tx : 0u);
         while (ok && seg.next(tile, ks0, ks1)) {
           int b, n0, m0;
-          w4_tile_coords(p, tile, mt, b, n0, m0);
+          w4_tile_coords<PAIR ? 2 * W4_BN : W4_BN>(p, tile, mt, b, n0, m0);
           for (int ks = ks0; ks < ks1; ++ks) {
             if (!mbar_wait(&raw_empty[st], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
             uint8_t* dst = raw_base + st * Cfg::RAW_BYTES;
             mbar_arrive_expect_tx(&raw_full[st], tx);
-            tma_load_3d(dst, &tmW, &raw_full[st], ks * (W4_SLAB_K / 2), n0, b);
+            tma_load_3d(dst, &tmW, &raw_full[st], ks * (W4_SLAB_K / 2), n0 + n_off, b);
             const int srow = (p.group <= W4_SLAB_K) ? ks * p.scale_rows : (ks * W4_SLAB_K) / p.group;
-            if (p.has_scales) tma_load_3d(dst + W4_RAW_PACKED, &tmS, &raw_full[st], n0, srow, b);
-            if (ZT) tma_load_3d(dst + W4_RAW_BYTES, &tmZ, &raw_full[st], n0, srow, b);
+            if (p.has_scales) tma_load_3d(dst + W4_RAW_PACKED, &tmS, &raw_full[st], n0 + n_off, srow, b);
+            if (ZT) tma_load_3d(dst + W4_RAW_BYTES, &tmZ, &raw_full[st], n0 + n_off, srow, b);
             issued_mask |= 1u << st;
             parity_mask = (parity_mask & ~(1u << st)) | (phase << st);
             if (++st == RS) { st = 0; phase ^= 1u; }
@@ -178,11 +200,16 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
         while (ok && seg.next(tile, ks0, ks1)) {
           int b, n0, m0;
-          w4_tile_coords(p, tile, mt, b, n0, m0);
+          w4_tile_coords<PAIR ? 2 * W4_BN : W4_BN>(p, tile, mt, b, n0, m0);
           for (int kb = 4 * ks0; kb < 4 * ks1; ++kb) {
             if (!mbar_wait(&a_empty[st], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
-            mbar_arrive_expect_tx(&a_full[st], (uint32_t)a_bytes);
-            tma_load_3d(a_base + st * a_bytes, &tmA, &a_full[st], kb * 64, m0, b);
+            if constexpr (PAIR) {  // both CTAs' bytes are counted on the leader's barrier
+              if (crank == 0) mbar_arrive_expect_tx(&a_full[st], 2u * (uint32_t)a_bytes);
+              tma_load_3d_pair(a_base + st * a_bytes, &tmA, mapa_u32(smem_u32(&a_full[st]), 0), kb * 64, m0 + crank * a_rows, b);
+            } else {
+              mbar_arrive_expect_tx(&a_full[st], (uint32_t)a_bytes);
+              tma_load_3d(a_base + st * a_bytes, &tmA, &a_full[st], kb * 64, m0, b);
+            }
             issued_mask |= 1u << st;
             parity_mask = (parity_mask & ~(1u << st)) | (phase << st);
             if (++st == AS) { st = 0; phase ^= 1u; }
@@ -194,6 +221,10 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         for (int s = 0; s < W4W_MAX_AS; ++s) {
           if (!(issued_mask & (1u << s))) continue;
           const uint64_t t0 = global_timer_ns();
+          if (PAIR && warp == 1 && crank != 0) {  // counted by the leader, which this CTA leaves with: what a copy may take
+            while (global_timer_ns() - t0 < 50000ull) {}
+            continue;
+          }
           while (!mbar_try_wait(&full[s], (parity_mask >> s) & 1u)) {
             if (global_timer_ns() - t0 > p.wait_limit_ns) {
               if (p.status) atomicMax(p.status, (uint32_t)ST_TIMEOUT_DRAIN);
@@ -205,13 +236,17 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------------ MMA issuer (converged warp, one elected lane)
-    const uint32_t idesc = make_idesc(ACC_F32, FMT_F16, FMT_F16, 0, 0, W4_BN, mt);
+    const uint32_t idesc = make_idesc(ACC_F32, FMT_F16, FMT_F16, 0, 0, PAIR ? 2 * W4_BN : W4_BN, mt);
     const uint64_t desc_hi = make_desc_kmajor(0);  // K-major activation descriptor without its start address
     const uint32_t a_base_u32 = smem_u32(a_base);
+    auto commit = [](uint64_t* bar) {
+      if constexpr (PAIR) umma_commit_pair(bar);
+      else umma_commit(bar);
+    };
     int as = 0, ws = 0, it = 0;
     uint32_t aphase = 0, wphase = 0;
     bool ok = true;
-    while (ok && seg.next(tile, ks0, ks1)) {
+    while ((!PAIR || crank == 0) && ok && seg.next(tile, ks0, ks1)) {  // PAIR: the leader's, for both CTAs
       const int buf = acc_bufs == 2 ? it & 1 : 0;
       const uint32_t tphase = (uint32_t)(acc_bufs == 2 ? it >> 1 : it) & 1u;
       ++it;
@@ -228,19 +263,22 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           const uint64_t adesc = desc_hi | (uint64_t)(((a_base_u32 + as * a_bytes) & 0x3FFFFu) >> 4);
           if (elect_one_sync()) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)  // 16 k per MMA: 8 tensor-memory columns, 32 bytes of a row
-              umma_f16_ts(d, tW + blk * 32 + kk * 8, adesc + 2 * kk, idesc, (h != 2 * ks0 || blk != 0 || kk != 0) ? 1u : 0u);
-            umma_commit(&a_empty[as]);
-            if (blk == 1) umma_commit(&w_empty[ws]);
+            for (int kk = 0; kk < 4; ++kk) {  // 16 k per MMA: 8 tensor-memory columns, 32 bytes of a row
+              const uint32_t add = (h != 2 * ks0 || blk != 0 || kk != 0) ? 1u : 0u;
+              if constexpr (PAIR) umma_f16_ts_pair(d, tW + blk * 32 + kk * 8, adesc + 2 * kk, idesc, add);
+              else umma_f16_ts(d, tW + blk * 32 + kk * 8, adesc + 2 * kk, idesc, add);
+            }
+            commit(&a_empty[as]);
+            if (blk == 1) commit(&w_empty[ws]);
           }
           if (++as == AS) { as = 0; aphase ^= 1u; }
         }
         if (++ws == WS) { ws = 0; wphase ^= 1u; }
       }
-      if (ok && elect_one_sync()) umma_commit(&tfull[buf]);  // the elected lane is the same one every time
+      if (ok && elect_one_sync()) commit(&tfull[buf]);  // the elected lane is the same one every time
     }
     if (!ok) {
-      if (elect_one_sync()) umma_commit(drain);
+      if (elect_one_sync()) commit(drain);
       if (lane == 0) {
         const uint64_t t0 = global_timer_ns();
         while (!mbar_try_wait(drain, 0)) {
@@ -259,11 +297,11 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const int buf = acc_bufs == 2 ? it & 1 : 0;
       const uint32_t tphase = (uint32_t)(acc_bufs == 2 ? it >> 1 : it) & 1u;
       int b, n0, m0;
-      w4_tile_coords(p, tile, mt, b, n0, m0);
-      const int n = n0 + nl;
+      w4_tile_coords<PAIR ? 2 * W4_BN : W4_BN>(p, tile, mt, b, n0, m0);
+      const int n = n0 + n_off + nl;
       uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
       const bool full_tile = (ks0 == 0 && ks1 == p.KS);
-      const int my_slot = (ks1 < p.KS) ? 2 * cta + 1 : 2 * cta;
+      const int my_slot = partial_slot(cta, ks1 < p.KS ? 1 : 0);
       float* part = p.ws_partials + (size_t)my_slot * ((size_t)mt * W4_BN) + nl;
       if (mbar_wait_warp(&tfull[buf], tphase, ctl, ST_TIMEOUT_EPILOGUE)) {
         tc_fence_after_sync();
@@ -286,7 +324,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[buf]);
+        if (lane == 0) arrive_leader(&tempty[buf]);
       }
       // Segment end.  The epilogue warps decide together whether to go on (a warp that left alone would leave the others
       // waiting at the named barrier for ever): a wait that gave up set the abort flag before its warp reached the first
@@ -305,7 +343,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       if (warp == W4W_FIRST_EPI_WARP && lane == 0) {
         uint32_t ctrl = *abort_flag ? 1u : 0u;
         // split tile: count arrivals; the last contributor (found without waiting) adds the partial sums
-        if (!ctrl && !full_tile && atomicAdd(p.ws_counters + b_first, 1u) == (uint32_t)(b_last - b_first)) ctrl |= 2u;
+        if (!ctrl && !full_tile && atomicAdd(counter(b_first), 1u) == (uint32_t)(b_last - b_first)) ctrl |= 2u;
         epi_flag[par] = ctrl;
       }
       w4g_epi_bar();
@@ -321,7 +359,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           for (int u = 0; u < 16; ++u) sum[u] = 0.0f;
 #pragma unroll 1
           for (int o = b_first; o <= b_last; ++o) {  // fixed order: results do not depend on arrival order
-            const int slot = (w4_range_begin(T, Gs, o + 1) >= first_item + p.KS) ? 2 * o : 2 * o + 1;
+            const int slot = partial_slot(o, w4_range_begin(T, Gs, o + 1) >= first_item + p.KS ? 0 : 1);
             const float* src = p.ws_partials + (size_t)slot * ((size_t)mt * W4_BN) + (size_t)c * W4_BN + nl;
             float v[16];
 #pragma unroll
@@ -398,7 +436,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&w_full[ws]);
+        if (lane == 0) arrive_leader(&w_full[ws]);
         ws ^= 2;
         if (ws < 2) wphase ^= 1u;
       }
@@ -408,9 +446,11 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   // ------------------------------------------------------------------ teardown
   tc_fence_before_sync();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // neither CTA leaves while the other may still reach into it
   if (warp == 3) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
 }
 
