@@ -50,3 +50,16 @@ def test_extreme_values():
     C = torch.zeros(M, N, dtype=torch.int32, device="cuda")
     out = q.w4a8_gemm_cv(M, N, K)(A.cuda(), qB.cuda(), ws, C)
     assert torch.equal(out.cpu(), oc.w4a8_gemm_ref(A, qB))
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 6144, 18960), (3, 6176, 21008), (16, 5888, 19200)])
+def test_whole_tiles_behind_cut_ones(M, K, N):
+    """Few tokens, long K and at least a round of tiles: the remainder's tiles are cut along K first, whole ones follow."""
+    import tilelang_ascend_b200 as q
+    from oracle import qgemm_oracle as oc
+    g = torch.Generator().manual_seed(M + K + N)
+    A = torch.randint(-128, 128, (M, K), dtype=torch.int8, generator=g)
+    qB = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g)
+    C = q.w4a8_gemm_cv(M, N, K)(A.cuda(), qB.cuda(), torch.empty((N, K), dtype=torch.int8, device="cuda"),
+                                torch.empty((M, N), dtype=torch.int32, device="cuda"))
+    assert torch.equal(C.cpu(), oc.w4a8_gemm_ref(A, qB))

@@ -90,6 +90,10 @@ int set_smem_w4i8() {
   using C = qg::W4I8Cfg<MT>;
   if (set_smem(qg::w4a8_gemm_kernel<MT, false>, C::SMEM_BYTES)) return -1;
   if (set_smem(qg::w4a8_gemm_kernel<MT, true>, C::SMEM_BYTES)) return -1;
+  if constexpr (MT == 16) {
+    if (set_smem(qg::w4a8_gemm_kernel<MT, false, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w4a8_gemm_kernel<MT, true, true>, C::SMEM_BYTES)) return -1;
+  }
   return 0;
 }
 template <int MT>
@@ -457,6 +461,12 @@ __global__ void unpack_int4_kernel(const uint8_t* __restrict__ packed, int8_t* _
 template <int MT>
 static int launch_w4i8(bool sgn, const CUtensorMap& tmW, const CUtensorMap& tmA, const qg::W4A8Params& p, int grid,
                        cudaStream_t s) {
+  if constexpr (MT == 16) {
+    if (p.dp_rounds > 0 && p.KS >= 24) {
+      if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+      return launch_pdl(qg::w4a8_gemm_kernel<MT, false, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+    }
+  }
   if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
   return launch_pdl(qg::w4a8_gemm_kernel<MT, false>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
 }
@@ -506,10 +516,14 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   p.K = (int)K;
   p.n_tiles = (int)((N + 127) / 128);
   p.KS = (int)((K + 255) / 256);
-  p.total_items = (long long)p.n_tiles * p.KS;
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
-  int64_t grid = grid_max < p.total_items ? grid_max : p.total_items;
+  const int64_t items = (int64_t)p.n_tiles * p.KS, grid = grid_max < items ? grid_max : items;
+  // As the group-sum kernel: whole tiles where there are enough, the remainder (with one whole round, when it is small) cut.
+  const int64_t rounds = p.n_tiles / grid, left = p.n_tiles % grid;
+  const bool borrow = rounds != 0 && left != 0 && 2 * left < grid;
+  p.dp_rounds = (int)(borrow ? rounds - 1 : rounds);
+  p.sk_tiles = (int)(borrow ? left + grid : left);
   // a programmatic dependent of whatever is in front: behind another call of this operator it is resident early
   if (X != nullptr) {
     if (launch_pdl(qg::w4a8_quant_prepare_activations, (int)M, 256, 0, s, static_cast<const uint4*>(X), x_is_bf16,

@@ -12,6 +12,7 @@
 #include "act_quant.cuh"
 #include "common.cuh"
 #include "w4a16.cuh"
+#include "w4a16_gs.cuh"
 
 namespace qg {
 
@@ -23,7 +24,7 @@ struct W4A8Params {
   int M, N, K;
   int n_tiles;           // 128-row weight tiles; one token tile (M <= MT)
   int KS;                // 256-wide K slabs per tile
-  long long total_items;
+  int sk_tiles, dp_rounds;  // WHOLE: the first sk_tiles tiles are cut over all CTAs, each of which then takes dp_rounds whole ones
   uint32_t* status;
   unsigned long long wait_limit_ns;
 };
@@ -148,7 +149,11 @@ w4a8_quant_prepare_activations(const uint4* __restrict__ X, int is_bf16, int rou
   }
 }
 
-template <int MT, bool SIGNED>
+// WHOLE: whole tiles per CTA where there is at least a round of them; the tiles that are cut come first, so that their hand-overs
+// run beside the whole tiles' stream and the launch ends with plain tile writes (16 x 8192 x 28672 with the quantiser 31.9 -> 30.4
+// us).  Its own instantiation, for 16 tokens and K above 5888: 32 x 8192 x 28672 35.0 / 35.2 and 8 x 4096 x 20000 18.7 / 18.7 gained
+// nothing, 4 x 1024 x 28672 took 12.6 us instead of 12.0, and in the one kernel 64 x 8192 x 28672 45.7 instead of 42.3.
+template <int MT, bool SIGNED, bool WHOLE = false>
 __global__ void __launch_bounds__(W4_THREADS, 1)
 w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
                  const W4A8Params p) {
@@ -216,8 +221,14 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   const int G = gridDim.x;
   const int cta = blockIdx.x;
-  const long long T = p.total_items;
-  W4SegIter seg{w4_range_begin(T, G, cta), w4_range_begin(T, G, cta + 1), p.KS};
+  const long long T = (long long)(WHOLE ? p.sk_tiles : p.n_tiles) * p.KS;
+  const W4SegIter cut{w4_range_begin(T, G, cta), w4_range_begin(T, G, cta + 1), p.KS};
+  const long long n_slabs = cut.end - cut.item + (WHOLE ? (long long)p.dp_rounds * p.KS : 0);  // slabs of this CTA, in order
+  auto segments = [&]() {
+    if constexpr (WHOLE) return W4HybridIter{cut, p.sk_tiles + cta, p.dp_rounds, G, p.KS};
+    else return cut;
+  };
+  auto seg = segments();
   int tile, ks0, ks1;
 
   if (warp == 0) {
@@ -482,7 +493,6 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
     for (int c = 0; c < 4; ++c) off[c] = row * 128 + (((4 * h + c) ^ sw) << 4);
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    const long long n_slabs = seg.end - seg.item;  // slabs of this CTA, in order
     bool ok = true;
     for (long long i = set; ok && i < n_slabs; i += 2) {
       const int rs = (int)(i % RS), ws = (int)(i % WS);
