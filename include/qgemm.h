@@ -62,9 +62,11 @@ void qgemm_set_wait_limit_ms(uint32_t ms);
 
 /* Test hook, off by default (no counterpart in the reference).  With 1 the small-token W4A16 kernel (two-launch
  * form) leaves one accumulator hand-over of the launch unsignalled; with 2 the single-launch form of small problems
- * keeps back one CTA's "my sums have arrived" signal inside the last cluster.  Either way one bounded wait of the
- * epilogue runs out: the launch ends after the wait limit with QGEMM_ST_TIMEOUT_EPILOGUE in `status` and an
- * unspecified C, nothing is left in flight and the next call works normally.  It exists so that a test can see the
+ * keeps back one CTA's "my sums have arrived" signal inside the last cluster; the kernels whose tiles are made by two
+ * CTAs (W8A8, wide W4A16) keep back the last accumulator of the last pair with 1, and with 3 / 4 the first / second CTA
+ * of the last pair copies no activations (W8A8: nothing).  Either way one or more bounded waits run out: the launch ends
+ * after the wait limit (with 3 and 4 twice that) with QGEMM_ST_TIMEOUT_EPILOGUE in `status` (3 and 4: the code of one of
+ * the waits) and an unspecified C, nothing is left in flight and the next call works normally.  It exists so that a test can see the
  * time-out paths end to end without faulting or hanging the device. */
 void qgemm_debug_withhold_commit(int on);
 

@@ -696,3 +696,28 @@ def test_wide_tiles_of_two_ctas(M, K, N, group, zeros, dt):
     ref, mag = a @ W.double().T, a.abs() @ W.double().abs().T
     eps = 2.0 ** -11 if dt == "float16" else 2.0 ** -8
     assert ((C - ref).abs() <= eps * ref.abs() + K * 2.0 ** -24 * mag + 1e-7).all()
+
+
+@pytest.mark.parametrize("hook,codes", [(1, [3]), (3, [1, 2, 3, 4]), (4, [1, 2, 3, 4])])
+def test_wide_tiles_of_two_ctas_give_up_cleanly(hook, codes):
+    """Bounded waits of the two-CTA wide tiles, made to run out in the safe way in the last pair: the last accumulators are never
+    handed over (1), or one of the two CTAs copies no activations while the other one fills its ring (3, 4).  The launch ends by
+    itself, without the code of a copy that never landed, and the next call is right."""
+    q = _q()
+    from tilelang_ascend_b200 import _lib
+    lib = _lib.load()
+    A, P, S = (t.cuda() for t in oc.make_w4a16_inputs(385, 8192, 9472, "float16", 128, seed=1))
+    want = q.w4a16_gemm(A, P, S, 8, 128)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    try:
+        lib.qgemm_set_wait_limit_ms(20)
+        lib.qgemm_debug_withhold_commit(hook)
+        q.w4a16_gemm(A, P, S, 8, 128, status=status)
+        torch.cuda.synchronize()  # returns: the kernel gave up by itself
+        assert int(status.item()) in codes
+    finally:
+        lib.qgemm_debug_withhold_commit(0)
+        lib.qgemm_set_wait_limit_ms(2000)
+    status.zero_()
+    assert torch.equal(q.w4a16_gemm(A, P, S, 8, 128, status=status), want)
+    assert int(status.item()) == 0

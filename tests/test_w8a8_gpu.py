@@ -320,3 +320,31 @@ def test_tiles_of_two_ctas_are_exact(batch, M, K, N, layout):
     _cmp(C, ref)
     acc = q.quant_matmul(A.cuda(), Bd, sb.cuda(), out_dtype="int32", b_layout=layout)
     assert torch.equal(acc.cpu(), acc_ref)
+
+
+@pytest.mark.parametrize("hook,codes", [(1, [3]), (3, [1, 2, 3]), (4, [1, 2, 3])])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_tiles_of_two_ctas_give_up_cleanly(layout, hook, codes):
+    """Bounded waits of the two-CTA form, made to run out in the safe way in its last pair: the last accumulators are never
+    handed over (1), or one of the two CTAs copies nothing while the other one fills its ring (3, 4).  The launch ends by itself,
+    without the code of a copy that never landed, and the next call is exact."""
+    q = _q()
+    from tilelang_ascend_b200 import _lib
+    lib = _lib.load()
+    A, B, sa, sb = (t.cuda() for t in oc.make_w8a8_inputs(0, 1300, 3072, 2064, seed=1))
+    if layout == "NK":
+        B = B.transpose(-1, -2).contiguous()
+    want = q.quant_matmul(A, B, sb, scale_a=sa, b_layout=layout)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    try:
+        lib.qgemm_set_wait_limit_ms(20)
+        lib.qgemm_debug_withhold_commit(hook)
+        q.quant_matmul(A, B, sb, scale_a=sa, b_layout=layout, status=status)
+        torch.cuda.synchronize()  # returns: the kernel gave up by itself
+        assert int(status.item()) in codes
+    finally:
+        lib.qgemm_debug_withhold_commit(0)
+        lib.qgemm_set_wait_limit_ms(2000)
+    status.zero_()
+    assert torch.equal(q.quant_matmul(A, B, sb, scale_a=sa, b_layout=layout, status=status), want)
+    assert int(status.item()) == 0

@@ -50,6 +50,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+// What the landing of `bytes` would do to the phase's count.
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -385,6 +389,42 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 // thread's earlier accesses (2 us a slab in w4a16_wide.cuh).
 __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapa_u32(smem_u32(bar), 0)) : "memory");
+}
+// The end of the producer in each CTA of a pair, whose copies are all counted on the leader's barriers `full`: `bytes` a CTA and
+// fill, fill i in stage i % stages.  Neither CTA may leave while a copy into its shared memory is under way, also when the
+// producers stopped at different fills because a wait gave up.  So the second CTA says how many fills it has issued, and the
+// leader, which leaves with it (cluster_sync_all), completes what only one of them has issued - at most `stages` fills, since a
+// stage is filled again only after both CTAs' copies in it have been used - and waits, bounded, for the last phase of every stage.
+// Nothing is waited for that the MMAs behind these copies have not waited for already, unless the launch gave up.
+__device__ __forceinline__ void pair_wait_copies(uint64_t* full, uint32_t stages, uint32_t bytes, uint32_t issued, int crank,
+                                                 uint64_t* reported, uint32_t* peer_issued, const WaitCtl& ctl) {
+  if (crank != 0) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(smem_u32(peer_issued), 0)), "r"(issued) : "memory");
+    mbar_arrive_cluster(mapa_u32(smem_u32(reported), 0));
+    return;
+  }
+  // twice the limit: the second CTA's last wait may have started as late as when this one's gave up
+  uint64_t t0 = global_timer_ns();
+  while (!mbar_try_wait_cluster(reported, 0)) {
+    if (global_timer_ns() - t0 > 2 * ctl.limit_ns) {
+      if (ctl.status) atomicMax(ctl.status, (uint32_t)ST_TIMEOUT_DRAIN);
+      return;
+    }
+  }
+  const uint32_t theirs = *reinterpret_cast<volatile uint32_t*>(peer_issued), all = max(issued, theirs);
+  for (uint32_t i = min(issued, theirs); i < all; ++i) {
+    if (i >= issued) mbar_arrive_expect_tx(&full[i % stages], bytes);  // the second CTA's copies alone
+    else mbar_complete_tx(&full[i % stages], bytes);                   // expected of it, never issued
+  }
+  for (uint32_t i = all > stages ? all - stages : 0; i < all; ++i) {
+    t0 = global_timer_ns();
+    while (!mbar_try_wait(&full[i % stages], (i / stages) & 1u)) {
+      if (global_timer_ns() - t0 > ctl.limit_ns) {
+        if (ctl.status) atomicMax(ctl.status, (uint32_t)ST_TIMEOUT_DRAIN);
+        return;
+      }
+    }
+  }
 }
 // ----------------------------------------------------------------- descriptors
 // 64-bit shared-memory matrix descriptor (tcgen05): start address, leading / stride byte offsets

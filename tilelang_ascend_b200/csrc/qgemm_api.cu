@@ -290,15 +290,15 @@ int launch_w4(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUt
 constexpr int64_t kW4MaxGrid = 1024;
 constexpr int64_t kW4CounterBytes = kW4MaxGrid * 4;
 
-// Test hook (qgemm_debug_withhold_commit): see W4GDebug.
-int g_w4g_withhold_commit = 0;
+// Test hook (qgemm_debug_withhold_commit): see W4GDebug, and `withhold` of W8A8Params and W4A16Params.
+int g_withhold = 0;
 
 // `tmZ` non-null: the zeros-tensor instantiation (not combined with the gathered form).
 template <int MT>
 int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap* tmZ, const qg::W4A16Params& p,
                int grid, cudaStream_t s) {
   qg::W4GDebug dbg;
-  dbg.withhold_last_commit = g_w4g_withhold_commit;
+  dbg.withhold_last_commit = g_withhold;
   constexpr int smem = qg::W4GCfg<MT>::SMEM_BYTES, smem_zt = qg::W4GCfg<MT, true>::SMEM_BYTES;
   if (tmZ != nullptr) {
     if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, p, dbg);
@@ -356,7 +356,7 @@ int launch_w4g_prepare(const void* A, void* out, const qg::W4A16Params& p, bool 
 int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const qg::W4A16Params& p, int grid, int cluster, cudaStream_t s) {
   static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   qg::W4GDebug dbg;
-  dbg.withhold_last_commit = g_w4g_withhold_commit;
+  dbg.withhold_last_commit = g_withhold;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)qg::W4G_THREADS);
@@ -551,7 +551,7 @@ const char* qgemm_last_error(void) { return g_err; }
 
 void qgemm_set_wait_limit_ms(uint32_t ms) { g_wait_limit_ns = (unsigned long long)ms * 1000000ull; }
 
-void qgemm_debug_withhold_commit(int on) { g_w4g_withhold_commit = (on == 2) ? 2 : (on ? 1 : 0); }
+void qgemm_debug_withhold_commit(int on) { g_withhold = on >= 2 && on <= 4 ? on : (on ? 1 : 0); }
 
 int qgemm_init(void) {
   int sms = 0;
@@ -744,6 +744,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.k_blocks = (int)((K + 127) / 128);
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
+  p.withhold = g_withhold;
   // with rows that no block can cover, a CTA per SM to clear them, whatever the number of tiles
   const bool sure_to_clear = p.zero_uncovered && M > num_blocks * qg::W8_BM;
   const int workers = use_pair ? sms / 2 : sms;  // CTAs, or pairs of them
@@ -1081,6 +1082,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   p.total_items = num_tiles * p.KS;
   p.status = status;
   p.wait_limit_ns = g_wait_limit_ns;
+  p.withhold = g_withhold;
   p.A_raw = nullptr;
   p.a_is_bf16 = a_dtype == QGEMM_DT_BF16 ? 1 : 0;
   p.w_interleaved = weight_format == QGEMM_W4_SEQUENTIAL ? 0 : 1;
@@ -1126,7 +1128,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   // 8.8 / 9.8 us; with more clusters than SMs (several waves) it loses.  QGEMM_W4_SMALL=0 keeps the two-launch form.
   {
     static const int small_on = getenv("QGEMM_W4_SMALL") ? atoi(getenv("QGEMM_W4_SMALL")) : 1;
-    if (small_on && use_gs && mt == 16 && gd == nullptr && zeros == nullptr && g_w4g_withhold_commit != 1) {
+    if (small_on && use_gs && mt == 16 && gd == nullptr && zeros == nullptr && g_withhold != 1) {
       int cluster = 0;
       for (int c = 1; c <= 4; c *= 2)  // clusters of eight were measured slower than the two-launch form (15.3 / 11.3 us)
         if (p.KS % c == 0 && p.KS / c <= qg::W4G_SMALL_MAX_SLABS) { cluster = c; break; }

@@ -54,6 +54,7 @@ struct W4A16Params {
   long long total_items;
   uint32_t* status;
   unsigned long long wait_limit_ns;
+  int withhold;          // test hook of the two-CTA wide tiles (qgemm_debug_withhold_commit)
   // Gathered form (column-sharded weights, one process per GPU): when n_dst > 0 the [M, N] result is written
   // into columns [col0, col0 + N) of n_dst row-major [M, ldc] buffers, one per rank (this rank's own and its
   // peers', mapped into this process), instead of into C.  Plain stores to peer memory: the transfer of the

@@ -211,6 +211,7 @@ struct W4HybridIter {
     --dp_left;
     return true;
   }
+  __device__ __forceinline__ bool done() const { return sk.item >= sk.end && dp_left <= 0; }
 };
 
 

@@ -98,9 +98,11 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint64_t* tfull = w_empty + WS;
   uint64_t* tempty = tfull + 2;
   uint64_t* drain = tempty + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  uint64_t* reported = drain + 1;  // PAIR: the second CTA's producer of activations has ended (pair_wait_copies)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  volatile uint32_t* epi_flag = tmem_slot + 2;
+  volatile uint32_t* epi_flag = tmem_slot + 2;  // two words
+  uint32_t* peer_issued = tmem_slot + 4;
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -128,6 +130,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       mbar_init(&tempty[i], (PAIR ? 2 : 1) * W4W_EPI_WARPS);
     }
     mbar_init(drain, 1);
+    mbar_init(reported, 1);
     *abort_flag = 0;
     epi_flag[0] = epi_flag[1] = 0;
     fence_barrier_init();
@@ -175,7 +178,7 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     // ------------------------------------------------------------------ producers
     if (lane == 0) {
       int st = 0;
-      uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
+      uint32_t phase = 0, issued_mask = 0, parity_mask = 0, fills = 0;
       bool ok = true;
       if (warp == 0) {
         const uint32_t row_tx = (uint32_t)p.scale_rows * 256u;
@@ -198,7 +201,8 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       } else {
         pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
-        while (ok && seg.next(tile, ks0, ks1)) {
+        const bool idle = PAIR && p.withhold == 3 + crank && cta == G - 1;  // test hook: this CTA copies nothing
+        while (!idle && ok && seg.next(tile, ks0, ks1)) {
           int b, n0, m0;
           w4_tile_coords<PAIR ? 2 * W4_BN : W4_BN>(p, tile, mt, b, n0, m0);
           for (int kb = 4 * ks0; kb < 4 * ks1; ++kb) {
@@ -210,21 +214,20 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
               mbar_arrive_expect_tx(&a_full[st], (uint32_t)a_bytes);
               tma_load_3d(a_base + st * a_bytes, &tmA, &a_full[st], kb * 64, m0, b);
             }
+            ++fills;
             issued_mask |= 1u << st;
             parity_mask = (parity_mask & ~(1u << st)) | (phase << st);
             if (++st == AS) { st = 0; phase ^= 1u; }
           }
         }
       }
-      if (!ok) {  // wait (bounded) for the copies still in flight before the CTA may exit
+      if (PAIR && warp == 1) {
+        pair_wait_copies(a_full, (uint32_t)AS, (uint32_t)a_bytes, fills, crank, reported, peer_issued, ctl);
+      } else if (!ok) {  // wait (bounded) for the copies still in flight before the CTA may exit
         uint64_t* full = warp == 0 ? raw_full : a_full;
         for (int s = 0; s < W4W_MAX_AS; ++s) {
           if (!(issued_mask & (1u << s))) continue;
           const uint64_t t0 = global_timer_ns();
-          if (PAIR && warp == 1 && crank != 0) {  // counted by the leader, which this CTA leaves with: what a copy may take
-            while (global_timer_ns() - t0 < 50000ull) {}
-            continue;
-          }
           while (!mbar_try_wait(&full[s], (parity_mask >> s) & 1u)) {
             if (global_timer_ns() - t0 > p.wait_limit_ns) {
               if (p.status) atomicMax(p.status, (uint32_t)ST_TIMEOUT_DRAIN);
@@ -275,7 +278,8 @@ w4a16_wide_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
         if (++ws == WS) { ws = 0; wphase ^= 1u; }
       }
-      if (ok && elect_one_sync()) commit(&tfull[buf]);  // the elected lane is the same one every time
+      const bool withheld = PAIR && p.withhold == 1 && cta == G - 1 && seg.done();
+      if (ok && !withheld && elect_one_sync()) commit(&tfull[buf]);  // the elected lane is the same one every time
     }
     if (!ok) {
       if (elect_one_sync()) commit(drain);

@@ -38,6 +38,7 @@ struct W8A8Params {
   // right half of tile split_from + i), so that the last, partly filled round of the persistent grid keeps
   // twice as many SMs busy for about half as long.  num_items = num_tiles when nothing is split.
   int split_from, num_items;
+  int withhold;   // test hook of the two-CTA form (qgemm_debug_withhold_commit)
   int tma_store;  // C is written with tiled bulk stores from a shared-memory staging tile (needs bn % 64 == 0)
 };
 
@@ -194,8 +195,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* drain = tempty + 2;
   uint64_t* stages_free = drain + 1;    // split form: the peer's MMAs have finished reading the peer's stages
   uint64_t* partial_full = drain + 2;   // split form: the peer's accumulators for this CTA's columns have arrived
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 3);
+  uint64_t* reported = drain + 3;       // two-CTA tiles: the second CTA's producer has ended (pair_wait_copies)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 4);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  uint32_t* peer_issued = tmem_slot + 2;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -219,6 +222,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     if (p.tma_store) tma_prefetch_desc(&tmC);
     mbar_init(drain, 1);
+    mbar_init(reported, 1);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmA);
@@ -244,9 +248,10 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       int stage = 0;
-      uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
+      uint32_t phase = 0, issued_mask = 0, parity_mask = 0, fills = 0;
       bool ok = true;
-      for (int tile = tile_first; ok && tile < p.num_items; tile += tile_stride) {
+      const bool idle = PAIR && p.withhold == 3 + crank && tile_first == tile_stride - 1;  // test hook: this CTA copies nothing
+      for (int tile = idle ? p.num_items : tile_first; ok && tile < p.num_items; tile += tile_stride) {
         const W8Tile t = w8_tile<PAIR>(p, tile, crank);
         const int m0 = t.m0, n0 = t.n0;
         const int b_boxes = B_NK ? 1 : (t.bn + 127) / 128;  // 128-column boxes of B actually needed
@@ -263,8 +268,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tma_load_3d_pair(sA, &tmA, bar, kb * W8_BK, m0, t.bA);
             if constexpr (B_NK) tma_load_3d_pair(sB, &tmB, bar, kb * W8_BK, nh, t.bB);
             else tma_load_3d_pair(sB, &tmB, bar, nh, kb * W8_BK, t.bB);
-            issued_mask |= 1u << stage;
-            parity_mask = (parity_mask & ~(1u << stage)) | (phase << stage);
+            ++fills;
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             continue;
           }
@@ -282,16 +286,13 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
-      if (!ok) {
-        // Gave up: wait (bounded) until every bulk copy already issued has landed before the CTA may exit.  PAIR: the counts are
-        // the leader's; the second CTA, which leaves with it, waits for what a copy may take.
+      if constexpr (PAIR) {
+        pair_wait_copies(full, STAGES, Cfg::STAGE_BYTES, fills, crank, reported, peer_issued, ctl);
+      } else if (!ok) {
+        // Gave up: wait (bounded) until every bulk copy already issued has landed before the CTA may exit.
         for (int s = 0; s < STAGES; ++s) {
           if (!(issued_mask & (1u << s))) continue;
           const uint64_t t0 = global_timer_ns();
-          if (PAIR && crank != 0) {
-            while (global_timer_ns() - t0 < 50000ull) {}
-            continue;
-          }
           while (!mbar_try_wait(&full[s], (parity_mask >> s) & 1u)) {
             if (global_timer_ns() - t0 > p.wait_limit_ns) {
               if (p.status) atomicMax(p.status, (uint32_t)ST_TIMEOUT_DRAIN);
@@ -342,8 +343,12 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
       if (ok && elect_one_sync()) {  // the elected lane is the same one every time
-        if constexpr (PAIR) umma_commit_pair(&tfull[buf]);
-        else umma_commit(&tfull[buf]);
+        if constexpr (PAIR) {
+          const bool withheld = p.withhold == 1 && tile_first == tile_stride - 1 && tile + tile_stride >= p.num_items;
+          if (!withheld) umma_commit_pair(&tfull[buf]);
+        } else {
+          umma_commit(&tfull[buf]);
+        }
       }
     }
     if (!ok) {
