@@ -63,3 +63,42 @@ def test_whole_tiles_behind_cut_ones(M, K, N):
     C = q.w4a8_gemm_cv(M, N, K)(A.cuda(), qB.cuda(), torch.empty((N, K), dtype=torch.int8, device="cuda"),
                                 torch.empty((M, N), dtype=torch.int32, device="cuda"))
     assert torch.equal(C.cpu(), oc.w4a8_gemm_ref(A, qB))
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (48, 4096, 4096), (2, 16384 + 256, 1024)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_behind_the_kernels_that_write_its_activations(M, K, N, fused):
+    """The pre-pass starts early behind the few-token W8A8 kernel and the quantiser, which still write the activations then: a
+    chain is bit-identical to the same chain with the device drained between the calls."""
+    import tilelang_ascend_b200 as q
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a0 = torch.randint(-128, 128, (M, K), dtype=torch.int8, generator=g, device="cuda")
+    Ws = [torch.randint(-128, 128, (K, K), dtype=torch.int8, generator=g, device="cuda") for _ in range(3)]
+    scale = torch.full((K,), 1e-4, device="cuda")
+    qB = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    ws = torch.empty((N, K), dtype=torch.int8, device="cuda")
+    kernel = q.w4a8_gemm_act_quant(M, N, K) if fused else q.w4a8_gemm_cv(M, N, K)
+
+    def chain(drain):
+        step = torch.cuda.synchronize if drain else lambda: None
+        out, a = [], a0
+        for i in range(9):
+            h = q.quant_matmul(a, Ws[i % 3], scale, out_dtype="bfloat16")
+            step()
+            C = torch.empty((M, N), dtype=torch.int32, device="cuda")
+            if fused:
+                C, s = kernel(h, qB, ws, C)
+                out.append(s)
+                step()
+            a, s = q.act_quant(h)
+            step()
+            if not fused:
+                C = kernel(a, qB, ws, C)
+                step()
+            out += [C, s]
+        return out
+
+    want = chain(True)
+    for _ in range(3):
+        assert all(torch.equal(x, y) for x, y in zip(chain(False), want))
+    assert len({int(c.view(-1)[0]) for c in want if c.dtype == torch.int32}) > 1  # the steps differ

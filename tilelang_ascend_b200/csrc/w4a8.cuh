@@ -52,11 +52,13 @@ struct W4I8Cfg {
 // Pre-pass: int8 activations [M, K] -> the same values with every group of eight k reordered to
 // 0,2,4,6,1,3,5,7 (the byte order the unpack produces), and the row sums.  One block per row.
 __global__ void __launch_bounds__(256)
-w4a8_prepare_activations(const uint2* __restrict__ in, uint2* __restrict__ out, int* __restrict__ row_sums,
+w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restrict__ row_sums,
                          uint32_t* __restrict__ counters, int n_counters, int K) {
   __shared__ int red[8];
   pdl_launch_dependents();
-  pdl_wait();  // behind another call of this operator: that call's kernel still reads the scratch until it is done
+  // behind another call of this operator: that call's kernel still reads the scratch until it is done; behind the quantiser
+  // or the few-token W8A8 kernel: the activations are still being written
+  pdl_wait();
   // the caller's scratch holds anything: the arrival counters start at zero
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0u;
   const int m = blockIdx.x;
@@ -64,7 +66,7 @@ w4a8_prepare_activations(const uint2* __restrict__ in, uint2* __restrict__ out, 
   uint2* dst = out + (size_t)m * (K / 8);
   int acc = 0;
   for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const uint2 v = src[i];
+    const uint2 v = ld_written(src + i);
     acc = __dp4a((int)v.x, 0x01010101, acc);
     acc = __dp4a((int)v.y, 0x01010101, acc);
     dst[i] = make_uint2(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.x, v.y, 0x7531));
@@ -88,13 +90,13 @@ w4a8_prepare_activations(const uint2* __restrict__ in, uint2* __restrict__ out, 
 // memory.  One block per row; a thread keeps up to eight 16-byte chunks of the row in registers between the abs-max
 // pass and the quantise pass (K <= 16384), longer rows are read again.
 __global__ void __launch_bounds__(256)
-w4a8_quant_prepare_activations(const uint4* __restrict__ X, int is_bf16, int round_scale, uint2* __restrict__ out,
+w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uint2* __restrict__ out,
                                int* __restrict__ row_sums, float* __restrict__ scales, uint32_t* __restrict__ counters,
                                int n_counters, int K) {
   __shared__ float redf[8];
   __shared__ int red[8];
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();  // as above
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0u;
   const int m = blockIdx.x;
   const int chunks = K >> 3;
@@ -107,12 +109,11 @@ w4a8_quant_prepare_activations(const uint4* __restrict__ X, int is_bf16, int rou
 #pragma unroll
   for (int i = 0; i < KEEP; ++i) {
     const int c = threadIdx.x + i * 256;
-    if (c < chunks) {
-      keep[i] = __ldg(x + c);
-      m2 = aq_absmax8(keep[i], bf16, m2);
-    }
+    keep[i] = c < chunks ? ld_written(x + c) : make_uint4(0u, 0u, 0u, 0u);
   }
-  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) m2 = aq_absmax8(__ldg(x + c), bf16, m2);
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) m2 = aq_absmax8(keep[i], bf16, m2);
+  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) m2 = aq_absmax8(ld_written(x + c), bf16, m2);
   float mx = aq_pair_max(m2, bf16);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -136,7 +137,7 @@ w4a8_quant_prepare_activations(const uint4* __restrict__ X, int is_bf16, int rou
     const int c = threadIdx.x + i * 256;
     if (c < chunks) emit(c, keep[i]);
   }
-  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) emit(c, __ldg(x + c));
+  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) emit(c, ld_written(x + c));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -401,10 +402,13 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
           if (full_tile) {
             if (n < p.N) {
+              int off[CH];
+#pragma unroll
+              for (int j = 0; j < CH; ++j) off[j] = SIGNED && c * CH + j < p.M ? 8 * ld_written(p.row_sums + c * CH + j) : 0;
 #pragma unroll
               for (int j = 0; j < CH; ++j) {
                 const int m = c * CH + j;
-                if (m < p.M) p.C[(size_t)m * p.N + n] = (int)r[j] - (SIGNED ? 8 * __ldg(p.row_sums + m) : 0);
+                if (m < p.M) p.C[(size_t)m * p.N + n] = (int)r[j] - off[j];
               }
             }
           } else {
@@ -452,7 +456,7 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           for (int mb = 0; mb < rows; mb += RU) {
             int sum[RU];
 #pragma unroll
-            for (int u = 0; u < RU; ++u) sum[u] = 0;
+            for (int u = 0; u < RU; ++u) sum[u] = SIGNED && mb + u < rows ? -8 * ld_written(p.row_sums + mb + u) : 0;
 #pragma unroll 1
             for (int c = b_first; c <= b_last; ++c) {
               const long long c_end = w4_range_begin(T, G, c + 1);
@@ -466,8 +470,7 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             }
 #pragma unroll
             for (int u = 0; u < RU; ++u) {
-              if (mb + u < rows)
-                p.C[(size_t)(mb + u) * p.N + n] = sum[u] - (SIGNED ? 8 * __ldg(p.row_sums + mb + u) : 0);
+              if (mb + u < rows) p.C[(size_t)(mb + u) * p.N + n] = sum[u];
             }
           }
         }
