@@ -150,3 +150,34 @@ def test_chain_of_quantisers_and_few_token_gemms(M, K, layers):
     for _ in range(3):
         assert torch.equal(chain(False), want)
     assert torch.isfinite(want.float()).all() and want.float().abs().max() > 0.1
+
+
+@pytest.mark.parametrize("M", [8, 40])
+def test_scales_written_in_front_of_the_quantiser(M):
+    """The int4 GEMM reads its scales without waiting for the kernel directly in front of it.  Here that is the quantiser, and the
+    kernel in front of the quantiser writes the scales: the chain is bit-identical to the one with the device drained between the
+    calls."""
+    K, N, rows = 4096, 4096, 32  # 32 groups of 128
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randint(-128, 128, (rows, K), dtype=torch.int8, generator=g, device="cuda")
+    Ws = [torch.randint(-128, 128, (K, N), dtype=torch.int8, generator=g, device="cuda") for _ in range(3)]
+    P = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    x = torch.randn((M, K), generator=g, device="cuda").half()
+    scale = torch.full((1,), 1e-8, device="cuda")
+
+    def chain(drain):
+        step = torch.cuda.synchronize if drain else lambda: None
+        out = []
+        for i in range(12):
+            S = q.quant_matmul(a, Ws[i % 3], scale, out_dtype="float16")
+            step()
+            y, s = q.act_quant(x)
+            step()
+            out += [q.w4a16_gemm(x, P, S, 8, 128), y, s]
+            step()
+        return out
+
+    want = chain(True)
+    for _ in range(3):
+        assert all(torch.equal(u, v) for u, v in zip(chain(False), want))
+    assert not torch.equal(want[0], want[3])

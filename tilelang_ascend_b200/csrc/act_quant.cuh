@@ -121,9 +121,11 @@ __device__ __forceinline__ float aq_pow2_ceil(float x) {
 // TPR threads share one row; a block holds AQ_THREADS / TPR rows; KEEP chunks per thread stay in registers.
 template <int TPR, int KEEP>
 __global__ void __launch_bounds__(AQ_THREADS, KEEP == 4 ? AQ_MIN_BLOCKS : 1) act_quant_kernel(const ActQuantParams p) {
-  // A W8A8 kernel behind this one may set up meanwhile; it waits for this whole grid before it reads anything.
-  pdl_launch_dependents();
   pdl_wait();  // a programmatic dependent itself: the kernel in front may have written X, and may still read Y and S
+  // A W8A8 kernel behind this one may set up meanwhile; it waits for this whole grid before it reads anything.  Not in front of
+  // the wait: an int4 GEMM behind this kernel reads its weights and scales at once, and whatever wrote those may be the kernel in
+  // front of this one.
+  pdl_launch_dependents();
   constexpr int ROWS = AQ_THREADS / TPR;
   constexpr int WPR = TPR / 32;  // warps per row
   __shared__ float red[AQ_THREADS / 32];
