@@ -670,8 +670,8 @@ def test_each_token_gets_its_own_sums(M, K, N):
 
 # Wide tiles made by two CTAs (256 weight rows): whole tiles and tiles cut along K; tokens that fill a tile or end in the first or
 # the second CTA's half of it; weight rows that end in either CTA's half; scale groups of 64 and 128; a zeros tensor.
-@pytest.mark.parametrize("M,K,N,group,zeros", [(500, 8192, 14344, 128, False), (1000, 2048, 20488, 128, False), (385, 8192, 9472, 128, False),
-                                               (800, 6144, 6016, 64, True), (2100, 4096, 4240, 128, False)])
+@pytest.mark.parametrize("M,K,N,group,zeros", [(500, 8192, 14344, 128, False), (1000, 2048, 20488, 128, False), (430, 8192, 9472, 128, False),
+                                               (860, 6144, 6016, 64, True), (2100, 4096, 4240, 128, False), (1586, 3584, 2832, 128, False)])
 @pytest.mark.parametrize("dt", ["float16", "bfloat16"])
 def test_wide_tiles_of_two_ctas(M, K, N, group, zeros, dt):
     """One-hot activations read columns of half(q - zero) * s (f16) back bit for bit, for every token and weight row; dense ones
@@ -706,7 +706,7 @@ def test_wide_tiles_of_two_ctas_give_up_cleanly(hook, codes):
     q = _q()
     from tilelang_ascend_b200 import _lib
     lib = _lib.load()
-    A, P, S = (t.cuda() for t in oc.make_w4a16_inputs(385, 8192, 9472, "float16", 128, seed=1))
+    A, P, S = (t.cuda() for t in oc.make_w4a16_inputs(430, 8192, 9472, "float16", 128, seed=1))
     want = q.w4a16_gemm(A, P, S, 8, 128)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     try:
@@ -721,3 +721,35 @@ def test_wide_tiles_of_two_ctas_give_up_cleanly(hook, codes):
     status.zero_()
     assert torch.equal(q.w4a16_gemm(A, P, S, 8, 128, status=status), want)
     assert int(status.item()) == 0
+
+
+def _call_workspaces(shapes, pair):
+    """qgemm_w4a16_call_workspace_bytes of (M, K, N), groups of 128, in a process with pairs of CTAs switched on or off."""
+    import json
+    import os
+    import subprocess
+    import sys
+    code = ("import json, sys; from tilelang_ascend_b200 import _lib; lib = _lib.load(); "
+            "print(json.dumps([lib.qgemm_w4a16_call_workspace_bytes(1, M, N, K, 128, 1, 0, 0) for M, K, N in json.loads(sys.argv[1])]))")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", code, json.dumps(shapes)], cwd=root, env={**os.environ, "QGEMM_W4_PAIR": pair},
+                         capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr
+    return json.loads(res.stdout.splitlines()[-1])
+
+
+def test_token_counts_of_two_cta_tiles():
+    """An MMA over two CTAs takes tokens in steps of 32: where pairs change a tile's height (read off the scratch that a call
+    needs), the height is a multiple of it."""
+    from tilelang_ascend_b200 import _lib
+    lib = _lib.load()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    shapes = [(M, K, N) for K, N in [(6144, 6664), (3328, 4384), (8192, 12896), (3072, 8704), (5120, 6960)]
+              for M in range(190, 2400, 53)]
+    height = lambda s, need: (need - lib.qgemm_w4a16_counter_bytes() - 2 * s[0] * s[1]) // (sms * 2 * 128 * 4)  # noqa: E731
+    changed = 0
+    for s, one, two in zip(shapes, _call_workspaces(shapes, "0"), _call_workspaces(shapes, "1")):
+        if one != two:
+            changed += 1
+            assert height(s, two) % 32 == 0, (s, height(s, two))
+    assert changed >= 5

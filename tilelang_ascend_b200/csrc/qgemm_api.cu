@@ -817,7 +817,7 @@ int qgemm_w8a8_grouped_zeroed(const int8_t* A, const int8_t* B, const float* sca
 int64_t qgemm_w4a16_counter_bytes(void) { return kW4CounterBytes; }
 
 // Wide tiles (w4a16_wide.cuh): the tile's tokens and the cut of the work.  Of the cuts into equal tiles (48 .. 256 tokens,
-// a multiple of 16, fewer when there are fewer tokens) and of three ways to deal T tiles to G CTAs the one with the
+// a multiple of 16 or, with two CTAs, of 32, fewer when there are fewer tokens) and of three ways to deal T tiles to G CTAs the one with the
 // smallest estimated time: whole tiles only; whole rounds of G tiles and each tile of the remainder cut into S equal K
 // ranges for S CTAs; or the remainder (with one whole round, when it is small) cut evenly over all CTAs.  The estimate is
 // fitted to a sweep of tile heights and cuts over K = 1024 .. 8192, N = 1024 .. 14336, 80 .. 2048 tokens (us): a slab
@@ -834,11 +834,11 @@ struct W4WidePlan {
   bool pair = false;
   double time = 0.0;  // estimated
 };
-static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, int64_t G) {
+static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, int64_t G, int64_t step) {
   W4WidePlan best;
   if (M <= 0 || weight_tiles <= 0 || KS <= 0) return best;  // a size query about an empty problem
   for (int64_t t = (M + qg::W4W_MAX_MT - 1) / qg::W4W_MAX_MT;; ++t) {
-    const int64_t mt = ((M + t - 1) / t + 15) / 16 * 16;
+    const int64_t mt = ((M + t - 1) / t + step - 1) / step * step;
     const int64_t tiles = weight_tiles * ((M + mt - 1) / mt), rounds = tiles / G, r = tiles % G;
     const double slab = std::max(0.95, 0.5 + 0.0048 * (double)mt), end = 2.0 + 0.015 * (double)mt;
     auto consider = [&](double slabs, double extra, int64_t sk_tiles, int64_t sk_grid) {
@@ -868,9 +868,9 @@ static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, 
 // 12.1 / 12.7.  QGEMM_W4_PAIR=0 disables pairs.
 static W4WidePlan w4_wide_plan(int64_t M, int64_t batch, int64_t N, int64_t KS, int64_t G) {
   static const int pair_on = getenv("QGEMM_W4_PAIR") ? atoi(getenv("QGEMM_W4_PAIR")) : 1;
-  const W4WidePlan one = w4_wide_plan_for(M, batch * ((N + 127) / 128), KS, G);
+  const W4WidePlan one = w4_wide_plan_for(M, batch * ((N + 127) / 128), KS, G, qg::W4W_MT_STEP);
   if (!pair_on || G < 2 || one.mt == 0) return one;
-  W4WidePlan two = w4_wide_plan_for(M, batch * ((N + 255) / 256), KS, G / 2);
+  W4WidePlan two = w4_wide_plan_for(M, batch * ((N + 255) / 256), KS, G / 2, qg::W4W_PAIR_MT_STEP);
   two.pair = true;
   return two.mt >= 192 && 0.93 * two.time + 2.5 < one.time ? two : one;
 }
@@ -1016,6 +1016,7 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   W4WidePlan plan;
   if (wide) plan = w4_wide_plan(M, batch, N, (K + 255) / 256, grid_max);
+  if (wide && (plan.mt <= 0 || plan.mt > qg::W4W_MAX_MT || plan.mt % (plan.pair ? qg::W4W_PAIR_MT_STEP : qg::W4W_MT_STEP) != 0)) return fail("qgemm_w4a16: no MMA has %d tokens", plan.mt);
   int mt = wide ? plan.mt : w4_pick_mt(M, use_gs);
   if (gd != nullptr && mt < 16) mt = 16;  // the register-operand decode kernel writes one destination only
 

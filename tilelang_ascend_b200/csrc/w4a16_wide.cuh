@@ -32,6 +32,10 @@
 namespace qg {
 
 constexpr int W4W_MAX_MT = 256;
+// A tile's tokens are the MMA's N: a multiple of 16 for one CTA's 128 rows.  For the 256 rows of two CTAs multiples of 32 are
+// taken, which every statement of the shape rules for cta_group::2 allows; some allow steps of 16 as well, some do not.
+constexpr int W4W_MT_STEP = 16, W4W_PAIR_MT_STEP = 32;
+static_assert(W4W_MAX_MT % W4W_PAIR_MT_STEP == 0, "tile heights");
 constexpr int W4W_FIRST_EPI_WARP = 4;
 constexpr int W4W_EPI_WARPS = 8;
 constexpr int W4W_FIRST_DQ_WARP = W4W_FIRST_EPI_WARP + W4W_EPI_WARPS;  // 12
