@@ -670,8 +670,8 @@ def test_each_token_gets_its_own_sums(M, K, N):
 
 # Wide tiles made by two CTAs (256 weight rows): whole tiles and tiles cut along K; tokens that fill a tile or end in the first or
 # the second CTA's half of it; weight rows that end in either CTA's half; scale groups of 64 and 128; a zeros tensor.
-@pytest.mark.parametrize("M,K,N,group,zeros", [(500, 8192, 14344, 128, False), (1000, 2048, 20488, 128, False), (430, 8192, 9472, 128, False),
-                                               (860, 6144, 6016, 64, True), (2100, 4096, 4240, 128, False), (1586, 3584, 2832, 128, False)])
+@pytest.mark.parametrize("M,K,N,group,zeros", [(500, 8192, 14344, 128, False), (1000, 3328, 20488, 128, False), (430, 8192, 9472, 128, False),
+                                               (860, 6144, 6016, 64, True), (1047, 4864, 3720, 128, False), (1588, 4608, 2992, 128, False)])
 @pytest.mark.parametrize("dt", ["float16", "bfloat16"])
 def test_wide_tiles_of_two_ctas(M, K, N, group, zeros, dt):
     """One-hot activations read columns of half(q - zero) * s (f16) back bit for bit, for every token and weight row; dense ones
@@ -753,3 +753,9 @@ def test_token_counts_of_two_cta_tiles():
             changed += 1
             assert height(s, two) % 32 == 0, (s, height(s, two))
     assert changed >= 5
+
+
+def test_short_k_stays_with_single_ctas():
+    """Below thirteen slabs of K a pair of CTAs gains nothing or is the slower one: the plan is the one without pairs."""
+    shapes = [(M, K, N) for K in (1024, 1536, 2048, 3072) for N in (1088, 4096, 13792, 25408) for M in (250, 700, 1152, 2221, 3468)]
+    assert _call_workspaces(shapes, "1") == _call_workspaces(shapes, "0")

@@ -861,18 +861,21 @@ static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, 
   return best;
 }
 // On G SMs: by single CTAs, or by pairs of them with tiles of 256 weight rows.  A pair halves what a CTA loads of the activations,
-// which counts from tiles of about 192 tokens on, and each hand-over between the two CTAs takes longer, which counts while there
-// are few of them: 0.93 of the time and 2.5 us.  us, one CTA / two, alone | back to back for seconds: 4096 x 8192 x 28672 1438 /
-// 1318 | 1648 / 1545, 500 x 8192 x 28672 177 / 167 | 208 / 198, 800 x 6144 x 6000 64.0 / 62.2 | 72.7 / 68.8, 700 x 3072 x 12288 46.4
-// / 46.9 | 53.5 / 52.0; not taken: 100 x 8192 x 28672 60.0 / 61.3 | 72.1 / 71.2, 256 x 8192 x 8192 41.7 / 43.9, 2000 x 1024 x 1024
-// 12.1 / 12.7.  QGEMM_W4_PAIR=0 disables pairs.
+// which counts from tiles of about 192 tokens on; each hand-over between the two CTAs takes longer, once per launch and once per
+// tile, and a tile of few slabs does not earn that back: 0.93 of the time, 2.5 us and 0.4 us per tile of a pair, from 13 slabs on.
+// Fitted to and checked on 265 shapes, K 1024 .. 8192, N 1024 .. 28672, 180 .. 4096 tokens, both ways in turn: 88 take pairs, four
+// of them 0.8 .. 1.6 % slower than one CTA, the mean 3.5 % faster.  us, one CTA / two: 4096 x 8192 x 28672 1448 / 1389, 500 x 8192
+// x 28672 184 / 174, 2235 x 4096 x 17440 260 / 247; not taken: 2286 x 2816 x 16576 175 / 171, 3314 x 2560 x 8736 130 / 134, 2628 x
+// 2048 x 21520 205 / 208, 1152 x 1536 x 13792 55.3 / 60.2, 3468 x 1024 x 25408 194 / 204.  QGEMM_W4_PAIR=0 disables pairs.
 static W4WidePlan w4_wide_plan(int64_t M, int64_t batch, int64_t N, int64_t KS, int64_t G) {
   static const int pair_on = getenv("QGEMM_W4_PAIR") ? atoi(getenv("QGEMM_W4_PAIR")) : 1;
   const W4WidePlan one = w4_wide_plan_for(M, batch * ((N + 127) / 128), KS, G, qg::W4W_MT_STEP);
-  if (!pair_on || G < 2 || one.mt == 0) return one;
-  W4WidePlan two = w4_wide_plan_for(M, batch * ((N + 255) / 256), KS, G / 2, qg::W4W_PAIR_MT_STEP);
+  if (!pair_on || G < 2 || one.mt == 0 || KS < 13) return one;
+  const int64_t weight_tiles = batch * ((N + 255) / 256);
+  W4WidePlan two = w4_wide_plan_for(M, weight_tiles, KS, G / 2, qg::W4W_PAIR_MT_STEP);
   two.pair = true;
-  return two.mt >= 192 && 0.93 * two.time + 2.5 < one.time ? two : one;
+  const double tiles_each = (double)(weight_tiles * ((M + two.mt - 1) / two.mt)) / (double)(G / 2);
+  return two.mt >= 192 && 0.93 * two.time + 2.5 + 0.4 * tiles_each < one.time ? two : one;
 }
 static int64_t w4_wide_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
