@@ -759,3 +759,28 @@ def test_short_k_stays_with_single_ctas():
     """Below thirteen slabs of K a pair of CTAs gains nothing or is the slower one: the plan is the one without pairs."""
     shapes = [(M, K, N) for K in (1024, 1536, 2048, 3072) for N in (1088, 4096, 13792, 25408) for M in (250, 700, 1152, 2221, 3468)]
     assert _call_workspaces(shapes, "1") == _call_workspaces(shapes, "0")
+
+
+@pytest.mark.parametrize("M,K,N", [(211, 6400, 12768), (218, 8192, 12896)])
+def test_scratch_for_single_ctas_is_enough(M, K, N):
+    """Where pairs of CTAs would take taller tiles, and so more scratch, the scratch that single CTAs need is still accepted,
+    a byte less is refused as it is without pairs, and the results agree within the fp32 sums' bound and the output's rounding."""
+    q = _q()
+    from tilelang_ascend_b200 import _lib
+    lib = _lib.load()
+    (small,), (large,) = _call_workspaces([(M, K, N)], "0"), _call_workspaces([(M, K, N)], "1")
+    assert small < large  # otherwise the shape shows nothing
+    A, P, S = (t.cuda() for t in oc.make_w4a16_inputs(M, K, N, "float16", 128, seed=M))
+    want = q.w4a16_gemm(A, P, S, 8, 128).double()
+    code = q.ops._ABI_DT[torch.float16]
+    ws = torch.empty(small, dtype=torch.uint8, device="cuda")
+    C = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    call = lambda size: lib.qgemm_w4a16_ex(A.data_ptr(), P.data_ptr(), S.data_ptr(), 0, 8, 0, 0, 128, C.data_ptr(), ws.data_ptr(),  # noqa: E731
+                                           size, 1, M, N, K, code, code, 0, torch.cuda.current_stream().cuda_stream)
+    assert call(small - 1) != 0
+    assert call(small) == 0, _lib.last_error()
+    # both ways add the same products in fp32, in another order: K 2^-24 of the sum of magnitudes each
+    nib = torch.stack([P & 15, P >> 4], dim=-1).view(N, K).half()
+    W = ((nib - 8) * S.T.repeat_interleave(128, dim=1)).double()
+    mag = A.double().abs() @ W.abs().T
+    assert ((C.double() - want).abs() <= 2.0 ** -10 * want.abs() + 2 * K * 2.0 ** -24 * mag + 1e-7).all()

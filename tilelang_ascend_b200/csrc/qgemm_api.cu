@@ -867,22 +867,25 @@ static W4WidePlan w4_wide_plan_for(int64_t M, int64_t weight_tiles, int64_t KS, 
 // of them 0.8 .. 1.6 % slower than one CTA, the mean 3.5 % faster.  us, one CTA / two: 4096 x 8192 x 28672 1448 / 1389, 500 x 8192
 // x 28672 184 / 174, 2235 x 4096 x 17440 260 / 247; not taken: 2286 x 2816 x 16576 175 / 171, 3314 x 2560 x 8736 130 / 134, 2628 x
 // 2048 x 21520 205 / 208, 1152 x 1536 x 13792 55.3 / 60.2, 3468 x 1024 x 25408 194 / 204.  QGEMM_W4_PAIR=0 disables pairs.
-static W4WidePlan w4_wide_plan(int64_t M, int64_t batch, int64_t N, int64_t KS, int64_t G) {
+static W4WidePlan w4_wide_plan(int64_t M, int64_t batch, int64_t N, int64_t KS, int64_t G, bool pairs = true) {
   static const int pair_on = getenv("QGEMM_W4_PAIR") ? atoi(getenv("QGEMM_W4_PAIR")) : 1;
   const W4WidePlan one = w4_wide_plan_for(M, batch * ((N + 127) / 128), KS, G, qg::W4W_MT_STEP);
-  if (!pair_on || G < 2 || one.mt == 0 || KS < 13) return one;
+  if (!pairs || !pair_on || G < 2 || one.mt == 0 || KS < 13) return one;
   const int64_t weight_tiles = batch * ((N + 255) / 256);
   W4WidePlan two = w4_wide_plan_for(M, weight_tiles, KS, G / 2, qg::W4W_PAIR_MT_STEP);
   two.pair = true;
   const double tiles_each = (double)(weight_tiles * ((M + two.mt - 1) / two.mt)) / (double)(G / 2);
   return two.mt >= 192 && 0.93 * two.time + 2.5 + 0.4 * tiles_each < one.time ? two : one;
 }
+// Scratch for tiles of mt tokens: arrival counters, two partial sums per CTA, the prepared activations.
+static int64_t w4_wide_bytes(int64_t batch, int64_t M, int64_t K, int64_t grid, int mt) {
+  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + batch * M * K * 2;
+}
 static int64_t w4_wide_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
   if (ensure_device(&sms)) return -1;
   const int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
-  const int mt = w4_wide_plan(M, batch, N, (K + 255) / 256, grid).mt;
-  return kW4CounterBytes + grid * 2 * (int64_t)mt * 128 * 4 + batch * M * K * 2;
+  return w4_wide_bytes(batch, M, K, grid, w4_wide_plan(M, batch, N, (K + 255) / 256, grid).mt);
 }
 
 // Which of the W4A16 kernels takes a call: the group-sum kernel (w4a16_gs.cuh) up to 64 tokens where it can (wide scale
@@ -1008,17 +1011,21 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   const bool use_gs = route == W4_GROUP_SUM, wide = route == W4_WIDE;
   int64_t need = w4_workspace_bytes(batch, M, N, K);
   if (need < 0) return -1;
-  const int64_t wide_need = wide ? w4_wide_workspace_bytes(batch, M, N, K) : 0;
+  int sms = 0;
+  if (ensure_device(&sms)) return -1;
+  const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
+  W4WidePlan plan;
+  if (wide) {
+    plan = w4_wide_plan(M, batch, N, (K + 255) / 256, grid_max);
+    // pairs may want taller tiles, and so more scratch: a workspace that does for single CTAs stays good for those
+    if (plan.pair && workspace_bytes < w4_wide_bytes(batch, M, K, grid_max, plan.mt)) plan = w4_wide_plan(M, batch, N, (K + 255) / 256, grid_max, false);
+  }
+  const int64_t wide_need = wide ? w4_wide_bytes(batch, M, K, grid_max, plan.mt) : 0;
   // a workspace too small for the wide tiles' partial sums will do if it has room for 128 tokens': no tile is split then
   if (wide) need = std::min(need, wide_need);
   const bool wide_unsplit = wide && workspace_bytes < wide_need;
   if (workspace == nullptr || workspace_bytes < need) return fail("qgemm_w4a16: workspace of %lld bytes needed (got %lld)", (long long)need, (long long)workspace_bytes);
 
-  int sms = 0;
-  if (ensure_device(&sms)) return -1;
-  const int64_t grid_max = sms < kW4MaxGrid ? sms : kW4MaxGrid;
-  W4WidePlan plan;
-  if (wide) plan = w4_wide_plan(M, batch, N, (K + 255) / 256, grid_max);
   if (wide && (plan.mt <= 0 || plan.mt > qg::W4W_MAX_MT || plan.mt % (plan.pair ? qg::W4W_PAIR_MT_STEP : qg::W4W_MT_STEP) != 0)) return fail("qgemm_w4a16: no MMA has %d tokens", plan.mt);
   int mt = wide ? plan.mt : w4_pick_mt(M, use_gs);
   if (gd != nullptr && mt < 16) mt = 16;  // the register-operand decode kernel writes one destination only
