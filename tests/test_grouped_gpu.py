@@ -89,3 +89,23 @@ def test_empty_and_rejects():
         q.grouped_quant_matmul(torch.zeros(8, 40, dtype=torch.int8, device="cuda"),
                                torch.zeros(2, 40, 64, dtype=torch.int8, device="cuda"),
                                q.build_block_metadata([8], 128, "cuda"), sb)
+
+
+@pytest.mark.parametrize("sizes", [(1700, 900), (2300,), (130, 64, 1200)])
+def test_few_groups_of_large_weights(sizes):
+    """Weights of more than 40 MB a group: the tiles are walked in bands as high as a group has row blocks in the mean.  Each group
+    equals the plain operator on its rows, bit for bit."""
+    K, N = 7184, 6160
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    A = torch.randint(-128, 128, (sum(sizes), K), dtype=torch.int8, generator=g, device="cuda")
+    B = torch.randint(-128, 128, (len(sizes), K, N), dtype=torch.int8, generator=g, device="cuda")
+    sb = torch.rand((len(sizes), N), generator=g, device="cuda") * 0.019 + 0.001
+    sa = torch.rand(sum(sizes), generator=g, device="cuda") * 0.019 + 0.001
+    kernel = q.grouped_quant_gemm(sizes, K, N, out_dtype="bfloat16")
+    C = kernel(A, B, kernel.block_metadata("cuda"), sb, sa)
+    first = 0
+    for i, rows in enumerate(sizes):
+        end = first + rows
+        want = q.quant_matmul(A[first:end].contiguous(), B[i], sb[i], scale_a=sa[first:end].contiguous(), out_dtype="bfloat16")
+        assert torch.equal(C[first:end], want)
+        first = end

@@ -215,13 +215,18 @@ int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaSt
 // streams through once per band.  As many row blocks as keep the band's A rows within 34 MB, at least 8: config 3
 // takes all 32 row blocks (16.8 MB, B read from DRAM once instead of four times: 172 -> 165 us; 16 or 24 row blocks:
 // 170 us).
-// Grouped form: 8 whatever K is.  A higher band holds row blocks of many groups, whose B tiles do not share anything, and comes
-// back to its A rows only after all of those (16 groups, 8192 x 7168 x 2048: 359 MB of DRAM reads for 294 MB of operands).  us, at
-// the power limit, bands of 34 MB / 8 / 16 row blocks: that shape 126.4 / 123.4 / 125.5; 32 groups, 8192 x 4096 x 4096 187 / 178 /
-// 180; 16 groups, 8192 x 1024 x 2048 27.9 / 26.7 / 27.5; four row blocks as eight.
-int w8_group_m(int64_t m_tiles, int64_t k_bytes, bool grouped) {
+// Grouped form (groups > 0): 8 while L2 keeps a group's B beside the band's A.  A higher band holds row blocks of several groups,
+// whose B tiles do not share anything, and comes back to its A rows only after all of those.  A B that L2 does not keep streams
+// through once per band: then all row blocks that a group has in the mean, within the 34 MB.  us, in turn, bands of 8 / of a
+// group's row blocks / of 34 MB: 16 groups, 8192 x 7168 x 2048 95.9 / 95.9 / 101; 4 groups, 8192 x 2048 x 4096 55.2 / 56.2 / 57.7;
+// one group, 4096 x 7168 x 4096 (29 MB of B) 85.1 / 87.1; 8192 x 4096 x 8192 (34 MB) 187.5 / 184.7, two groups 189.2 / 188.3; 4096
+// x 7168 x 7168 (51 MB) 149.0 / 143.5; 8192 x 4096 x 14336 (59 MB), one group 337 / 324, two 338 / 328 / 328, four 341 / 334 / 337,
+// eight 345 / 345 / 354.
+int w8_group_m(int64_t m_tiles, int64_t k_bytes, int64_t groups, int64_t b_bytes) {
   static const int forced = getenv("QGEMM_W8_GROUP_M") ? atoi(getenv("QGEMM_W8_GROUP_M")) : 0;  // tuning override
-  int64_t g = forced > 0 ? forced : (grouped ? 8 : (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1)));
+  int64_t g = (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1));
+  if (groups > 0) g = b_bytes <= (40ll << 20) ? 8 : std::min(g, m_tiles / groups);
+  if (forced > 0) g = forced;
   if (g < 8) g = 8;
   if (g > m_tiles) g = m_tiles;
   return (int)(g > 0 ? g : 1);
@@ -735,7 +740,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.sb_mode = (scale_b_len == 1) ? 0 : ((scale_b_len == N) ? 1 : 2);
   p.sa_mode = (scale_a == nullptr) ? 0 : ((scale_a_len == M) ? 1 : 2);
   p.m_tiles = (int)m_tiles;
-  p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K, false) + 1) / 2 : w8_group_m(m_tiles, K, meta != nullptr);
+  p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K, 0, 0) + 1) / 2 : w8_group_m(m_tiles, K, meta ? batch : 0, N * K);
   p.n_tiles = (int)((N + bn_eff - 1) / bn_eff);
   p.bn = bn_eff;
   const int64_t num_tiles = batchA * p.m_tiles * p.n_tiles;
