@@ -41,7 +41,9 @@ struct W4I8Cfg {
   static constexpr int ACC_COLS = 2 * MMAW * MT;
   static constexpr int TMEM_COLS = 512;
   static constexpr int BAR_BYTES = 512;
-  static constexpr int SMEM_BYTES = RAW_STAGES * W4_RAW_PACKED + A_STAGES * A_BYTES + BAR_BYTES + 1024;
+  static constexpr int ROW_SUM_BYTES = MT * 4;
+  static constexpr int SMEM_BYTES = RAW_STAGES * W4_RAW_PACKED + A_STAGES * A_BYTES + BAR_BYTES + ROW_SUM_BYTES + 1024;
+  static_assert(SMEM_BYTES <= 232448, "shared memory of a CTA");
   static constexpr int CH = (MT < 32) ? 16 : 32;
   static_assert(ACC_COLS + W_STAGES * W4I8_W_COLS <= 512, "tensor memory budget");
   // an MMA issuer takes every MMAW-th slab: with ring depths that are multiples of MMAW it always meets the same
@@ -112,7 +114,8 @@ w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uin
     keep[i] = c < chunks ? ld_written(x + c) : make_uint4(0u, 0u, 0u, 0u);
   }
 #pragma unroll
-  for (int i = 0; i < KEEP; ++i) m2 = aq_absmax8(keep[i], bf16, m2);
+  for (int i = 0; i < KEEP; ++i)
+    if (threadIdx.x + i * 256 < chunks) m2 = aq_absmax8(keep[i], bf16, m2);
   for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) m2 = aq_absmax8(ld_written(x + c), bf16, m2);
   float mx = aq_pair_max(m2, bf16);
 #pragma unroll
@@ -181,6 +184,7 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* epi_flag = tmem_slot + 2;
+  int* bias = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + Cfg::BAR_BYTES);  // 8 * sum_k a[m,k], signed nibbles
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -369,6 +373,10 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     int it = 0, seg_idx = 0;
     long long first_slab = 0;  // CTA-local index of the segment's first slab: issuer (first_slab + i) % MMAW took slab i
     pdl_wait();  // row sums and zeroed counters come from the pre-pass kernel
+    // Handed round through shared memory, once per CTA: the pre-pass may still have been writing them when this kernel started,
+    // which __ldg must not be used for, and ordinary loads at every tile's end made 128 x 4096 x 14336 37.1 us (__ldg 34.0, so 33.0).
+    if (SIGNED && nl < MT) bias[nl] = nl < p.M ? 8 * ld_written(p.row_sums + nl) : 0;
+    w4_epi_bar();
     while (seg.next(tile, ks0, ks1)) {
       const int buf = it & 1;
       const uint32_t tphase = (it >> 1) & 1;
@@ -402,13 +410,10 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           }
           if (full_tile) {
             if (n < p.N) {
-              int off[CH];
-#pragma unroll
-              for (int j = 0; j < CH; ++j) off[j] = SIGNED && c * CH + j < p.M ? 8 * ld_written(p.row_sums + c * CH + j) : 0;
 #pragma unroll
               for (int j = 0; j < CH; ++j) {
                 const int m = c * CH + j;
-                if (m < p.M) p.C[(size_t)m * p.N + n] = (int)r[j] - off[j];
+                if (m < p.M) p.C[(size_t)m * p.N + n] = (int)r[j] - (SIGNED ? bias[m] : 0);
               }
             }
           } else {
@@ -456,7 +461,7 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           for (int mb = 0; mb < rows; mb += RU) {
             int sum[RU];
 #pragma unroll
-            for (int u = 0; u < RU; ++u) sum[u] = SIGNED && mb + u < rows ? -8 * ld_written(p.row_sums + mb + u) : 0;
+            for (int u = 0; u < RU; ++u) sum[u] = 0;
 #pragma unroll 1
             for (int c = b_first; c <= b_last; ++c) {
               const long long c_end = w4_range_begin(T, G, c + 1);
@@ -470,7 +475,7 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             }
 #pragma unroll
             for (int u = 0; u < RU; ++u) {
-              if (mb + u < rows) p.C[(size_t)(mb + u) * p.N + n] = sum[u];
+              if (mb + u < rows) p.C[(size_t)(mb + u) * p.N + n] = sum[u] - (SIGNED ? bias[mb + u] : 0);
             }
           }
         }
