@@ -696,10 +696,9 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   const bool use_pair = meta == nullptr && !use_splitk && w8_pair_pays(batch, M, N, k_blocks, b_layout == QGEMM_B_KN, sms);
   const int BN = (N > 128 && (tiles256 >= sms || use_splitk || use_pair)) ? 256 : 128;
   const int64_t m_tiles = use_pair ? (M + 255) / 256 : row_blocks;  // of 128 rows, of 256 for two CTAs
-  // Width actually computed per tile (a multiple of 32, at most BN).  Narrower tiles that fill the last
-  // round of the persistent grid better were measured slower on B200 (224 instead of 256 columns on the
-  // 4096 x 4096 x 14336 shape: 235 us against 231 us), so the full width is used.
-  const int bn_eff = BN;
+  // Tiles are BN columns wide: narrower ones that fill the last round of the persistent grid better were slower (224 instead of
+  // 256 columns on the 4096 x 4096 x 14336 shape, by an earlier form of the kernel: 235 us against 231), and the epilogue wants
+  // multiples of 128.
   if (b_layout == QGEMM_B_KN) {
     const uint64_t dims[3] = {(uint64_t)N, (uint64_t)K, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)N, (uint64_t)K * (uint64_t)N};
@@ -715,7 +714,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   // C as a tensor map for the epilogue's tiled stores: boxes of 64 outputs x 32 rows, 128-byte swizzle.
   CUtensorMap tmC = tmA;
   static const int tma_store_on = getenv("QGEMM_W8_TMA_STORE") ? atoi(getenv("QGEMM_W8_TMA_STORE")) : 1;  // 0: per-row stores
-  const bool tma_store = tma_store_on && C != nullptr && (bn_eff % 64) == 0;
+  const bool tma_store = tma_store_on && C != nullptr;
   if (tma_store) {
     const uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)batchA};
     const uint64_t str[2] = {(uint64_t)N * 2, (uint64_t)M * (uint64_t)N * 2};
@@ -741,8 +740,8 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   p.sa_mode = (scale_a == nullptr) ? 0 : ((scale_a_len == M) ? 1 : 2);
   p.m_tiles = (int)m_tiles;
   p.group_m = use_pair ? (w8_group_m(2 * m_tiles, K, 0, 0) + 1) / 2 : w8_group_m(m_tiles, K, meta ? batch : 0, N * K);
-  p.n_tiles = (int)((N + bn_eff - 1) / bn_eff);
-  p.bn = bn_eff;
+  p.n_tiles = (int)((N + BN - 1) / BN);
+  p.bn = BN;
   const int64_t num_tiles = batchA * p.m_tiles * p.n_tiles;
   if (num_tiles > 0x7fffffff) return fail("qgemm_w8a8: too many tiles");
   p.num_tiles = (int)num_tiles;

@@ -25,7 +25,7 @@ struct W8A8Params {
   int m_tiles, n_tiles, num_tiles, k_blocks;
   int group_m;  // tile rasterisation: the tiles of `group_m` row blocks are walked column block by column block
 
-  int bn;            // columns per tile actually computed: a multiple of 32, at most the kernel's BN
+  int bn;            // columns per tile: the kernel's BN
   uint32_t* status;  // nullable device word
   unsigned long long wait_limit_ns;
   // Grouped (ragged) form: A and C are [M, K] / [M, N] stacks of row groups, B is [groups, ...]; row block i
@@ -39,7 +39,7 @@ struct W8A8Params {
   // twice as many SMs busy for about half as long.  num_items = num_tiles when nothing is split.
   int split_from, num_items;
   int withhold;   // test hook of the two-CTA form (qgemm_debug_withhold_commit)
-  int tma_store;  // C is written with tiled bulk stores from a shared-memory staging tile (needs bn % 64 == 0)
+  int tma_store;  // C is written with tiled bulk stores from a shared-memory staging tile
 };
 
 // One output tile's coordinates: batch index of B / scale_b, batch index of A / C / scale_a, first row, valid rows.
@@ -183,6 +183,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   using Cfg = W8Cfg<BN, FORM>;
   constexpr int STAGES = Cfg::STAGES;
   constexpr bool SPLITK = FORM == W8_SPLITK, PAIR = FORM == W8_PAIR;
+  // Two warps share the columns of 32 rows and store them in pieces of 64: an item of 128 columns at least (a half-width one, or
+  // a CTA's half of a tile whose K is cut, comes from 256).
+  static_assert(BN == 128 || (BN == 256 && (BN / 2) % 128 == 0), "columns of a tile");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
