@@ -52,17 +52,37 @@ def test_extreme_values():
     assert torch.equal(out.cpu(), oc.w4a8_gemm_ref(A, qB))
 
 
-@pytest.mark.parametrize("M,K,N", [(16, 6144, 18960), (3, 6176, 21008), (16, 5888, 19200)])
-def test_whole_tiles_behind_cut_ones(M, K, N):
-    """Few tokens, long K and at least a round of tiles: the remainder's tiles are cut along K first, whole ones follow."""
-    import tilelang_ascend_b200 as q
-    from oracle import qgemm_oracle as oc
-    g = torch.Generator().manual_seed(M + K + N)
-    A = torch.randint(-128, 128, (M, K), dtype=torch.int8, generator=g)
-    qB = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g)
-    C = q.w4a8_gemm_cv(M, N, K)(A.cuda(), qB.cuda(), torch.empty((N, K), dtype=torch.int8, device="cuda"),
-                                torch.empty((M, N), dtype=torch.int32, device="cuda"))
-    assert torch.equal(C.cpu(), oc.w4a8_gemm_ref(A, qB))
+# Weight tiles for a number of SMs, and whether there are whole ones in the form for few tokens and K of at least 24 slabs: a round
+# of whole tiles and nothing cut; a remainder of at least half a round, cut; two rounds and one tile, cut with one of the rounds; and
+# one round and one tile, all of which are cut.
+TILES = [(lambda sms: sms, True), (lambda sms: sms + (sms + 1) // 2 + 2, True), (lambda sms: 2 * sms + 1, True), (lambda sms: sms + 1, False)]
+
+
+@pytest.mark.parametrize("tiles,whole", TILES)
+@pytest.mark.parametrize("M,K", [(16, 6144), (1, 6176), (7, 5888), (17, 6144)])
+@pytest.mark.parametrize("form", ["signed", "unsigned", "quantised"])
+def test_whole_tiles_behind_cut_ones(form, M, K, tiles, whole):
+    """Few tokens, long K and at least a round of tiles: the remainder's tiles are cut along K first, whole ones follow.  K = 5888
+    (23 slabs) and 17 tokens stay with the other form.  Exact, against float64 sums."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = tiles(sms)
+    assert (n // sms - (1 if 0 < 2 * (n % sms) < sms else 0) > 0) == whole
+    N = 128 * n - 48
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    qB = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    W = torch.stack([qB & 15, qB >> 4], dim=-1).view(N, K).double()
+    if form != "unsigned":
+        W = torch.where(W >= 8, W - 16, W)
+    ws, C = torch.empty((N, K), dtype=torch.int8, device="cuda"), torch.empty((M, N), dtype=torch.int32, device="cuda")
+    if form == "quantised":
+        x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+        A, scale = q.act_quant(x)
+        C, s = q.w4a8_gemm_act_quant(M, N, K)(x, qB, ws, C)
+        assert torch.equal(s.view(-1), scale.view(-1))
+    else:
+        A = torch.randint(-128, 128, (M, K), dtype=torch.int8, generator=g, device="cuda")
+        C = q.w4a8_gemm_cv(M, N, K)(A, qB, ws, C) if form == "signed" else q.dequant_gemm_int8_wrapper(M, N, K, 128, 128, 64)(A, qB)
+    assert torch.equal(C.double(), A.double() @ W.T)
 
 
 @pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (48, 4096, 4096), (2, 16384 + 256, 1024)])
