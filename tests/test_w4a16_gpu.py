@@ -784,3 +784,31 @@ def test_scratch_for_single_ctas_is_enough(M, K, N):
     W = ((nib - 8) * S.T.repeat_interleave(128, dim=1)).double()
     mag = A.double().abs() @ W.abs().T
     assert ((C.double() - want).abs() <= 2.0 ** -10 * want.abs() + 2 * K * 2.0 ** -24 * mag + 1e-7).all()
+
+
+def test_switch_for_wide_tiles_of_two_ctas():
+    """QGEMM_W4_PAIR=0 (read once per process, hence a child process): single CTAs make the tiles, so that the test hook of the
+    two-CTA form changes nothing; one-hot activations read columns of (q - 8) * s back bit for bit."""
+    import os
+    import subprocess
+    import sys
+    code = r"""
+import torch
+from oracle import qgemm_oracle as oc
+import tilelang_ascend_b200 as q
+from tilelang_ascend_b200 import _lib
+_lib.load().qgemm_debug_withhold_commit(1)
+M, K, N = 430, 8192, 9472
+_, P, S = (t.cuda() for t in oc.make_w4a16_inputs(16, K, N, "float16", 128, seed=1))
+W = (torch.stack([P & 15, P >> 4], dim=-1).view(N, K).half() - 8) * S.T.repeat_interleave(128, dim=1)
+k = (torch.arange(M, device="cuda") * 2654435761) % K
+A = torch.zeros(M, K, dtype=torch.float16, device="cuda")
+A[torch.arange(M, device="cuda"), k] = 1.0
+status = torch.zeros(1, dtype=torch.int32, device="cuda")
+assert torch.equal(q.w4a16_gemm(A, P, S, 8, 128, status=status), W[:, k].T) and int(status.item()) == 0
+print("single ok")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, QGEMM_W4_PAIR="0"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "single ok" in r.stdout, r.stdout + r.stderr

@@ -348,3 +348,29 @@ def test_tiles_of_two_ctas_give_up_cleanly(layout, hook, codes):
     status.zero_()
     assert torch.equal(q.quant_matmul(A, B, sb, scale_a=sa, b_layout=layout, status=status), want)
     assert int(status.item()) == 0
+
+
+def test_switch_for_tiles_of_two_ctas():
+    """QGEMM_W8_PAIR=0 (read once per process, hence a child process): single CTAs make the tiles, so that the test hook of the
+    two-CTA form changes nothing, with the same bits."""
+    import os
+    import subprocess
+    import sys
+    code = r"""
+import torch
+from oracle import qgemm_oracle as oc
+import tilelang_ascend_b200 as q
+from tilelang_ascend_b200 import _lib
+_lib.load().qgemm_debug_withhold_commit(1)
+for batch, M, K, N in [(0, 1300, 3072, 2064), (3, 520, 4112, 2048)]:
+    A, B, sa, sb = oc.make_w8a8_inputs(batch, M, K, N, seed=M + N)
+    ref, acc_ref = oc.quant_matmul_ref(A, B, sb, "bfloat16", scale_a=sa, return_acc=True)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    C, acc = q.quant_matmul(A.cuda(), B.cuda(), sb.cuda(), scale_a=sa.cuda(), out_dtype="bfloat16", return_accumulators=True, status=status)
+    assert torch.equal(C.cpu(), ref) and torch.equal(acc.cpu(), acc_ref) and int(status.item()) == 0, (batch, M, K, N)
+print("single ok")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, QGEMM_W8_PAIR="0"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "single ok" in r.stdout, r.stdout + r.stderr

@@ -591,10 +591,13 @@ static int w8_rows_split(int64_t tiles, int64_t k_blocks, int64_t tokens, int sm
 
 // Whether two CTAs per tile of 256 x 256 (PAIR of w8a8.cuh) are faster than one per tile of 128 x 256 or 128 x 128.  Counted in
 // rounds of 128 x 256 tiles over the SMs: a last round that is cut in half-width items counts 0.6, a round of 128 x 128 tiles
-// 0.55, a round of pairs 0.87; the pairs' longer start and hand-over of a tile count the less the longer K is.  From a sweep over
-// 400 shapes, K 512 .. 8192, 64 .. 3500 tiles of 128 x 256, both layouts (us, one / two CTAs per tile): 4096 x 4096 x 14336
-// 166 / 150, 4096 x 2048 x 4096 31.5 / 30.0, 1300 x 2048 x 8192 23.8 / 24.7 (2.6 rounds against 3), 512 x 8192 x 5120 36.2 / 28.9,
-// but 4096 x 1024 x 4096 19.6 / 22.4.  QGEMM_W8_PAIR=0 disables it.
+// 0.55, a round of pairs 0.87; the pairs' longer start and hand-over of a tile count the less the longer K is.  The constants come
+// from a sweep with hand-overs at cluster scope, which cost pairs more than the plain ones now; they err on the side of one CTA.
+// Both ways in turn over 150 shapes, K 2048 .. 8192, both layouts: no shape that takes pairs is slower for it, and the choice is
+// 0.9 % behind the better one in the mean.  us, one / two CTAs per tile: 4096 x 4096 x 14336 166 / 148, 4096 x 2048 x 4096 30.2 /
+// 27.3, 16 x 512 x 7168 x 2048 [K, N] 94.7 / 89.3, [N, K] 100.9 / 89.0, 512 x 8192 x 5120 36.7 / 27.3, 3895 x 5824 x 1056 36.3 /
+// 31.0; not taken, though as fast or faster: 1300 x 2048 x 8192 23.5 / 22.8, 4096 x 1024 x 4096 19.4 / 18.9, and most shapes
+// with K below 2048.  QGEMM_W8_PAIR=0 disables it.
 static bool w8_pair_pays(int64_t batch, int64_t M, int64_t N, int64_t k_blocks, bool kn, int64_t sms) {
   static const int pair_on = getenv("QGEMM_W8_PAIR") ? atoi(getenv("QGEMM_W8_PAIR")) : 1;
   if (!pair_on || N <= 128 || k_blocks < 16) return false;

@@ -845,7 +845,9 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         uint16_t* Cout = reinterpret_cast<uint16_t*>(p.C) + (size_t)b * p.M * p.N;
         const int n = n0 + 4 * lane;  // four rows of the tile per lane
         const int rows = min(MT, p.M - m0);
-        constexpr int RU = 4, CU = 2;  // four tokens of two contributors in flight
+        // four tokens of two contributors in flight; of one at 33 .. 64 tokens: 64 x 8192 x 1024 27.6 us instead of 21.9, 64 x 8192 x
+        // 4096 17.6 / 16.5, 2 x 58 x 2304 x 1008 20.6 / 17.8, 64 x 8192 x 28672 37.5 / 38.0 (32 bytes of spills either way)
+        constexpr int RU = 4, CU = 2;
         // every contributor but the last one stops short of the tile's end: its partial tile is its second one (slot 2 c + 1)
         auto part = [&](int c, int m) {
           return reinterpret_cast<const float4*>(p.ws_partials + (size_t)(c == b_last ? 2 * c : 2 * c + 1) * (MT * W4_BN) +

@@ -155,12 +155,12 @@ w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uin
 
 // WHOLE: whole tiles per CTA where there is at least a round of them; the tiles that are cut come first, so that their hand-overs
 // run beside the whole tiles' stream and the launch ends with plain tile writes.  Its own instantiation, for 16 tokens and at least
-// 24 slabs of K.  us without / with it, 16 tokens with the quantiser, 148 | 188 | 224 | 297 tiles on 148 SMs: K = 4096 13.1 / 13.6 |
-// 18.0 / 17.9 | 19.4 / 19.8 | 21.7 / 21.5, 5120 15.7 / 15.8 | 21.0 / 21.0 | 22.6 / 22.5 | 26.3 / 25.5, 5888 16.8 / 16.9 | 22.7 / 22.8 |
-// 24.8 / 24.2 | 29.3 / 28.2, 6144 17.7 / 17.7 | 23.2 / 23.2 | 25.4 / 24.6 | 30.0 / 27.8, 8192 22.3 / 22.2 | 28.0 / 28.0 | 30.8 / 29.7 |
-// 36.7 / 34.9; 2048 x 28672 14.2 / 15.8.  So up to 5 % are lost with 16 slabs, 2 % up to 23 (5 tokens), nothing beyond 0.7 % from 24
-// on, where two rounds and more gain 3 to 8 %.  32 x 8192 x 28672 35.0 / 35.2; in the one kernel 64 x 8192 x 28672 took 45.7 instead
-// of 42.3.
+// 24 slabs of K.  us a call without / with it, 16 tokens with the quantiser, calls one after another, 148 | 224 | 260 | 297 | 371 |
+// 560 tiles on 148 SMs: K = 8192 19.9 / 20.0 | 29.1 / 28.3 | 32.5 / 31.0 | 35.3 / 33.3 | 41.4 / 39.3 | 56.8 / 53.9; 6144 15.6 / 15.6 |
+// 24.2 / 23.8 | 26.7 / 25.8 | 28.6 / 27.2 | 33.9 / 32.2 | 45.5 / 44.2; 5120 14.0 / 14.0 | 21.4 / 21.5 | 23.6 / 23.6 | 25.5 / 24.8 |
+// 29.8 / 28.0 | 39.5 / 38.8; 4096 12.8 / 12.7 | 18.6 / 19.3 | 20.1 / 20.8 | 21.5 / 21.9 | 25.3 / 24.6 | 33.4 / 34.7.  As one graph the
+// same up to two rounds but for 20 and 16 slabs, where 224 tiles take 20.5 / 21.1 and 17.5 / 18.8: so from 24 slabs on, where
+// nothing loses.  In the one kernel 64 x 8192 x 28672 took 8 % longer.
 template <int MT, bool SIGNED, bool WHOLE = false>
 __global__ void __launch_bounds__(W4_THREADS, 1)
 w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,

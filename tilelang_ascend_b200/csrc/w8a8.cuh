@@ -174,8 +174,8 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
 // CTA 32 KB of loads instead of 48, so that six of them are in flight instead of four, and B crosses from L2 once for 256 rows.
 // The leader (rank 0) issues; all bytes are counted on its barriers; its commits signal both CTAs, and the epilogue warps of both
 // hand an accumulator back to it.  Traffic is what bounds these shapes, for what it costs in time and, at the power limit, in
-// clock: 4096 x 4096 x 14336 166 -> 150 us (back to back for seconds 190 -> 175; 3.2 POPS, cuBLASLt's plain int8 GEMM 3.0),
-// 16 x 512 x 7168 x 2048 [N, K] 101 -> 91.  Which shapes take it: w8_pair_pays in qgemm_api.cu.
+// clock: 4096 x 4096 x 14336 166 -> 148 us (3.2 POPS, cuBLASLt's plain int8 GEMM 3.0; tensor pipe 92 % of active cycles instead of
+// 79, 1.9 GB from L2 into the SMs instead of 2.8), 16 x 512 x 7168 x 2048 [N, K] 101 -> 89.  Which shapes take it: w8_pair_pays in qgemm_api.cu.
 template <int BN, bool B_NK, bool OUT_BF16, W8Form FORM = W8_ALONE>
 __global__ void __launch_bounds__(W8_THREADS, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
