@@ -218,10 +218,10 @@ int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaSt
 // Grouped form (groups > 0): 8 while L2 keeps a group's B beside the band's A.  A higher band holds row blocks of several groups,
 // whose B tiles do not share anything, and comes back to its A rows only after all of those.  A B that L2 does not keep streams
 // through once per band: then all row blocks that a group has in the mean, within the 34 MB.  us, in turn, bands of 8 / of a
-// group's row blocks / of 34 MB: 16 groups, 8192 x 7168 x 2048 95.9 / 95.9 / 101; 4 groups, 8192 x 2048 x 4096 55.2 / 56.2 / 57.7;
-// one group, 4096 x 7168 x 4096 (29 MB of B) 85.1 / 87.1; 8192 x 4096 x 8192 (34 MB) 187.5 / 184.7, two groups 189.2 / 188.3; 4096
-// x 7168 x 7168 (51 MB) 149.0 / 143.5; 8192 x 4096 x 14336 (59 MB), one group 337 / 324, two 338 / 328 / 328, four 341 / 334 / 337,
-// eight 345 / 345 / 354.
+// group's row blocks / of 34 MB: 16 groups, 8192 x 7168 x 2048 95.9 / 95.9 / 100.4 (of 32 row blocks); 4 groups, 8192 x 2048 x 4096
+// 55.2 / 56.2 / 57.7; one group, 4096 x 7168 x 4096 (29 MB of B) 85.1 / 87.1; 8192 x 4096 x 8192 (34 MB) 187.5 / 184.7, two groups
+// 189.2 / 188.3; 4096 x 7168 x 7168 (51 MB) 149.0 / 143.5; 8192 x 4096 x 14336 (59 MB), one group 337 / 324, two 338 / 328 / 328,
+// four 341 / 334 / 337, eight 345 / 345 / 354.
 int w8_group_m(int64_t m_tiles, int64_t k_bytes, int64_t groups, int64_t b_bytes) {
   static const int forced = getenv("QGEMM_W8_GROUP_M") ? atoi(getenv("QGEMM_W8_GROUP_M")) : 0;  // tuning override
   int64_t g = (34ll << 20) / (128 * (k_bytes > 0 ? k_bytes : 1));
