@@ -812,3 +812,26 @@ print("single ok")
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, QGEMM_W4_PAIR="0"), capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "single ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("batch,M,K,N", [
+    # one (row, slab) per warp of the pre-pass; a last slab that is cut; two in registers; three and ten in shared memory; rounds of
+    # several, the last one partly filled; as many blocks as an SM holds
+    (1, 1, 288, 40), (3, 5, 1312, 64), (1, 48, 4384, 72), (2, 33, 6432, 40), (23, 16, 4096, 48), (40, 16, 4096, 64), (9, 64, 8192, 40),
+    (1, 64, 8224, 128), (19, 61, 5152, 40)])
+@pytest.mark.parametrize("dt", ["float16", "bfloat16"])
+def test_pre_pass_of_the_group_sum_kernel(batch, M, K, N, dt):
+    """Small integer activations and scales of one: the fp32 sums are exact, so the result is the float64 product rounded once.
+    The scratch starts as NaN: activation rows beyond M are not written and must not reach an output."""
+    q = _q()
+    g = torch.Generator(device="cuda").manual_seed(K + 64 * M + batch)
+    A = torch.randint(-3, 4, (batch, M, K), generator=g, device="cuda").to(getattr(torch, dt))
+    P = torch.randint(0, 256, (batch, N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    S = torch.ones((batch, 1, N), dtype=torch.float16, device="cuda")
+    W = torch.stack([P & 15, P >> 4], dim=-1).view(batch, N, K).double() - 8
+    want = (A.double() @ W.transpose(1, 2)).to(getattr(torch, dt))
+    if batch == 1:
+        A, P, S, want = A[0], P[0], S[0], want[0]
+    poison = torch.full((1 << 24,), float("nan"), device="cuda")  # the scratch comes from this block
+    del poison
+    assert torch.equal(q.w4a16_gemm(A, P, S, 8, K), want)

@@ -300,21 +300,21 @@ int g_withhold = 0;
 
 // `tmZ` non-null: the zeros-tensor instantiation (not combined with the gathered form).
 template <int MT>
-int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap* tmZ, const qg::W4A16Params& p,
-               int grid, cudaStream_t s) {
+int launch_w4g(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, const CUtensorMap* tmZ, const CUtensorMap& tmA,
+               const qg::W4A16Params& p, int grid, cudaStream_t s) {
   qg::W4GDebug dbg;
   dbg.withhold_last_commit = g_withhold;
   constexpr int smem = qg::W4GCfg<MT>::SMEM_BYTES, smem_zt = qg::W4GCfg<MT, true>::SMEM_BYTES;
   if (tmZ != nullptr) {
-    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, p, dbg);
-    return launch_pdl(qg::w4a16_gs_kernel<MT, false, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, p, dbg);
+    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, tmA, p, dbg);
+    return launch_pdl(qg::w4a16_gs_kernel<MT, false, false, true>, grid, qg::W4G_THREADS, smem_zt, s, tmW, tmS, *tmZ, tmA, p, dbg);
   }
   if (p.n_dst > 0) {
-    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
-    return launch_pdl(qg::w4a16_gs_kernel<MT, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+    if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
+    return launch_pdl(qg::w4a16_gs_kernel<MT, false, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
   }
-  if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
-  return launch_pdl(qg::w4a16_gs_kernel<MT, false>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, p, dbg);
+  if (bf) return launch_pdl(qg::w4a16_gs_kernel<MT, true>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
+  return launch_pdl(qg::w4a16_gs_kernel<MT, false>, grid, qg::W4G_THREADS, smem, s, tmW, tmS, tmS, tmA, p, dbg);
 }
 
 // The wide tiles, `workers` CTAs or pairs of them; a programmatic dependent of the pre-pass.
@@ -345,15 +345,21 @@ int launch_w4w(bool bf, bool zt, const CUtensorMap& tmW, const CUtensorMap& tmS,
   return bf ? launch_w4w<true, false, PAIR>(tmW, tmS, tmZ, tmA, p, mt, 0, workers, s) : launch_w4w<false, false, PAIR>(tmW, tmS, tmZ, tmA, p, mt, 0, workers, s);
 }
 
-// The pre-pass of the group-sum kernel: activations -> stage images.
-template <int MT>
-int launch_w4g_prepare(const void* A, void* out, const qg::W4A16Params& p, bool is_bf16, cudaStream_t s) {
-  const long long threads = (long long)p.batch * p.m_tiles * (2 * p.KS) * MT * 4;
-  const long long blocks = (threads + 127) / 128;
-  if (blocks > 0x7fffffffll) return fail("qgemm_w4a16: activation tensor too large");
-  return launch_pdl(qg::w4g_prepare_activations<MT>, (int)blocks, 128, 0, s, static_cast<const uint4*>(A),
-                    static_cast<uint8_t*>(out), p.batch, p.M, p.K, p.m_tiles, 2 * p.KS, is_bf16 ? 1 : 0,
-                    p.ws_counters, (int)(kW4CounterBytes / 4));
+// The pre-pass of the group-sum kernel.
+int launch_w4g_prepare(const void* A, void* out, const qg::W4A16Params& p, bool is_bf16, int sms, cudaStream_t s) {
+  constexpr int warps = qg::W4G_PREP_THREADS / 32;
+  const long long rows = (long long)p.batch * p.M, slabs = rows * p.KS;
+  if (p.m_tiles != 1 || slabs > 0x3fffffffll) return fail("qgemm_w4a16: activation tensor too large");
+  // A block per SM at most, so that all are resident early, and each warp's share in equal rounds.  From four rounds on throughput
+  // counts for more than an early start: as many blocks as an SM holds.  us, one / eleven blocks per SM (one for every 128 chunks
+  // of 32 k, before): 24 x 60 x 7424 x 1408 51.9 / 45.8 (50.5), 32 x 64 x 8192 x 1024 63.6 / 51.3 (58.2); from two rounds on 20 x 48
+  // x 4096 x 2048 33.9 / 35.8 (37.0), 8 x 64 x 8192 x 1024 25.4 / 27.5 (28.0), but 24 x 64 x 4096 x 4096 70.3 / 69.0.
+  const long long each = (slabs + warps * sms - 1) / (warps * sms), rounds = (each + qg::W4G_PREP_LANDING - 1) / qg::W4G_PREP_LANDING;
+  const int per = (int)((each + rounds - 1) / rounds);
+  const int grid = (int)std::min<long long>(sms * (rounds > 4 ? 11 : 1), (slabs + warps * per - 1) / (warps * per));
+  auto kernel = per <= qg::W4G_PREP_REGS ? qg::w4g_prepare_activations<false> : qg::w4g_prepare_activations<true>;
+  return launch_pdl(kernel, grid, qg::W4G_PREP_THREADS, 0, s, static_cast<const uint4*>(A), static_cast<uint8_t*>(out), (int)rows, p.M,
+                    p.K, p.KS, is_bf16 ? 1 : 0, per, reinterpret_cast<uint4*>(p.ws_counters), (int)(kW4CounterBytes / 4));
 }
 
 // Single-launch form of the group-sum kernel (see its SMALL parameter): clusters of `cluster` CTAs, one tile per cluster,
@@ -376,8 +382,8 @@ int launch_w4g_small(bool bf, const CUtensorMap& tmW, const CUtensorMap& tmS, co
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
-  if (bf) CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, true, false, false, true>, tmW, tmS, tmS, p, dbg));
-  else CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, false, false, false, true>, tmW, tmS, tmS, p, dbg));
+  if (bf) CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, true, false, false, true>, tmW, tmS, tmS, tmS, p, dbg));
+  else CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w4a16_gs_kernel<16, false, false, false, true>, tmW, tmS, tmS, tmS, p, dbg));
   return 0;
 }
 
@@ -910,7 +916,8 @@ static W4Route w4_route(int64_t M, int64_t K, int64_t group, bool has_scales, bo
 
 // Scratch of the kernels for few tokens: the arrival counters first (fixed place whatever the tile height), then two
 // partial slots of [MT][128] fp32 per CTA, then the prepared activations - plain f16 [M, K] in the kernel's K order, or
-// the group-sum kernel's stage images (token tiles padded).
+// in blocks of
+// 64 k for the group-sum kernel (counted with its token tile).
 static int64_t w4_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
   if (ensure_device(&sms)) return -1;
@@ -1160,10 +1167,15 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   if (use_gs) {
     const CUtensorMap* tz = zeros != nullptr ? &tmZ : nullptr;
     const bool a_bf = a_dtype == QGEMM_DT_BF16;
-    p.A_raw = a_prepared;
-    if (mt == 16) return launch_w4g_prepare<16>(A, a_prepared, p, a_bf, s) || launch_w4g<16>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
-    if (mt == 32) return launch_w4g_prepare<32>(A, a_prepared, p, a_bf, s) || launch_w4g<32>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
-    return launch_w4g_prepare<64>(A, a_prepared, p, a_bf, s) || launch_w4g<64>(bf, tmW, tmS, tz, p, (int)grid, s) ? -1 : 0;
+    // prepared activations: [batch][64-k block][M][64], K padded to whole slabs
+    const uint64_t dims[3] = {64, (uint64_t)M, (uint64_t)batch * (uint64_t)p.KS * 4};
+    const uint64_t str[2] = {128, (uint64_t)M * 128};
+    const uint32_t box[3] = {64, (uint32_t)mt, 4};
+    if (encode_map(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, a_prepared, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+    if (launch_w4g_prepare(A, a_prepared, p, a_bf, sms, s)) return -1;
+    if (mt == 16) return launch_w4g<16>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
+    if (mt == 32) return launch_w4g<32>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
+    return launch_w4g<64>(bf, tmW, tmS, tz, tmA, p, (int)grid, s);
   }
   {
     const long long n_chunks = (long long)batch * M * K / 8;

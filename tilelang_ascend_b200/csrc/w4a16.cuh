@@ -46,8 +46,8 @@ struct W4A16Params {
   // whole tiles sk_tiles + c + j * grid.  The other kernels deal all (tile, slab) items evenly (total_items).
   int sk_tiles, dp_rounds;
   int sk_grid;  // wide tiles only: the first sk_tiles tiles are cut over this many CTAs
-  // Group-sum kernel: the prepared activations (stage images) or, in its single-launch form (no pre-pass), the caller's
-  // activations [batch, M, K] and whether they are bf16; and whether the weight layout is the interleaved one.
+  // Group-sum kernel: in its single-launch form (no pre-pass) the caller's activations [batch, M, K], and whether they are
+  // bf16; and whether the weight layout is the interleaved one.
   const void* A_raw;
   int a_is_bf16, w_interleaved;
   int scale_rows;       // scale rows fetched per slab (256 / group, at least 1)

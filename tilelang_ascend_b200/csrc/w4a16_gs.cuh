@@ -15,14 +15,15 @@
 //    40.8 / 40.5; only raw nibbles, 64 tokens, 38.0 / 39.5.  And a large
 //    activation at a weight equal to zero then costs all other terms of the half their low bits: 18 to 400 times the
 //    bound of test_large_activations_at_the_zero_point; an infinite one makes the difference NaN.)
-//  - Activations are laid out by the pre-pass in the exact image of a shared-memory stage (swizzle, K order), so that a
-//    stage is one untiled bulk copy.
+//  - Activations are laid out by the pre-pass in the kernel's K order, so that a stage is one copy.  (Four, one for every 64 k, which
+//    could leave out the rows beyond M without a tensor map, are more than the producer gets to issue: one token of 8192 x 28672
+//    29.9 us instead of 26.5.)
 //  - All hand-overs are by whole slabs; one commit per slab signals one barrier that the weight stage, the activation
 //    stage and the accumulators share; the group scales arrive with the packed bytes and need no barrier of their own.
 //
 // Structure (persistent; the K slabs of the tiles are dealt to the CTAs, see W4HybridIter):
 //   warp 0        TMA: packed weights [128 rows x 128 B] per slab into the raw ring, the slab's scale (and zero) rows
-//   warp 1        bulk copies: prepared activations
+//   warp 1        TMA: prepared activations
 //   warps 2, 3    tcgen05.mma kind::f16 issuers (A = weights from tensor memory, B = activations from shared memory):
 //                 issuer w takes the slabs i with i % 2 == w, each of the two halves into its own accumulator
 //   warps 4..11   drain: tcgen05.ld of a half's accumulator, fp32 FMA with the half's scale into register sums, in two sets of
@@ -190,13 +191,6 @@ __device__ __forceinline__ void w4g_fma2(float& d0, float& d1, uint32_t a0, uint
 // Named barrier of the eight drain warps.
 __device__ __forceinline__ void w4g_epi_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// Untiled bulk copy global -> shared memory.
-__device__ __forceinline__ void w4g_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
 // The segments of a CTA: those of its stream-K range, then its whole tiles (first_dp, first_dp + stride, ...).
 struct W4HybridIter {
   W4SegIter sk;
@@ -233,14 +227,13 @@ __device__ __forceinline__ uint4 w4g_to_f16(uint4 v, bool is_bf16) {
   }
   return v;
 }
-// Byte offset of 16-byte piece j (0..15) of row r inside a half's image: 64-k block j / 8, 128-byte swizzle.
+// Byte offset of 16-byte piece j (0..15) of row r inside a half of an activation stage: 64-k block j / 8, 128-byte swizzle.
 template <int MT>
 __device__ __forceinline__ uint32_t w4g_a_offset(int r, int j) {
   return (uint32_t)((j >> 3) * (MT * 128) + r * 128 + (((j & 7) ^ (r & 7)) << 4));
 }
 
-// One 32-k chunk (chunk c of four) of row r: four 16-byte loads already in v -> the half's image at dst (global or shared
-// memory).
+// One 32-k chunk (chunk c of four) of row r: four 16-byte loads already in v -> a half of a stage (single-launch form).
 template <int MT>
 __device__ __forceinline__ void w4g_emit_chunk(uint8_t* dst, int r, int c, const uint4 (&v)[4]) {
   uint2 lo[4], hi[4];
@@ -252,38 +245,87 @@ __device__ __forceinline__ void w4g_emit_chunk(uint8_t* dst, int r, int c, const
   *reinterpret_cast<uint4*>(dst + w4g_a_offset<MT>(r, 4 * c + 3)) = make_uint4(hi[2].x, hi[2].y, hi[3].x, hi[3].y);
 }
 
-// Pre-pass: activations [batch, M, K] (f16 or bf16) -> [batch][token tile][half] images (rows beyond M and k beyond K are
-// zero).  One thread per 32-k chunk.  Block 0 also zeroes the split-K arrival counters, so every call starts from clean
-// counters whatever an earlier (possibly aborted) call left in the scratch.
-template <int MT>
-__global__ void __launch_bounds__(128)
-w4g_prepare_activations(const uint4* __restrict__ in, uint8_t* __restrict__ out, int batch, int M, int K, int m_tiles,
-                        int halves, int is_bf16, uint32_t* __restrict__ counters, int n_counters) {
+// Pre-pass: activations [batch, M, K] (f16 or bf16) -> f16 [batch][64-k block][M][64] in the kernel's K order, whose blocks a tiled
+// copy lays out as an activation stage wants them, rows beyond M zero.  (Rows that are left as they were reach nobody's sums but
+// cost power: one token of 8192 x 28672 29.7 us for seconds instead of 28.1.)  A warp takes the 256 k of a slab of one
+// row at a time, eight values a lane, `per` of them in flight.  k beyond K are zero.  Block 0 also zeroes the split-K arrival
+// counters, so every call starts from clean counters whatever an earlier (possibly aborted) call left in the scratch.
+// What bounds it is latency, between the end of the kernel in front and the GEMM kernel's first MMA, so all of its blocks should
+// be waiting on an SM each when that kernel ends.  Behind another call of this operator, whose CTAs hold every SM, that takes
+// blocks that fit beside a CTA of the GEMM kernel - 128 threads of 32 registers, what its 768 x 80 leave of the register file, and
+// what its shared memory leaves - and no more of them than SMs (but see launch_w4g_prepare).  More blocks than that (one for every 128 chunks of 32 k of all
+// MT rows) waited for the first SMs to become free, filled these, 16 to an SM, and kept the next call's GEMM CTAs off them for up
+// to 10 us: 32 x 16 x 4096 x 4096 61.9 -> 59.2 us, 11 x 2 x 4352 x 1344 18.3 -> 14.4, 16 x 48 x 4096 x 2048 32.1 -> 28.3.
+// LANDING: the values in flight wait in shared memory, since 32 registers hold two; with one or two the way through shared
+// memory is the longer one (2 x 1280 x 14752 5.70 us, 5.60 without).
+constexpr int W4G_PREP_THREADS = 128;
+constexpr int W4G_PREP_REGS = 2;      // (row, slab) in flight per warp in registers,
+constexpr int W4G_PREP_LANDING = 10;  // in shared memory: 20 KB, what a CTA of the 64-token kernel leaves
+__device__ __forceinline__ void w4g_prep_emit(uint8_t* out, uint4 v, bool is_bf16, int M, int b, int m, int KS, int ks, int lane) {
+  const int w = lane & 3, piece = (lane & 4) + (w >> 1);  // word w of the block's 32-k chunk (lane / 4) % 2
+  uint2 lo, hi;
+  w4g_split_word(w4g_to_f16(v, is_bf16), lo, hi);
+  uint8_t* dst = out + ((((size_t)b * KS + ks) * 4 + (lane >> 3)) * M + m) * 128 + piece * 16 + (w & 1) * 8;
+  *reinterpret_cast<uint2*>(dst) = lo;
+  *reinterpret_cast<uint2*>(dst + 32) = hi;
+}
+template <bool LANDING>
+__global__ void __launch_bounds__(W4G_PREP_THREADS, 16)
+w4g_prepare_activations(const uint4* in, uint8_t* __restrict__ out, int rows, int M, int K, int KS, int is_bf16, int per,
+                        uint4* __restrict__ counters, int n_counters) {
   pdl_launch_dependents();  // the GEMM kernel behind may set up and start streaming weights meanwhile
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = (int)(i & 3);
-  const int r = (int)((i >> 2) % MT);
-  const long long blk = (i >> 2) / MT;  // (b * m_tiles + tile) * halves + half
-  const int half = (int)(blk % halves);
-  const long long bt = blk / halves;
-  const int tile = (int)(bt % m_tiles);
-  const long long b = bt / m_tiles;
+  const int lane = threadIdx.x & 31, warp = (int)(blockIdx.x * (W4G_PREP_THREADS / 32) + (threadIdx.x >> 5));
+  const int first = per * warp, step = per * (int)gridDim.x * (W4G_PREP_THREADS / 32);
+  int row = first / KS, ks = first - row * KS;  // row: of all problems'
   pdl_wait();  // the kernel in front (another call's GEMM, which lets its dependents start early) is done
-  if (blockIdx.x == 0)
-    for (int k = threadIdx.x; k < n_counters; k += blockDim.x) counters[k] = 0u;
-  if (b >= batch) return;
-  const int m = tile * MT + r, k0 = half * 128 + c * 32;
-  uint4 v[4];
+  auto src = [&](int r, int k) { return in + ((size_t)r * (size_t)K + k * W4_SLAB_K) / 8 + lane; };  // K is a multiple of 32
+  auto in_row = [&](int k) { return k * W4_SLAB_K + lane * 8 < K; };
+  while (row < rows) {
+    int r = row, k = ks, b = row / M, m = row - b * M;
+    auto next = [&]() {
+      if (++k == KS) {
+        k = 0;
+        ++r;
+        if (++m == M) { m = 0; ++b; }
+      }
+    };
+    if constexpr (LANDING) {
+      __shared__ uint4 landing[W4G_PREP_LANDING * W4G_PREP_THREADS];
+      const uint4* mine = landing + threadIdx.x;  // a thread reads only what it has copied itself
+      const int n = min(per, (rows - row) * KS - ks);
+      for (int u = 0; u < n; ++u) {
+        if (in_row(k)) cp_async16(smem_u32(mine + u * W4G_PREP_THREADS), src(r, k));
+        if (++k == KS) { k = 0; ++r; }
+      }
+      cp_async_wait();
+      r = row;
+      k = ks;
+#pragma unroll 1
+      for (int u = 0; u < n; ++u) {
+        w4g_prep_emit(out, in_row(k) ? mine[u * W4G_PREP_THREADS] : make_uint4(0u, 0u, 0u, 0u), is_bf16 != 0, M, b, m, KS, k, lane);
+        next();
+      }
+    } else {
+      uint4 v[W4G_PREP_REGS];
 #pragma unroll
-  for (int w = 0; w < 4; ++w) v[w] = make_uint4(0u, 0u, 0u, 0u);
-  if (m < M && k0 < K) {  // K is a multiple of 32
-    const uint4* src = in + ((size_t)b * M + m) * (size_t)(K / 8) + k0 / 8;
+      for (int u = 0; u < W4G_PREP_REGS; ++u) {
+        v[u] = u < per && r < rows && in_row(k) ? ld_written(src(r, k)) : make_uint4(0u, 0u, 0u, 0u);
+        if (++k == KS) { k = 0; ++r; }
+      }
+      r = row;
+      k = ks;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) v[w] = ld_written(src + w);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) v[w] = w4g_to_f16(v[w], is_bf16 != 0);
+      for (int u = 0; u < W4G_PREP_REGS; ++u) {
+        if (u < per && r < rows) w4g_prep_emit(out, v[u], is_bf16 != 0, M, b, m, KS, k, lane);
+        next();
+      }
+    }
+    ks += step;
+    row += ks / KS;
+    ks %= KS;
   }
-  w4g_emit_chunk<MT>(out + (size_t)blk * w4g_half_bytes(MT), r, c, v);
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < n_counters / 4; i += W4G_PREP_THREADS) counters[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // Sixteen packed bytes (32 weights) -> eight f16x2 words of the low nibbles' q - zero, then eight of the high ones', K order
@@ -352,14 +394,15 @@ __device__ __forceinline__ void w4g_store_tile(const W4A16Params& p, int b, int 
 // clusters of C = KS / (slabs per CTA) CTAs, one tile per cluster, CTA r taking the r-th K range; there is no pre-pass
 // and no scratch memory:
 //  - the drain warps first fetch the CTA's own piece of the activations straight from the caller's tensor and write the
-//    stage images the pre-pass would have written;
+//    stages as the copies of what the pre-pass makes would have;
 //  - at the end CTAs 1 .. C-1 write their sums through distributed shared memory into the unused upper half of the
 //    first CTA's raw ring, and the first CTA adds them in rank order and writes the tile - no counters, no partial
 //    sums in global memory, the same fixed summation order on every run.
 template <int MT, bool OUT_BF16, bool GATHER = false, bool ZT = false, bool SMALL = false>
 __global__ void __launch_bounds__(W4G_THREADS, 1)
 w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
-                const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ W4A16Params p, const W4GDebug dbg) {
+                const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ W4A16Params p,
+                const W4GDebug dbg) {
   using Cfg = W4GCfg<MT, ZT>;
   constexpr int RS = Cfg::RS;
   constexpr int AS = Cfg::AS;
@@ -414,6 +457,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     tma_prefetch_desc(&tmW);
     if (p.has_scales) tma_prefetch_desc(&tmS);
     if (ZT) tma_prefetch_desc(&tmZ);
+    if (!SMALL) tma_prefetch_desc(&tmA);
   }
   if (warp == W4G_FIRST_MMA_WARP + 1) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -479,11 +523,12 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         int srow = (ks / spg) * row_step, in_group = ks % spg;
         int st = 0;
         uint32_t phase = 0;
+        const uint64_t once = l2_policy_evict_first();
         while (i < n_slabs) {
           w4g_wait<W4G_RAW_EMPTY, ST_TIMEOUT_PRODUCER>(bar0 + 8 * st, phase ^ 1u, ctl, fail);
           if (fail) break;
           mbar_arrive_expect_tx(&raw_full[st], tx);
-          tma_load_3d(raw_base + st * W4_RAW_PACKED, &tmW, &raw_full[st], ks * (W4_SLAB_K / 2), n0, b);
+          tma_load_3d_hint(raw_base + st * W4_RAW_PACKED, &tmW, &raw_full[st], ks * (W4_SLAB_K / 2), n0, b, once);
           // scale rows of the slab: two when the groups are 128 wide, else the one row of the slab's group
           if (p.has_scales) tma_load_3d(sc_base + (i % Cfg::SS) * W4G_SC_BYTES, &tmS, &raw_full[st], n0, srow, b);
           if (ZT) tma_load_3d(z_base + st * W4G_SC_BYTES, &tmZ, &raw_full[st], n0, srow, b);
@@ -502,12 +547,6 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
       } else {
         pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
-        const uint32_t a0 = smem_u32(a_base);
-        const uint8_t* base = reinterpret_cast<const uint8_t*>(p.A_raw);
-        auto tile_src = [&](int k) {
-          return base + (((size_t)b * p.m_tiles + (size_t)(m0 / MT)) * (size_t)p.KS + (size_t)k) * Cfg::A_BYTES;
-        };
-        const uint8_t* src = tile_src(ks);
         int st = 0;
         while (i < n_slabs) {
           if (i >= AS)  // the slab that used this stage has been multiplied
@@ -515,17 +554,17 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           if (fail) break;
           uint64_t* bar = &a_full[i % W4G_BARS];
           mbar_arrive_expect_tx(bar, Cfg::A_BYTES);
-          w4g_bulk_load(a0 + st * Cfg::A_BYTES, src, Cfg::A_BYTES, smem_u32(bar));
+          tma_load_3d(a_base + st * Cfg::A_BYTES, &tmA, bar, 0, 0, (b * p.KS + ks) * 4);  // four blocks of 64 k, MT rows each
           issued_mask |= 1u << (i % W4G_BARS);
           parity_mask = (parity_mask & ~(1u << (i % W4G_BARS))) | (((uint32_t)(i / W4G_BARS) & 1u) << (i % W4G_BARS));
           if (++st == AS) st = 0;
           ++i;
-          src += Cfg::A_BYTES;
+          ++ks;
           if (--left == 0) {
             tile = i == n_sk ? p.sk_tiles + cta : tile + (i < n_sk ? 1 : G);
+            ks = 0;
             left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
             w4_tile_coords(p, tile, MT, b, n0, m0);
-            src = tile_src(0);
           }
         }
       }
