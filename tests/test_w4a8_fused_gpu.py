@@ -122,3 +122,26 @@ def test_behind_the_kernels_that_write_its_activations(M, K, N, fused):
     for _ in range(3):
         assert all(torch.equal(x, y) for x, y in zip(chain(False), want))
     assert len({int(c.view(-1)[0]) for c in want if c.dtype == torch.int32}) > 1  # the steps differ
+
+
+# blocks per row of the pre-pass: eight, as many as leave one per SM, one; rows of more chunks than it keeps in shared memory; parts
+# that are not whole multiples of a block's threads
+@pytest.mark.parametrize("M,K", [(1, 4128), (18, 4128), (19, 8224), (37, 8192), (49, 8224), (74, 4096), (75, 4128), (128, 8224), (5, 16416)])
+@pytest.mark.parametrize("dt", ["bfloat16", "float16"])
+def test_parts_of_the_pre_pass(M, K, dt):
+    """Quantised activations and their row sums, made by several blocks per row: exact against the quantiser's int8 values, with
+    weights whose sums the row sums decide."""
+    N = 5120
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    x = (torch.randn((M, K), generator=g, device="cuda") + 0.5).to(getattr(torch, dt))
+    x[:, -1] = 7.0  # the largest value of a row belongs to its last part
+    qB = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    W = torch.stack([qB & 15, qB >> 4], dim=-1).view(N, K).double()
+    W = torch.where(W >= 8, W - 16, W)
+    ws = torch.full((N, K), 0x55, dtype=torch.int8, device="cuda")
+    C = torch.empty((M, N), dtype=torch.int32, device="cuda")
+    A, scale = q.act_quant(x)
+    want = A.double() @ W.T
+    got, s = q.w4a8_gemm_act_quant(M, N, K)(x, qB, ws, C)
+    assert torch.equal(s.view(-1), scale.view(-1)) and torch.equal(got.double(), want)
+    assert torch.equal(q.w4a8_gemm_cv(M, N, K)(A, qB, ws, torch.empty_like(C)).double(), want)

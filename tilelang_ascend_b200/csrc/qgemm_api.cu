@@ -502,7 +502,10 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   if (need > N * K) return 1;  // the caller's workspace is [N, K] int8
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   uint8_t* a_prepared = ws + kW4CounterBytes + partial_bytes;
-  int* row_sums = reinterpret_cast<int*>(a_prepared + a_bytes);
+  // Blocks of the pre-pass per row: as many as leave one block for every SM.  The sums over their parts of K stand behind the
+  // counters that are used.
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>({qg::W4I8_PREP_MAX_PARTS, sms / M, (kW4MaxGrid - grid_max) / M}));
+  int* row_sums = parts > 1 ? reinterpret_cast<int*>(ws) + grid_max : reinterpret_cast<int*>(a_prepared + a_bytes);
 
   CUtensorMap tmW, tmA;
   {
@@ -522,6 +525,7 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   p.ws_counters = reinterpret_cast<uint32_t*>(ws);
   p.ws_partials = reinterpret_cast<int*>(ws + kW4CounterBytes);
   p.row_sums = row_sums;
+  p.row_parts = parts;
   p.M = (int)M;
   p.N = (int)N;
   p.K = (int)K;
@@ -537,13 +541,13 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   p.sk_tiles = (int)(borrow ? left + grid : left);
   // a programmatic dependent of whatever is in front: behind another call of this operator it is resident early
   if (X != nullptr) {
-    if (launch_pdl(qg::w4a8_quant_prepare_activations, (int)M, 256, 0, s, static_cast<const uint4*>(X), x_is_bf16,
-                   round_scale, reinterpret_cast<uint2*>(a_prepared), row_sums, scale_out,
-                   reinterpret_cast<uint32_t*>(ws), (int)(kW4CounterBytes / 4), (int)K))
+    if (launch_pdl(qg::w4a8_quant_prepare_activations, (int)M * parts, qg::W4I8_PREP_THREADS, 16 * (int)std::min<int64_t>(K / 8, qg::W4I8_PREP_KEPT), s, static_cast<const uint4*>(X),
+                   x_is_bf16, round_scale, reinterpret_cast<uint2*>(a_prepared), row_sums, scale_out, p.ws_counters, (int)grid_max,
+                   (int)K, (int)M, parts))
       return -1;
-  } else if (launch_pdl(qg::w4a8_prepare_activations, (int)M, 256, 0, s, reinterpret_cast<const uint2*>(A),
-                        reinterpret_cast<uint2*>(a_prepared), row_sums, reinterpret_cast<uint32_t*>(ws),
-                        (int)(kW4CounterBytes / 4), (int)K))
+  } else if (launch_pdl(qg::w4a8_prepare_activations, (int)M * parts, qg::W4I8_PREP_THREADS, 0, s,
+                        reinterpret_cast<const uint2*>(A), reinterpret_cast<uint2*>(a_prepared), row_sums, p.ws_counters,
+                        (int)grid_max, (int)K, (int)M, parts))
     return -1;
   const bool sgn = signed_nibbles != 0;
   switch (mt) {

@@ -19,8 +19,9 @@ namespace qg {
 struct W4A8Params {
   int* C;                // [M, N] int32
   int* ws_partials;      // scratch: 2 * grid slots of [MT][128] int32
-  uint32_t* ws_counters; // scratch: grid counters, zeroed by the pre-pass kernel of every call
-  const int* row_sums;   // [M] sum_k A[m,k] (signed nibbles only)
+  uint32_t* ws_counters; // scratch: a counter per CTA, zeroed by the pre-pass kernel of every call
+  const int* row_sums;   // [row_parts][M] sums over parts of K of A[m,k] (signed nibbles only)
+  int row_parts;
   int M, N, K;
   int n_tiles;           // 128-row weight tiles; one token tile (M <= MT)
   int KS;                // 256-wide K slabs per tile
@@ -52,36 +53,46 @@ struct W4I8Cfg {
 };
 
 // Pre-pass: int8 activations [M, K] -> the same values with every group of eight k reordered to
-// 0,2,4,6,1,3,5,7 (the byte order the unpack produces), and the row sums.  One block per row.
-__global__ void __launch_bounds__(256)
-w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restrict__ row_sums,
-                         uint32_t* __restrict__ counters, int n_counters, int K) {
-  __shared__ int red[8];
+// 0,2,4,6,1,3,5,7 (the byte order the unpack produces), and the row sums.  `parts` blocks share a row: block (m, part) takes
+// the part-th range of its chunks of eight k and leaves their sum in row_sums[part * M + m].
+// What bounds both pre-passes is latency, between the end of the kernel in front and the GEMM kernel's first MMA, so their blocks
+// should all be waiting, on SMs of their own, when that kernel ends: few enough for one per SM, and 128 threads of 40 registers at
+// most, which fit beside a CTA of the GEMM kernel (832 threads of 72).  Blocks of 256 threads and 63 registers, a row each, did
+// not: behind another call of this operator they waited for the first SMs to become free, shared these, and kept the next call's
+// GEMM CTAs off them for 8 us: 16 x 8192 x 28672 26.2 -> 24.7 us, 12 x 6912 x 7792 14.9 -> 13.2.
+constexpr int W4I8_PREP_THREADS = 128;
+constexpr int W4I8_PREP_MAX_PARTS = 8;
+constexpr int W4I8_PREP_KEPT = 1024;  // chunks of a row that the quantising pre-pass keeps in shared memory
+__device__ __forceinline__ int w4i8_block_sum(int acc, int* red) {  // in thread 0
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  return red[0] + red[1] + red[2] + red[3];
+}
+__global__ void __launch_bounds__(W4I8_PREP_THREADS, 12)
+w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restrict__ row_sums, uint32_t* __restrict__ counters,
+                         int n_counters, int K, int M, int parts) {
+  __shared__ int red[W4I8_PREP_THREADS / 32];
   pdl_launch_dependents();
   // behind another call of this operator: that call's kernel still reads the scratch until it is done; behind the quantiser
   // or the few-token W8A8 kernel: the activations are still being written
   pdl_wait();
-  // the caller's scratch holds anything: the arrival counters start at zero
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0u;
-  const int m = blockIdx.x;
-  const uint2* src = in + (size_t)m * (K / 8);
-  uint2* dst = out + (size_t)m * (K / 8);
+  const int m = (int)blockIdx.x / parts, part = (int)blockIdx.x - m * parts, chunks = K / 8;
+  const int c0 = (int)((long long)chunks * part / parts), c1 = (int)((long long)chunks * (part + 1) / parts);
+  const uint2* src = in + (size_t)m * chunks;
+  uint2* dst = out + (size_t)m * chunks;
   int acc = 0;
-  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
+  for (int i = c0 + (int)threadIdx.x; i < c1; i += W4I8_PREP_THREADS) {
     const uint2 v = ld_written(src + i);
     acc = __dp4a((int)v.x, 0x01010101, acc);
     acc = __dp4a((int)v.y, 0x01010101, acc);
     dst[i] = make_uint2(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.x, v.y, 0x7531));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < 8; ++w) s += red[w];
-    row_sums[m] = s;
-  }
+  // the caller's scratch holds anything: the arrival counters start at zero
+  for (int i = blockIdx.x * W4I8_PREP_THREADS + threadIdx.x; i < n_counters; i += gridDim.x * W4I8_PREP_THREADS) counters[i] = 0u;
+  const int sum = w4i8_block_sum(acc, red);
+  if (threadIdx.x == 0) row_sums[part * M + m] = sum;
 }
 
 // The same pre-pass with the per-token activation quantiser in front of it, fused: bf16 / f16 activations [M, K] ->
@@ -89,67 +100,51 @@ w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restri
 // straight in the kernel's byte order, and their row sums.  The arithmetic is act_quant_kernel's (act_quant.cuh),
 // so the int8 values and scales are bit-identical to running that kernel first
 // (examples/deepseek_v4/act_quant.py:112-142); what disappears is one launch and the int8 round trip through
-// memory.  One block per row; a thread keeps up to eight 16-byte chunks of the row in registers between the abs-max
-// pass and the quantise pass (K <= 16384), longer rows are read again.
-__global__ void __launch_bounds__(256)
+// memory.  Every block of a row takes the abs-max of all of it (four instructions per eight values), then quantises its own part
+// (about a hundred), which it reads again from L1.
+__global__ void __launch_bounds__(W4I8_PREP_THREADS, 12)
 w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uint2* __restrict__ out,
                                int* __restrict__ row_sums, float* __restrict__ scales, uint32_t* __restrict__ counters,
-                               int n_counters, int K) {
-  __shared__ float redf[8];
-  __shared__ int red[8];
+                               int n_counters, int K, int M, int parts) {
+  __shared__ float redf[W4I8_PREP_THREADS / 32];
+  __shared__ int red[W4I8_PREP_THREADS / 32];
   pdl_launch_dependents();
-  pdl_wait();  // as above
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0u;
-  const int m = blockIdx.x;
-  const int chunks = K >> 3;
+  const int m = (int)blockIdx.x / parts, part = (int)blockIdx.x - m * parts, chunks = K / 8;
+  const int c0 = (int)((long long)chunks * part / parts), c1 = (int)((long long)chunks * (part + 1) / parts);
   const bool bf16 = is_bf16 != 0;
   const uint4* x = X + (size_t)m * chunks;
+  pdl_wait();  // as above
   uint2* dst = out + (size_t)m * chunks;
-  constexpr int KEEP = 8;
-  uint4 keep[KEEP];
+  extern __shared__ uint4 row[];  // the first `kept` chunks
+  const int kept = min(chunks, W4I8_PREP_KEPT);
+  for (int c = threadIdx.x; c < kept; c += W4I8_PREP_THREADS) cp_async16(smem_u32(row + c), x + c);
   uint32_t m2 = 0u;
-#pragma unroll
-  for (int i = 0; i < KEEP; ++i) {
-    const int c = threadIdx.x + i * 256;
-    keep[i] = c < chunks ? ld_written(x + c) : make_uint4(0u, 0u, 0u, 0u);
-  }
-#pragma unroll
-  for (int i = 0; i < KEEP; ++i)
-    if (threadIdx.x + i * 256 < chunks) m2 = aq_absmax8(keep[i], bf16, m2);
-  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) m2 = aq_absmax8(ld_written(x + c), bf16, m2);
+  for (int c = kept + (int)threadIdx.x; c < chunks; c += W4I8_PREP_THREADS) m2 = aq_absmax8(ld_written(x + c), bf16, m2);
+  cp_async_wait();
+  for (int c = threadIdx.x; c < kept; c += W4I8_PREP_THREADS) m2 = aq_absmax8(row[c], bf16, m2);
+  for (int i = blockIdx.x * W4I8_PREP_THREADS + threadIdx.x; i < n_counters; i += gridDim.x * W4I8_PREP_THREADS) counters[i] = 0u;
   float mx = aq_pair_max(m2, bf16);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) redf[threadIdx.x >> 5] = mx;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 8; ++w) mx = fmaxf(mx, redf[w]);
+  for (int w = 0; w < W4I8_PREP_THREADS / 32; ++w) mx = fmaxf(mx, redf[w]);
   const float amax = fmaxf(mx, 1e-4f);
   float scale = __fdiv_rn(amax, 127.0f);
   if (round_scale) scale = aq_pow2_ceil(scale);
   const float rcp = __frcp_rn(scale);
   int acc = 0;
-  auto emit = [&](int c, const uint4& v) {
-    const uint2 q = aq_quant8(v, bf16, scale, rcp);  // eight int8 values in K order
+  for (int c = c0 + (int)threadIdx.x; c < c1; c += W4I8_PREP_THREADS) {
+    const uint2 q = aq_quant8(c < kept ? row[c] : ld_written(x + c), bf16, scale, rcp);  // eight int8 values in K order
     acc = __dp4a((int)q.x, 0x01010101, acc);
     acc = __dp4a((int)q.y, 0x01010101, acc);
     dst[c] = make_uint2(__byte_perm(q.x, q.y, 0x6420), __byte_perm(q.x, q.y, 0x7531));
-  };
-#pragma unroll
-  for (int i = 0; i < KEEP; ++i) {
-    const int c = threadIdx.x + i * 256;
-    if (c < chunks) emit(c, keep[i]);
   }
-  for (int c = threadIdx.x + KEEP * 256; c < chunks; c += 256) emit(c, ld_written(x + c));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
+  const int sum = w4i8_block_sum(acc, red);
   if (threadIdx.x == 0) {
-    int sum = 0;
-    for (int w = 0; w < 8; ++w) sum += red[w];
-    row_sums[m] = sum;
-    scales[m] = scale;
+    row_sums[part * M + m] = sum;
+    if (part == 0) scales[m] = scale;
   }
 }
 
@@ -247,13 +242,14 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
       bool ok = true;
       const uint32_t tx = W4_RAW_PACKED;
+      const uint64_t once = l2_policy_evict_first();
       while (ok && seg.next(tile, ks0, ks1)) {
         const int n0 = tile * W4_BN;
         for (int ks = ks0; ks < ks1; ++ks) {
           if (!mbar_wait(&raw_empty[rs], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* dst = raw_base + rs * W4_RAW_PACKED;
           mbar_arrive_expect_tx(&raw_full[rs], tx);
-          tma_load_2d(dst, &tmW, &raw_full[rs], ks * (W4_SLAB_K / 2), n0);
+          tma_load_2d_hint(dst, &tmW, &raw_full[rs], ks * (W4_SLAB_K / 2), n0, once);
           issued_mask |= 1u << rs;
           parity_mask = (parity_mask & ~(1u << rs)) | (phase << rs);
           if (++rs == RS) { rs = 0; phase ^= 1u; }
@@ -379,7 +375,12 @@ w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     pdl_wait();  // row sums and zeroed counters come from the pre-pass kernel
     // Handed round through shared memory, once per CTA: the pre-pass may still have been writing them when this kernel started,
     // which __ldg must not be used for, and ordinary loads at every tile's end made 128 x 4096 x 14336 37.1 us (__ldg 34.0, so 33.0).
-    if (SIGNED && nl < MT) bias[nl] = nl < p.M ? 8 * ld_written(p.row_sums + nl) : 0;
+    if (SIGNED && nl < MT) {
+      int sum = 0;
+      if (nl < p.M)
+        for (int i = 0; i < p.row_parts; ++i) sum += ld_written(p.row_sums + i * p.M + nl);
+      bias[nl] = 8 * sum;
+    }
     w4_epi_bar();
     while (seg.next(tile, ks0, ks1)) {
       const int buf = it & 1;
