@@ -181,3 +181,43 @@ def test_scales_written_in_front_of_the_quantiser(M):
     for _ in range(3):
         assert all(torch.equal(u, v) for u, v in zip(chain(False), want))
     assert not torch.equal(want[0], want[3])
+
+
+# tiles of 128 x 128, a K cut over two CTAs, 128 x 256, tiles of two CTAs; more and fewer quantiser blocks than SMs
+@pytest.mark.parametrize("M,K,layers,layout", [(300, 1024, 12, "KN"), (130, 8192, 6, "KN"), (1150, 4096, 6, "NK"), (1200, 4096, 6, "KN"),
+                                               (4096, 2048, 6, "NK"), (777, 512, 12, "KN")])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_chain_of_quantisers_and_tile_gemms(M, K, layers, layout, grouped):
+    """The tile kernels are programmatic dependents too, of the quantiser and of each other, and let the quantiser start early: a
+    chain whose steps read what the one in front has just written - every other step two products in a row, into buffers that the
+    allocator hands out again at once - is bit-identical to the same chain with the device drained between the calls."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    scale = torch.rand(K, generator=g, device="cuda") / (0.577 * 74 * K ** 0.5)  # a layer keeps its input's magnitude
+    if grouped:
+        sizes = (M // 3, 0, M - M // 3 - 7, 7)
+        W = torch.randint(-128, 128, (4, K, K), dtype=torch.int8, generator=g, device="cuda")
+        kernel = q.grouped_quant_gemm(sizes, K, K, out_dtype="bfloat16")
+        meta, scales = kernel.block_metadata("cuda"), scale.expand(4, K).contiguous()
+        product = lambda a, sa: kernel(a, W, meta, scales, sa)
+    else:
+        W = torch.randint(-128, 128, (K, K), dtype=torch.int8, generator=g, device="cuda")
+        product = lambda a, sa: q.quant_matmul(a, W, scale, scale_a=sa, out_dtype="bfloat16", b_layout=layout)
+
+    def chain(drain):
+        step = torch.cuda.synchronize if drain else lambda: None
+        h, first = x, None
+        for i in range(layers):
+            a, sa = q.act_quant(h)
+            step()
+            if i % 2:
+                first = product(a, sa.view(-1))
+                step()
+            h = product(a, sa.view(-1))
+            step()
+        return h, first
+
+    want = chain(True)
+    for _ in range(3):
+        assert all(torch.equal(u, v) for u, v in zip(chain(False), want))
+    assert torch.isfinite(want[0].float()).all() and want[0].float().abs().max() > 0.1

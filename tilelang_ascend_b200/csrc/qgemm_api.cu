@@ -192,9 +192,9 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 // Launch `kernel` so that it may start while the kernel in front of it on the stream is still running
 // (programmatic dependent launch); the kernel itself waits before it reads that kernel's results.
-// QGEMM_PDL=0 falls back to plain stream order.
+// QGEMM_PDL=0 falls back to plain stream order, as `early` = false does.
 template <typename... KArgs, typename... Args>
-int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
+int launch_maybe_pdl(bool early, void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
   static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -205,9 +205,13 @@ int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaSt
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = pdl && early ? 1 : 0;
   CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
   return 0;
+}
+template <typename... KArgs, typename... Args>
+int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
+  return launch_maybe_pdl(true, kernel, grid, threads, smem, s, std::forward<Args>(args)...);
 }
 
 // Rasterisation band: the tiles of `group_m` consecutive row blocks are walked column block by column block, so a
@@ -235,27 +239,27 @@ int w8_group_m(int64_t m_tiles, int64_t k_bytes, int64_t groups, int64_t b_bytes
 template <int BN, bool NK, bool BF>
 int launch_w8(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p, int grid,
               cudaStream_t s) {
-  qg::w8a8_gemm_kernel<BN, NK, BF><<<grid, qg::W8_THREADS, qg::W8Cfg<BN>::SMEM_BYTES, s>>>(tmA, tmB, tmC, p);
-  CUDA_OK(cudaGetLastError());
-  return 0;
+  return launch_pdl(qg::w8a8_gemm_kernel<BN, NK, BF>, grid, qg::W8_THREADS, qg::W8Cfg<BN>::SMEM_BYTES, s, tmA, tmB, tmC, p);
 }
 
 // The forms in which a cluster of two CTAs makes a tile: `clusters` of them.
 template <bool NK, bool BF, qg::W8Form FORM>
 int launch_w8_clusters(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const qg::W8A8Params& p,
                        int clusters, cudaStream_t s) {
+  static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * clusters));
   cfg.blockDim = dim3((unsigned)qg::W8_THREADS);
   cfg.dynamicSmemBytes = (size_t)qg::W8Cfg<256, FORM>::SMEM_BYTES;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl ? 2 : 1;
   CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, FORM>, tmA, tmB, tmC, p));
   return 0;
 }
@@ -777,6 +781,12 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
       p.num_items = (int)(num_tiles + R);
     }
   }
+  // The next kernel's CTAs then come to the SMs in the order in which these become free.  Grouped calls of several rounds, whose
+  // neighbouring CTAs share tiles of L2, lose more by that than a late start costs: 16 groups, 8192 x 7168 x 2048 120.6 us, 126.0 with
+  // it, 25 groups, 3751 x 4992 x 3664 118.4 / 120.5; of one or two rounds 14 groups, 150 x 4256 x 1568 26.2 / 25.5, 17 groups, 1903 x
+  // 1184 x 1216 12.6 / 11.9.  Plain and batched calls gain throughout: 16 x 512 x 7168 x 2048 116.6 / 112.5, 1097 x 2496 x 1680 11.7 /
+  // 10.9, 519 x 1344 x 2400 7.2 / 6.6, and with the quantiser in front 4096 x 4096 x 14336 188.7 / 186.4, 300 x 2048 x 4096 13.6 / 12.1.
+  p.early = meta == nullptr || p.num_items <= 2 * grid ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool nk = b_layout == QGEMM_B_NK;
   const bool bf = out_dtype == QGEMM_DT_BF16;
@@ -1364,14 +1374,19 @@ int qgemm_act_quant(const void* X, int8_t* Y, float* S, int64_t M, int64_t N, in
   const int64_t grid = (M + rows_per_block - 1) / rows_per_block;
   if (grid > 0x7fffffffll) return fail("qgemm_act_quant: too many rows (%lld)", (long long)M);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // A programmatic dependent: behind the few-token W8A8 kernel it is resident when that kernel ends.
+  // A programmatic dependent: behind a W8A8 kernel it is resident when that kernel ends.  Not with more blocks than SMs: the SMs that
+  // kernel leaves idle would be filled with them and the others get few.  us with the GEMM behind it, plain stream order / early from
+  // any number of blocks up to four per SM: 1000 x 2048 x 2048 13.2 / 16.3, 3000 x 1024 x 1024 13.2 / 16.4, 600 x 4096 x 4096 21.5 / 22.6.
+  int sms = 0;
+  if (ensure_device(&sms)) return -1;
+  const bool early = grid <= sms;
   switch (tpr) {
-    case 32: return launch_pdl(qg::act_quant_kernel<32, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
-    case 64: return launch_pdl(qg::act_quant_kernel<64, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
-    case 128: return launch_pdl(qg::act_quant_kernel<128, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 32: return launch_maybe_pdl(early, qg::act_quant_kernel<32, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 64: return launch_maybe_pdl(early, qg::act_quant_kernel<64, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 128: return launch_maybe_pdl(early, qg::act_quant_kernel<128, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
     default:
-      if (keep8) return launch_pdl(qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS>, (int)grid, qg::AQ_THREADS, 0, st, p);
-      return launch_pdl(qg::act_quant_kernel<256, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+      if (keep8) return launch_maybe_pdl(early, qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS>, (int)grid, qg::AQ_THREADS, 0, st, p);
+      return launch_maybe_pdl(early, qg::act_quant_kernel<256, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
   }
 }
 

@@ -38,6 +38,7 @@ struct W8A8Params {
   // right half of tile split_from + i), so that the last, partly filled round of the persistent grid keeps
   // twice as many SMs busy for about half as long.  num_items = num_tiles when nothing is split.
   int split_from, num_items;
+  int early;      // let the next kernel on the stream set up beside this one (w8a8_impl says when)
   int withhold;   // test hook of the two-CTA form (qgemm_debug_withhold_commit)
   int tma_store;  // C is written with tiled bulk stores from a shared-memory staging tile
 };
@@ -103,10 +104,10 @@ __device__ __forceinline__ W8Tile w8_tile(const W8A8Params& p, int item, int cra
     t.m0 = PAIR ? (2 * m_blk + crank) * W8_BM : m_blk * W8_BM;  // PAIR: a row block is 256 rows, 128 for each CTA
     t.rows = min(W8_BM, p.M - t.m0);
   } else {
-    t.bB = __ldg(p.meta + 3 * m_blk);
+    t.bB = ld_written(p.meta + 3 * m_blk);
     t.bA = 0;
-    t.m0 = __ldg(p.meta + 3 * m_blk + 1);
-    t.rows = min(__ldg(p.meta + 3 * m_blk + 2), W8_BM);
+    t.m0 = ld_written(p.meta + 3 * m_blk + 1);
+    t.rows = min(ld_written(p.meta + 3 * m_blk + 2), W8_BM);
     // a table entry that points outside the tensors computes nothing (loads are bounds-checked by TMA)
     if (t.bB < 0 || t.bB >= p.groups || t.m0 < 0 || t.m0 >= p.M) { t.bB = 0; t.m0 = 0; t.rows = 0; }
     t.rows = min(t.rows, p.M - t.m0);
@@ -135,8 +136,8 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
     for (int i = lane; open_rows != 0 && i - lane < p.num_blocks; i += 32) {
       uint32_t mine = 0;
       if (i < p.num_blocks) {
-        const int g = __ldg(p.meta + 3 * i), first = __ldg(p.meta + 3 * i + 1);
-        const int rows = min(__ldg(p.meta + 3 * i + 2), W8_BM);
+        const int g = ld_written(p.meta + 3 * i), first = ld_written(p.meta + 3 * i + 1);
+        const int rows = min(ld_written(p.meta + 3 * i + 2), W8_BM);
         if (g >= 0 && g < p.groups && first >= 0 && first < p.M && rows > 0) {  // as in w8_tile
           const int lo = max(first - row0, 0), hi = min(first - row0 + rows, 32);
           if (lo < hi) mine = (hi - lo == 32 ? 0xffffffffu : (1u << (hi - lo)) - 1u) << lo;
@@ -231,6 +232,13 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
   }
+  if constexpr (FORM != W8_ALONE) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
+  else __syncthreads();
+  // Launched as a programmatic dependent: set up beside the end of the kernel in front (the quantiser and the W8A8 kernels let
+  // theirs start early), but nothing is read, written or taken from the SM's tensor memory before that kernel is done.  Then the
+  // next kernel may set up beside this one.  The first loads do not wait for the tensor memory.
+  pdl_wait();
+  if (p.early) pdl_launch_dependents();
   if (warp == 1) {
     if constexpr (PAIR) {
       tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
@@ -240,11 +248,13 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tmem_relinquish();
     }
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  if constexpr (FORM != W8_ALONE) cluster_sync_all();  // both CTAs' barriers exist before either signals the other's
-  const uint32_t tmem_base = *tmem_slot;
+  uint32_t tmem_base = 0;
+  if (warp != 0) {
+    tc_fence_before_sync();
+    asm volatile("bar.sync 1, %0;" ::"n"(W8_THREADS - 32) : "memory");
+    tc_fence_after_sync();
+    tmem_base = *tmem_slot;
+  }
   const WaitCtl ctl{abort_flag, p.status, p.wait_limit_ns};
 
   if (warp == 0) {
@@ -391,11 +401,11 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int m = t.m0 + q * 32 + lane;
       const bool row_ok = q * 32 + lane < t.rows;
       float sa = 1.0f;
-      if (p.sa_mode != 0 && row_ok) sa = __ldg(p.scale_a + (p.sa_mode == 2 ? (size_t)t.bA * p.M : 0) + m);
+      if (p.sa_mode != 0 && row_ok) sa = ld_written(p.scale_a + (p.sa_mode == 2 ? (size_t)t.bA * p.M : 0) + m);
       const float* sbp = p.scale_b + (p.sb_mode == 2 ? (size_t)t.bB * p.N : 0);
       auto column_scale = [&](int c) {  // of this lane's column of chunk c
         const int n = t.n0 + c * 32 + lane;
-        return p.C == nullptr ? 0.f : (p.sb_mode == 0 ? __ldg(sbp) : (n < p.N ? __ldg(sbp + n) : 0.f));
+        return p.C == nullptr ? 0.f : (p.sb_mode == 0 ? ld_written(sbp) : (n < p.N ? ld_written(sbp + n) : 0.f));
       };
       // This warp's chunks of 32 columns.  Split form: of the half of the tile that this CTA finishes.
       const int own_chunks = (SPLITK ? t.bn >> 6 : t.bn >> 5) >> 1;
