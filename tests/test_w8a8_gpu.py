@@ -374,3 +374,23 @@ print("single ok")
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, QGEMM_W8_PAIR="0"), capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "single ok" in r.stdout, r.stdout + r.stderr
+
+
+# On 148 SMs: one CTA each that fits an SM or shares it; a cut in two from eight k blocks on, in four from six, in eight from 32, and the
+# sizes at either side of each; clusters of four on 136 and 140 SMs; 96 and 208 KB of pipeline, more k blocks than stages, up to 128
+# tokens, and one token more.
+@pytest.mark.parametrize("batch,M,K,N", [
+    (0, 32, 896, 9472), (0, 33, 1024, 9472), (0, 17, 1024, 9488), (0, 48, 640, 4352), (0, 16, 768, 4480), (0, 8, 4096, 4352), (0, 40, 2048, 18944),
+    (0, 5, 1536, 18960), (0, 24, 4080, 1168), (0, 60, 8192, 1168), (0, 128, 4096, 2048), (0, 129, 1152, 1040), (3, 72, 4864, 6016),
+    (2, 1, 4224, 1024)])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_plans_for_few_tokens_are_exact(batch, M, K, N, layout):
+    g = torch.Generator(device="cuda").manual_seed(K + M + N)
+    lead = (batch,) if batch else ()
+    A = torch.randint(-128, 128, lead + (M, K), dtype=torch.int8, generator=g, device="cuda")
+    B = torch.randint(-128, 128, lead + ((K, N) if layout == "KN" else (N, K)), dtype=torch.int8, generator=g, device="cuda")
+    sb, sa = torch.rand(lead + (N,), generator=g, device="cuda"), torch.rand(lead + (M,), generator=g, device="cuda")
+    acc = A.double() @ (B if layout == "KN" else B.transpose(-1, -2)).double()
+    want = ((acc.float() * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.bfloat16)
+    import tilelang_ascend_b200 as q
+    assert torch.equal(q.quant_matmul(A, B, sb, scale_a=sa, out_dtype="bfloat16", b_layout=layout), want)

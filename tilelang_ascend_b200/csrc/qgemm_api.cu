@@ -122,10 +122,11 @@ int set_smem_w4g() {
 }
 
 int set_smem_w8r() {
-  if (set_smem(qg::w8a8_rows_kernel<false, false>, qg::W8R_SMEM_BYTES)) return -1;
-  if (set_smem(qg::w8a8_rows_kernel<false, true>, qg::W8R_SMEM_BYTES)) return -1;
-  if (set_smem(qg::w8a8_rows_kernel<true, false>, qg::W8R_SMEM_BYTES)) return -1;
-  return set_smem(qg::w8a8_rows_kernel<true, true>, qg::W8R_SMEM_BYTES);
+  constexpr int smem = qg::W8R_RING_BYTES_ONE + qg::W8R_EXTRA_BYTES;
+  if (set_smem(qg::w8a8_rows_kernel<false, false>, smem)) return -1;
+  if (set_smem(qg::w8a8_rows_kernel<false, true>, smem)) return -1;
+  if (set_smem(qg::w8a8_rows_kernel<true, false>, smem)) return -1;
+  return set_smem(qg::w8a8_rows_kernel<true, true>, smem);
 }
 template <bool PAIR>
 int set_smem_w4w() {
@@ -277,7 +278,7 @@ int launch_w8_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const qg::W8R
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(qg::W8R_THREADS);
-  cfg.dynamicSmemBytes = (size_t)qg::W8R_SMEM_BYTES;
+  cfg.dynamicSmemBytes = (size_t)(p.ring + qg::W8R_EXTRA_BYTES);
   cfg.stream = s;
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -577,30 +578,34 @@ int qgemm_init(void) {
   return ensure_device(&sms);
 }
 
-// Over how many CTAs the few-token form (w8a8_rows.cuh) cuts the K of its `tiles` tiles; 0: w8a8.cuh is the faster one.
-// The cut.  A CTA per SM, at least two 128-k blocks each; a second one per SM, or clusters of eight on more than half of the
-// SMs (they rarely find eight SMs close together), from eight blocks each on.  us, cut so / two CTAs per SM whatever their K: 32
-// tokens 1024 x 8192 6.1 / 7.3, 2048 x 2048 4.9 / 6.6, 64 tokens 4096 x 4096 8.3 / 10.0.
-// The choice.  Per tile this form pays for its tokens (8.4 ns each, not shared when K is not cut) and saves the k blocks that
-// other CTAs of the cluster take.  So up to 48 tokens always; up to 64 unless nothing is cut, K is long and there are more
-// tiles than SMs; above that when the cut saves enough blocks.  us, this form / w8a8.cuh: 32 tokens 1024 x 8192 6.1 / 7.3, 128
-// tokens 512 x 14336 7.9 / 6.0, 1024 x 1024 7.0 / 7.1, 2048 x 2048 7.9 / 8.9, 4096 x 14336 18.3 / 20.3, 10 x 96 x 2048 x 3072
-// 18.0 / 16.7.  Over 1739 shapes (1 .. 10 problems of 16 .. 512 tokens, K and N 128 .. 14336, weights from DRAM) the choice is
-// within 1 % of the better one in the mean and 5 % behind w8a8.cuh at worst ([N, K] weights).
-static int w8_rows_split(int64_t tiles, int64_t k_blocks, int64_t tokens, int sms) {
-  int S = 1;
-  while (S < qg::W8R_MAX_SPLIT) {
-    const int n = 2 * S;
-    const int64_t ctas = tiles * n;
-    const bool fits = k_blocks >= 2 * n && ctas <= (n == qg::W8R_MAX_SPLIT ? sms / 2 : sms);
-    if (!fits && !(k_blocks >= 8 * n && ctas <= 2 * sms)) break;
-    S = n;
-  }
-  const int64_t saved = k_blocks - (k_blocks + S - 1) / S, ctas = tiles * S;
-  if (tokens <= 48) return S;
-  if (tokens <= 64) return saved >= 4 || k_blocks <= 12 || tiles <= sms ? S : 0;
-  if (ctas > sms) return saved >= 16 ? S : 0;
-  return saved >= (tokens <= 96 ? 7 : 9) || (saved >= 6 && 2 * ctas <= sms) ? S : 0;
+// How the few-token form (w8a8_rows.cuh) takes `tiles` tiles: over how many CTAs it cuts their K, and the bytes of a CTA's pipeline.
+// split 0: w8a8.cuh is the faster one.
+// The cut.  One CTA per SM, as long as it saves each CTA four k blocks; clusters of eight from 32 k blocks on, and where they fit
+// easily.  A second CTA per SM by a further cut does not pay.
+// The pipeline.  208 KB (one CTA per SM) where all CTAs find an SM of their own, else, and for up to 32 tokens of [K, N] weights, 96 KB.
+// Clusters of four do not fill all SMs with one CTA each: 12 fewer.
+// The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take.  So up to 48 tokens always, up to
+// 64 unless nothing is cut, K is long and there are more tiles than SMs, above that when the cut saves enough blocks.
+// From 150 shapes (1 .. 10 problems of 1 .. 512 tokens, K 512 .. 8192, N 512 .. 14336, weights from DRAM; every cut, both pipelines and
+// the other kernel in turn): 1.0 % behind the best in the mean, where the rule before (two CTAs per SM from eight blocks each on, 96 KB)
+// was 4.1 %.  us, before / after: 24 x 4096 x 14336 14.7 / 13.6, 128 x 8192 x 8192 20.7 / 18.5, 71 tokens of 140 tiles, K = 4864 17.5 /
+// 15.3, 24 x 8192 x 4096 12.1 / 11.1, 13 x 512 x 3008 4.2 / 3.6; 256 x 1024 x 1024 6.4 by this form, 5.9 by w8a8.cuh.
+struct W8RowsPlan {
+  int split, ring;
+};
+static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, bool kn, int64_t sms) {
+  auto saved = [&](int64_t n) { return k_blocks - (k_blocks + n - 1) / n; };
+  int64_t S = 1;
+  if (2 * tiles <= sms && saved(2) >= 4) S = 2;
+  if (4 * tiles <= sms && saved(4) >= 4) S = 4;
+  if (8 * tiles <= (kn ? sms - 20 : sms / 2) && k_blocks >= 32) S = 8;
+  static_assert(qg::W8R_MAX_SPLIT == 8, "cuts above");
+  const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 12);
+  const W8RowsPlan plan{(int)S, alone && (!kn || tokens > 32) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
+  if (tokens <= 48) return plan;
+  if (tokens <= 64) return saved(S) >= 4 || k_blocks <= 12 || tiles <= sms ? plan : none;
+  if (plan.ring == qg::W8R_RING_BYTES_ONE && k_blocks >= 32) return plan;
+  return saved(S) >= (tokens <= 96 ? 7 : 9) ? plan : none;
 }
 
 // Whether two CTAs per tile of 256 x 256 (PAIR of w8a8.cuh) are faster than one per tile of 128 x 256 or 128 x 128.  Counted in
@@ -659,7 +664,10 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
 
   CUtensorMap tmA, tmB;
   const int64_t k_blocks = (K + 127) / 128, n_tiles128 = (N + 127) / 128, row_tiles = (M + qg::W8R_MAX_MT - 1) / qg::W8R_MAX_MT;
-  const int S = meta == nullptr && acc_out == nullptr ? w8_rows_split(batch * n_tiles128 * row_tiles, k_blocks, (M + row_tiles - 1) / row_tiles, sms) : 0;
+  W8RowsPlan rows_plan{0, 0};
+  if (meta == nullptr && acc_out == nullptr)
+    rows_plan = w8_rows_plan(batch * n_tiles128 * row_tiles, k_blocks, (M + row_tiles - 1) / row_tiles, b_layout == QGEMM_B_KN, sms);
+  const int S = rows_plan.split;
   if (S > 0) {
     const int64_t n_tiles = n_tiles128, m_tiles = row_tiles, tiles = batch * n_tiles * m_tiles;
     if (tiles > 0x7fffffff / qg::W8R_MAX_SPLIT) return fail("qgemm_w8a8: too many tiles");
@@ -677,6 +685,7 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
     p.m_tiles = (int)m_tiles;
     p.mt = (int)(((M + m_tiles - 1) / m_tiles + unit - 1) / unit * unit);
     p.tmem_cols = p.mt <= 32 ? 32 : (p.mt <= 64 ? 64 : 128);
+    p.ring = rows_plan.ring;
     p.status = status;
     p.wait_limit_ns = g_wait_limit_ns;
     const uint64_t dims_a[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)batch};

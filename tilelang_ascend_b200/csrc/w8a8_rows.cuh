@@ -4,10 +4,10 @@
 // Few tokens make the product a stream of the weights, so what counts is how many SMs load and how much each has in
 // flight.  w8a8.cuh gives a 128-token row block to one CTA per 128 or 256 columns: 112 CTAs (14336 columns), 64 (8192) or 32
 // (4096) of one tile each, whose pipeline fill, int32 exchange and store follow one another.  Here a tile is 128 weight
-// columns x up to 128 tokens, K is cut over a cluster of S = 1, 2, 4 or 8 CTAs, and two CTAs share an SM, so that one loads
-// while the other starts up or finishes.  24 tokens, K = 4096, N = 14336: 22.6 -> 15 us (58.7 MB at 6.5 TB/s: 9), with the
-// quantiser in front 28.7 -> 20.6; 8192 x 8192: 26.6 -> 15.9; 1024 x 1024: 8.2 -> 4.9.  What is left is the start of the
-// launch, the pipeline's first loads and the two cluster barriers.
+// columns x up to 128 tokens and K is cut over a cluster of S = 1, 2, 4 or 8 CTAs, one CTA per SM where that is enough, with most of
+// the SM's shared memory as its pipeline (w8_rows_plan).  24 tokens, K = 4096, N = 14336: 22.6 us by w8a8.cuh, 14.7 with two CTAs
+// per SM and a pipeline of 96 KB each, now 13.6 (58.7 MB at 6.5 TB/s: 9), with the quantiser in front 28.7, 18.5, now 16.8; 8192 x
+// 8192, 128 tokens 20.7 -> 18.5.  What is left is the start of the launch, the pipeline's first loads and the two cluster barriers.
 //   warp 0      TMA: [128 columns x 128 k] of weights ([N, K]: K-major rows; [K, N]: MN-major) and [tokens x 128 k] of A
 //   warp 1      tcgen05.mma kind::i8 (M = 128 weight columns, N = tokens rounded up to 16), allocates tensor memory
 //   warps 2..5  epilogue
@@ -27,10 +27,12 @@ namespace qg {
 constexpr int W8R_THREADS = 192;
 constexpr int W8R_MAX_MT = 128;
 constexpr int W8R_MAX_SPLIT = 8;
-constexpr int W8R_RING_BYTES = 96 * 1024;  // two CTAs per SM
-constexpr int W8R_MAX_STAGES = 8;
+constexpr int W8R_RING_BYTES = 96 * 1024;       // two CTAs per SM
+constexpr int W8R_RING_BYTES_ONE = 208 * 1024;  // one
+constexpr int W8R_MAX_STAGES = 12;
 constexpr int W8R_W_BYTES = 128 * 128;
-constexpr int W8R_SMEM_BYTES = W8R_RING_BYTES + 256 + 1024;  // ring, barriers, alignment slack
+constexpr int W8R_EXTRA_BYTES = 256 + 1024;  // barriers, alignment slack
+static_assert(W8R_RING_BYTES_ONE + W8R_EXTRA_BYTES <= 232448 && 8 * (2 * W8R_MAX_STAGES + 2) + 8 <= 256, "shared memory of a CTA");
 
 struct W8RowsParams {
   const float* scale_b;
@@ -41,6 +43,7 @@ struct W8RowsParams {
   int n_tiles, m_tiles, k_blocks;
   int mt;                // tokens per tile: M rounded up to 16, at least 4 per CTA of the cluster
   int tmem_cols;         // power of two >= max(mt, 32)
+  int ring;              // bytes of the pipeline's stages
   uint32_t* status;
   unsigned long long wait_limit_ns;
 };
@@ -50,7 +53,7 @@ __global__ void __launch_bounds__(W8R_THREADS, 2)
 w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const W8RowsParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + W8R_RING_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.ring);
   uint64_t* empty = full + W8R_MAX_STAGES;
   uint64_t* tfull = empty + W8R_MAX_STAGES;
   uint64_t* drain = tfull + 1;
@@ -62,7 +65,7 @@ w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int S = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
   const int mt = p.mt;
   const int stage_bytes = W8R_W_BYTES + mt * 128;
-  const int stages = min(W8R_MAX_STAGES, W8R_RING_BYTES / stage_bytes);
+  const int stages = min(W8R_MAX_STAGES, p.ring / stage_bytes);
   const int tile = (int)blockIdx.x / S;
   const int b = tile / (p.n_tiles * p.m_tiles);
   const int in_b = tile - b * (p.n_tiles * p.m_tiles);
@@ -85,16 +88,20 @@ w8a8_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // dependents start early), but nothing is read, written or taken from the SM's tensor memory before that kernel is done.
   // Then the next kernel may set up beside this one (the quantiser and this kernel wait for this whole grid before they touch
   // anything): 1 x 2048 x 2048 4.9 -> 4.2 us a call, 64 x 1024 x 1024 5.2 -> 4.6, 256 x 1024 x 1024 6.5 -> 6.2, each as one graph.
+  __syncthreads();
   pdl_wait();
   pdl_launch_dependents();
   if (warp == 1) {
     tmem_alloc(tmem_slot, (uint32_t)p.tmem_cols);
     tmem_relinquish();
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  uint32_t tmem_base = 0;
+  if (warp != 0) {  // the first loads do not wait for the tensor memory (256 x 1024 x 1024 by this form 6.15 -> 5.81 us)
+    tc_fence_before_sync();
+    asm volatile("bar.sync 1, %0;" ::"n"(W8R_THREADS - 32) : "memory");
+    tc_fence_after_sync();
+    tmem_base = *tmem_slot;
+  }
   const WaitCtl ctl{abort_flag, p.status, p.wait_limit_ns};
   const int q = warp & 3;
   const int nl = q * 32 + lane;  // weight column inside the tile == TMEM lane
