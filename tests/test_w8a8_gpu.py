@@ -394,3 +394,20 @@ def test_plans_for_few_tokens_are_exact(batch, M, K, N, layout):
     want = ((acc.float() * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.bfloat16)
     import tilelang_ascend_b200 as q
     assert torch.equal(q.quant_matmul(A, B, sb, scale_a=sa, out_dtype="bfloat16", b_layout=layout), want)
+
+
+# Tiles of two CTAs at short K, down to fewer k blocks than pipeline stages, and tiles of 128 x 128 or 128 x 256 where these are taken
+# instead, on 148 SMs.
+@pytest.mark.parametrize("batch,M,K,N", [(0, 3100, 288, 1296), (0, 3100, 400, 3600), (0, 1300, 640, 2320), (0, 2310, 1024, 2576),
+                                         (12, 640, 672, 560), (0, 169, 800, 4400), (0, 602, 2048, 6896), (0, 4096, 16, 2320)])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_short_k_is_exact(batch, M, K, N, layout):
+    import tilelang_ascend_b200 as q
+    g = torch.Generator(device="cuda").manual_seed(K + M + N)
+    lead = (batch,) if batch else ()
+    A = torch.randint(-128, 128, lead + (M, K), dtype=torch.int8, generator=g, device="cuda")
+    B = torch.randint(-128, 128, lead + ((K, N) if layout == "KN" else (N, K)), dtype=torch.int8, generator=g, device="cuda")
+    sb, sa = torch.rand(lead + (N,), generator=g, device="cuda"), torch.rand(lead + (M,), generator=g, device="cuda")
+    acc = (A.double() @ (B if layout == "KN" else B.transpose(-1, -2)).double()).float()  # below 2^24: exact
+    C = q.quant_matmul(A, B, sb, scale_a=sa, out_dtype="float16", b_layout=layout)
+    assert torch.equal(C, ((acc * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.float16))

@@ -610,24 +610,23 @@ static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, 
 
 // Whether two CTAs per tile of 256 x 256 (PAIR of w8a8.cuh) are faster than one per tile of 128 x 256 or 128 x 128.  Counted in
 // rounds of 128 x 256 tiles over the SMs: a last round that is cut in half-width items counts 0.6, a round of 128 x 128 tiles
-// 0.55, a round of pairs 0.87; the pairs' longer start and hand-over of a tile count the less the longer K is.  The constants come
-// from a sweep with hand-overs at cluster scope, which cost pairs more than the plain ones now; they err on the side of one CTA.
-// Both ways in turn over 150 shapes, K 2048 .. 8192, both layouts: no shape that takes pairs is slower for it, and the choice is
-// 0.9 % behind the better one in the mean.  us, one / two CTAs per tile: 4096 x 4096 x 14336 166 / 148, 4096 x 2048 x 4096 30.2 /
-// 27.3, 16 x 512 x 7168 x 2048 [K, N] 94.7 / 89.3, [N, K] 100.9 / 89.0, 512 x 8192 x 5120 36.7 / 27.3, 3895 x 5824 x 1056 36.3 /
-// 31.0; not taken, though as fast or faster: 1300 x 2048 x 8192 23.5 / 22.8, 4096 x 1024 x 4096 19.4 / 18.9, and most shapes
-// with K below 2048.  QGEMM_W8_PAIR=0 disables it.
+// 0.5, a round of pairs 0.76; the pairs' longer start and hand-over of a tile count the less the longer K is.  Both ways in turn
+// over 370 shapes (1 .. 16 problems of 160 .. 4096 rows, K 512 .. 8192, N 512 .. 14336, both layouts): the choice is 0.1 % behind
+// the better one in the mean, 11 % at worst (16 x 279 x 5664 x 13136 468 / 521, seconds at the power limit); constants that were
+// fitted to an earlier kernel and K from 2048 on only were 4.4 % and 33 % behind.  us, one / two CTAs per tile: 4096 x 4096 x 14336
+// 166 / 148, 2026 x 2464 x 12912 62.6 / 50.6, 14 x 2283 x 1024 x 7568 284 / 227, 12 x 2065 x 672 x 560 22.7 / 20.1, 2228 x 5152 x 3632
+// 41.6 / 34.7; not taken: 169 x 800 x 4400 6.6 / 8.0, and, though as fast, 602 x 2048 x 13776 24.0 / 23.2.  QGEMM_W8_PAIR=0 disables it.
 static bool w8_pair_pays(int64_t batch, int64_t M, int64_t N, int64_t k_blocks, bool kn, int64_t sms) {
   static const int pair_on = getenv("QGEMM_W8_PAIR") ? atoi(getenv("QGEMM_W8_PAIR")) : 1;
-  if (!pair_on || N <= 128 || k_blocks < 16) return false;
+  if (!pair_on || N <= 128) return false;
   auto rounds = [](int64_t tiles, int64_t workers, bool halves) {
     const int64_t whole = tiles / workers, left = tiles % workers;
     return (double)whole + (left == 0 ? 0.0 : (halves && whole != 0 && 2 * left <= workers ? 0.6 : 1.0));
   };
   const int64_t row_blocks = (M + 127) / 128, tiles256 = batch * row_blocks * ((N + 255) / 256);
-  const double one = tiles256 >= sms ? rounds(tiles256, sms, kn) : 0.55 * rounds(batch * row_blocks * ((N + 127) / 128), sms, false);
+  const double one = tiles256 >= sms ? rounds(tiles256, sms, kn) : 0.5 * rounds(batch * row_blocks * ((N + 127) / 128), sms, false);
   const double two = rounds(batch * ((M + 255) / 256) * ((N + 255) / 256), sms / 2, true);
-  return two * (0.87 + 1.3 / (double)k_blocks) + 2.4 / (double)k_blocks < one;
+  return two * (0.76 + 0.5 / (double)k_blocks) + 1.2 / (double)k_blocks < one;
 }
 
 // Plain / batched form: meta == nullptr.  Grouped form: A and C are single [M, K] / [M, N] stacks, B holds
