@@ -221,3 +221,20 @@ def test_chain_of_quantisers_and_tile_gemms(M, K, layers, layout, grouped):
     for _ in range(3):
         assert all(torch.equal(u, v) for u, v in zip(chain(False), want))
     assert torch.isfinite(want[0].float()).all() and want[0].float().abs().max() > 0.1
+
+
+# one, two, four and eight chunks of eight per thread; rows shared by 32 .. 1024 threads, full and one chunk over; the last number of
+# rows that is spread on 148 SMs, and the next
+@pytest.mark.parametrize("M,N", [(3, 256), (3, 264), (318, 4096), (317, 4104), (5, 4096), (5, 4104), (158, 8192), (159, 8192), (159, 8200),
+                                 (160, 8200), (7, 16384), (7, 16392), (636, 2048), (637, 2048), (1271, 2056), (1273, 2056), (5089, 256),
+                                 (5088, 512), (5089, 512)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("round_scale", [False, True])
+def test_threads_per_row(M, N, dt, round_scale):
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, N, generator=g).to(dt)
+    x[M // 2] = 0
+    x[M - 1, N - 1] = 60.0
+    y, s = q.act_quant(x.cuda(), round_scale)
+    y_ref, s_ref = oc.act_quant_torch_ref(x, round_scale)
+    assert torch.equal(y.cpu(), y_ref) and torch.equal(s.cpu().view(-1), s_ref.view(-1))

@@ -9,9 +9,9 @@
 // The device kernel it replaces is act_quant_kernel_int8_optimized (act_quant.py:33-92).
 //
 // HBM bound: every element is read once (2 bytes) and written once (1 byte).  A row is held in registers
-// between the abs-max pass and the quantise pass: 4 or 8 16-byte chunks per thread; rows longer than
+// between the abs-max pass and the quantise pass: 1 to 8 16-byte chunks per thread; rows longer than
 // 256 * AQ_MAX_CHUNKS * 8 elements are read a second time (from L2).  The host picks how many
-// threads share a row (32, 64, 128 or 256) so that short rows do not leave most of a block idle.
+// threads share a row, 32 to 1024 (qgemm_act_quant).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -118,17 +118,18 @@ __device__ __forceinline__ float aq_pow2_ceil(float x) {
   return __uint_as_float((uint32_t)e << 23);
 }
 
-// TPR threads share one row; a block holds AQ_THREADS / TPR rows; KEEP chunks per thread stay in registers.
+// TPR threads share one row; a block holds max(AQ_THREADS, TPR) / TPR rows; KEEP chunks per thread stay in registers.
+__host__ __device__ constexpr int aq_block(int tpr) { return tpr > AQ_THREADS ? tpr : AQ_THREADS; }
 template <int TPR, int KEEP>
-__global__ void __launch_bounds__(AQ_THREADS, KEEP == 4 ? AQ_MIN_BLOCKS : 1) act_quant_kernel(const ActQuantParams p) {
+__global__ void __launch_bounds__(aq_block(TPR), KEEP == 4 ? AQ_MIN_BLOCKS : 1) act_quant_kernel(const ActQuantParams p) {
   pdl_wait();  // a programmatic dependent itself: the kernel in front may have written X, and may still read Y and S
   // A W8A8 kernel behind this one may set up meanwhile; it waits for this whole grid before it reads anything.  Not in front of
   // the wait: an int4 GEMM behind this kernel reads its weights and scales at once, and whatever wrote those may be the kernel in
   // front of this one.
   pdl_launch_dependents();
-  constexpr int ROWS = AQ_THREADS / TPR;
+  constexpr int ROWS = aq_block(TPR) / TPR;
   constexpr int WPR = TPR / 32;  // warps per row
-  __shared__ float red[AQ_THREADS / 32];
+  __shared__ float red[aq_block(TPR) / 32];
   const int t = threadIdx.x % TPR;
   const int r = threadIdx.x / TPR;
   const int warp = threadIdx.x >> 5;

@@ -1374,27 +1374,57 @@ int qgemm_act_quant(const void* X, int8_t* Y, float* S, int64_t M, int64_t N, in
   p.is_bf16 = x_dtype == QGEMM_DT_BF16;
   p.round_scale = round_scale != 0;
   const int64_t chunks = N / 8;
-  // threads per row: the fewest of 32..256 that keep a row in at most 4 chunks per thread (8 at 256)
-  int tpr = 32;
-  while (tpr < qg::AQ_THREADS && chunks > (int64_t)tpr * 4) tpr *= 2;
-  const bool keep8 = chunks > (int64_t)tpr * 4;
-  const int64_t rows_per_block = qg::AQ_THREADS / tpr;
+  int sms = 0;
+  if (ensure_device(&sms)) return -1;
+  // Threads per row.  While the rows leave threads idle, latency counts, and what a thread does one after another: one chunk each in
+  // rows of up to 512 chunks, else two, as long as that is no more than about half of the threads that the SMs hold.  Above that the
+  // fewest of 32..256 that keep a row in at most 4 chunks per thread (8 at 256).  us, four / two / one chunk per thread: 24 x 4096
+  // 2.74 / 1.95 / 1.78, 148 x 1024 2.70 / 1.98 / 1.72, 600 x 2048 3.66 / 2.85 / 2.73, 1200 x 2048 4.81 / 3.60 / 3.97, 300 x 8192 4.25 / 3.81 /
+  // 6.05, 148 x 14336 4.66 / 3.43 / -; not taken: 600 x 8192 6.19 / 6.54 / 10.81, 4096 x 2048 9.10 / 9.98 / 9.92.  With a product behind it,
+  // 4096 columns, 24 x 4096 10.5 -> 9.0, 300 x 2048 13.2 -> 11.1.
+  auto threads_for = [&](int keep) {
+    int t = 32;
+    while (t < 1024 && chunks > (int64_t)t * keep) t *= 2;
+    return t;
+  };
+  int keep = 4, tpr = 32;
+  if (threads_for(1) <= 512 && chunks <= 512 && M * threads_for(1) <= 1100ll * sms) keep = 1;
+  else if (chunks <= 2048 && M * threads_for(2) <= 1100ll * sms) keep = 2;
+  if (keep < 4) {
+    tpr = threads_for(keep);
+  } else {
+    while (tpr < qg::AQ_THREADS && chunks > (int64_t)tpr * 4) tpr *= 2;
+    if (chunks > (int64_t)tpr * 4) keep = qg::AQ_MAX_CHUNKS;
+  }
+  const int block = qg::aq_block(tpr);
+  const int64_t rows_per_block = block / tpr;
   const int64_t grid = (M + rows_per_block - 1) / rows_per_block;
   if (grid > 0x7fffffffll) return fail("qgemm_act_quant: too many rows (%lld)", (long long)M);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // A programmatic dependent: behind a W8A8 kernel it is resident when that kernel ends.  Not with more blocks than SMs: the SMs that
   // kernel leaves idle would be filled with them and the others get few.  us with the GEMM behind it, plain stream order / early from
   // any number of blocks up to four per SM: 1000 x 2048 x 2048 13.2 / 16.3, 3000 x 1024 x 1024 13.2 / 16.4, 600 x 4096 x 4096 21.5 / 22.6.
-  int sms = 0;
-  if (ensure_device(&sms)) return -1;
   const bool early = grid <= sms;
+  auto launch = [&](auto kernel) { return launch_maybe_pdl(early, kernel, (int)grid, block, 0, st, p); };
+  auto launch_few = [&](auto keep_) {  // one or two chunks per thread
+    constexpr int KEEP = decltype(keep_)::value;
+    switch (tpr) {
+      case 32: return launch(qg::act_quant_kernel<32, KEEP>);
+      case 64: return launch(qg::act_quant_kernel<64, KEEP>);
+      case 128: return launch(qg::act_quant_kernel<128, KEEP>);
+      case 256: return launch(qg::act_quant_kernel<256, KEEP>);
+      case 512: return launch(qg::act_quant_kernel<512, KEEP>);
+      default: return launch(qg::act_quant_kernel<1024, 2>);
+    }
+  };
+  if (keep == 1) return launch_few(std::integral_constant<int, 1>{});
+  if (keep == 2) return launch_few(std::integral_constant<int, 2>{});
+  if (keep == qg::AQ_MAX_CHUNKS) return launch(qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS>);
   switch (tpr) {
-    case 32: return launch_maybe_pdl(early, qg::act_quant_kernel<32, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
-    case 64: return launch_maybe_pdl(early, qg::act_quant_kernel<64, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
-    case 128: return launch_maybe_pdl(early, qg::act_quant_kernel<128, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
-    default:
-      if (keep8) return launch_maybe_pdl(early, qg::act_quant_kernel<256, qg::AQ_MAX_CHUNKS>, (int)grid, qg::AQ_THREADS, 0, st, p);
-      return launch_maybe_pdl(early, qg::act_quant_kernel<256, 4>, (int)grid, qg::AQ_THREADS, 0, st, p);
+    case 32: return launch(qg::act_quant_kernel<32, 4>);
+    case 64: return launch(qg::act_quant_kernel<64, 4>);
+    case 128: return launch(qg::act_quant_kernel<128, 4>);
+    default: return launch(qg::act_quant_kernel<256, 4>);
   }
 }
 
