@@ -411,3 +411,19 @@ def test_short_k_is_exact(batch, M, K, N, layout):
     acc = (A.double() @ (B if layout == "KN" else B.transpose(-1, -2)).double()).float()  # below 2^24: exact
     C = q.quant_matmul(A, B, sb, scale_a=sa, out_dtype="float16", b_layout=layout)
     assert torch.equal(C, ((acc * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.float16))
+
+
+# K cut over two CTAs: at least 50 k blocks, weights [K, N], accumulators wanted; ragged M, N and K, and either side of the limits.
+@pytest.mark.parametrize("batch,M,K,N", [(0, 256, 6400, 1024), (2, 200, 6416, 528), (0, 130, 8192, 2064), (3, 256, 6272, 1024), (0, 1100, 6544, 1040)])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_long_k_of_few_tiles_is_exact(batch, M, K, N, layout):
+    import tilelang_ascend_b200 as q
+    g = torch.Generator(device="cuda").manual_seed(K + M + N)
+    lead = (batch,) if batch else ()
+    A = torch.randint(-128, 128, lead + (M, K), dtype=torch.int8, generator=g, device="cuda")
+    B = torch.randint(-128, 128, lead + ((K, N) if layout == "KN" else (N, K)), dtype=torch.int8, generator=g, device="cuda")
+    sb, sa = torch.rand(lead + (N,), generator=g, device="cuda"), torch.rand(lead + (M,), generator=g, device="cuda")
+    want = A.double() @ (B if layout == "KN" else B.transpose(-1, -2)).double()
+    C, acc = q.quant_matmul(A, B, sb, scale_a=sa, out_dtype="float16", b_layout=layout, return_accumulators=True)
+    assert torch.equal(acc.double(), want)
+    assert torch.equal(C, ((want.float() * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.float16))

@@ -584,8 +584,10 @@ int qgemm_init(void) {
 // easily.  A second CTA per SM by a further cut does not pay.
 // The pipeline.  208 KB (one CTA per SM) where all CTAs find an SM of their own, else, and for up to 32 tokens of [K, N] weights, 96 KB.
 // Clusters of four do not fill all SMs with one CTA each: 12 fewer.
-// The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take.  So up to 48 tokens always, up to
-// 64 unless nothing is cut, K is long and there are more tiles than SMs, above that when the cut saves enough blocks.
+// The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take: up to 48 tokens always, above that
+// when the cut saves three blocks, and one more for every eight tokens, up to 64 also uncut from eleven blocks on.  (220 shapes of
+// 41 .. 128 tokens per tile: 0.5 % behind the better one in the mean.)  The time by w8a8.cuh over this form's: 124 tokens, 188 tiles,
+// K = 4608 0.64; 54 tokens, 73 tiles, K = 640 0.96; 60 tokens, 112 tiles, K = 2048 1.16; 109 tokens, 5 tiles cut in four, K = 1920 1.04.
 // From 150 shapes (1 .. 10 problems of 1 .. 512 tokens, K 512 .. 8192, N 512 .. 14336, weights from DRAM; every cut, both pipelines and
 // the other kernel in turn): 1.0 % behind the best in the mean, where the rule before (two CTAs per SM from eight blocks each on, 96 KB)
 // was 4.1 %.  us, before / after: 24 x 4096 x 14336 14.7 / 13.6, 128 x 8192 x 8192 20.7 / 18.5, 71 tokens of 140 tiles, K = 4864 17.5 /
@@ -602,10 +604,8 @@ static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, 
   static_assert(qg::W8R_MAX_SPLIT == 8, "cuts above");
   const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 12);
   const W8RowsPlan plan{(int)S, alone && (!kn || tokens > 32) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
-  if (tokens <= 48) return plan;
-  if (tokens <= 64) return saved(S) >= 4 || k_blocks <= 12 || tiles <= sms ? plan : none;
-  if (plan.ring == qg::W8R_RING_BYTES_ONE && k_blocks >= 32) return plan;
-  return saved(S) >= (tokens <= 96 ? 7 : 9) ? plan : none;
+  const bool uncut = tokens <= 64 && k_blocks > 10 && tiles <= sms;
+  return tokens <= 48 || uncut || 25 * saved(S) > 3 * (tokens - 40) + 50 ? plan : none;
 }
 
 // Whether two CTAs per tile of 256 x 256 (PAIR of w8a8.cuh) are faster than one per tile of 128 x 256 or 128 x 128.  Counted in
@@ -710,13 +710,13 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   }
   const int64_t row_blocks = meta ? num_blocks : (M + 127) / 128;
   const int64_t tiles256 = batchA * row_blocks * ((N + 255) / 256);
-  // Fewer 256-wide tiles than half the SMs: split K over pairs of CTAs (one tile per pair, twice as many SMs at
-  // work on full-width tiles) instead of falling back to 128-wide tiles - when K is long enough to pay for the
-  // cluster launch and the exchange: on 2 x 512 x K x 2048, split against 128-wide tiles, K = 7168: 19.8 / 23.6 us,
-  // 4096: 14.9 / 16.2, 3072: 13.7 / 13.3, and 256 x 1024 x 1024: 9.9 / 7.0, so the split starts at K = 4096.
-  // QGEMM_W8_SPLITK=0 disables it.
+  // A very long K and fewer 128-wide tiles than half the SMs, weights [K, N]: split K over pairs of CTAs (one tile of 256 columns per
+  // pair).  Everything else of few tiles is faster by tiles of 128 columns, whose pipeline is six stages deep.  us, split / 128-wide:
+  // 256-row problems of 51 tiles, K = 7296 23.0 / 26.8, 63 tiles, K = 8192 22.0 / 24.2, but 24 tiles, K = 5504 21.6 / 22.0; not taken: 40
+  // tiles, K = 6656, [N, K] 17.9 / 16.8, 99 tiles, K = 4352 18.3 / 15.1, 114 tiles, K = 4992 18.4 / 15.7.  Without accumulators the
+  // few-token form takes these shapes.  QGEMM_W8_SPLITK=0 disables it.
   static const int splitk_on = getenv("QGEMM_W8_SPLITK") ? atoi(getenv("QGEMM_W8_SPLITK")) : 1;
-  const bool use_splitk = splitk_on && meta == nullptr && N > 128 && 2 * tiles256 <= sms && (K + 127) / 128 >= 32;
+  const bool use_splitk = splitk_on && meta == nullptr && b_layout == QGEMM_B_KN && N > 128 && 2 * batchA * row_blocks * n_tiles128 <= sms && k_blocks >= 50;
   // Otherwise two CTAs per tile of 256 x 256 where that is the faster one (w8_pair_pays).
   const bool use_pair = meta == nullptr && !use_splitk && w8_pair_pays(batch, M, N, k_blocks, b_layout == QGEMM_B_KN, sms);
   const int BN = (N > 128 && (tiles256 >= sms || use_splitk || use_pair)) ? 256 : 128;

@@ -160,8 +160,7 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
   }
 }
 
-// SPLITK = true is the form for grids that would leave more than half of the SMs idle (fewer 128 x 256 tiles than
-// half the SM count): the kernel is launched in clusters of two CTAs, one tile per cluster; each CTA accumulates
+// SPLITK is the form for very long K on grids that would leave half of the SMs idle (w8a8_impl): the kernel is launched in clusters of two CTAs, one tile per cluster; each CTA accumulates
 // one half of the K range in its own tensor memory; then each CTA writes its int32 accumulators of the OTHER CTA's
 // half of the columns into that CTA's shared memory (the pipeline stages, idle by then) through distributed shared
 // memory, adds what it received to its own half and runs the epilogue for that half - an exact integer sum, so the
