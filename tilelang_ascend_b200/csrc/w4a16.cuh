@@ -314,6 +314,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       int rs = 0;
       uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
       bool ok = true;
+      const uint64_t once = l2_policy_evict_first();
       const uint32_t tx = W4_RAW_PACKED + (p.has_scales ? p.scale_rows * 256 : 0);
       while (ok && seg.next(tile, ks0, ks1)) {
         int b, n0, m0;
@@ -322,7 +323,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           if (!mbar_wait(&raw_empty[rs], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* dst = raw_base + rs * W4_RAW_BYTES;
           mbar_arrive_expect_tx(&raw_full[rs], tx);
-          tma_load_3d(dst, &tmW, &raw_full[rs], ks * (W4_SLAB_K / 2), n0, b);
+          tma_load_3d_hint(dst, &tmW, &raw_full[rs], ks * (W4_SLAB_K / 2), n0, b, once);
           if (p.has_scales) {
             const int srow = (p.group <= W4_SLAB_K) ? ks * p.scale_rows : (ks * W4_SLAB_K) / p.group;
             tma_load_3d(dst + W4_RAW_PACKED, &tmS, &raw_full[rs], n0, srow, b);

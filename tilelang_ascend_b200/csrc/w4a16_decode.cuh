@@ -137,6 +137,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       int s = 0;
       uint32_t phase = 0, issued_mask = 0, parity_mask = 0;
       bool ok = true;
+      const uint64_t once = l2_policy_evict_first();
       const uint32_t tx = W4_RAW_PACKED + (SCALED ? p.scale_rows * 256 : 0) + 4 * Cfg::A_KB_BYTES;
       bool waited = false;  // the activations come from the pre-pass kernel in front: wait for it once, after
                             // the first weight loads are on their way
@@ -147,7 +148,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
           if (!mbar_wait(&empty[s], phase ^ 1u, ctl, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* dst = smem + s * Cfg::STAGE_BYTES;
           mbar_arrive_expect_tx(&full[s], tx);
-          tma_load_3d(dst, &tmW, &full[s], ks * (W4_SLAB_K / 2), n0, b);
+          tma_load_3d_hint(dst, &tmW, &full[s], ks * (W4_SLAB_K / 2), n0, b, once);
           if (SCALED) {
             const int srow = (p.group <= W4_SLAB_K) ? ks * p.scale_rows : (ks * W4_SLAB_K) / p.group;
             tma_load_3d(dst + W4_RAW_PACKED, &tmS, &full[s], n0, srow, b);
