@@ -479,12 +479,12 @@ static int launch_w4i8(bool sgn, const CUtensorMap& tmW, const CUtensorMap& tmA,
                        cudaStream_t s) {
   if constexpr (MT == 16) {
     if (p.dp_rounds > 0 && p.KS >= 24) {
-      if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
-      return launch_pdl(qg::w4a8_gemm_kernel<MT, false, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+      if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true, true>, grid, qg::W4I8Cfg<MT>::THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+      return launch_pdl(qg::w4a8_gemm_kernel<MT, false, true>, grid, qg::W4I8Cfg<MT>::THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
     }
   }
-  if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
-  return launch_pdl(qg::w4a8_gemm_kernel<MT, false>, grid, qg::W4_THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+  if (sgn) return launch_pdl(qg::w4a8_gemm_kernel<MT, true>, grid, qg::W4I8Cfg<MT>::THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
+  return launch_pdl(qg::w4a8_gemm_kernel<MT, false>, grid, qg::W4I8Cfg<MT>::THREADS, qg::W4I8Cfg<MT>::SMEM_BYTES, s, tmW, tmA, p);
 }
 
 // Fused path of qgemm_w4a8 for up to 128 tokens: no int8 copy of the weights; the caller's [N, K] workspace
@@ -507,9 +507,9 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   if (need > N * K) return 1;  // the caller's workspace is [N, K] int8
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   uint8_t* a_prepared = ws + kW4CounterBytes + partial_bytes;
-  // Blocks of the pre-pass per row: as many as leave one block for every SM.  The sums over their parts of K stand behind the
-  // counters that are used.
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>({qg::W4I8_PREP_MAX_PARTS, sms / M, (kW4MaxGrid - grid_max) / M}));
+  // Blocks of the pre-pass per row: as many as leave one block for every SM, four above 64 tokens, where they do not fit beside a CTA
+  // of the GEMM kernel.  The sums over their parts of K stand behind the counters that are used.
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>({qg::W4I8_PREP_MAX_PARTS, M <= 64 ? sms / M : 4 * sms / M, (kW4MaxGrid - grid_max) / M}));
   int* row_sums = parts > 1 ? reinterpret_cast<int*>(ws) + grid_max : reinterpret_cast<int*>(a_prepared + a_bytes);
 
   CUtensorMap tmW, tmA;

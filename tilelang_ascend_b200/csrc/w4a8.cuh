@@ -35,7 +35,8 @@ template <int MT>
 struct W4I8Cfg {
   static constexpr int RAW_STAGES = 8;                 // even, like W_STAGES: a stage always belongs to one warp set
   static constexpr int A_STAGES = (MT <= 32) ? 8 : (MT == 64 ? 4 : 3);
-  static constexpr int MMAW = (MT <= 32) ? 4 : (MT == 64 ? 2 : 1);
+  static constexpr int MMAW = MT == 16 ? 4 : (MT <= 64 ? 2 : 1);
+  static constexpr int THREADS = (W4_FIRST_XMMA_WARP + MMAW - 1) * 32;  // two issuers: with room for a block of the pre-pass
   static constexpr int W_STAGES = 4;
   static constexpr int A_KB_BYTES = MT * 128;          // one 128-wide K block of int8 activations
   static constexpr int A_BYTES = 2 * A_KB_BYTES;       // one 256-wide slab
@@ -57,9 +58,11 @@ struct W4I8Cfg {
 // the part-th range of its chunks of eight k and leaves their sum in row_sums[part * M + m].
 // What bounds both pre-passes is latency, between the end of the kernel in front and the GEMM kernel's first MMA, so their blocks
 // should all be waiting, on SMs of their own, when that kernel ends: few enough for one per SM, and 128 threads of 40 registers at
-// most, which fit beside a CTA of the GEMM kernel (832 threads of 72).  Blocks of 256 threads and 63 registers, a row each, did
+// most, which fit beside a CTA of the GEMM kernel of up to 64 tokens (832 threads of 64 registers or 768 of 72; more tokens leave no
+// shared memory, and then more blocks are faster: 128 x 8192 x 8192 41.7 us with one per row, 38.1 with four).  Blocks of 256 threads and 63 registers, a row each, did
 // not: behind another call of this operator they waited for the first SMs to become free, shared these, and kept the next call's
-// GEMM CTAs off them for 8 us: 16 x 8192 x 28672 26.2 -> 24.7 us, 12 x 6912 x 7792 14.9 -> 13.2.
+// GEMM CTAs off them for 8 us: 16 x 8192 x 28672 26.2 -> 24.7 us, 20 x 8192 x 28672
+// 31.2 -> 27.5, 12 x 6912 x 7792 14.9 -> 13.2.
 constexpr int W4I8_PREP_THREADS = 128;
 constexpr int W4I8_PREP_MAX_PARTS = 8;
 constexpr int W4I8_PREP_KEPT = 1024;  // chunks of a row that the quantising pre-pass keeps in shared memory
