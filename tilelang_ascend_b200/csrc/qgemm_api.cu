@@ -584,7 +584,8 @@ int qgemm_init(void) {
 // The cut.  One CTA per SM, as long as it saves each CTA four k blocks; clusters of eight from 32 k blocks on, and where they fit
 // easily.  A second CTA per SM by a further cut does not pay.
 // The pipeline.  208 KB (one CTA per SM) where all CTAs find an SM of their own, else, and for up to 32 tokens of [K, N] weights, 96 KB.
-// Clusters of four do not fill all SMs with one CTA each: 12 fewer.
+// Clusters of four do not fill all SMs with one CTA each, 128 of 148 or a few more, by where the chip's working SMs are: 24 fewer (57 x
+// 1824 x 4240, 34 clusters, 10.3 us with 208 KB, 7.0 with 96).
 // The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take: up to 48 tokens always, above that
 // when the cut saves three blocks, and one more for every eight tokens, up to 64 also uncut from eleven blocks on.  (220 shapes of
 // 41 .. 128 tokens per tile: 0.5 % behind the better one in the mean.)  The time by w8a8.cuh over this form's: 124 tokens, 188 tiles,
@@ -603,7 +604,7 @@ static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, 
   if (4 * tiles <= sms && saved(4) >= 4) S = 4;
   if (8 * tiles <= (kn ? sms - 20 : sms / 2) && k_blocks >= 32) S = 8;
   static_assert(qg::W8R_MAX_SPLIT == 8, "cuts above");
-  const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 12);
+  const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 24);
   const W8RowsPlan plan{(int)S, alone && (!kn || tokens > 32) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
   const bool uncut = tokens <= 64 && k_blocks > 10 && tiles <= sms;
   return tokens <= 48 || uncut || 25 * saved(S) > 3 * (tokens - 40) + 50 ? plan : none;
@@ -792,10 +793,10 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   }
   // The next kernel's CTAs then come to the SMs in the order in which these become free.  Grouped calls of several rounds, whose
   // neighbouring CTAs share tiles of L2, lose more by that than a late start costs: 16 groups, 8192 x 7168 x 2048 120.6 us, 126.0 with
-  // it, 25 groups, 3751 x 4992 x 3664 118.4 / 120.5; of one or two rounds 14 groups, 150 x 4256 x 1568 26.2 / 25.5, 17 groups, 1903 x
-  // 1184 x 1216 12.6 / 11.9.  Plain and batched calls gain throughout: 16 x 512 x 7168 x 2048 116.6 / 112.5, 1097 x 2496 x 1680 11.7 /
+  // it, 25 groups, 3751 x 4992 x 3664 118.4 / 120.5, of two rounds 9 groups, 6844 x 2464 x 1232 31.6 / 32.2; of one round 14 groups, 150 x
+  // 4256 x 1568 26.2 / 25.5, or of tiles of 128 columns, 17 groups, 1903 x 1184 x 1216 12.2 / 11.5.  Plain and batched calls gain throughout: 16 x 512 x 7168 x 2048 116.6 / 112.5, 1097 x 2496 x 1680 11.7 /
   // 10.9, 519 x 1344 x 2400 7.2 / 6.6, and with the quantiser in front 4096 x 4096 x 14336 188.7 / 186.4, 300 x 2048 x 4096 13.6 / 12.1.
-  p.early = meta == nullptr || p.num_items <= 2 * grid ? 1 : 0;
+  p.early = meta == nullptr || BN == 128 || p.num_items <= grid ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool nk = b_layout == QGEMM_B_NK;
   const bool bf = out_dtype == QGEMM_DT_BF16;
