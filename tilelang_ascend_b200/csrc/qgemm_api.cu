@@ -581,11 +581,14 @@ int qgemm_init(void) {
 
 // How the few-token form (w8a8_rows.cuh) takes `tiles` tiles: over how many CTAs it cuts their K, and the bytes of a CTA's pipeline.
 // split 0: w8a8.cuh is the faster one.
-// The cut.  One CTA per SM, as long as it saves each CTA four k blocks; clusters of eight from 32 k blocks on, and where they fit
-// easily.  A second CTA per SM by a further cut does not pay.
+// The cut.  One CTA per SM, as long as it saves each CTA four k blocks; clusters of eight from 32 k blocks on, as long as each CTA of
+// theirs finds an SM of its own: 15 of them did on the chip this was measured on, and one is left as a margin.  us, cut in four / in
+// eight, 8, 32 and 128 tokens: 1792 columns (14 clusters), K = 4096 5.32 / 5.41, 6.20 / 5.67, 7.64 / 7.57, K = 8192 7.74 / 7.31, 9.09 /
+// 7.36, 10.00 / 9.95 ([N, K] weights 5.26 / 5.28, 5.84 / 5.41, 7.75 / 7.37, 7.59 / 7.36, 8.12 / 7.51, 10.27 / 9.84); 2048 columns (16),
+// K = 4096 5.50 / 7.03, 6.15 / 7.06, 7.86 / 9.75.  A second CTA per SM by a further cut does not pay.
 // The pipeline.  208 KB (one CTA per SM) where all CTAs find an SM of their own, else, and for up to 32 tokens of [K, N] weights, 96 KB.
-// Clusters of four do not fill all SMs with one CTA each, 128 of 148 or a few more, by where the chip's working SMs are: 24 fewer (57 x
-// 1824 x 4240, 34 clusters, 10.3 us with 208 KB, 7.0 with 96).
+// Clusters of four do not fill all SMs with one CTA each either, 132 of 148 on that chip, 128 on another: 24 fewer (57 x 1824 x 4240, 34
+// clusters, 10.3 us with 208 KB, 7.0 with 96).
 // The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take: up to 48 tokens always, above that
 // when the cut saves three blocks, and one more for every eight tokens, up to 64 also uncut from eleven blocks on.  (220 shapes of
 // 41 .. 128 tokens per tile: 0.5 % behind the better one in the mean.)  The time by w8a8.cuh over this form's: 124 tokens, 188 tiles,
@@ -602,7 +605,7 @@ static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, 
   int64_t S = 1;
   if (2 * tiles <= sms && saved(2) >= 4) S = 2;
   if (4 * tiles <= sms && saved(4) >= 4) S = 4;
-  if (8 * tiles <= (kn ? sms - 20 : sms / 2) && k_blocks >= 32) S = 8;
+  if (8 * tiles <= sms - 36 && k_blocks >= 32) S = 8;
   static_assert(qg::W8R_MAX_SPLIT == 8, "cuts above");
   const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 24);
   const W8RowsPlan plan{(int)S, alone && (!kn || tokens > 32) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
