@@ -377,11 +377,11 @@ print("single ok")
 
 
 # On 148 SMs: one CTA each that fits an SM or shares it; a cut in two from eight k blocks on, in four from six, in eight from 32 and up
-# to 14 clusters, and the sizes at either side of each; clusters of four on 136 and 140 SMs; 96 and 208 KB of pipeline, more k blocks than stages, up to 128
-# tokens, and one token more.
+# to 14 clusters, and the sizes at either side of each; clusters of four on 136 and 140 SMs; 96 and 208 KB of pipeline, a K that the
+# shorter one just holds and one block more, more k blocks than stages, up to 128 tokens, and one token more.
 @pytest.mark.parametrize("batch,M,K,N", [
     (0, 32, 896, 9472), (0, 33, 1024, 9472), (0, 17, 1024, 9488), (0, 48, 640, 4352), (0, 16, 768, 4480), (0, 8, 4096, 4352), (0, 40, 2048, 18944),
-    (0, 5, 1536, 18960), (0, 24, 4080, 1168), (0, 60, 8192, 1168), (0, 128, 4096, 2048), (0, 12, 4096, 1792), (0, 100, 4112, 1808), (0, 129, 1152, 1040), (3, 72, 4864, 6016),
+    (0, 5, 1536, 18960), (0, 24, 4080, 1168), (0, 60, 8192, 1168), (0, 128, 4096, 2048), (0, 12, 4096, 1792), (0, 30, 1024, 8192), (0, 48, 1056, 8192), (0, 16, 640, 9488), (0, 16, 656, 9488), (0, 100, 4112, 1808), (0, 129, 1152, 1040), (3, 72, 4864, 6016),
     (2, 1, 4224, 1024)])
 @pytest.mark.parametrize("layout", ["KN", "NK"])
 def test_plans_for_few_tokens_are_exact(batch, M, K, N, layout):

@@ -586,7 +586,12 @@ int qgemm_init(void) {
 // eight, 8, 32 and 128 tokens: 1792 columns (14 clusters), K = 4096 5.32 / 5.41, 6.20 / 5.67, 7.64 / 7.57, K = 8192 7.74 / 7.31, 9.09 /
 // 7.36, 10.00 / 9.95 ([N, K] weights 5.26 / 5.28, 5.84 / 5.41, 7.75 / 7.37, 7.59 / 7.36, 8.12 / 7.51, 10.27 / 9.84); 2048 columns (16),
 // K = 4096 5.50 / 7.03, 6.15 / 7.06, 7.86 / 9.75.  A second CTA per SM by a further cut does not pay.
-// The pipeline.  208 KB (one CTA per SM) where all CTAs find an SM of their own, else, and for up to 32 tokens of [K, N] weights, 96 KB.
+// The pipeline.  96 KB, beside which the next call's CTA finds room, where that holds a CTA's whole K (64 tiles of K = 1024, cut in two,
+// 96 / 208 KB: 17 tokens 4.54 / 4.87 us, 40 tokens 6.3 / 6.5), for up to 16 tokens of [K, N] weights, and where CTAs share SMs; else 208
+// KB.  us, calls one after another: [K, N] 16 x 8192 x 8192 14.2 / 14.8, 16 x 4096 x 14336 12.6 / 12.8, 17 x 4096 x 14336 14.5 / 13.5, 32 x
+// 2048 x 14336 9.4 / 8.7, 32 x 1024 x 14336 6.7 / 6.6, [N, K] 16 x 8192 x 8192 15.0 / 14.9, 32 x 8192 x 8192 16.7 / 15.0, 8 x 1024 x 14336 5.9 /
+// 5.9, 8 x 1536 x 12288 6.9 / 6.8.  ([K, N], 110 shapes: at 4, 12 and 16 tokens 208 KB is 2 % slower in the mean, 3 % above eight blocks a
+// CTA; at 17 .. 32 tokens 1 and 3 % faster.)
 // Clusters of four do not fill all SMs with one CTA each either, 132 of 148 on that chip, 128 on another: 24 fewer (57 x 1824 x 4240, 34
 // clusters, 10.3 us with 208 KB, 7.0 with 96).
 // The choice.  Per tile this form pays for its tokens and saves the k blocks that other CTAs take: up to 48 tokens always, above that
@@ -608,7 +613,8 @@ static W8RowsPlan w8_rows_plan(int64_t tiles, int64_t k_blocks, int64_t tokens, 
   if (8 * tiles <= sms - 36 && k_blocks >= 32) S = 8;
   static_assert(qg::W8R_MAX_SPLIT == 8, "cuts above");
   const bool alone = S < 4 ? S * tiles <= sms : (S == 4 && S * tiles <= sms - 24);
-  const W8RowsPlan plan{(int)S, alone && (!kn || tokens > 32) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
+  const bool held = (k_blocks + S - 1) / S * (qg::W8R_W_BYTES + 128 * tokens) <= qg::W8R_RING_BYTES;
+  const W8RowsPlan plan{(int)S, alone && !held && (!kn || tokens > 16) ? qg::W8R_RING_BYTES_ONE : qg::W8R_RING_BYTES}, none{0, 0};
   const bool uncut = tokens <= 64 && k_blocks > 10 && tiles <= sms;
   return tokens <= 48 || uncut || 25 * saved(S) > 3 * (tokens - 40) + 50 ? plan : none;
 }
