@@ -835,3 +835,25 @@ def test_pre_pass_of_the_group_sum_kernel(batch, M, K, N, dt):
     poison = torch.full((1 << 24,), float("nan"), device="cuda")  # the scratch comes from this block
     del poison
     assert torch.equal(q.w4a16_gemm(A, P, S, 8, K), want)
+
+
+# On 148 SMs, slabs per CTA and the tiles they belong to: fewer than the activation stages (one, two, three), as many, one more; a change
+# of tile after one slab, after two, after three, with a batch, and from a shared tile to a whole one; one token and M below the tile.
+@pytest.mark.parametrize("batch,M,K,N", [
+    (1, 1, 8192, 560), (1, 1, 1792, 6288), (1, 3, 3584, 4096), (1, 16, 1024, 20000), (1, 9, 1280, 20000), (1, 2, 512, 30000),
+    (1, 1, 768, 24000), (3, 13, 2304, 7296), (19, 5, 512, 1072)])
+@pytest.mark.parametrize("zeros", ["scalar", "tensor"])
+def test_first_activations_of_a_cta(batch, M, K, N, zeros):
+    """Small integer activations and scales of one, as above: the fp32 sums are exact."""
+    q = _q()
+    g = torch.Generator(device="cuda").manual_seed(K + 64 * M + batch)
+    A = torch.randint(-3, 4, (batch, M, K), generator=g, device="cuda").to(torch.bfloat16)
+    P = torch.randint(0, 256, (batch, N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    S = torch.ones((batch, K // 256, N), dtype=torch.float16, device="cuda")
+    Z = torch.randint(0, 16, (batch, K // 256, N), generator=g, device="cuda").to(torch.float16)
+    W = torch.stack([P & 15, P >> 4], dim=-1).view(batch, N, K).double()
+    W -= 8 if zeros == "scalar" else Z.double().transpose(1, 2).repeat_interleave(256, dim=2)
+    want = (A.double() @ W.transpose(1, 2)).to(torch.bfloat16)
+    for _ in range(2):  # the second call starts beside the first one
+        got = [q.w4a16_gemm(A, P, S, 8, 256) if zeros == "scalar" else q.w4a16_gemm(A, P, S, Z, 256, zeros_mode="quantized") for _ in range(3)]
+        assert all(torch.equal(x, want) for x in got)

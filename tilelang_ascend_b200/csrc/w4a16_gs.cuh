@@ -277,11 +277,12 @@ w4g_prepare_activations(const uint4* in, uint8_t* __restrict__ out, int rows, in
   const int lane = threadIdx.x & 31, warp = (int)(blockIdx.x * (W4G_PREP_THREADS / 32) + (threadIdx.x >> 5));
   const int first = per * warp, step = per * (int)gridDim.x * (W4G_PREP_THREADS / 32);
   int row = first / KS, ks = first - row * KS;  // row: of all problems'
+  int b0 = row / M, m0 = row - b0 * M;
   pdl_wait();  // the kernel in front (another call's GEMM, which lets its dependents start early) is done
   auto src = [&](int r, int k) { return in + ((size_t)r * (size_t)K + k * W4_SLAB_K) / 8 + lane; };  // K is a multiple of 32
   auto in_row = [&](int k) { return k * W4_SLAB_K + lane * 8 < K; };
   while (row < rows) {
-    int r = row, k = ks, b = row / M, m = row - b * M;
+    int r = row, k = ks, b = b0, m = m0;
     auto next = [&]() {
       if (++k == KS) {
         k = 0;
@@ -323,6 +324,8 @@ w4g_prepare_activations(const uint4* in, uint8_t* __restrict__ out, int rows, in
     ks += step;
     row += ks / KS;
     ks %= KS;
+    b0 = row / M;
+    m0 = row - b0 * M;
   }
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < n_counters / 4; i += W4G_PREP_THREADS) counters[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -546,18 +549,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           }
         }
       } else {
-        pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
-        int st = 0;
-        while (i < n_slabs) {
-          if (i >= AS)  // the slab that used this stage has been multiplied
-            w4g_wait<W4G_DONE, ST_TIMEOUT_PRODUCER>(bar0 + 8 * ((i - AS) % W4G_BARS), (uint32_t)((i - AS) / W4G_BARS) & 1u, ctl, fail);
-          if (fail) break;
-          uint64_t* bar = &a_full[i % W4G_BARS];
-          mbar_arrive_expect_tx(bar, Cfg::A_BYTES);
-          tma_load_3d(a_base + st * Cfg::A_BYTES, &tmA, bar, 0, 0, (b * p.KS + ks) * 4);  // four blocks of 64 k, MT rows each
-          issued_mask |= 1u << (i % W4G_BARS);
-          parity_mask = (parity_mask & ~(1u << (i % W4G_BARS))) | (((uint32_t)(i / W4G_BARS) & 1u) << (i % W4G_BARS));
-          if (++st == AS) st = 0;
+        auto advance = [&]() {
           ++i;
           ++ks;
           if (--left == 0) {
@@ -566,6 +558,37 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
             left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
             w4_tile_coords(p, tile, MT, b, n0, m0);
           }
+        };
+        // A CTA's first copies are what the kernel waits for when it has few slabs, so up to 16 tokens all that can be done for
+        // them without the activations is done in front of the wait, and they are issued in one go behind it (1 x 1792 x 6288 9.5 ->
+        // 8.9 us, 16 x 3584 x 4096 10.5 -> 9.5; 64 x 8192 x 28672 43.7 instead of 42.2).
+        constexpr int EARLY = MT == 16 ? AS : 0;
+        int first_z[AS];
+#pragma unroll
+        for (int j = 0; j < EARLY; ++j) {
+          first_z[j] = (b * p.KS + ks) * 4;
+          if (j < n_slabs) {
+            mbar_arrive_expect_tx(&a_full[j], Cfg::A_BYTES);
+            advance();
+          }
+        }
+        pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
+#pragma unroll
+        for (int j = 0; j < EARLY; ++j)
+          if (j < n_slabs) tma_load_3d(a_base + j * Cfg::A_BYTES, &tmA, &a_full[j], 0, 0, first_z[j]);
+        issued_mask = (1u << min(n_slabs, EARLY)) - 1u;
+        int st = 0;
+        while (i < n_slabs) {
+          if (EARLY == AS || i >= AS)  // the slab that used this stage has been multiplied
+            w4g_wait<W4G_DONE, ST_TIMEOUT_PRODUCER>(bar0 + 8 * ((i - AS) % W4G_BARS), (uint32_t)((i - AS) / W4G_BARS) & 1u, ctl, fail);
+          if (fail) break;
+          uint64_t* bar = &a_full[i % W4G_BARS];
+          mbar_arrive_expect_tx(bar, Cfg::A_BYTES);
+          tma_load_3d(a_base + st * Cfg::A_BYTES, &tmA, bar, 0, 0, (b * p.KS + ks) * 4);  // four blocks of 64 k, MT rows each
+          issued_mask |= 1u << (i % W4G_BARS);
+          parity_mask = (parity_mask & ~(1u << (i % W4G_BARS))) | (((uint32_t)(i / W4G_BARS) & 1u) << (i % W4G_BARS));
+          if (++st == AS) st = 0;
+          advance();
         }
       }
       if (fail) {  // wait (bounded) for the copies still in flight before the CTA may exit
