@@ -547,12 +547,13 @@ static int w4a8_fused(const int8_t* A, const uint8_t* qB, int8_t* workspace, int
   p.sk_tiles = (int)(borrow ? left + grid : left);
   // a programmatic dependent of whatever is in front: behind another call of this operator it is resident early
   if (X != nullptr) {
-    if (launch_pdl(qg::w4a8_quant_prepare_activations, (int)M * parts, qg::W4I8_PREP_THREADS, 16 * (int)std::min<int64_t>(K / 8, qg::W4I8_PREP_KEPT), s, static_cast<const uint4*>(X),
-                   x_is_bf16, round_scale, reinterpret_cast<uint2*>(a_prepared), row_sums, scale_out, p.ws_counters, (int)grid_max,
-                   (int)K, (int)M, parts))
+    auto prepare = M <= 16 ? qg::w4a8_quant_prepare_activations<12> : qg::w4a8_quant_prepare_activations<16>;
+    const int kept = 16 * (int)std::min<int64_t>(K / 8, qg::W4I8_PREP_KEPT);
+    if (launch_pdl(prepare, (int)M * parts, qg::W4I8_PREP_THREADS, kept, s, static_cast<const uint4*>(X), x_is_bf16, round_scale,
+                   reinterpret_cast<uint2*>(a_prepared), row_sums, scale_out, p.ws_counters, (int)grid_max, (int)K, (int)M, parts))
       return -1;
-  } else if (launch_pdl(qg::w4a8_prepare_activations, (int)M * parts, qg::W4I8_PREP_THREADS, 0, s,
-                        reinterpret_cast<const uint2*>(A), reinterpret_cast<uint2*>(a_prepared), row_sums, p.ws_counters,
+  } else if (launch_pdl(M <= 16 ? qg::w4a8_prepare_activations<12> : qg::w4a8_prepare_activations<16>, (int)M * parts,
+                        qg::W4I8_PREP_THREADS, 0, s, reinterpret_cast<const uint2*>(A), reinterpret_cast<uint2*>(a_prepared), row_sums, p.ws_counters,
                         (int)grid_max, (int)K, (int)M, parts))
     return -1;
   const bool sgn = signed_nibbles != 0;

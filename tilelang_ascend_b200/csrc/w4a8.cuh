@@ -36,7 +36,9 @@ struct W4I8Cfg {
   static constexpr int RAW_STAGES = 8;                 // even, like W_STAGES: a stage always belongs to one warp set
   static constexpr int A_STAGES = (MT <= 32) ? 8 : (MT == 64 ? 4 : 3);
   static constexpr int MMAW = MT == 16 ? 4 : (MT <= 64 ? 2 : 1);
-  static constexpr int THREADS = (W4_FIRST_XMMA_WARP + MMAW - 1) * 32;  // two issuers: with room for a block of the pre-pass
+  // Two issuers leave room for a block of the pre-pass.  The kernel is compiled for what it is launched with: at the 72 registers of
+  // 832 threads it spilled, and 64 x 5888 x 22384 took 31.0 us (29.5 with 80 registers), 32 x 6144 x 11792 19.3 (18.2).
+  static constexpr int THREADS = (W4_FIRST_XMMA_WARP + MMAW - 1) * 32;
   static constexpr int W_STAGES = 4;
   static constexpr int A_KB_BYTES = MT * 128;          // one 128-wide K block of int8 activations
   static constexpr int A_BYTES = 2 * A_KB_BYTES;       // one 256-wide slab
@@ -57,12 +59,12 @@ struct W4I8Cfg {
 // 0,2,4,6,1,3,5,7 (the byte order the unpack produces), and the row sums.  `parts` blocks share a row: block (m, part) takes
 // the part-th range of its chunks of eight k and leaves their sum in row_sums[part * M + m].
 // What bounds both pre-passes is latency, between the end of the kernel in front and the GEMM kernel's first MMA, so their blocks
-// should all be waiting, on SMs of their own, when that kernel ends: few enough for one per SM, and 128 threads of 40 registers at
-// most, which fit beside a CTA of the GEMM kernel of up to 64 tokens (832 threads of 64 registers or 768 of 72; more tokens leave no
-// shared memory, and then more blocks are faster: 128 x 8192 x 8192 41.7 us with one per row, 38.1 with four).  Blocks of 256 threads and 63 registers, a row each, did
-// not: behind another call of this operator they waited for the first SMs to become free, shared these, and kept the next call's
-// GEMM CTAs off them for 8 us: 16 x 8192 x 28672 26.2 -> 24.7 us, 20 x 8192 x 28672
-// 31.2 -> 27.5, 12 x 6912 x 7792 14.9 -> 13.2.
+// should all be waiting, on SMs of their own, when that kernel ends: few enough for one per SM, and 128 threads of 40 registers up to
+// 16 tokens, 32 above, which fit beside a CTA of the GEMM kernel of up to 64 tokens (832 threads of 64 registers, or 768 of 80; more
+// tokens leave no shared memory, and then more blocks are faster: 128 x 8192 x 8192 41.7 us with one per row, 38.1 with four).  Blocks
+// of 256 threads and 63 registers, a row each, did not: behind another call of this operator they waited for the first SMs to become
+// free, shared these, and kept the next call's GEMM CTAs off them for 8 us: 16 x 8192 x 28672 26.2 -> 24.7 us, 20 x 8192 x 28672 31.2 ->
+// 27.5, 12 x 6912 x 7792 14.9 -> 13.2.
 constexpr int W4I8_PREP_THREADS = 128;
 constexpr int W4I8_PREP_MAX_PARTS = 8;
 constexpr int W4I8_PREP_KEPT = 1024;  // chunks of a row that the quantising pre-pass keeps in shared memory
@@ -73,7 +75,8 @@ __device__ __forceinline__ int w4i8_block_sum(int acc, int* red) {  // in thread
   __syncthreads();
   return red[0] + red[1] + red[2] + red[3];
 }
-__global__ void __launch_bounds__(W4I8_PREP_THREADS, 12)
+template <int BLOCKS>  // per SM, i.e. 40 or 32 registers
+__global__ void __launch_bounds__(W4I8_PREP_THREADS, BLOCKS)
 w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restrict__ row_sums, uint32_t* __restrict__ counters,
                          int n_counters, int K, int M, int parts) {
   __shared__ int red[W4I8_PREP_THREADS / 32];
@@ -105,7 +108,8 @@ w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restri
 // (examples/deepseek_v4/act_quant.py:112-142); what disappears is one launch and the int8 round trip through
 // memory.  Every block of a row takes the abs-max of all of it (four instructions per eight values), then quantises its own part
 // (about a hundred), which it reads again from L1.
-__global__ void __launch_bounds__(W4I8_PREP_THREADS, 12)
+template <int BLOCKS>  // per SM, i.e. 40 or 32 registers
+__global__ void __launch_bounds__(W4I8_PREP_THREADS, BLOCKS)
 w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uint2* __restrict__ out,
                                int* __restrict__ row_sums, float* __restrict__ scales, uint32_t* __restrict__ counters,
                                int n_counters, int K, int M, int parts) {
@@ -160,7 +164,7 @@ w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uin
 // same up to two rounds but for 20 and 16 slabs, where 224 tiles take 20.5 / 21.1 and 17.5 / 18.8: so from 24 slabs on, where
 // nothing loses.  In the one kernel 64 x 8192 x 28672 took 8 % longer.
 template <int MT, bool SIGNED, bool WHOLE = false>
-__global__ void __launch_bounds__(W4_THREADS, 1)
+__global__ void __launch_bounds__(W4I8Cfg<MT>::THREADS, 1)
 w4a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
                  const W4A8Params p) {
   using Cfg = W4I8Cfg<MT>;
