@@ -354,14 +354,17 @@ int launch_w4w(bool bf, bool zt, const CUtensorMap& tmW, const CUtensorMap& tmS,
 int launch_w4g_prepare(const void* A, void* out, const qg::W4A16Params& p, bool is_bf16, int sms, cudaStream_t s) {
   constexpr int warps = qg::W4G_PREP_THREADS / 32;
   const long long rows = (long long)p.batch * p.M, slabs = rows * p.KS;
-  if (p.m_tiles != 1 || slabs > 0x3fffffffll) return fail("qgemm_w4a16: activation tensor too large");
-  // A block per SM at most, so that all are resident early, and each warp's share in equal rounds.  From four rounds on throughput
-  // counts for more than an early start: as many blocks as an SM holds.  us, one / eleven blocks per SM (one for every 128 chunks
-  // of 32 k, before): 24 x 60 x 7424 x 1408 51.9 / 45.8 (50.5), 32 x 64 x 8192 x 1024 63.6 / 51.3 (58.2); from two rounds on 20 x 48
-  // x 4096 x 2048 33.9 / 35.8 (37.0), 8 x 64 x 8192 x 1024 25.4 / 27.5 (28.0), but 24 x 64 x 4096 x 4096 70.3 / 69.0.
+  if (slabs > 0x3fffffffll) return fail("qgemm_w4a16: activation tensor too large");
+  // A block per SM at most, so that all are resident early, and each warp's share in equal rounds.  Above four rounds throughput
+  // counts for more than an early start: a block for every round.  Ten of them are resident on an SM (20 KB of shared memory and 1 KB
+  // beside it each), but with no more than ten launched warps of the last round come to a second one.  us, one block per SM / a block
+  // for every round (one for every 128 chunks of 32 k, before): 24 x 60 x 7424 x 1408 51.9 / 46.4 (51.0), 32 x 64 x 8192 x 1024 63.6 /
+  // 52.7 (58.7; ten per SM 54.6), 40 x 64 x 8192 x 1024 - / 65.6 (72.6; ten per SM 67.0, eleven 67.0); from two rounds on 20 x 48 x 4096
+  // x 2048 33.9 / 35.8 (37.0), 8 x 64 x 8192 x 1024 25.4 / 27.5 (28.0), but 24 x 64 x 4096 x 4096 70.3 / 69.0.
   const long long each = (slabs + warps * sms - 1) / (warps * sms), rounds = (each + qg::W4G_PREP_LANDING - 1) / qg::W4G_PREP_LANDING;
   const int per = (int)((each + rounds - 1) / rounds);
-  const int grid = (int)std::min<long long>(sms * (rounds > 4 ? 11 : 1), (slabs + warps * per - 1) / (warps * per));
+  const long long blocks = (slabs + warps * per - 1) / (warps * per);
+  const int grid = (int)(rounds > 4 ? blocks : std::min<long long>(sms, blocks));
   auto kernel = per <= qg::W4G_PREP_REGS ? qg::w4g_prepare_activations<false> : qg::w4g_prepare_activations<true>;
   return launch_pdl(kernel, grid, qg::W4G_PREP_THREADS, 0, s, static_cast<const uint4*>(A), static_cast<uint8_t*>(out), (int)rows, p.M,
                     p.K, p.KS, is_bf16 ? 1 : 0, per, reinterpret_cast<uint4*>(p.ws_counters), (int)(kW4CounterBytes / 4));
