@@ -67,8 +67,6 @@ int set_smem_w8() {
   if constexpr (BN == 256) {  // the forms of two CTAs
     if (set_smem(qg::w8a8_gemm_kernel<256, false, false, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
     if (set_smem(qg::w8a8_gemm_kernel<256, false, true, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, false, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w8a8_gemm_kernel<256, true, true, qg::W8_SPLITK>, C::SMEM_BYTES)) return -1;
     constexpr int pair_bytes = qg::W8Cfg<256, qg::W8_PAIR>::SMEM_BYTES;
     if (set_smem(qg::w8a8_gemm_kernel<256, false, false, qg::W8_PAIR>, pair_bytes)) return -1;
     if (set_smem(qg::w8a8_gemm_kernel<256, false, true, qg::W8_PAIR>, pair_bytes)) return -1;
@@ -264,13 +262,6 @@ int launch_w8_clusters(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   CUDA_OK(cudaLaunchKernelEx(&cfg, qg::w8a8_gemm_kernel<256, NK, BF, FORM>, tmA, tmB, tmC, p));
   return 0;
 }
-template <qg::W8Form FORM>
-int launch_w8_clusters(bool nk, bool bf, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
-                       const qg::W8A8Params& p, int clusters, cudaStream_t s) {
-  if (nk) return bf ? launch_w8_clusters<true, true, FORM>(tmA, tmB, tmC, p, clusters, s) : launch_w8_clusters<true, false, FORM>(tmA, tmB, tmC, p, clusters, s);
-  return bf ? launch_w8_clusters<false, true, FORM>(tmA, tmB, tmC, p, clusters, s) : launch_w8_clusters<false, false, FORM>(tmA, tmB, tmC, p, clusters, s);
-}
-
 // Few-token form: clusters of S CTAs, a programmatic dependent of whatever is in front of it on the stream.
 template <bool NK, bool BF>
 int launch_w8_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const qg::W8RowsParams& p, int grid, int S, cudaStream_t s) {
@@ -813,8 +804,15 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool nk = b_layout == QGEMM_B_NK;
   const bool bf = out_dtype == QGEMM_DT_BF16;
-  if (use_splitk) return launch_w8_clusters<qg::W8_SPLITK>(nk, bf, tmA, tmB, tmC, p, (int)num_tiles, s);
-  if (use_pair) return launch_w8_clusters<qg::W8_PAIR>(nk, bf, tmA, tmB, tmC, p, grid, s);
+  if (use_splitk) {  // [K, N] only
+    constexpr auto form = qg::W8_SPLITK;
+    return bf ? launch_w8_clusters<false, true, form>(tmA, tmB, tmC, p, (int)num_tiles, s) : launch_w8_clusters<false, false, form>(tmA, tmB, tmC, p, (int)num_tiles, s);
+  }
+  if (use_pair) {
+    constexpr auto form = qg::W8_PAIR;
+    if (nk) return bf ? launch_w8_clusters<true, true, form>(tmA, tmB, tmC, p, grid, s) : launch_w8_clusters<true, false, form>(tmA, tmB, tmC, p, grid, s);
+    return bf ? launch_w8_clusters<false, true, form>(tmA, tmB, tmC, p, grid, s) : launch_w8_clusters<false, false, form>(tmA, tmB, tmC, p, grid, s);
+  }
   if (BN == 256) {
     if (nk) return bf ? launch_w8<256, true, true>(tmA, tmB, tmC, p, grid, s) : launch_w8<256, true, false>(tmA, tmB, tmC, p, grid, s);
     return bf ? launch_w8<256, false, true>(tmA, tmB, tmC, p, grid, s) : launch_w8<256, false, false>(tmA, tmB, tmC, p, grid, s);

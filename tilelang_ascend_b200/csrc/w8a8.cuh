@@ -160,7 +160,8 @@ __device__ __forceinline__ void w8_zero_uncovered(const W8A8Params& p, int warp4
   }
 }
 
-// SPLITK is the form for very long K on grids that would leave half of the SMs idle (w8a8_impl): the kernel is launched in clusters of two CTAs, one tile per cluster; each CTA accumulates
+// SPLITK is the form for weights [K, N] and a very long K on grids that would leave half of the SMs idle (w8a8_impl): the kernel is
+// launched in clusters of two CTAs, one tile per cluster; each CTA accumulates
 // one half of the K range in its own tensor memory; then each CTA writes its int32 accumulators of the OTHER CTA's
 // half of the columns into that CTA's shared memory (the pipeline stages, idle by then) through distributed shared
 // memory, adds what it received to its own half and runs the epilogue for that half - an exact integer sum, so the
@@ -183,6 +184,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   using Cfg = W8Cfg<BN, FORM>;
   constexpr int STAGES = Cfg::STAGES;
   constexpr bool SPLITK = FORM == W8_SPLITK, PAIR = FORM == W8_PAIR;
+  static_assert(!(SPLITK && B_NK), "K is cut for weights [K, N] only");
   // Two warps share the columns of 32 rows and store them in pieces of 64: an item of 128 columns at least (a half-width one, or
   // a CTA's half of a tile whose K is cut, comes from 256).
   static_assert(BN == 128 || (BN == 256 && (BN / 2) % 128 == 0), "columns of a tile");
