@@ -167,15 +167,19 @@ def test_config3_full_size_properties():
 
 
 # (with accumulators; without them the few-token form takes these shapes)
-SPLITK_SHAPES = [(0, 256, 4096, 1024), (2, 200, 4224, 528), (0, 130, 7168, 272), (3, 256, 4608, 1024),
-                 (0, 200, 4112, 2064), (2, 300, 4096, 1040)]
+SPLITK_SHAPES = [(0, 256, 6400, 1024), (2, 200, 6416, 528), (0, 130, 7168, 272), (3, 256, 6544, 1024), (0, 200, 6288, 2064),
+                 (2, 300, 7296, 1040), (0, 129, 8192, 144)]
+# too short a K, or too many tiles
+UNSPLIT_SHAPES = [(0, 256, 4096, 1024), (2, 200, 4224, 528), (3, 256, 4608, 1024), (0, 200, 4112, 2064), (2, 300, 4096, 1040),
+                  (0, 256, 6272, 1024), (2, 300, 6400, 1680)]
 
 
-@pytest.mark.parametrize("batch,M,K,N", SPLITK_SHAPES)
+@pytest.mark.parametrize("batch,M,K,N", SPLITK_SHAPES + UNSPLIT_SHAPES)
 def test_k_split_over_cta_pairs_is_exact(batch, M, K, N):
     """Few tiles and a long K: the kernel runs in clusters of two CTAs that each accumulate half of K and exchange
-    halves of the tile through distributed shared memory.  Ragged M, N and K, both layouts: accumulators and outputs
-    bit-exact against the oracle."""
+    halves of the tile through distributed shared memory, for weights [K, N] and at least 50 k blocks.  Ragged M, N and K, even
+    and odd numbers of k blocks, batches, shapes on the other side of the rule, and [N, K] weights, whose K is never cut:
+    accumulators and outputs bit-exact against the oracle."""
     q = _q()
     A, B, sa, sb = oc.make_w8a8_inputs(batch, M, K, N, seed=M + K)
     ref, acc_ref = oc.quant_matmul_ref(A, B, sb, "bfloat16", scale_a=sa, return_acc=True)
@@ -413,7 +417,8 @@ def test_short_k_is_exact(batch, M, K, N, layout):
     assert torch.equal(C, ((acc * sa.unsqueeze(-1)) * sb.unsqueeze(-2)).to(torch.float16))
 
 
-# K cut over two CTAs: at least 50 k blocks, weights [K, N], accumulators wanted; ragged M, N and K, and either side of the limits.
+# K cut over two CTAs: at least 50 k blocks, weights [K, N], accumulators wanted.  Ragged M, N and K, and beyond the limits: too short a
+# K, too many tiles, weights [N, K].
 @pytest.mark.parametrize("batch,M,K,N", [(0, 256, 6400, 1024), (2, 200, 6416, 528), (0, 130, 8192, 2064), (3, 256, 6272, 1024), (0, 1100, 6544, 1040)])
 @pytest.mark.parametrize("layout", ["KN", "NK"])
 def test_long_k_of_few_tiles_is_exact(batch, M, K, N, layout):
