@@ -815,8 +815,10 @@ print("single ok")
 
 
 @pytest.mark.parametrize("batch,M,K,N", [
-    # one (row, slab) per warp of the pre-pass; a last slab that is cut; two in registers; three and ten in shared memory; rounds of
-    # several, the last one partly filled; a block for every round, one and several waves of them
+    # one (row, slab) per warp of the pre-pass, one and a few rows; a last slab that is cut; two in registers; three and ten in shared
+    # memory; rounds of several, the last one partly filled; a block for every round, one and several waves of them; and, up to 16
+    # tokens of a short K, no pre-pass
+    (1, 1, 8192, 40), (1, 5, 8224, 64), (1, 16, 8224, 64), (3, 13, 6432, 64), (60, 15, 4128, 40),
     (13, 64, 8192, 40), (75, 37, 6432, 40),
     (1, 1, 288, 40), (3, 5, 1312, 64), (1, 48, 4384, 72), (2, 33, 6432, 40), (23, 16, 4096, 48), (40, 16, 4096, 64), (9, 64, 8192, 40),
     (1, 64, 8224, 128), (19, 61, 5152, 40)])
