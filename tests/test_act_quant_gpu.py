@@ -183,7 +183,8 @@ def test_scales_written_in_front_of_the_quantiser(M):
     assert not torch.equal(want[0], want[3])
 
 
-# tiles of 128 x 128, a K cut over two CTAs, 128 x 256, tiles of two CTAs; more and fewer quantiser blocks than SMs
+# On 148 SMs: tiles of 128 x 128, grouped ones of 128 x 256 in several rounds, tiles of two CTAs; more and fewer quantiser blocks than
+# SMs.  (130 x 8192 by tiles of 128 x 128 too: its K is not cut, see the test below.)
 @pytest.mark.parametrize("M,K,layers,layout", [(300, 1024, 12, "KN"), (130, 8192, 6, "KN"), (1150, 4096, 6, "NK"), (1200, 4096, 6, "KN"),
                                                (4096, 2048, 6, "NK"), (777, 512, 12, "KN")])
 @pytest.mark.parametrize("grouped", [False, True])
@@ -223,11 +224,49 @@ def test_chain_of_quantisers_and_tile_gemms(M, K, layers, layout, grouped):
     assert torch.isfinite(want[0].float()).all() and want[0].float().abs().max() > 0.1
 
 
+# On 148 SMs the tile kernels' other forms: a K cut over two CTAs (even and odd number of k blocks; with accumulators only), tiles of
+# 128 x 256 with a tail of half-width ones, grouped ones of exactly one round.
+@pytest.mark.parametrize("form,M,K,layers", [("split", 100, 6400, 6), ("split", 128, 6528, 6), ("whole", 9500, 288, 10), ("grouped", 4600, 1024, 8)])
+def test_chain_through_the_other_forms_of_the_tile_gemm(form, M, K, layers):
+    """These start early behind the quantiser and behind each other too, and let the next kernel start: same chain, same bits."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    scale = torch.rand(K, generator=g, device="cuda") / (0.577 * 74 * K ** 0.5)
+    if form == "grouped":
+        W = torch.randint(-128, 128, (4, K, K), dtype=torch.int8, generator=g, device="cuda")
+        kernel = q.grouped_quant_gemm((M // 3, 0, M - M // 3 - 7, 7), K, K, out_dtype="bfloat16")
+        meta, scales = kernel.block_metadata("cuda"), scale.expand(4, K).contiguous()
+        product = lambda a, sa: (kernel(a, W, meta, scales, sa),)
+    else:
+        W = torch.randint(-128, 128, (K, K), dtype=torch.int8, generator=g, device="cuda")
+        product = lambda a, sa: q.quant_matmul(a, W, scale, scale_a=sa, out_dtype="bfloat16", return_accumulators=True) if form == "split" \
+            else (q.quant_matmul(a, W, scale, scale_a=sa, out_dtype="bfloat16"),)
+
+    def chain(drain):
+        step = torch.cuda.synchronize if drain else lambda: None
+        h, first = (x,), (x,)
+        for i in range(layers):
+            a, sa = q.act_quant(h[0])
+            step()
+            if i % 2:
+                first = product(a, sa.view(-1))
+                step()
+            h = product(a, sa.view(-1))
+            step()
+        return (*h, *first)
+
+    want = chain(True)
+    for _ in range(3):
+        assert all(torch.equal(u, v) for u, v in zip(chain(False), want))
+    assert torch.isfinite(want[0].float()).all() and want[0].float().abs().max() > 0.1
+
+
 # one, two, four and eight chunks of eight per thread; rows shared by 32 .. 1024 threads, full and one chunk over; the last number of
-# rows that is spread on 148 SMs, and the next
+# rows that is spread on 148 SMs (rows x threads <= 1100 x 148), and the next
 @pytest.mark.parametrize("M,N", [(3, 256), (3, 264), (318, 4096), (317, 4104), (5, 4096), (5, 4104), (158, 8192), (159, 8192), (159, 8200),
                                  (160, 8200), (7, 16384), (7, 16392), (636, 2048), (637, 2048), (1271, 2056), (1273, 2056), (5089, 256),
-                                 (5088, 512), (5089, 512)])
+                                 (5088, 512), (5089, 512), (317, 4096), (635, 2048), (158, 8200), (635, 2056), (636, 2056), (5087, 512), (5087, 256),
+                                 (5088, 256), (317, 8192), (318, 8192)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("round_scale", [False, True])
 def test_threads_per_row(M, N, dt, round_scale):
