@@ -51,10 +51,19 @@ std::mutex g_mu;
 DeviceState g_dev[kMaxDevices];
 EncodeTiledFn g_encode = nullptr;
 
+// Kernels that are to be resident beside one another - a GEMM kernel and the next call's pre-pass - want all of an SM's memory that
+// can be as shared memory.  The driver by itself takes as little as one of them needs, 196 KB for the 187 of the 16-token group-sum
+// kernel, beside which the pre-pass's 21 KB found no room: 8 x 16 x 4096 x 4096, call after call, 22.0 us instead of 18.6, 27 x 15 x
+// 1024 x 3120 17.0 / 14.8, W4A8 27 x 3328 x 2320 20.3 / 18.1, 64 x 4096 x 14336 23.7 / 22.0 (as one graph it mostly did find room).
+template <typename K>
+int most_shared_memory(K kernel) {
+  CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  return 0;
+}
 template <typename K>
 int set_smem(K kernel, int bytes) {
   CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  return 0;
+  return most_shared_memory(kernel);
 }
 
 template <int BN>
@@ -161,6 +170,10 @@ int ensure_device(int* sm_count) {
     if (set_smem_w4g<16>() || set_smem_w4g<32>() || set_smem_w4g<64>()) return -1;
     if (set_smem_w4i8<16>() || set_smem_w4i8<32>() || set_smem_w4i8<64>() || set_smem_w4i8<128>()) return -1;
     if (set_smem_w8r() || set_smem_w4w<false>() || set_smem_w4w<true>()) return -1;
+    if (most_shared_memory(qg::w4g_prepare_activations<false>) || most_shared_memory(qg::w4g_prepare_activations<true>)) return -1;
+    if (most_shared_memory(qg::w4a8_prepare_activations<12>) || most_shared_memory(qg::w4a8_prepare_activations<16>)) return -1;
+    if (most_shared_memory(qg::w4a8_quant_prepare_activations<12>) || most_shared_memory(qg::w4a8_quant_prepare_activations<16>)) return -1;
+    if (most_shared_memory(qg::w4a16_prepare_activations)) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
     st.ready.store(true, std::memory_order_release);
