@@ -860,3 +860,22 @@ def test_first_activations_of_a_cta(batch, M, K, N, zeros):
     for _ in range(2):  # the second call starts beside the first one
         got = [q.w4a16_gemm(A, P, S, 8, 256) if zeros == "scalar" else q.w4a16_gemm(A, P, S, Z, 256, zeros_mode="quantized") for _ in range(3)]
         assert all(torch.equal(x, want) for x in got)
+
+
+# On 148 SMs: every tile's K in equal ranges, one per CTA.  Whole tiles on 61 and 66 CTAs, on 60 with 8.9 slabs a CTA more than an even
+# deal has, on 60 with 10.1 more (not taken), on 59 (not taken); ranges of two on 99 and 108, of three on 99; halves with 4.9 and with
+# 5.1 slabs more (not taken).
+@pytest.mark.parametrize("batch,M,K,N", [
+    (1, 64, 1280, 7728), (1, 40, 2816, 8400), (1, 20, 3840, 7680), (1, 20, 4352, 7680), (1, 17, 1280, 7504), (1, 16, 4608, 1312),
+    (1, 32, 3072, 2256), (1, 3, 6912, 1312), (1, 12, 5632, 5248), (4, 12, 5632, 1280)])
+def test_equal_ranges_of_k(batch, M, K, N):
+    """Small integer activations and scales of one: the fp32 sums are exact whatever the cut."""
+    q = _q()
+    g = torch.Generator(device="cuda").manual_seed(K + 64 * M + batch)
+    A = torch.randint(-3, 4, (batch, M, K), generator=g, device="cuda").half()
+    P = torch.randint(0, 256, (batch, N, K // 2), dtype=torch.uint8, generator=g, device="cuda")
+    S = torch.ones((batch, K // 128, N), dtype=torch.float16, device="cuda")
+    W = torch.stack([P & 15, P >> 4], dim=-1).view(batch, N, K).double() - 8
+    want = (A.double() @ W.transpose(1, 2)).half()
+    for _ in range(2):
+        assert all(torch.equal(x, want) for x in [q.w4a16_gemm(A, P, S, 8, 128) for _ in range(3)])

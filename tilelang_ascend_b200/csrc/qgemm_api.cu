@@ -1162,13 +1162,19 @@ static int w4a16_impl(const void* A, const uint8_t* B_packed, const void* scales
   int64_t grid = sms < kW4MaxGrid ? sms : kW4MaxGrid;
   if (plan.pair) grid /= 2;  // pairs of CTAs
   if (p.total_items < grid) grid = p.total_items;
-  // Small problems (a few slabs per CTA): prefer a slightly smaller grid that cuts every tile into equal K ranges,
-  // one per CTA, over an even deal that leaves most CTAs with two partial tiles and so two split-K hand-overs.
+  // Small problems (a few slabs per CTA): prefer a smaller grid that cuts every tile into equal K ranges, one per CTA, over an even
+  // deal that leaves most CTAs with two partial tiles and so two split-K hand-overs, each of which takes longer than several slabs.
+  // The group-sum kernel: down to two fifths of the SMs, as long as a CTA gets no more than five slabs more by it, nine where the
+  // tiles are whole and nothing is handed over.  us, even / equal: 16 x 4608 x 1312 12.3 / 8.3 (99 CTAs), 32 x 3072 x 2256 14.2 / 9.4 (108),
+  // 20 x 5376 x 1200 16.0 / 10.7 (70), 64 x 6912 x 3040 18.4 / 16.2 (72), whole tiles 64 x 1280 x 7728 14.1 / 8.0 (61), 2 x 20 x 3840 x 3888
+  // 12.2 / 11.1 (62); not taken: 8 x 7168 x 5296 11.2 / 11.8 (84 CTAs of 14 slabs instead of 8), 4 x 20 x 6656 x 1088 13.1 / 14.6 (72 of 13).
+  // (120 shapes of 1 .. 64 tokens, thirty for each step from three quarters down: 28 % faster in the mean in each.)
   if (!wide && p.total_items <= 8 * grid && p.total_items > grid) {
-    for (int64_t g2 = grid; g2 * 4 >= grid * 3; --g2) {
+    const int64_t least = use_gs ? (2 * grid + 4) / 5 : (3 * grid + 3) / 4;
+    for (int64_t g2 = grid; g2 >= least; --g2) {
       if (p.total_items % g2 != 0) continue;
       const int64_t per = p.total_items / g2;
-      if (p.KS % per == 0) {
+      if (p.KS % per == 0 && per * grid - p.total_items <= (per == p.KS ? 9 : 5) * grid) {
         grid = g2;
         break;
       }
