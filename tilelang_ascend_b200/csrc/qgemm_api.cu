@@ -204,9 +204,9 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 // Launch `kernel` so that it may start while the kernel in front of it on the stream is still running
 // (programmatic dependent launch); the kernel itself waits before it reads that kernel's results.
-// QGEMM_PDL=0 falls back to plain stream order, as `early` = false does.
+// QGEMM_PDL=0 falls back to plain stream order.
 template <typename... KArgs, typename... Args>
-int launch_maybe_pdl(bool early, void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
+int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
   static const int pdl = getenv("QGEMM_PDL") ? atoi(getenv("QGEMM_PDL")) : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -217,13 +217,9 @@ int launch_maybe_pdl(bool early, void (*kernel)(KArgs...), int grid, int threads
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl && early ? 1 : 0;
+  cfg.numAttrs = pdl ? 1 : 0;
   CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
   return 0;
-}
-template <typename... KArgs, typename... Args>
-int launch_pdl(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t s, Args&&... args) {
-  return launch_maybe_pdl(true, kernel, grid, threads, smem, s, std::forward<Args>(args)...);
 }
 
 // Rasterisation band: the tiles of `group_m` consecutive row blocks are walked column block by column block, so a
@@ -1433,11 +1429,12 @@ int qgemm_act_quant(const void* X, int8_t* Y, float* S, int64_t M, int64_t N, in
   const int64_t grid = (M + rows_per_block - 1) / rows_per_block;
   if (grid > 0x7fffffffll) return fail("qgemm_act_quant: too many rows (%lld)", (long long)M);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // A programmatic dependent: behind a W8A8 kernel it is resident when that kernel ends.  Not with more blocks than SMs: the SMs that
-  // kernel leaves idle would be filled with them and the others get few.  us with the GEMM behind it, plain stream order / early from
-  // any number of blocks up to four per SM: 1000 x 2048 x 2048 13.2 / 16.3, 3000 x 1024 x 1024 13.2 / 16.4, 600 x 4096 x 4096 21.5 / 22.6.
-  const bool early = grid <= sms;
-  auto launch = [&](auto kernel) { return launch_maybe_pdl(early, kernel, (int)grid, block, 0, st, p); };
+  // A programmatic dependent: behind a W8A8 kernel it is resident when that kernel ends, and behind any other its launch is ready.
+  // With more blocks than SMs they first fill the SMs that a GEMM kernel leaves idle in its last round, but in plain stream order the
+  // launch costs more.  us, plain / early, calls one after another: by itself 4096 x 4096 16.5 / 14.6, 8192 x 1024 10.3 / 8.5, with the GEMM
+  // behind it 600 x 4096 x 4096 22.0 / 20.1, 361 x 2464 x 2768 14.4 / 12.5, but 3000 x 1024 x 1024 15.6 / 16.1, 775 x 3968 x 11056 47.1 / 48.3; 60
+  // such pairs of 150 .. 4096 rows 6 % faster in the mean (as one graph, where a plain launch costs less, 1 % slower).
+  auto launch = [&](auto kernel) { return launch_pdl(kernel, (int)grid, block, 0, st, p); };
   auto launch_few = [&](auto keep_) {  // one or two chunks per thread
     constexpr int KEEP = decltype(keep_)::value;
     switch (tpr) {
