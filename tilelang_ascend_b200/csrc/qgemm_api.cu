@@ -55,15 +55,16 @@ EncodeTiledFn g_encode = nullptr;
 // can be as shared memory.  The driver by itself takes as little as one of them needs, 196 KB for the 187 of the 16-token group-sum
 // kernel, beside which the pre-pass's 21 KB found no room: 8 x 16 x 4096 x 4096, call after call, 22.0 us instead of 18.6, 27 x 15 x
 // 1024 x 3120 17.0 / 14.8, W4A8 27 x 3328 x 2320 20.3 / 18.1, 64 x 4096 x 14336 23.7 / 22.0 (as one graph it mostly did find room).
+// A kernel by itself is the slower for the smaller cache: 16 x 4096 x 4096 in a single launch 8.46, 8.37 with 196 KB.
 template <typename K>
 int most_shared_memory(K kernel) {
   CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   return 0;
 }
 template <typename K>
-int set_smem(K kernel, int bytes) {
+int set_smem(K kernel, int bytes, bool beside_pre_pass = false) {
   CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  return most_shared_memory(kernel);
+  return beside_pre_pass ? most_shared_memory(kernel) : 0;
 }
 
 template <int BN>
@@ -95,11 +96,11 @@ int set_smem_w4d() {
 template <int MT>
 int set_smem_w4i8() {
   using C = qg::W4I8Cfg<MT>;
-  if (set_smem(qg::w4a8_gemm_kernel<MT, false>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a8_gemm_kernel<MT, true>, C::SMEM_BYTES)) return -1;
+  if (set_smem(qg::w4a8_gemm_kernel<MT, false>, C::SMEM_BYTES, true)) return -1;
+  if (set_smem(qg::w4a8_gemm_kernel<MT, true>, C::SMEM_BYTES, true)) return -1;
   if constexpr (MT == 16) {
-    if (set_smem(qg::w4a8_gemm_kernel<MT, false, true>, C::SMEM_BYTES)) return -1;
-    if (set_smem(qg::w4a8_gemm_kernel<MT, true, true>, C::SMEM_BYTES)) return -1;
+    if (set_smem(qg::w4a8_gemm_kernel<MT, false, true>, C::SMEM_BYTES, true)) return -1;
+    if (set_smem(qg::w4a8_gemm_kernel<MT, true, true>, C::SMEM_BYTES, true)) return -1;
   }
   return 0;
 }
@@ -115,12 +116,12 @@ template <int MT>
 int set_smem_w4g() {
   using C = qg::W4GCfg<MT>;
   constexpr int zt_bytes = qg::W4GCfg<MT, true>::SMEM_BYTES;
-  if (set_smem(qg::w4a16_gs_kernel<MT, false>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, false, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, true, true>, C::SMEM_BYTES)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, false, false, true>, zt_bytes)) return -1;
-  if (set_smem(qg::w4a16_gs_kernel<MT, true, false, true>, zt_bytes)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, false>, C::SMEM_BYTES, true)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, true>, C::SMEM_BYTES, true)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, false, true>, C::SMEM_BYTES, true)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, true, true>, C::SMEM_BYTES, true)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, false, false, true>, zt_bytes, true)) return -1;
+  if (set_smem(qg::w4a16_gs_kernel<MT, true, false, true>, zt_bytes, true)) return -1;
   if constexpr (MT == 16) {
     if (set_smem(qg::w4a16_gs_kernel<16, false, false, false, true>, C::SMEM_BYTES)) return -1;
     if (set_smem(qg::w4a16_gs_kernel<16, true, false, false, true>, C::SMEM_BYTES)) return -1;
@@ -173,7 +174,6 @@ int ensure_device(int* sm_count) {
     if (most_shared_memory(qg::w4g_prepare_activations<false>) || most_shared_memory(qg::w4g_prepare_activations<true>)) return -1;
     if (most_shared_memory(qg::w4a8_prepare_activations<12>) || most_shared_memory(qg::w4a8_prepare_activations<16>)) return -1;
     if (most_shared_memory(qg::w4a8_quant_prepare_activations<12>) || most_shared_memory(qg::w4a8_quant_prepare_activations<16>)) return -1;
-    if (most_shared_memory(qg::w4a16_prepare_activations)) return -1;
     if (set_smem_w4d<0>() || set_smem_w4d<1>() || set_smem_w4d<2>() || set_smem_w4d<4>()) return -1;
     st.sm_count = prop.multiProcessorCount;
     st.ready.store(true, std::memory_order_release);

@@ -562,7 +562,7 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         // A CTA's first copies are what the kernel waits for when it has few slabs, so up to 16 tokens all that can be done for
         // them without the activations is done in front of the wait, and they are issued in one go behind it (1 x 1792 x 6288 9.5 ->
         // 8.9 us, 16 x 3584 x 4096 10.5 -> 9.5; 64 x 8192 x 28672 43.7 instead of 42.2).
-        constexpr int EARLY = MT == 16 ? AS : 0;
+        constexpr int EARLY = MT == 16 && !SMALL ? AS : 0;
         int first_z[AS];
 #pragma unroll
         for (int j = 0; j < EARLY; ++j) {
