@@ -561,13 +561,16 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         };
         // A CTA's first copies are what the kernel waits for when it has few slabs, so up to 16 tokens all that can be done for
         // them without the activations is done in front of the wait, and they are issued in one go behind it (1 x 1792 x 6288 9.5 ->
-        // 8.9 us, 16 x 3584 x 4096 10.5 -> 9.5; 64 x 8192 x 28672 43.7 instead of 42.2).
+        // 8.9 us, 16 x 3584 x 4096 10.5 -> 9.5; 64 x 8192 x 28672 43.7 instead of 42.2).  Not with less than five thirds of a slab
+        // per CTA in the mean, some with one and some with two, where it is slower (2 x 4864 x 1104 11.0 -> 12.1, 4 x 3328 x 1696 9.9 ->
+        // 11.1, 16 x 4864 x 1104 11.3 -> 12.1; from there on 2 x 3328 x 2624 9.3 -> 9.1, 2 x 4352 x 2784 10.7 -> 9.4).
         constexpr int EARLY = MT == 16 && !SMALL ? AS : 0;
+        const int n_first = 3 * p.total_items >= 5 * G ? min(n_slabs, EARLY) : 0;
         int first_z[AS];
 #pragma unroll
         for (int j = 0; j < EARLY; ++j) {
           first_z[j] = (b * p.KS + ks) * 4;
-          if (j < n_slabs) {
+          if (j < n_first) {
             mbar_arrive_expect_tx(&a_full[j], Cfg::A_BYTES);
             advance();
           }
@@ -575,11 +578,11 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
 #pragma unroll
         for (int j = 0; j < EARLY; ++j)
-          if (j < n_slabs) tma_load_3d(a_base + j * Cfg::A_BYTES, &tmA, &a_full[j], 0, 0, first_z[j]);
-        issued_mask = (1u << min(n_slabs, EARLY)) - 1u;
-        int st = 0;
+          if (j < n_first) tma_load_3d(a_base + j * Cfg::A_BYTES, &tmA, &a_full[j], 0, 0, first_z[j]);
+        issued_mask = (1u << n_first) - 1u;
+        int st = n_first == AS ? 0 : n_first;
         while (i < n_slabs) {
-          if (EARLY == AS || i >= AS)  // the slab that used this stage has been multiplied
+          if (i >= AS)  // the slab that used this stage has been multiplied
             w4g_wait<W4G_DONE, ST_TIMEOUT_PRODUCER>(bar0 + 8 * ((i - AS) % W4G_BARS), (uint32_t)((i - AS) / W4G_BARS) & 1u, ctl, fail);
           if (fail) break;
           uint64_t* bar = &a_full[i % W4G_BARS];
