@@ -169,7 +169,8 @@ __device__ __forceinline__ uint4 ld_written(const uint4* p) {
   return v;
 }
 
-// Sixteen bytes global -> shared memory past L1; only the thread that copied them may read them after cp_async_wait().
+// Sixteen bytes global -> shared memory past L1; after cp_async_wait() the thread that copied them may read them, others behind a
+// barrier that follows it.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }

@@ -807,8 +807,9 @@ static int w8a8_impl(const int8_t* A, const int8_t* B, const float* scale_b, con
   // The next kernel's CTAs then come to the SMs in the order in which these become free.  Grouped calls of several rounds, whose
   // neighbouring CTAs share tiles of L2, lose more by that than a late start costs: 16 groups, 8192 x 7168 x 2048 120.6 us, 126.0 with
   // it, 25 groups, 3751 x 4992 x 3664 118.4 / 120.5, of two rounds 9 groups, 6844 x 2464 x 1232 31.6 / 32.2; of one round 14 groups, 150 x
-  // 4256 x 1568 26.2 / 25.5, or of tiles of 128 columns, 17 groups, 1903 x 1184 x 1216 12.2 / 11.5.  Plain and batched calls gain throughout: 16 x 512 x 7168 x 2048 116.6 / 112.5, 1097 x 2496 x 1680 11.7 /
-  // 10.9, 519 x 1344 x 2400 7.2 / 6.6, and with the quantiser in front 4096 x 4096 x 14336 188.7 / 186.4, 300 x 2048 x 4096 13.6 / 12.1.
+  // 4256 x 1568 26.2 / 25.5, or of tiles of 128 columns, 17 groups, 1903 x 1184 x 1216 12.2 / 11.5.  Plain and batched calls gain
+  // throughout: 1097 x 2496 x 1680 11.7 / 10.9, 519 x 1344 x 2400 7.2 / 6.6, and with the quantiser in front 300 x 2048 x 4096 13.6 / 12.1
+  // (calls of 100 us and more by no more than repeats differ).
   p.early = meta == nullptr || BN == 128 || p.num_items <= grid ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool nk = b_layout == QGEMM_B_NK;
@@ -960,8 +961,7 @@ static W4Route w4_route(int64_t M, int64_t K, int64_t group, bool has_scales, bo
 
 // Scratch of the kernels for few tokens: the arrival counters first (fixed place whatever the tile height), then two
 // partial slots of [MT][128] fp32 per CTA, then the prepared activations - plain f16 [M, K] in the kernel's K order, or
-// in blocks of
-// 64 k for the group-sum kernel (counted with its token tile).
+// in blocks of 64 k for the group-sum kernel (counted with its token tile).
 static int64_t w4_workspace_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   int sms = 0;
   if (ensure_device(&sms)) return -1;
@@ -1416,7 +1416,7 @@ int qgemm_act_quant(const void* X, int8_t* Y, float* S, int64_t M, int64_t N, in
     return t;
   };
   int keep = 4, tpr = 32;
-  if (threads_for(1) <= 512 && chunks <= 512 && M * threads_for(1) <= 1100ll * sms) keep = 1;
+  if (chunks <= 512 && M * threads_for(1) <= 1100ll * sms) keep = 1;
   else if (chunks <= 2048 && M * threads_for(2) <= 1100ll * sms) keep = 2;
   if (keep < 4) {
     tpr = threads_for(keep);

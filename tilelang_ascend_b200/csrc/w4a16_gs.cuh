@@ -253,9 +253,9 @@ __device__ __forceinline__ void w4g_emit_chunk(uint8_t* dst, int r, int c, const
 // What bounds it is latency, between the end of the kernel in front and the GEMM kernel's first MMA, so all of its blocks should
 // be waiting on an SM each when that kernel ends.  Behind another call of this operator, whose CTAs hold every SM, that takes
 // blocks that fit beside a CTA of the GEMM kernel - 128 threads of 32 registers, what its 768 x 80 leave of the register file, and
-// what its shared memory leaves - and no more of them than SMs (but see launch_w4g_prepare).  More blocks than that (one for every 128 chunks of 32 k of all
-// MT rows) waited for the first SMs to become free, filled these, 16 to an SM, and kept the next call's GEMM CTAs off them for up
-// to 10 us: 32 x 16 x 4096 x 4096 61.9 -> 59.2 us, 11 x 2 x 4352 x 1344 18.3 -> 14.4, 16 x 48 x 4096 x 2048 32.1 -> 28.3.
+// what its shared memory leaves - and no more of them than SMs (but see launch_w4g_prepare).  More blocks than that (one for every
+// 128 chunks of 32 k of all MT rows) waited for the first SMs to become free, filled these, 16 to an SM, and kept the next call's
+// GEMM CTAs off them for up to 10 us: 32 x 16 x 4096 x 4096 61.9 -> 59.2 us, 11 x 2 x 4352 x 1344 18.3 -> 14.4, 16 x 48 x 4096 x 2048 32.1 -> 28.3.
 // LANDING: the values in flight wait in shared memory, since 32 registers hold two; with one or two the way through shared
 // memory is the longer one (2 x 1280 x 14752 5.70 us, 5.60 without).
 constexpr int W4G_PREP_THREADS = 128;

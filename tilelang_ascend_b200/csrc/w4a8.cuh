@@ -107,7 +107,7 @@ w4a8_prepare_activations(const uint2* in, uint2* __restrict__ out, int* __restri
 // so the int8 values and scales are bit-identical to running that kernel first
 // (examples/deepseek_v4/act_quant.py:112-142); what disappears is one launch and the int8 round trip through
 // memory.  Every block of a row takes the abs-max of all of it (four instructions per eight values), then quantises its own part
-// (about a hundred), which it reads again from L1.
+// (about a hundred), which it reads again from shared memory, beyond the first W4I8_PREP_KEPT chunks from global memory.
 template <int BLOCKS>  // per SM, i.e. 40 or 32 registers
 __global__ void __launch_bounds__(W4I8_PREP_THREADS, BLOCKS)
 w4a8_quant_prepare_activations(const uint4* X, int is_bf16, int round_scale, uint2* __restrict__ out,

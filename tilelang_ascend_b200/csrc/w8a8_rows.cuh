@@ -6,8 +6,9 @@
 // (4096) of one tile each, whose pipeline fill, int32 exchange and store follow one another.  Here a tile is 128 weight
 // columns x up to 128 tokens and K is cut over a cluster of S = 1, 2, 4 or 8 CTAs, one CTA per SM where that is enough, with most of
 // the SM's shared memory as its pipeline (w8_rows_plan).  24 tokens, K = 4096, N = 14336: 22.6 us by w8a8.cuh, 14.7 with two CTAs
-// per SM and a pipeline of 96 KB each, now 13.6 (58.7 MB at 6.5 TB/s: 9), with the quantiser in front 28.7, 18.5, now 16.8; 8192 x
-// 8192, 128 tokens 20.7 -> 18.5.  What is left is the start of the launch, the pipeline's first loads and the two cluster barriers.
+// per SM and a pipeline of 96 KB each, now 13.6 (58.7 MB at 6.5 TB/s: 9), each as one graph; with the quantiser in front, calls one
+// after another, 28.7, 19.1, now 15.9; 8192 x 8192, 128 tokens 20.7 -> 18.5.  What is left is the start of the launch, the pipeline's
+// first loads and the two cluster barriers.
 //   warp 0      TMA: [128 columns x 128 k] of weights ([N, K]: K-major rows; [K, N]: MN-major) and [tokens x 128 k] of A
 //   warp 1      tcgen05.mma kind::i8 (M = 128 weight columns, N = tokens rounded up to 16), allocates tensor memory
 //   warps 2..5  epilogue
