@@ -549,38 +549,39 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           }
         }
       } else {
-        auto advance = [&]() {
-          ++i;
-          ++ks;
-          if (--left == 0) {
-            tile = i == n_sk ? p.sk_tiles + cta : tile + (i < n_sk ? 1 : G);
-            ks = 0;
-            left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
-            w4_tile_coords(p, tile, MT, b, n0, m0);
-          }
-        };
+        int st = 0;
         // A CTA's first copies are what the kernel waits for when it has few slabs, so up to 16 tokens all that can be done for
         // them without the activations is done in front of the wait, and they are issued in one go behind it (1 x 1792 x 6288 9.5 ->
-        // 8.9 us, 16 x 3584 x 4096 10.5 -> 9.5; 64 x 8192 x 28672 43.7 instead of 42.2).  Not with less than five thirds of a slab
-        // per CTA in the mean, some with one and some with two, where it is slower (2 x 4864 x 1104 11.0 -> 12.1, 4 x 3328 x 1696 9.9 ->
-        // 11.1, 16 x 4864 x 1104 11.3 -> 12.1; from there on 2 x 3328 x 2624 9.3 -> 9.1, 2 x 4352 x 2784 10.7 -> 9.4).
-        constexpr int EARLY = MT == 16 && !SMALL ? AS : 0;
-        const int n_first = 3 * p.total_items >= 5 * G ? min(n_slabs, EARLY) : 0;
-        int first_z[AS];
+        // 8.9 us, 16 x 3584 x 4096 10.4 -> 8.8; 64 x 8192 x 28672 43.7 instead of 42.2).  Not with less than two slabs per CTA in
+        // the mean, some with one and some with two, where all then hand over at once and it is slower (2 x 4864 x 1104 11.3 -> 12.1, 4 x
+        // 3328 x 1696 9.9 -> 11.1, 8 x 4352 x 2048 9.8 -> 11.5; from there on 2 x 4352 x 2784 10.7 -> 9.5, 12 x 3328 x 3872 10.6 -> 9.4).
+        if (MT == 16 && !SMALL && p.total_items >= 2 * G) {
+          int first_z[AS];
+          const int n_first = min(n_slabs, AS);
 #pragma unroll
-        for (int j = 0; j < EARLY; ++j) {
-          first_z[j] = (b * p.KS + ks) * 4;
-          if (j < n_first) {
-            mbar_arrive_expect_tx(&a_full[j], Cfg::A_BYTES);
-            advance();
+          for (int j = 0; j < AS; ++j) {
+            first_z[j] = (b * p.KS + ks) * 4;
+            if (j < n_first) {  // as below
+              mbar_arrive_expect_tx(&a_full[j], Cfg::A_BYTES);
+              ++ks;
+              if (--left == 0) {
+                tile = j + 1 == n_sk ? p.sk_tiles + cta : tile + (j + 1 < n_sk ? 1 : G);
+                ks = 0;
+                left = j + 1 < n_sk ? min(n_sk - (j + 1), p.KS) : p.KS;
+                w4_tile_coords(p, tile, MT, b, n0, m0);
+              }
+            }
           }
-        }
-        pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
+          pdl_wait();
 #pragma unroll
-        for (int j = 0; j < EARLY; ++j)
-          if (j < n_first) tma_load_3d(a_base + j * Cfg::A_BYTES, &tmA, &a_full[j], 0, 0, first_z[j]);
-        issued_mask = (1u << n_first) - 1u;
-        int st = n_first == AS ? 0 : n_first;
+          for (int j = 0; j < AS; ++j)
+            if (j < n_first) tma_load_3d(a_base + j * Cfg::A_BYTES, &tmA, &a_full[j], 0, 0, first_z[j]);
+          issued_mask = (1u << n_first) - 1u;
+          i = n_first;
+          st = n_first == AS ? 0 : n_first;
+        } else {
+          pdl_wait();  // the prepared activations come from the pre-pass kernel in front of this one
+        }
         while (i < n_slabs) {
           if (i >= AS)  // the slab that used this stage has been multiplied
             w4g_wait<W4G_DONE, ST_TIMEOUT_PRODUCER>(bar0 + 8 * ((i - AS) % W4G_BARS), (uint32_t)((i - AS) / W4G_BARS) & 1u, ctl, fail);
@@ -591,7 +592,14 @@ w4a16_gs_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           issued_mask |= 1u << (i % W4G_BARS);
           parity_mask = (parity_mask & ~(1u << (i % W4G_BARS))) | (((uint32_t)(i / W4G_BARS) & 1u) << (i % W4G_BARS));
           if (++st == AS) st = 0;
-          advance();
+          ++i;
+          ++ks;
+          if (--left == 0) {
+            tile = i == n_sk ? p.sk_tiles + cta : tile + (i < n_sk ? 1 : G);
+            ks = 0;
+            left = i < n_sk ? min(n_sk - i, p.KS) : p.KS;
+            w4_tile_coords(p, tile, MT, b, n0, m0);
+          }
         }
       }
       if (fail) {  // wait (bounded) for the copies still in flight before the CTA may exit
